@@ -137,7 +137,7 @@ struct egg_ctx {
     int8_t *d_vfit = nullptr;           // fitness at every vector's window of table columns; votes of the vectors
     int32_t *d_vvotes = nullptr;
     int32_t *d_votes = nullptr;         // partial vote matrices of a batch: [splits][weights]
-    int *d_wide = nullptr;              // bit 0: some fitness value lies beyond -1..1, bit 1: beyond int8
+    int *d_wide = nullptr;              // bit 0: some fitness value lies beyond -1..1, bit 1: beyond int8, bit 2: its product with the noise does
     void *upd_base = nullptr;           // one allocation of the plan's descriptors and the update's buffers
     // Newton-Schulz of square, wide and tall matrices on a side stream and workspace each: batches of small matrices leave SMs free
     uint8_t *muon_ws[3] = {nullptr, nullptr, nullptr};
@@ -1382,11 +1382,11 @@ static int apply_update_async(egg_ctx *c, uint32_t step_seed, float lr) {
     uint8_t *changed = c->scales_on ? c->d_changed : nullptr;
     int rc;
     if ((rc = PROF(EGG_PROF_UPD_OPERANDS, launch_upd_table(st, pl, c->d_tab, step_seed, cf.device_mask, cf.device_gaussian, c->d_updates, c->d_wide, c->d_norm2)))) return rc;
-    if ((rc = PROF(EGG_PROF_UPD_OPERANDS, launch_upd_masks(st, pl, c->d_fit, c->d_masks, c->d_vfit, c->d_vvotes, c->d_wide)))) return rc;
+    if ((rc = PROF(EGG_PROF_UPD_OPERANDS, launch_upd_masks(st, pl, c->d_fit, c->d_masks, c->d_vfit, c->d_vvotes, c->d_wide, cf.device_gaussian ? 3 * cf.device_mask : cf.device_mask)))) return rc;
     if (!pl.vecs.empty() && (rc = PROFN(EGG_PROF_UPD_VECTOR, 2, launch_upd_vectors(st, pl, c->d_tab, c->d_masks, c->d_vfit, c->d_vvotes, c->d_wide, c->d_fit, cf.device_gaussian, c->d_model, c->d_opt, h, c->d_updates, changed, c->num_sms)))) return rc;
     for (const UpdBatch &b : pl.batches) {
         if ((rc = PROF(EGG_PROF_UPD_OPERANDS, launch_upd_operands(st, pl, b, c->d_tab, c->d_masks, c->d_wide, c->d_fit, c->d_fn)))) return rc;
-        if ((rc = PROF(EGG_PROF_UPD_GEMM, launch_upd_votes(st, pl, b, c->d_tab, c->d_fn, c->d_votes, c->d_err, c->num_sms)))) return rc;
+        if ((rc = PROF(EGG_PROF_UPD_GEMM, launch_upd_votes(st, pl, b, c->d_tab, c->d_fn, c->d_wide, c->d_votes, c->d_err, c->num_sms)))) return rc;
         if (b.any_adam && (rc = PROF(EGG_PROF_UPD_APPLY, launch_upd_adam(st, pl, b, c->d_votes, c->d_model, c->d_opt, c->d_shadow, h, c->d_updates, changed)))) return rc;
         if ((rc = muon_steps(c, (int)(&b - pl.batches.data()), lr))) return rc;
     }

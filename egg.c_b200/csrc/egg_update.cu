@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <map>
 #include <cuda.h>
+#include <limits.h>
 #include <string.h>
 
 namespace egg {
@@ -67,7 +68,7 @@ int launch_upd_table(cudaStream_t st, const UpdPlan &pl, int8_t *tab, uint32_t s
 }
 
 // ------------------------------------------------------------------ fitness as byte masks, at every alignment, and as vector windows
-__global__ void upd_masks_kernel(const int32_t *fit, int pairs, int kp, uint8_t *masks, int *range, const UpdVec *vecs, int nvec, int vec_pad, int pitch,
+__global__ void upd_masks_kernel(const int32_t *fit, int pairs, int kp, uint8_t *masks, int *range, int most, const UpdVec *vecs, int nvec, int vec_pad, int pitch,
                                  const UpdVecCols *vcols, int ncols, int8_t *vfit, int32_t *vvotes, int len_long) {
     chain_next();
     chain_wait();
@@ -85,6 +86,7 @@ __global__ void upd_masks_kernel(const int32_t *fit, int pairs, int kp, uint8_t 
             if (f > 0) pos |= 0xFFu << (8 * k);
             if (f < 0) neg |= 0xFFu << (8 * k);
             if (f > 1 || f < -1) wide |= (f > 127 || f < -127) ? 3 : 1;
+            if (f > most || f < -most) wide |= 4;
         }
         *reinterpret_cast<uint32_t *>(masks + (int64_t)r * kp + j) = pos;
         *reinterpret_cast<uint32_t *>(masks + (int64_t)(16 + r) * kp + j) = neg;
@@ -110,9 +112,9 @@ __global__ void upd_masks_kernel(const int32_t *fit, int pairs, int kp, uint8_t 
 int64_t upd_vfit_bytes(const UpdPlan &pl) { return (int64_t)pl.vec_pad * pl.pitch; }
 int64_t upd_vvotes_elems(const UpdPlan &pl) { return (int64_t)pl.vec_pad * pl.len_long; }
 
-int launch_upd_masks(cudaStream_t st, const UpdPlan &pl, const int32_t *fit, uint8_t *masks, int8_t *vfit, int32_t *vvotes, int *range) {
+int launch_upd_masks(cudaStream_t st, const UpdPlan &pl, const int32_t *fit, uint8_t *masks, int8_t *vfit, int32_t *vvotes, int *range, int amp) {
     EGG_CUDA(launch_chained(upd_masks_kernel, dim3((unsigned)((pl.kp / 4 + 255) / 256), (unsigned)(16 + pl.vec_pad)), 256, 0, st, fit, pl.pairs, pl.kp, masks,
-                            range, pl.d_vecs, (int)pl.vecs.size(), pl.vec_pad, pl.pitch, pl.d_vcols, (int)pl.vcols.size(), vfit, vvotes, pl.len_long));
+                            range, amp > 0 ? 127 / amp : INT_MAX, pl.d_vecs, (int)pl.vecs.size(), pl.vec_pad, pl.pitch, pl.d_vcols, (int)pl.vcols.size(), vfit, vvotes, pl.len_long));
     return EGG_OK;
 }
 
@@ -123,7 +125,7 @@ __device__ __forceinline__ uint32_t neg4(uint32_t n) {
 }
 // fitness (as masks) times noise
 __device__ __forceinline__ uint32_t fit_times(uint32_t n, uint32_t pos, uint32_t neg) { return (n & pos) | (neg4(n) & neg); }
-// byte-wise product with general fitness values, truncated to int8 as the reference's operand is
+// byte-wise product with general fitness values; beyond a byte it wraps
 __device__ __forceinline__ uint32_t fit_times_wide(uint32_t n, const int32_t *fit, int p, int pairs) {
     uint32_t o = 0;
 #pragma unroll
@@ -312,36 +314,45 @@ int launch_upd_vectors(cudaStream_t st, const UpdPlan &pl, const int8_t *tab, co
 constexpr int FN_ROWS = 8;            // rows per block: the masks are read once for all of them
 
 __global__ void __launch_bounds__(256, 6) upd_operands_kernel(const UpdMat *mats, int nmats, const int8_t *tab, int pitch, const uint8_t *masks, int kp,
-                                                           const int *range, const int32_t *fit, int pairs, int8_t *fn) {
+                                                           const int *range, const int32_t *fit, int pairs, int rows1, int8_t *fn) {
     chain_next();
-    const int row0 = (int)blockIdx.x * FN_ROWS;
-    int lo = 0, hi = nmats - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (mats[mid].fn_row0 <= row0) lo = mid; else hi = mid - 1;
-    }
-    const UpdMat m = mats[lo];                    // (descriptors are older than the chain)
+    int row0 = (int)blockIdx.x * FN_ROWS;
+    auto find = [&](int form) {
+        int lo = 0, hi = nmats - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (mats[mid].form[form].fn_row0 <= row0) lo = mid; else hi = mid - 1;
+        }
+        return mats[lo].form[form];
+    };
+    UpdForm m = find(0);                          // (descriptors are older than the chain)
     chain_wait();
-    const bool wide = *range != 0;
-    const int x = m.x_fn, sh = (x & 3) * 8, r = m.r;
-    const bool by2 = x & 8, by1 = x & 4;
-    const int8_t *src0 = tab + (int64_t)(row0 - m.fn_row0) * pitch + (x & ~15);
-    const uint8_t *mp = masks + (int64_t)r * kp, *mn = masks + (int64_t)(16 + r) * kp;
-    for (int j = (int)(blockIdx.y * blockDim.x + threadIdx.x) * 16; j < kp; j += (int)(gridDim.y * blockDim.x) * 16) {
-        const uint4 ps = *reinterpret_cast<const uint4 *>(mp + j), ng = *reinterpret_cast<const uint4 *>(mn + j);
+    const int rg = *range;
+    const bool wide = rg != 0;
+    // the grid covers form 0's rows; products that wrap take form 1's, more of them, in as many trips as it needs
+    const int rows = rg & 4 ? rows1 : row0 + 1;
+    for (; row0 < rows; row0 += (int)gridDim.x * FN_ROWS) {
+        if (rg & 4) m = find(1);
+        const int x = m.x_fn, sh = (x & 3) * 8, r = m.r;
+        const bool by2 = x & 8, by1 = x & 4;
+        const int8_t *src0 = tab + (int64_t)(row0 - m.fn_row0) * pitch + (x & ~15);
+        const uint8_t *mp = masks + (int64_t)r * kp, *mn = masks + (int64_t)(16 + r) * kp;
+        for (int j = (int)(blockIdx.y * blockDim.x + threadIdx.x) * 16; j < kp; j += (int)(gridDim.y * blockDim.x) * 16) {
+            const uint4 ps = *reinterpret_cast<const uint4 *>(mp + j), ng = *reinterpret_cast<const uint4 *>(mn + j);
 #pragma unroll 2
-        for (int e = 0; e < FN_ROWS; e++) {
-            // 16 bytes from any byte offset: two aligned words of 16, shifted by words, then by bytes
-            const uint4 *src = reinterpret_cast<const uint4 *>(src0 + (int64_t)e * pitch + j);
-            const uint4 a = src[0], b = src[1];
-            uint32_t w0 = a.x, w1 = a.y, w2 = a.z, w3 = a.w, w4 = b.x, w5 = b.y;
-            if (by2) { w0 = w2; w1 = w3; w2 = w4; w3 = w5; w4 = b.z; w5 = b.w; }
-            if (by1) { w0 = w1; w1 = w2; w2 = w3; w3 = w4; w4 = w5; }
-            uint4 n = make_uint4(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh), __funnelshift_r(w2, w3, sh), __funnelshift_r(w3, w4, sh));
-            if (!wide) n = make_uint4(fit_times(n.x, ps.x, ng.x), fit_times(n.y, ps.y, ng.y), fit_times(n.z, ps.z, ng.z), fit_times(n.w, ps.w, ng.w));
-            else n = make_uint4(fit_times_wide(n.x, fit, j - r, pairs), fit_times_wide(n.y, fit, j - r + 4, pairs), fit_times_wide(n.z, fit, j - r + 8, pairs),
-                                fit_times_wide(n.w, fit, j - r + 12, pairs));
-            *reinterpret_cast<uint4 *>(fn + (int64_t)(row0 + e) * kp + j) = n;
+            for (int e = 0; e < FN_ROWS; e++) {
+                // 16 bytes from any byte offset: two aligned words of 16, shifted by words, then by bytes
+                const uint4 *src = reinterpret_cast<const uint4 *>(src0 + (int64_t)e * pitch + j);
+                const uint4 a = src[0], b = src[1];
+                uint32_t w0 = a.x, w1 = a.y, w2 = a.z, w3 = a.w, w4 = b.x, w5 = b.y;
+                if (by2) { w0 = w2; w1 = w3; w2 = w4; w3 = w5; w4 = b.z; w5 = b.w; }
+                if (by1) { w0 = w1; w1 = w2; w2 = w3; w3 = w4; w4 = w5; }
+                uint4 n = make_uint4(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh), __funnelshift_r(w2, w3, sh), __funnelshift_r(w3, w4, sh));
+                if (!wide) n = make_uint4(fit_times(n.x, ps.x, ng.x), fit_times(n.y, ps.y, ng.y), fit_times(n.z, ps.z, ng.z), fit_times(n.w, ps.w, ng.w));
+                else n = make_uint4(fit_times_wide(n.x, fit, j - r, pairs), fit_times_wide(n.y, fit, j - r + 4, pairs), fit_times_wide(n.z, fit, j - r + 8, pairs),
+                                    fit_times_wide(n.w, fit, j - r + 12, pairs));
+                *reinterpret_cast<uint4 *>(fn + (int64_t)(row0 + e) * kp + j) = n;
+            }
         }
     }
 }
@@ -350,8 +361,8 @@ int launch_upd_operands(cudaStream_t st, const UpdPlan &pl, const UpdBatch &b, c
                         const int32_t *fit, int8_t *fn) {
     int gy = (pl.kp / 16 + 255) / 256;
     if (gy > 65535) gy = 65535;
-    EGG_CUDA(launch_chained(upd_operands_kernel, dim3((unsigned)(b.fn_rows / FN_ROWS), (unsigned)gy), 256, 0, st, pl.d_mats + b.first, b.count, tab, pl.pitch, masks, pl.kp, range,
-                                                                                            fit, pl.pairs, fn));
+    EGG_CUDA(launch_chained(upd_operands_kernel, dim3((unsigned)(b.fn_rows[0] / FN_ROWS), (unsigned)gy), 256, 0, st, pl.d_mats + b.first, b.count, tab, pl.pitch, masks, pl.kp, range,
+                            fit, pl.pairs, b.fn_rows[1], fn));
     EGG_CUDA(cudaGetLastError());
     return EGG_OK;
 }
@@ -378,6 +389,7 @@ struct UpdVoteSmem {
 
 struct UpdVoteParams {
     const UpdMat *mats; int nmats, tiles, splits, num_kb;
+    const int *range;
     int32_t *votes; int64_t split_stride;
     int *err;
 };
@@ -422,13 +434,15 @@ upd_votes_kernel(const __grid_constant__ CUtensorMap tab_a, const __grid_constan
         if (ptx::elect_one()) {
             uint32_t it = 0;
             bool ok = true;
+            const int form = *p.range >> 2 & 1;
             for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
                 const int split = item / p.tiles, tile = item - split * p.tiles;
                 const UpdMat &m = p.mats[find(tile)];
+                const UpdForm f = m.form[form];
                 const int local = tile - m.tile0, tm = local / m.tiles_n, tn = local - tm * m.tiles_n;
-                const int ya = tm * UV_BM + (m.fn_is_n ? m.fn_row0 : 0), yb = tn * UV_BN + (m.fn_is_n ? 0 : m.fn_row0);
-                const int xa = m.fn_is_n ? 0 : m.x_tab, xb = m.fn_is_n ? m.x_tab : 0;
-                const CUtensorMap *ta = m.fn_is_n ? &fn_a : &tab_a, *tb = m.fn_is_n ? &tab_b : &fn_b;
+                const int ya = tm * UV_BM + (f.fn_is_n ? f.fn_row0 : 0), yb = tn * UV_BN + (f.fn_is_n ? 0 : f.fn_row0);
+                const int xa = f.fn_is_n ? 0 : f.x_tab, xb = f.fn_is_n ? f.x_tab : 0;
+                const CUtensorMap *ta = f.fn_is_n ? &fn_a : &tab_a, *tb = f.fn_is_n ? &tab_b : &fn_b;
                 const int kb1 = min(p.num_kb, (split + 1) * kb_per);
                 for (int kb = split * kb_per; kb < kb1; kb++, it++) {
                     const int s = it % UV_STAGES;
@@ -514,15 +528,16 @@ int upd_init() {
     return EGG_OK;
 }
 
-int launch_upd_votes(cudaStream_t st, const UpdPlan &pl, const UpdBatch &b, const int8_t *tab, const int8_t *fn, int32_t *votes, int *err, int num_sms) {
+int launch_upd_votes(cudaStream_t st, const UpdPlan &pl, const UpdBatch &b, const int8_t *tab, const int8_t *fn, const int *range, int32_t *votes, int *err, int num_sms) {
     CUtensorMap ta, tb, fa, fb;
     int rc;
+    const uint64_t fn_rows = (uint64_t)std::max(b.fn_rows[0], b.fn_rows[1]);
     if ((rc = upd_tensor_map(&ta, tab, (uint64_t)pl.W, (uint64_t)pl.pitch, UV_BM)) || (rc = upd_tensor_map(&tb, tab, (uint64_t)pl.W, (uint64_t)pl.pitch, UV_BN)) ||
-        (rc = upd_tensor_map(&fa, fn, (uint64_t)b.fn_rows, (uint64_t)pl.kp, UV_BM)) || (rc = upd_tensor_map(&fb, fn, (uint64_t)b.fn_rows, (uint64_t)pl.kp, UV_BN)))
+        (rc = upd_tensor_map(&fa, fn, fn_rows, (uint64_t)pl.kp, UV_BM)) || (rc = upd_tensor_map(&fb, fn, fn_rows, (uint64_t)pl.kp, UV_BN)))
         return rc;
     UpdVoteParams p;
     p.mats = pl.d_mats + b.first; p.nmats = b.count; p.tiles = b.tiles; p.splits = b.splits; p.num_kb = pl.kp / UV_BK;
-    p.votes = votes; p.split_stride = b.votes; p.err = err;
+    p.range = range; p.votes = votes; p.split_stride = b.votes; p.err = err;
     const int items = b.tiles * b.splits;
     EGG_CUDA(launch_chained(upd_votes_kernel, items < num_sms ? items : num_sms, UV_THREADS, sizeof(UpdVoteSmem) + 1024, st, ta, tb, fa, fb, p));
     EGG_CUDA(cudaGetLastError());
@@ -694,7 +709,7 @@ int upd_plan_build(UpdPlan &pl, const std::vector<ParamDesc> &params, const std:
             const int64_t waves = ((int64_t)b.tiles * s + num_sms - 1) / num_sms, cost = waves * (per + 6) * 16 + s;
             if (best < 0 || cost < best) { best = cost; b.splits = s; }
         }
-        pl.fn_bytes = std::max(pl.fn_bytes, (int64_t)b.fn_rows * pl.kp);
+        pl.fn_bytes = std::max(pl.fn_bytes, (int64_t)std::max(b.fn_rows[0], b.fn_rows[1]) * pl.kp);
         pl.votes_elems = std::max(pl.votes_elems, b.votes * b.splits);
         pl.batches.push_back(b);
     };
@@ -704,17 +719,23 @@ int upd_plan_build(UpdPlan &pl, const std::vector<ParamDesc> &params, const std:
         if (!d.rows_k || (!use.empty() && !use[i])) continue;
         UpdMat m;
         memset(&m, 0, sizeof(m));
-        m.rows_k = d.rows_k; m.cols_n = d.cols_n; m.fn_is_n = d.cols_n <= d.rows_k;
-        const int fr = m.fn_is_n ? d.cols_n : d.rows_k;
+        m.rows_k = d.rows_k; m.cols_n = d.cols_n;
+        const int fr = std::min(d.cols_n, d.rows_k);
         const int64_t wts = (int64_t)d.rows_k * d.cols_n;
-        if (b.count && (b.count == UV_MAX_MATS || (int64_t)(b.fn_rows + fr) * pl.kp > UPD_FN_BYTES || b.votes + wts > UPD_VOTE_ELEMS)) { close(); fresh(); }
+        if (b.count && (b.count == UV_MAX_MATS || (int64_t)(b.fn_rows[0] + fr) * pl.kp > UPD_FN_BYTES || b.votes + wts > UPD_VOTE_ELEMS)) { close(); fresh(); }
         const int s_n = d.seed_base + d.off_a + UPD_ORIGIN, s_k = d.seed_base + d.off_b + UPD_ORIGIN;
-        const int s_tab = m.fn_is_n ? s_k : s_n, s_fn = m.fn_is_n ? s_n : s_k;
-        m.r = s_tab & 15; m.x_tab = s_tab & ~15; m.x_fn = s_fn - m.r;
-        m.fn_row0 = b.fn_rows; m.tile0 = b.tiles; m.tiles_n = (d.rows_k + UV_BN - 1) / UV_BN; m.blk0 = b.blocks; m.muon = d.muon;
+        for (int form = 0; form < 2; form++) {
+            UpdForm &f = m.form[form];
+            f.fn_is_n = form || d.cols_n <= d.rows_k;
+            const int s_tab = f.fn_is_n ? s_k : s_n, s_fn = f.fn_is_n ? s_n : s_k;
+            f.r = s_tab & 15; f.x_tab = s_tab & ~15; f.x_fn = s_fn - f.r;
+            f.fn_row0 = b.fn_rows[form];
+            b.fn_rows[form] += f.fn_is_n ? d.cols_n : d.rows_k;
+        }
+        m.tile0 = b.tiles; m.tiles_n = (d.rows_k + UV_BN - 1) / UV_BN; m.blk0 = b.blocks; m.muon = d.muon;
         m.lr_scale = d.lr_scale; m.model_off = d.model_off; m.opt_off = d.opt_off; m.shadow_off = d.shadow_off; m.votes_off = b.votes;
         m.ov_in = d.ov_in; m.ov_out = d.ov_out;
-        b.fn_rows += fr; b.tiles += d.cols_n / UV_BM * m.tiles_n; b.blocks += d.cols_n / 32 * (d.rows_k / 128); b.votes += wts; b.count++;
+        b.tiles += d.cols_n / UV_BM * m.tiles_n; b.blocks += d.cols_n / 32 * (d.rows_k / 128); b.votes += wts; b.count++;
         b.any_adam |= !d.muon;
         pl.mats.push_back(m);
         pl.mat_param.push_back((int)i);

@@ -16,13 +16,18 @@ constexpr int UPD_ORIGIN = 16;        // columns before the first seed: windows 
 
 // One matrix of a batch.  The contraction index j of its vote product starts 0..15 columns before its first pair so that the
 // table serves as one operand in place (a TMA copy starts on a 16-byte boundary); the other operand, fitness times noise,
-// is written out with the same alignment for the smaller of the two dimensions.
-struct UpdMat {
-    int rows_k, cols_n;
+// is written out with the same alignment.  Which side carries the fitness makes no difference while the products fit a byte, so
+// form 0 writes the smaller of the two dimensions; where they wrap, the side is part of the result and form 1 writes the outputs n,
+// as the isolated update does.
+struct UpdForm {
     int fn_is_n;                      // 1: the written operand runs over the outputs n, the table over k; 0: the other way round
     int fn_row0;                      // first row of the written operand
     int x_fn;                         // table column of its contraction index 0 (any alignment)
     int x_tab, r;                     // table column of the in-place operand's index 0 (multiple of 16); index of the first pair
+};
+struct UpdMat {
+    int rows_k, cols_n;
+    UpdForm form[2];
     int tile0, tiles_n;               // first tile of the batch, tiles along k
     int blk0;                         // first block of the optimiser step
     int muon;
@@ -40,7 +45,8 @@ struct UpdHyper { float lr, beta1, beta2, eps, wd, mu; };
 
 struct UpdBatch {
     int first, count;                 // matrices
-    int tiles, splits, fn_rows, blocks;
+    int tiles, splits, blocks;
+    int fn_rows[2];                   // rows of the written operand in either form
     int64_t votes;                    // weights of the batch (elements of one partial vote array)
     bool any_adam;
 };
@@ -81,8 +87,8 @@ int launch_upd_table(cudaStream_t st, const UpdPlan &pl, int8_t *tab, uint32_t s
                      double *norm2);
 // masks[sign][16][kp]: bytes 0xFF where the fitness of pair (index - shift) is +1 / -1.  vfit[vec_pad][pitch]: the fitness as
 // bytes, placed at every vector's own window of table columns; vvotes[vec_pad][len_long] is cleared.  *range: bit 0 when some
-// |f| > 1, bit 1 when some |f| > 127.
-int launch_upd_masks(cudaStream_t st, const UpdPlan &pl, const int32_t *fit, uint8_t *masks, int8_t *vfit, int32_t *vvotes, int *range);
+// |f| > 1, bit 1 when some |f| > 127, bit 2 when some |f| times the largest noise value `amp` is.
+int launch_upd_masks(cudaStream_t st, const UpdPlan &pl, const int32_t *fit, uint8_t *masks, int8_t *vfit, int32_t *vvotes, int *range, int amp);
 int64_t upd_vfit_bytes(const UpdPlan &pl);
 int64_t upd_vvotes_elems(const UpdPlan &pl);
 // votes of all vectors (noise magnitudes up to 15), then their optimiser steps
@@ -90,7 +96,7 @@ int launch_upd_vectors(cudaStream_t st, const UpdPlan &pl, const int8_t *tab, co
                        const int32_t *fit, int gaussian, int8_t *model, uint8_t *opt, const UpdHyper &h, unsigned long long *total, uint8_t *changed, int num_sms);
 int launch_upd_operands(cudaStream_t st, const UpdPlan &pl, const UpdBatch &b, const int8_t *tab, const uint8_t *masks, const int *range,
                         const int32_t *fit, int8_t *fn);
-int launch_upd_votes(cudaStream_t st, const UpdPlan &pl, const UpdBatch &b, const int8_t *tab, const int8_t *fn, int32_t *votes, int *err, int num_sms);
+int launch_upd_votes(cudaStream_t st, const UpdPlan &pl, const UpdBatch &b, const int8_t *tab, const int8_t *fn, const int *range, int32_t *votes, int *err, int num_sms);
 int launch_upd_adam(cudaStream_t st, const UpdPlan &pl, const UpdBatch &b, const int32_t *votes, int8_t *model, uint8_t *opt, int8_t *shadow,
                     const UpdHyper &h, unsigned long long *total, uint8_t *changed);
 // one pass over all overlays (update_overlay_kernel, d-eggs/src/kernels.cu:61-77); entries whose `active` byte is 0 stay as they are

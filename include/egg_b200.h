@@ -223,6 +223,8 @@ int egg_update_owner_plan(const egg_config *cfg, int world, int32_t *owner_out, 
  * rebuilds vote = Σ_p fit_p·a_p·b_pᵀ for every parameter from the device
  * fitness vector and applies ES-AdamW (or Muon for hidden matrices when
  * use_muon), emb_bias at 0.1·lr.  *total_updates ≙ d_total_updates.
+ * Of a matrix the product fit_p·a_p (the side of the outputs) is one byte: exact while |fit| * (largest
+ * noise magnitude) <= 127, it wraps beyond, as in egg_update_matrix without split.  Vectors are exact.
  */
 int egg_apply_update(egg_ctx *ctx, uint32_t step_seed, float learning_rate,
                      uint64_t *total_updates);

@@ -1,0 +1,152 @@
+// A CUDA runtime and NCCL for host-side tests: device memory is host memory, kernels do nothing, and every launch, copy, event
+// and wait is logged.  Loaded in front of the real runtime (LD_PRELOAD), so that the library's host code runs without a GPU
+// and a test can make any single call fail.
+#include <dlfcn.h>
+#include <stdint.h>
+#include <stdio.h>
+#include <stdlib.h>
+#include <string.h>
+#include <sys/mman.h>
+
+#include <map>
+#include <mutex>
+#include <string>
+
+namespace {
+std::mutex m;
+std::string log_text;
+std::map<const void *, std::string> kernels;
+std::map<const void *, size_t> symbols;
+std::map<uintptr_t, size_t> device, pinned;
+std::map<const void *, void *> symbol_mem;
+uintptr_t next_handle = 0x1000;
+long mallocs = 0, fail_malloc = -1, host_allocs = 0;
+std::string fail_kernel;
+long fail_kernel_after = 0;
+struct Config { unsigned g[3], b[3]; size_t smem; void *st; } pushed;
+
+void note(const char *what, const std::string &rest) { log_text += std::string(what) + " " + rest + "\n"; }
+std::string hex(const void *p) { char s[32]; snprintf(s, sizeof s, "%p", p); return s; }
+void *take(size_t n) { return mmap(nullptr, n ? n : 1, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_NORESERVE, -1, 0); }
+int launch(const void *f, void *st) {
+    std::lock_guard<std::mutex> l(m);
+    const std::string &name = kernels[f];
+    if (!fail_kernel.empty() && name.find(fail_kernel) != std::string::npos && fail_kernel_after-- == 0) { note("failed", name + " " + hex(st)); return 719; }
+    note("launch", name + " " + hex(st));
+    return 0;
+}
+int encode_tiled(void *, int, uint32_t, void *base, const uint64_t *, const uint64_t *, const uint32_t *, const uint32_t *, int, int, int, int) {
+    return (reinterpret_cast<uintptr_t>(base) & 15) ? 1 : 0;
+}
+}  // namespace
+
+extern "C" {
+// ---- control ----
+const char *fake_log() { return log_text.c_str(); }
+void fake_clear() { log_text.clear(); }
+void fake_fail_malloc(long nth) { fail_malloc = nth < 0 ? -1 : mallocs + nth; }       // 0: the next one
+void fake_fail_kernel(const char *part, long after) { fail_kernel = part; fail_kernel_after = after; }
+long fake_mallocs() { return mallocs; }
+long fake_host_allocs() { return host_allocs; }
+long long fake_device_bytes() { long long n = 0; for (auto &d : device) n += (long long)d.second; return n; }
+long long fake_pinned_bytes() { long long n = 0; for (auto &d : pinned) n += (long long)d.second; return n; }
+
+// ---- runtime ----
+int cudaMalloc(void **p, size_t n) {
+    std::lock_guard<std::mutex> l(m);
+    if (mallocs++ == fail_malloc) return 2;
+    *p = take(n);
+    device[reinterpret_cast<uintptr_t>(*p)] = n;
+    return 0;
+}
+int cudaFree(void *p) {
+    std::lock_guard<std::mutex> l(m);
+    auto it = device.find(reinterpret_cast<uintptr_t>(p));
+    if (it == device.end()) return p ? 1 : 0;
+    mprotect(p, it->second ? it->second : 1, PROT_NONE);        // a later use of it is a fault here and now
+    note("free", hex(p));
+    device.erase(it);
+    return 0;
+}
+int cudaHostAlloc(void **p, size_t n, unsigned) {
+    std::lock_guard<std::mutex> l(m);
+    host_allocs++;
+    *p = take(n);
+    pinned[reinterpret_cast<uintptr_t>(*p)] = n;
+    return 0;
+}
+int cudaFreeHost(void *p) {
+    std::lock_guard<std::mutex> l(m);
+    auto it = pinned.find(reinterpret_cast<uintptr_t>(p));
+    if (it == pinned.end()) return 1;
+    munmap(p, it->second);
+    pinned.erase(it);
+    return 0;
+}
+int cudaMemcpyAsync(void *d, const void *s, size_t n, int, void *st) { memcpy(d, s, n); std::lock_guard<std::mutex> l(m); note("copy", hex(st)); return 0; }
+int cudaMemcpy(void *d, const void *s, size_t n, int) { memcpy(d, s, n); return 0; }
+int cudaMemset(void *d, int v, size_t n) { memset(d, v, n); return 0; }
+int cudaMemsetAsync(void *d, int v, size_t n, void *st) { memset(d, v, n); std::lock_guard<std::mutex> l(m); note("memset", hex(st)); return 0; }
+int cudaMemGetInfo(size_t *f, size_t *t) { *f = *t = (size_t)8 << 30; return 0; }
+int cudaPointerGetAttributes(void *a, const void *) { memset(a, 0, 16); return 0; }
+int cudaGetDeviceCount(int *n) { *n = 1; return 0; }
+int cudaGetDevice(int *d) { *d = 0; return 0; }
+int cudaSetDevice(int) { return 0; }
+int cudaDeviceGetAttribute(int *v, int a, int) { *v = a == 75 ? 10 : (a == 16 ? 148 : 0); return 0; }
+int cudaGetDriverEntryPoint(const char *, void **fn, unsigned long long, int *res) { *fn = (void *)encode_tiled; if (res) *res = 0; return 0; }
+int cudaGetLastError() { return 0; }
+const char *cudaGetErrorString(int e) { return e == 2 ? "out of memory" : "a failure the test asked for"; }
+int cudaFuncSetAttribute(const void *, int, int) { return 0; }
+int cudaOccupancyMaxActiveClusters(int *n, const void *, const void *) { *n = 74; return 0; }
+int cudaGetSymbolAddress(void **p, const void *s) {
+    std::lock_guard<std::mutex> l(m);
+    if (!symbol_mem[s]) symbol_mem[s] = take(symbols[s]);
+    *p = symbol_mem[s];
+    return 0;
+}
+int cudaStreamCreateWithFlags(void **s, unsigned) { std::lock_guard<std::mutex> l(m); *s = (void *)(next_handle += 16); return 0; }
+int cudaStreamDestroy(void *) { return 0; }
+int cudaStreamSynchronize(void *s) { std::lock_guard<std::mutex> l(m); note("sync", hex(s)); return 0; }
+int cudaStreamWaitEvent(void *s, void *e, unsigned) { std::lock_guard<std::mutex> l(m); note("wait", hex(s) + " " + hex(e)); return 0; }
+int cudaEventCreateWithFlags(void **e, unsigned) { std::lock_guard<std::mutex> l(m); *e = (void *)(next_handle += 16); return 0; }
+int cudaEventCreate(void **e) { return cudaEventCreateWithFlags(e, 0); }
+int cudaEventDestroy(void *) { return 0; }
+int cudaEventRecord(void *e, void *s) { std::lock_guard<std::mutex> l(m); note("record", hex(e) + " " + hex(s)); return 0; }
+int cudaEventSynchronize(void *) { return 0; }
+int cudaEventElapsedTime(float *t, void *, void *) { *t = 0; return 0; }
+int cudaStreamBeginCapture(void *, int) { return 0; }
+int cudaStreamEndCapture(void *, void **g) { *g = (void *)1; return 0; }
+int cudaGraphInstantiate(void **e, void *, unsigned long long) { *e = (void *)1; return 0; }
+int cudaGraphDestroy(void *) { return 0; }
+int cudaGraphExecDestroy(void *) { return 0; }
+int cudaGraphLaunch(void *, void *st) { std::lock_guard<std::mutex> l(m); note("graph", hex(st)); return 0; }
+int cudaLaunchKernel(const void *f, uint64_t, uint32_t, uint64_t, uint32_t, void **, size_t, void *st) { return launch(f, st); }
+int cudaLaunchKernelExC(const void *cfg, const void *f, void **) { return launch(f, *reinterpret_cast<void *const *>(static_cast<const char *>(cfg) + 32)); }
+
+// ---- what the compiler's start-up code calls ----
+void **__cudaRegisterFatBinary(void *) { static void *h; return &h; }
+void __cudaRegisterFatBinaryEnd(void **) {}
+void __cudaUnregisterFatBinary(void **) {}
+void __cudaRegisterFunction(void **, const char *f, char *, const char *name, int, void *, void *, void *, void *, int *) { kernels[f] = name; }
+void __cudaRegisterVar(void **, char *v, char *, const char *, int, size_t n, int, int) { symbols[v] = n; }
+unsigned __cudaPushCallConfiguration(uint64_t gxy, uint32_t gz, uint64_t bxy, uint32_t bz, size_t smem, void *st) {
+    pushed = Config{{(unsigned)gxy, (unsigned)(gxy >> 32), gz}, {(unsigned)bxy, (unsigned)(bxy >> 32), bz}, smem, st};
+    return 0;
+}
+int __cudaPopCallConfiguration(void *g, void *b, size_t *smem, void **st) {
+    memcpy(g, pushed.g, 12); memcpy(b, pushed.b, 12); *smem = pushed.smem; *st = pushed.st;
+    return 0;
+}
+
+// ---- NCCL ----
+int ncclGetUniqueId(void *id) { memset(id, 1, 128); return 0; }
+struct fake_id { char b[128]; };
+int ncclCommInitRank(void **c, int, fake_id, int) { *c = (void *)1; return 0; }
+int ncclCommDestroy(void *) { return 0; }
+const char *ncclGetErrorString(int) { return "nccl"; }
+int ncclAllGather(const void *, void *, size_t, int, void *, void *) { return 0; }
+int ncclBroadcast(const void *, void *, size_t, int, int, void *, void *) { return 0; }
+int ncclAllReduce(const void *, void *, size_t, int, int, void *, void *) { return 0; }
+int ncclGroupStart() { return 0; }
+int ncclGroupEnd() { return 0; }
+}

@@ -35,3 +35,42 @@ def test_update_against_oracle(kw, amp):
         assert (ctx.download_model() == model).all(), step
         assert (ctx.download_opt_state() == opt).all(), step
     ctx.close()
+
+
+@pytest.mark.parametrize("amp,kw", [
+    (8, dict(device_mask=15)),                                     # 120: still inside a byte
+    (9, dict(device_mask=15)),                                     # 135: the first that wraps
+    (127, dict(device_mask=1, device_gaussian=1)),                 # sums of three noise values
+    (200, dict(device_mask=3, vocab_size=768)),                    # beyond int8 itself, more outputs than four widths
+    (100000, dict(device_mask=15)),
+])
+def test_products_that_wrap_equal_the_isolated_update(amp, kw):
+    """Fitness times noise beyond a byte wraps on the outputs' side whatever the matrix's shape: every matrix of the model
+    update equals the isolated update of that matrix, which has no other form."""
+    import torch
+    pkg = load_pkg()
+    H, V = 128, kw.get("vocab_size", 256)
+    pop = 614
+    cfg = pkg.default_config(hidden_dim=H, n_layers=1, seq_len=16, population_size=pop, **kw)
+    ctx = pkg.Context(cfg, 0, 2)
+    rng = np.random.RandomState(amp)
+    model = rng.randint(-127, 128, pkg.model_bytes(cfg)).astype(np.int8)
+    fit = rng.randint(-amp, amp + 1, pop // 2).astype(np.int32)
+    ctx.upload_model(model)
+    ctx.write_fitness(fit)
+    ctx.apply_update(77, 0.4)
+    got, state = ctx.download_model(), ctx.download_opt_state().view(np.float32).reshape(-1, 3)
+    after_init = V * H + 3 * H + 4 * H * H + 4 * H + 4 * H * H + H
+    w_q = after_init + 2 * H
+    w_up = w_q + 4 * H * H + 2 * H
+    w_down = w_up + 4 * H * H + 4 * H
+    d_fit = torch.from_numpy(fit).cuda()
+    for off, rows, cols, a, b in ((0, H, V, 0, H), (V * H + 3 * H, H, 4 * H, 510, 511), (V * H + 3 * H + 4 * H * H + 4 * H, 4 * H, H, 512, 513),
+                                  (w_q, H, H, 200, 201), (w_up, H, 4 * H, 400, 401), (w_down, 4 * H, H, 402, 403)):
+        w = torch.from_numpy(model[off:off + rows * cols].copy()).cuda()
+        opt = torch.zeros(rows * cols, 3, device="cuda")
+        torch.cuda.synchronize()
+        ctx.update_matrix(w.data_ptr(), opt.data_ptr(), rows, cols, a, b, 0, d_fit.data_ptr(), pop // 2, 77, 0.4, 0, False)
+        assert (opt.cpu().numpy() == state[off:off + rows * cols]).all(), (rows, cols, a)
+        assert (w.cpu().numpy() == got[off:off + rows * cols]).all(), (rows, cols, a)
+    ctx.close()
