@@ -427,6 +427,7 @@ static int prepare_update(egg_ctx *c) {
 }
 
 static int noalloc_scratch_address(int device, int8_t **out);
+static bool fused_shifts(const egg_config &c);
 
 extern "C" int egg_ctx_create(const egg_config *cfg, int device, int wave_members, egg_ctx **out) {
     if (!cfg || !out) { set_error("null argument"); return EGG_E_INVALID; }
@@ -458,7 +459,7 @@ extern "C" int egg_ctx_create(const egg_config *cfg, int device, int wave_member
 #define TRYC(x) do { cudaError_t e_ = (x); if (e_ != cudaSuccess) { set_error("%s: %s", #x, cudaGetErrorString(e_)); egg_ctx_destroy(c); return EGG_E_CUDA; } } while (0)
     TRYC(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     TRYC(cudaEventCreate(&c->t0)); TRYC(cudaEventCreate(&c->t1));
-    c->SP = member_rows(cfg->hidden_dim, cfg->seq_len);
+    c->SP = fused_shifts(*cfg) ? member_rows(cfg->hidden_dim, cfg->seq_len) : cfg->seq_len;
     const int64_t H = cfg->hidden_dim, S = cfg->seq_len, SP = c->SP, POP = cfg->population_size;
     c->SL = scales_layout(*cfg);
     std::vector<NoiseSeg> segs(32 + 32 * cfg->n_layers);
@@ -804,8 +805,11 @@ static int ensure_pre(egg_ctx *c) {
     return a.commit(&c->pre_base);
 }
 
+// Whether the residual projections' shifts allow the row-owning form; larger ones take the two-kernel form at every shape.
+static bool fused_shifts(const egg_config &c) { return std::max(c.shift_out, c.shift_mlp_down) + c.fixed_point + c.sigma_shift <= PRESHIFT_MAX; }
+
 static bool use_fused(const egg_ctx *c) {
-    return c->fused_level > 0 && fused_supported(c->cfg.hidden_dim, c->SP);
+    return c->fused_level > 0 && fused_shifts(c->cfg) && fused_supported(c->cfg.hidden_dim, c->SP);
 }
 
 static FusedParams base_fused(egg_ctx *c, int M, int K, int parts) {

@@ -212,7 +212,7 @@ int launch_gemm_fused(cudaStream_t st, int mode, const int8_t *A, const int8_t *
         set_error("unsupported row-owning GEMM shape M=%d H=%d K=%d parts=%d seq_len=%d", p.M, p.H, p.K, p.parts, p.seq_len);
         return EGG_E_INVALID;
     }
-    if (mode != FUSED_QKV && p.out_shift + p.rank1_shift > 20) {     // (bias + noise) << (both shifts) joins a product below 2^30
+    if (mode != FUSED_QKV && p.out_shift + p.rank1_shift > PRESHIFT_MAX) {
         set_error("shifts %d + %d too large for the pre-shifted bias table", p.out_shift, p.rank1_shift);
         return EGG_E_INVALID;
     }
@@ -299,7 +299,7 @@ int launch_gemm(cudaStream_t st, int epi, const int8_t *A, const int8_t *B, cons
     p.fd_head = make_fastdiv(p.head_dim);
     p.lut_stride = 32 * 4;
     p.one = 1;
-    if (epi == EPI_GELU && p.out_shift + p.rank1_shift > 20) {       // (bias + noise) << (both shifts) joins a product below 2^30
+    if (epi == EPI_GELU && p.out_shift + p.rank1_shift > PRESHIFT_MAX) {
         set_error("shifts %d + %d too large for the pre-shifted bias table", p.out_shift, p.rank1_shift);
         return EGG_E_INVALID;
     }

@@ -153,6 +153,9 @@ int launch_gemm_fused(cudaStream_t st, int mode, const int8_t *A, const int8_t *
 // whether the row-owning kernels can run a configuration (whole 32-row groups of one member, a row fits tensor memory)
 int fused_cluster_size(int hidden);       // blocks per unit of the row-owning GEMM (two also where units are few), 0 when the width is unsupported
 inline bool fused_supported(int hidden, int seq_len) { return seq_len % 32 == 0 && fused_cluster_size(hidden) > 0; }
+// Largest output shift + rank-1 shift of the projections that add their bias before both (the row-owning residual projections
+// and MLP-up): (bias + noise) << (both shifts) joins a product below 2^30.
+constexpr int PRESHIFT_MAX = 20;
 // Rows that hold one member's seq_len tokens: padded to whole 32-row groups where that opens the row-owning kernels and the
 // row-per-lane epilogues for at most a third more rows (48 -> 64 costs 1.33; 16 -> 32 would double the work).
 inline int member_rows(int hidden, int seq_len) {

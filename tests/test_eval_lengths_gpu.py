@@ -26,6 +26,24 @@ def test_losses_match_oracle(seq, hidden):
     ctx.close()
 
 
+@pytest.mark.parametrize("kw", [
+    dict(hidden_dim=128, seq_len=48, shift_out=14), dict(hidden_dim=256, seq_len=128, shift_mlp_down=15, fixed_point=5),
+    dict(hidden_dim=640, seq_len=32, fixed_point=6, sigma_shift=6),
+])
+def test_shifts_beyond_the_row_owning_form(kw):
+    """Output shift plus rank-1 shift above 20: the two-kernel form at lengths and widths that otherwise never take it."""
+    pkg, O = load_pkg(), load_oracle()
+    kw = dict(kw, n_layers=1, population_size=8, device_mask=15)
+    cfg, ocfg, model, data = make_case(kw, data_len=9000, model_kind="random_all", model_seed=1)
+    ctx = pkg.Context(cfg, 0, 0)
+    ctx.upload_model(model)
+    ctx.set_dataset(data)
+    assert ctx.fused_epilogues_active() == 0
+    ctx.eval_chunk(0xBEEF, 40, 0, 8)
+    assert (ctx.read_losses(0, 8) == O.eval_losses(ocfg, model, data, 40, 0xBEEF, 0, 8)).all()
+    ctx.close()
+
+
 @pytest.mark.parametrize("hidden,seq", [(128, 48), (256, 64), (384, 80), (512, 32), (640, 96), (768, 32), (896, 16), (1024, 64)])
 def test_overlays_match_oracle(hidden, seq):
     pkg, O = load_pkg(), load_oracle()

@@ -1,0 +1,66 @@
+"""The library's host code without a GPU: its decisions and its error paths, run in child processes on the CUDA runtime of
+fake_cuda.cpp, whose kernels do nothing, which logs every launch and wait and fails the call a test names."""
+import json
+import os
+import subprocess
+import sys
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+PRELUDE = """
+import ctypes as C, json, sys
+sys.path.insert(0, %r)
+import numpy as np
+from common import load_pkg
+pkg = load_pkg()
+fake = C.CDLL(None)
+fake.fake_log.restype = C.c_char_p
+for f in (fake.fake_device_bytes, fake.fake_pinned_bytes): f.restype = C.c_longlong
+for f in (fake.fake_mallocs, fake.fake_host_allocs): f.restype = C.c_long
+fake.fake_fail_malloc.argtypes = [C.c_long]
+fake.fake_fail_kernel.argtypes = [C.c_char_p, C.c_long]
+def log(): return fake.fake_log().decode().splitlines()
+def launches(part): return sum(l.startswith("launch") and part in l for l in log())
+def context(wave=2, **kw):
+    ctx = pkg.Context(pkg.default_config(**kw), 0, wave)
+    ctx.upload_model(np.zeros(pkg.model_bytes(ctx.cfg), np.int8))
+    ctx.set_dataset(np.zeros(5000, np.uint8 if ctx.cfg.vocab_size == 256 else np.uint32))
+    return ctx
+def error(call):
+    try: call()
+    except pkg.EggError as e: return e.code
+    return 0
+out = {}
+""" % HERE
+
+
+@pytest.fixture(scope="session")
+def fake_cuda(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("fake") / "fake_cuda.so")
+    subprocess.run(["g++", "-O1", "-shared", "-fPIC", "-o", so, os.path.join(HERE, "fake_cuda.cpp")], check=True)
+
+    def run(code):
+        r = subprocess.run([sys.executable, "-c", PRELUDE + code + "\nprint(json.dumps(out))"], capture_output=True, text=True, timeout=300,
+                           env=dict(os.environ, LD_PRELOAD=so, EGG_NCCL_LIB=so))
+        assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
+        return json.loads(r.stdout.splitlines()[-1])
+    return run
+
+
+@pytest.mark.parametrize("kw,fused", [
+    (dict(hidden_dim=512, seq_len=256), True),
+    (dict(hidden_dim=896, seq_len=192, shift_out=11, fixed_point=6, sigma_shift=4), False),      # 21
+    (dict(hidden_dim=384, seq_len=48, shift_mlp_down=14), False),
+    (dict(hidden_dim=384, seq_len=48, shift_mlp_down=13), True),                                 # 20: the largest sum
+])
+def test_shifts_beyond_the_row_owning_form(fake_cuda, kw, fused):
+    """Shifts that the row-owning projections cannot take go to the two-kernel form, unpadded, instead of being refused."""
+    out = fake_cuda("""
+ctx = context(n_layers=1, population_size=8, **%r)
+ctx.eval_chunk(1, 0, 0, 8)
+out["fused"], out["active"] = launches("gemm_fused_kernel"), ctx.fused_epilogues_active()
+""" % kw)
+    assert (out["fused"] > 0) == fused and (out["active"] > 0) == fused
+
