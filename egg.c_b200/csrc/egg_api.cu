@@ -1139,8 +1139,9 @@ extern "C" int egg_generate(egg_ctx *c, uint8_t *host_tokens, int seed_len, int 
     EGG_CUDA(cudaMemsetAsync(tok, 0, (size_t)cf.seq_len + 258, c->stream));
     EGG_CUDA(cudaMemcpyAsync(tok, host_tokens, (size_t)seed_len, cudaMemcpyHostToDevice, c->stream));
     // every given token but the last only leaves its keys and values: from 12 on, one pass of the evaluation kernels over all of
-    // them (310 us at H 512, 4 layers, window 256) is shorter than a decode step each (38 us)
-    const int start = seed_len - 1 >= 12 ? seed_len - 1 : 0;
+    // them (310 us at H 512, 4 layers, window 256) is shorter than a decode step each (38 us).  Decoding takes any shift, the
+    // evaluation's MLP-up does not.
+    const int start = seed_len - 1 >= 12 && cf.shift_mlp_up + cf.fixed_point + cf.sigma_shift <= PRESHIFT_MAX ? seed_len - 1 : 0;
     if (start && gen_len > 0) {
         ChainScope chain(true);
         const Prefill pf = {tok, start, kv};

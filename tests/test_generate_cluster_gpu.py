@@ -36,6 +36,7 @@ def test_every_width_against_oracle(hidden, layers, given, new):
     (384, 48, 47, {}), (512, 48, 18, {}),            # windows shorter than the cache
     (896, 256, 250, {}), (1024, 80, 64, {}),
     (256, 512, 200, dict(device_mask=15)), (256, 64, 30, dict(device_mask=15, device_gaussian=1)),
+    (128, 64, 20, dict(shift_mlp_up=14)),            # a shift the evaluation's kernels do not take
 ])
 def test_given_bytes_in_one_pass(hidden, seq_len, given, kw):
     """The cache that the evaluation kernels fill equals the one that decoding fills, also with overlays loaded."""

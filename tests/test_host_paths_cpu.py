@@ -64,3 +64,13 @@ out["fused"], out["active"] = launches("gemm_fused_kernel"), ctx.fused_epilogues
 """ % kw)
     assert (out["fused"] > 0) == fused and (out["active"] > 0) == fused
 
+
+@pytest.mark.parametrize("shift,prefill", [(13, True), (14, False)])
+def test_sampling_takes_any_shift(fake_cuda, shift, prefill):
+    """Given bytes are decoded one by one where the evaluation's kernels do not take the model's shifts."""
+    out = fake_cuda("""
+ctx = context(hidden_dim=128, n_layers=1, seq_len=64, population_size=8, shift_mlp_up=%d)
+out["rc"] = error(lambda: ctx.generate(np.zeros(20, np.uint8), 4, 1))
+out["prefill"], out["decode"] = launches("kv_gather"), launches("generate_kernel")
+""" % shift)
+    assert out == {"rc": 0, "prefill": int(prefill), "decode": 1}
