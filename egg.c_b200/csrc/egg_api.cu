@@ -132,16 +132,18 @@ struct egg_ctx {
     void *arena = nullptr;              // the buffers of fixed size
     void *pre_base = nullptr;           // d_pre and d_rowmax3, allocated when the two-kernel form first runs
     UpdPlan plan;                       // of the parameters this context steps (all, or its own ones when the update is sharded)
-    int8_t *d_tab = nullptr, *d_fn = nullptr;      // noise table; written operands of a batch
-    uint8_t *d_masks = nullptr;
-    int8_t *d_vfit = nullptr;           // fitness at every vector's window of table columns; votes of the vectors
-    int32_t *d_vvotes = nullptr;
-    int32_t *d_votes = nullptr;         // partial vote matrices of a batch: [splits][weights]
-    int *d_wide = nullptr;              // bit 0: some fitness value lies beyond -1..1, bit 1: beyond int8, bit 2: its product with the noise does
-    void *upd_base = nullptr;           // one allocation of the plan's descriptors and the update's buffers
-    // Newton-Schulz of square, wide and tall matrices on a side stream and workspace each: batches of small matrices leave SMs free
-    uint8_t *muon_ws[3] = {nullptr, nullptr, nullptr};
-    double *d_norm2 = nullptr;          // [plan list]
+    struct UpdBuffers {
+        void *base = nullptr;           // one allocation of the plan's descriptors and all of these
+        int8_t *tab = nullptr, *fn = nullptr;      // noise table; written operands of a batch
+        uint8_t *masks = nullptr;
+        int8_t *vfit = nullptr;         // fitness at every vector's window of table columns; votes of the vectors
+        int32_t *vvotes = nullptr;
+        int32_t *votes = nullptr;       // partial vote matrices of a batch: [splits][weights]
+        int *wide = nullptr;            // bit 0: some fitness value lies beyond -1..1, bit 1: beyond int8, bit 2: its product with the noise does
+        // Newton-Schulz of square, wide and tall matrices on a side stream and workspace each: batches of small matrices leave SMs free
+        uint8_t *muon_ws[3] = {nullptr, nullptr, nullptr};
+        double *norm2 = nullptr;        // [plan list]
+    } upd;
     cudaStream_t side[3] = {nullptr, nullptr, nullptr};
     cudaEvent_t ev_m = nullptr, ev_done[3] = {nullptr, nullptr, nullptr};
     bool side_used[3] = {false, false, false};
@@ -384,7 +386,7 @@ extern "C" void egg_ctx_destroy(egg_ctx *c) {
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     if (c->comm && g_nccl.CommDestroy) g_nccl.CommDestroy(c->comm);
-    void *ptrs[] = {c->arena, c->upd_base, c->pre_base, c->d_data};
+    void *ptrs[] = {c->arena, c->upd.base, c->pre_base, c->d_data};
     host_stage_free(c->stage);
     pinned_give(reinterpret_cast<uint8_t *>(c->pin));
     pinned_release();
@@ -409,21 +411,30 @@ static int prepare_update(egg_ctx *c) {
         use.resize(c->params.size());
         for (size_t i = 0; i < use.size(); i++) use[i] = c->owner[i] == c->rank;
     }
-    int rc = upd_plan_build(c->plan, c->params, use, c->cfg.hidden_dim, c->cfg.vocab_size, c->cfg.population_size / 2, c->num_sms);
+    // The new plan takes the old one's place only when it is complete: a context whose request fails goes on as it was.
+    UpdPlan plan;
+    egg_ctx::UpdBuffers b;
+    int rc = upd_plan_build(plan, c->params, use, c->cfg.hidden_dim, c->cfg.vocab_size, c->cfg.population_size / 2, c->num_sms);
     if (rc) return rc;
-    if (c->upd_base) { EGG_CUDA(cudaStreamSynchronize(c->stream)); cudaFree(c->upd_base); c->upd_base = nullptr; }
     int64_t ws[3] = {0, 0, 0};
-    for (const MuonGroup &g : c->plan.groups) ws[g.slot] = std::max(ws[g.slot], ns_ws_bytes(g.rows, g.cols, g.count));
+    for (const MuonGroup &g : plan.groups) ws[g.slot] = std::max(ws[g.slot], ns_ws_bytes(g.rows, g.cols, g.count));
     DeviceArena a;
     uint8_t *desc = nullptr;
-    a.add(&desc, (int64_t)c->plan.descriptors.size());
-    a.add(&c->d_tab, upd_table_bytes(c->plan)); a.add(&c->d_fn, c->plan.fn_bytes); a.add(&c->d_masks, upd_mask_bytes(c->plan));
-    a.add(&c->d_votes, c->plan.votes_elems);
-    a.add(&c->d_vfit, upd_vfit_bytes(c->plan)); a.add(&c->d_vvotes, upd_vvotes_elems(c->plan));
-    for (int i = 0; i < 3; i++) a.add(&c->muon_ws[i], ws[i]);
-    a.add(&c->d_norm2, (int64_t)c->plan.list.size()); a.add(&c->d_wide, 1);
-    if ((rc = a.commit(&c->upd_base))) return rc;
-    return upd_plan_upload(c->plan, desc, c->stream);
+    a.add(&desc, (int64_t)plan.descriptors.size());
+    a.add(&b.tab, upd_table_bytes(plan)); a.add(&b.fn, plan.fn_bytes); a.add(&b.masks, upd_mask_bytes(plan));
+    a.add(&b.votes, plan.votes_elems);
+    a.add(&b.vfit, upd_vfit_bytes(plan)); a.add(&b.vvotes, upd_vvotes_elems(plan));
+    for (int i = 0; i < 3; i++) a.add(&b.muon_ws[i], ws[i]);
+    a.add(&b.norm2, (int64_t)plan.list.size()); a.add(&b.wide, 1);
+    if ((rc = a.commit(&b.base))) return rc;
+    if ((rc = upd_plan_upload(plan, desc, c->stream))) { cudaFree(b.base); return rc; }
+    if (c->upd.base) {
+        EGG_CUDA(cudaStreamSynchronize(c->stream));
+        cudaFree(c->upd.base);
+    }
+    c->plan = std::move(plan);
+    c->upd = b;
+    return EGG_OK;
 }
 
 static int noalloc_scratch_address(int device, int8_t **out);
@@ -1244,18 +1255,24 @@ extern "C" int egg_set_update_sharding(egg_ctx *c, int enable) {
             if (rc) return rc;
             EGG_CUDA(cudaStreamSynchronize(c->stream));
         }
-        const bool was = c->shard_update;
+        if (!c->shard_update) return EGG_OK;
+        EGG_CUDA(cudaSetDevice(c->device));
+        EGG_CUDA(cudaStreamSynchronize(c->stream));
         c->shard_update = false;
-        if (was) { EGG_CUDA(cudaSetDevice(c->device)); EGG_CUDA(cudaStreamSynchronize(c->stream)); return prepare_update(c); }
-        return EGG_OK;
+        int rc = prepare_update(c);
+        if (rc) c->shard_update = true;
+        return rc;
     }
     if (!c->comm || c->world < 2) { set_error("update sharding needs a communicator over at least two ranks"); return EGG_E_STATE; }
     if (c->scales_on) { set_error("update sharding is not combined with adaptive-noise overlays"); return EGG_E_STATE; }
-    plan_owners(c->params, c->world, c->owner);
-    c->shard_update = true;
     EGG_CUDA(cudaSetDevice(c->device));
     EGG_CUDA(cudaStreamSynchronize(c->stream));
-    return prepare_update(c);
+    const bool was = c->shard_update;
+    plan_owners(c->params, c->world, c->owner);
+    c->shard_update = true;
+    int rc = prepare_update(c);
+    if (rc) c->shard_update = was;
+    return rc;
 }
 
 extern "C" int egg_allgather_fitness(egg_ctx *c) {
@@ -1354,8 +1371,8 @@ static int muon_steps(egg_ctx *c, int batch, float lr) {
     for (const MuonGroup &g : pl.groups) {
         if (g.batch != batch) continue;
         any = true;
-        if ((rc = PROF(EGG_PROF_UPD_APPLY, launch_muon_momentum(c->stream, pl.d_mats, pl.d_list + g.first, g.count, g.rows, g.cols, c->d_votes, b.splits, b.votes,
-                                                                c->d_opt, cf.muon_momentum, c->d_norm2 + g.first)))) return rc;
+        if ((rc = PROF(EGG_PROF_UPD_APPLY, launch_muon_momentum(c->stream, pl.d_mats, pl.d_list + g.first, g.count, g.rows, g.cols, c->upd.votes, b.splits, b.votes,
+                                                                c->d_opt, cf.muon_momentum, c->upd.norm2 + g.first)))) return rc;
     }
     if (!any) return EGG_OK;
     EGG_CUDA(cudaEventRecord(c->ev_m, c->stream));
@@ -1364,9 +1381,9 @@ static int muon_steps(egg_ctx *c, int batch, float lr) {
         cudaStream_t st = c->side[g.slot];
         EGG_CUDA(cudaStreamWaitEvent(st, c->ev_m, 0));
         NsWs ws;
-        ns_ws_carve(ws, c->muon_ws[g.slot], g.rows, g.cols, g.count);
+        ns_ws_carve(ws, c->upd.muon_ws[g.slot], g.rows, g.cols, g.count);
         ProfScope ps(c, EGG_PROF_MUON, 12, st);
-        if ((rc = launch_muon_split(st, pl.d_mats, pl.d_list + g.first, g.count, g.rows, g.cols, c->d_opt, c->d_norm2 + g.first, ws))) return rc;
+        if ((rc = launch_muon_split(st, pl.d_mats, pl.d_list + g.first, g.count, g.rows, g.cols, c->d_opt, c->upd.norm2 + g.first, ws))) return rc;
         if ((rc = launch_newton_schulz(st, ws, g.rows, g.cols, g.count, c->d_err, c->num_sms))) return rc;
         if ((rc = launch_muon_apply(st, pl.d_mats, pl.d_list + g.first, g.count, g.rows, g.cols, ws.y, c->d_model, c->d_opt, c->d_shadow,
                                     lr * cf.muon_lr_scale, cf.adam_weight_decay, c->d_updates))) return rc;
@@ -1386,13 +1403,13 @@ static int apply_update_async(egg_ctx *c, uint32_t step_seed, float lr) {
     h.lr = lr; h.beta1 = cf.adam_beta1; h.beta2 = cf.adam_beta2; h.eps = cf.adam_eps; h.wd = cf.adam_weight_decay; h.mu = cf.muon_momentum;
     uint8_t *changed = c->scales_on ? c->d_changed : nullptr;
     int rc;
-    if ((rc = PROF(EGG_PROF_UPD_OPERANDS, launch_upd_table(st, pl, c->d_tab, step_seed, cf.device_mask, cf.device_gaussian, c->d_updates, c->d_wide, c->d_norm2)))) return rc;
-    if ((rc = PROF(EGG_PROF_UPD_OPERANDS, launch_upd_masks(st, pl, c->d_fit, c->d_masks, c->d_vfit, c->d_vvotes, c->d_wide, cf.device_gaussian ? 3 * cf.device_mask : cf.device_mask)))) return rc;
-    if (!pl.vecs.empty() && (rc = PROFN(EGG_PROF_UPD_VECTOR, 2, launch_upd_vectors(st, pl, c->d_tab, c->d_masks, c->d_vfit, c->d_vvotes, c->d_wide, c->d_fit, cf.device_gaussian, c->d_model, c->d_opt, h, c->d_updates, changed, c->num_sms)))) return rc;
+    if ((rc = PROF(EGG_PROF_UPD_OPERANDS, launch_upd_table(st, pl, c->upd.tab, step_seed, cf.device_mask, cf.device_gaussian, c->d_updates, c->upd.wide, c->upd.norm2)))) return rc;
+    if ((rc = PROF(EGG_PROF_UPD_OPERANDS, launch_upd_masks(st, pl, c->d_fit, c->upd.masks, c->upd.vfit, c->upd.vvotes, c->upd.wide, cf.device_gaussian ? 3 * cf.device_mask : cf.device_mask)))) return rc;
+    if (!pl.vecs.empty() && (rc = PROFN(EGG_PROF_UPD_VECTOR, 2, launch_upd_vectors(st, pl, c->upd.tab, c->upd.masks, c->upd.vfit, c->upd.vvotes, c->upd.wide, c->d_fit, cf.device_gaussian, c->d_model, c->d_opt, h, c->d_updates, changed, c->num_sms)))) return rc;
     for (const UpdBatch &b : pl.batches) {
-        if ((rc = PROF(EGG_PROF_UPD_OPERANDS, launch_upd_operands(st, pl, b, c->d_tab, c->d_masks, c->d_wide, c->d_fit, c->d_fn)))) return rc;
-        if ((rc = PROF(EGG_PROF_UPD_GEMM, launch_upd_votes(st, pl, b, c->d_tab, c->d_fn, c->d_wide, c->d_votes, c->d_err, c->num_sms)))) return rc;
-        if (b.any_adam && (rc = PROF(EGG_PROF_UPD_APPLY, launch_upd_adam(st, pl, b, c->d_votes, c->d_model, c->d_opt, c->d_shadow, h, c->d_updates, changed)))) return rc;
+        if ((rc = PROF(EGG_PROF_UPD_OPERANDS, launch_upd_operands(st, pl, b, c->upd.tab, c->upd.masks, c->upd.wide, c->d_fit, c->upd.fn)))) return rc;
+        if ((rc = PROF(EGG_PROF_UPD_GEMM, launch_upd_votes(st, pl, b, c->upd.tab, c->upd.fn, c->upd.wide, c->upd.votes, c->d_err, c->num_sms)))) return rc;
+        if (b.any_adam && (rc = PROF(EGG_PROF_UPD_APPLY, launch_upd_adam(st, pl, b, c->upd.votes, c->d_model, c->d_opt, c->d_shadow, h, c->d_updates, changed)))) return rc;
         if ((rc = muon_steps(c, (int)(&b - pl.batches.data()), lr))) return rc;
     }
     // UPDATE_OVERLAY of every parameter (worker.cu:445-455)

@@ -35,8 +35,14 @@ int launch(const void *f, void *st) {
     note("launch", name + " " + hex(st));
     return 0;
 }
+// refuses what is not aligned and what is not allocated any more
 int encode_tiled(void *, int, uint32_t, void *base, const uint64_t *, const uint64_t *, const uint32_t *, const uint32_t *, int, int, int, int) {
-    return (reinterpret_cast<uintptr_t>(base) & 15) ? 1 : 0;
+    const uintptr_t p = reinterpret_cast<uintptr_t>(base);
+    std::lock_guard<std::mutex> l(m);
+    auto it = device.upper_bound(p);
+    if ((p & 15) || it == device.begin()) return 1;
+    --it;
+    return p < it->first + it->second ? 0 : 1;
 }
 }  // namespace
 

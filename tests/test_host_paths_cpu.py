@@ -74,3 +74,25 @@ out["rc"] = error(lambda: ctx.generate(np.zeros(20, np.uint8), 4, 1))
 out["prefill"], out["decode"] = launches("kv_gather"), launches("generate_kernel")
 """ % shift)
     assert out == {"rc": 0, "prefill": int(prefill), "decode": 1}
+
+
+@pytest.mark.parametrize("muon", [0, 1])
+def test_update_survives_a_failed_change_of_sharding(fake_cuda, muon):
+    """Out of memory while the update's buffers are replaced: the change is refused and the context goes on with the ones it has."""
+    out = fake_cuda("""
+ctx = context(hidden_dim=128, n_layers=2, seq_len=32, population_size=64, use_muon=%d)
+ctx.comm_init(bytes(128), 0, 2)
+out["steps"] = []
+for target, fails in ((1, 1), (1, 0), (0, 1), (0, 0), (1, 1)):
+    fake.fake_fail_malloc(0 if fails else -1)
+    before = fake.fake_device_bytes()
+    rc = error(lambda: ctx.set_update_sharding(target))
+    same = fake.fake_device_bytes() == before
+    fake.fake_clear()
+    out["steps"].append([rc, same, error(lambda: ctx.apply_update(1, 0.1)), launches("upd_votes_kernel")])
+""" % muon)
+    nomem = out["steps"][0][0]
+    assert nomem < 0
+    assert [s[0] for s in out["steps"]] == [nomem, 0, nomem, 0, nomem]
+    assert [s[1] for s in out["steps"]] == [True, False, True, False, True]
+    assert all(s[2] == 0 and s[3] > 0 for s in out["steps"]), out
