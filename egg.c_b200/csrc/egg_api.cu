@@ -144,6 +144,7 @@ struct egg_ctx {
         uint8_t *muon_ws[3] = {nullptr, nullptr, nullptr};
         double *norm2 = nullptr;        // [plan list]
     } upd;
+    int64_t upd_share = 0;              // plan_share() of the plan: a communicator may be replaced under it
     cudaStream_t side[3] = {nullptr, nullptr, nullptr};
     cudaEvent_t ev_m = nullptr, ev_done[3] = {nullptr, nullptr, nullptr};
     bool side_used[3] = {false, false, false};
@@ -404,10 +405,15 @@ extern "C" void egg_ctx_destroy(egg_ctx *c) {
     delete c;
 }
 
+static bool update_is_sharded(const egg_ctx *c) { return c->shard_update && c->comm && c->world > 1 && !c->scales_on; }
+
+// Which parameters a plan covers: all (0), or one rank's share of so many.
+static int64_t plan_share(const egg_ctx *c) { return update_is_sharded(c) ? (int64_t)c->world << 32 | c->rank : 0; }
+
 // Update plan over the parameters this rank steps, and its buffers.
 static int prepare_update(egg_ctx *c) {
     std::vector<char> use;
-    if (c->shard_update) {
+    if (update_is_sharded(c)) {
         use.resize(c->params.size());
         for (size_t i = 0; i < use.size(); i++) use[i] = c->owner[i] == c->rank;
     }
@@ -434,6 +440,7 @@ static int prepare_update(egg_ctx *c) {
     }
     c->plan = std::move(plan);
     c->upd = b;
+    c->upd_share = plan_share(c);
     return EGG_OK;
 }
 
@@ -1193,6 +1200,8 @@ extern "C" int egg_nccl_unique_id(void *id128) {
     return EGG_OK;
 }
 
+static void plan_owners(const std::vector<ParamDesc> &params, int world, std::vector<int> &owner);
+
 extern "C" int egg_comm_init(egg_ctx *c, const void *id128, int rank, int world) {
     if (!c || !id128 || world < 1 || rank < 0 || rank >= world) { set_error("bad communicator arguments"); return EGG_E_INVALID; }
     if ((c->cfg.population_size / 2) % world) { set_error("POP/2 = %d pairs do not divide over %d ranks", c->cfg.population_size / 2, world); return EGG_E_INVALID; }
@@ -1204,6 +1213,7 @@ extern "C" int egg_comm_init(egg_ctx *c, const void *id128, int rank, int world)
     ncclResult_t r = g_nccl.CommInitRank(&c->comm, world, id, rank);
     if (r != ncclSuccess) { set_error("ncclCommInitRank failed (%d)", (int)r); return EGG_E_NCCL; }
     c->rank = rank; c->world = world;
+    if (c->shard_update && world > 1) plan_owners(c->params, world, c->owner);      // the next update takes the new shares
     return EGG_OK;
 }
 
@@ -1338,8 +1348,6 @@ static int run_matrix_update(egg_ctx *c, const MatrixUpdate &u, uint32_t step_se
     return launch_muon_apply(c->stream, dm, list, 1, u.rows_k, u.cols_n, ws.y, u.w_packed, opt, nullptr, u.lr * cf.muon_lr_scale, cf.adam_weight_decay, c->d_updates);
 }
 
-static bool update_is_sharded(const egg_ctx *c) { return c->shard_update && c->comm && c->world > 1 && !c->scales_on; }
-
 // One grouped broadcast per parameter from its owner: of the int8 weights, or of the optimiser state.
 static int broadcast_params(egg_ctx *c, bool opt_state) {
     if (!g_nccl.Broadcast || !g_nccl.GroupStart || !g_nccl.GroupEnd) { set_error("this NCCL build lacks ncclBroadcast / group calls"); return EGG_E_NCCL; }
@@ -1395,6 +1403,8 @@ static int muon_steps(egg_ctx *c, int batch, float lr) {
 
 static int apply_update_async(egg_ctx *c, uint32_t step_seed, float lr) {
     const egg_config &cf = c->cfg;
+    int rc;
+    if (c->upd_share != plan_share(c) && (rc = prepare_update(c))) return rc;
     const UpdPlan &pl = c->plan;
     cudaStream_t st = c->stream;
     ChainScope chain(c->model_bytes <= CHAIN_MAX_WEIGHTS);
@@ -1402,7 +1412,6 @@ static int apply_update_async(egg_ctx *c, uint32_t step_seed, float lr) {
     UpdHyper h;
     h.lr = lr; h.beta1 = cf.adam_beta1; h.beta2 = cf.adam_beta2; h.eps = cf.adam_eps; h.wd = cf.adam_weight_decay; h.mu = cf.muon_momentum;
     uint8_t *changed = c->scales_on ? c->d_changed : nullptr;
-    int rc;
     if ((rc = PROF(EGG_PROF_UPD_OPERANDS, launch_upd_table(st, pl, c->upd.tab, step_seed, cf.device_mask, cf.device_gaussian, c->d_updates, c->upd.wide, c->upd.norm2)))) return rc;
     if ((rc = PROF(EGG_PROF_UPD_OPERANDS, launch_upd_masks(st, pl, c->d_fit, c->upd.masks, c->upd.vfit, c->upd.vvotes, c->upd.wide, cf.device_gaussian ? 3 * cf.device_mask : cf.device_mask)))) return rc;
     if (!pl.vecs.empty() && (rc = PROFN(EGG_PROF_UPD_VECTOR, 2, launch_upd_vectors(st, pl, c->upd.tab, c->upd.masks, c->upd.vfit, c->upd.vvotes, c->upd.wide, c->d_fit, cf.device_gaussian, c->d_model, c->d_opt, h, c->d_updates, changed, c->num_sms)))) return rc;

@@ -28,11 +28,11 @@ struct Config { unsigned g[3], b[3]; size_t smem; void *st; } pushed;
 void note(const char *what, const std::string &rest) { log_text += std::string(what) + " " + rest + "\n"; }
 std::string hex(const void *p) { char s[32]; snprintf(s, sizeof s, "%p", p); return s; }
 void *take(size_t n) { return mmap(nullptr, n ? n : 1, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_NORESERVE, -1, 0); }
-int launch(const void *f, void *st) {
+int launch(const void *f, void *st, unsigned gx, unsigned gy, unsigned gz) {
     std::lock_guard<std::mutex> l(m);
     const std::string &name = kernels[f];
     if (!fail_kernel.empty() && name.find(fail_kernel) != std::string::npos && fail_kernel_after-- == 0) { note("failed", name + " " + hex(st)); return 719; }
-    note("launch", name + " " + hex(st));
+    note("launch", name + " " + hex(st) + " " + std::to_string(gx) + "," + std::to_string(gy) + "," + std::to_string(gz));
     return 0;
 }
 // refuses what is not aligned and what is not allocated any more
@@ -126,8 +126,11 @@ int cudaGraphInstantiate(void **e, void *, unsigned long long) { *e = (void *)1;
 int cudaGraphDestroy(void *) { return 0; }
 int cudaGraphExecDestroy(void *) { return 0; }
 int cudaGraphLaunch(void *, void *st) { std::lock_guard<std::mutex> l(m); note("graph", hex(st)); return 0; }
-int cudaLaunchKernel(const void *f, uint64_t, uint32_t, uint64_t, uint32_t, void **, size_t, void *st) { return launch(f, st); }
-int cudaLaunchKernelExC(const void *cfg, const void *f, void **) { return launch(f, *reinterpret_cast<void *const *>(static_cast<const char *>(cfg) + 32)); }
+int cudaLaunchKernel(const void *f, uint64_t gxy, uint32_t gz, uint64_t, uint32_t, void **, size_t, void *st) { return launch(f, st, (unsigned)gxy, (unsigned)(gxy >> 32), gz); }
+int cudaLaunchKernelExC(const void *cfg, const void *f, void **) {
+    const unsigned *g = static_cast<const unsigned *>(cfg);
+    return launch(f, *reinterpret_cast<void *const *>(static_cast<const char *>(cfg) + 32), g[0], g[1], g[2]);
+}
 
 // ---- what the compiler's start-up code calls ----
 void **__cudaRegisterFatBinary(void *) { static void *h; return &h; }

@@ -96,3 +96,24 @@ for target, fails in ((1, 1), (1, 0), (0, 1), (0, 0), (1, 1)):
     assert [s[0] for s in out["steps"]] == [nomem, 0, nomem, 0, nomem]
     assert [s[1] for s in out["steps"]] == [True, False, True, False, True]
     assert all(s[2] == 0 and s[3] > 0 for s in out["steps"]), out
+
+
+def test_update_follows_a_replaced_communicator(fake_cuda):
+    """The shares of a sharded update belong to a communicator: alone again a rank steps every parameter, among more ranks fewer."""
+    out = fake_cuda("""
+ctx = context(hidden_dim=128, n_layers=4, seq_len=32, population_size=64)
+def blocks():
+    fake.fake_clear()
+    ctx.apply_update(1, 0.1)
+    return [l.split()[-1] for l in log() if "upd_adam_kernel" in l]
+out["all"] = blocks()
+ctx.comm_init(bytes(128), 0, 2)
+ctx.set_update_sharding(True)
+out["two"] = blocks()
+ctx.comm_init(bytes(128), 0, 8)
+out["eight"] = blocks()
+ctx.comm_init(bytes(128), 0, 1)
+out["alone"] = blocks()
+""")
+    n = {k: sum(int(g.split(",")[0]) for g in v) for k, v in out.items()}
+    assert n["alone"] == n["all"] and n["eight"] < n["two"] < n["all"], n
