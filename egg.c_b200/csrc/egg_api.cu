@@ -1499,6 +1499,10 @@ extern "C" int egg_perturbed_projection(egg_ctx *c, const int8_t *x, const int8_
         set_error("projection shape unsupported (rows %lld, K %d, N %d, rows/member %d)", (long long)rows, K, N, rows_per_member);
         return EGG_E_INVALID;
     }
+    if (on_device && ((reinterpret_cast<uintptr_t>(x) & 15) || ((reinterpret_cast<uintptr_t>(w_packed) | reinterpret_cast<uintptr_t>(y)) & 3))) {
+        set_error("device pointers of a projection: x needs 16-byte alignment, w_packed and y 4-byte (%p, %p, %p)", (const void *)x, (const void *)w_packed, (void *)y);
+        return EGG_E_INVALID;
+    }
     EGG_CUDA(cudaSetDevice(c->device));
     cudaStream_t st = c->stream;
     const int64_t pairs = rows / rows_per_member / 2;
@@ -1529,6 +1533,8 @@ extern "C" int egg_perturbed_projection(egg_ctx *c, const int8_t *x, const int8_
     memset(&g, 0, sizeof(g));
     g.M = (int)rows; g.N = N; g.K = K; g.seq_len = g.tok_len = rows_per_member; g.nt = d_nt; g.nt_stride = stride; g.nt_a_off = 0; g.nt_c_off = -1; g.nt_d_off = -1;
     g.xb = d_xb; g.xb_stride = 1; g.rank1_shift = rank1_shift; g.out_shift = out_shift; g.out8 = d_y; g.err = c->d_err;
+    // the row-per-lane epilogue stores 16-byte boxes or 8-byte words, the other one 4-byte words
+    if (reinterpret_cast<uintptr_t>(d_y) & 15) g.rpl = -1;
     PTRY(launch_gemm(st, EPI_CLIP8, d_x, d_wt, g, c->num_sms));
     if (!on_device) PTRYC(cudaMemcpyAsync(y, d_y, (size_t)(rows * N), cudaMemcpyDeviceToHost, st));
     PTRYC(cudaStreamSynchronize(st));

@@ -249,7 +249,8 @@ int egg_generation_host(egg_ctx *ctx, const void *host_tokens, int64_t n_tokens,
  *   y[r][n] = clip((Σ_k x[r][k]·W[k][n] + ((xb_r·a_j[n]·ns_r) >> rank1_shift)) >> out_shift)
  * with member = r / rows_per_member, j = member/2, ns = +1/-1 for even/odd
  * member, a_j[n] = noise(seed + j + off_a, n), b_j[k] = noise(seed + j + off_b, k),
- * xb_r = Σ_k x[r][k]·b_j[k].  W is in the packed [K/4][N][4] layout.
+ * xb_r = Σ_k x[r][k]·b_j[k].  W is in the packed [K/4][N][4] layout.  Device pointers: x 16-byte aligned,
+ * w_packed and y 4-byte; a y that is 16-byte aligned as well takes the faster stores.
  */
 int egg_perturbed_projection(egg_ctx *ctx, const int8_t *x, const int8_t *w_packed,
                              int8_t *y, int64_t rows, int k_dim, int n_dim,

@@ -117,3 +117,23 @@ out["alone"] = blocks()
 """)
     n = {k: sum(int(g.split(",")[0]) for g in v) for k, v in out.items()}
     assert n["alone"] == n["all"] and n["eight"] < n["two"] < n["all"], n
+
+
+@pytest.mark.parametrize("rows_per_member,offset,rpl", [(64, 0, 1), (64, 16, 1), (64, 4, 0), (64, 8, 0), (20, 0, 0), (20, 4, 0), (64, 2, None)])
+@pytest.mark.parametrize("n", [256, 384, 4096])
+def test_projection_into_unaligned_memory(fake_cuda, n, rows_per_member, offset, rpl):
+    """The row-per-lane epilogue stores 16 bytes at a time: results elsewhere take the one that stores words, and what is not even
+    word-aligned is refused on the host."""
+    out = fake_cuda("""
+ctx = context(hidden_dim=128, n_layers=1, seq_len=32, population_size=8)
+rows, n, k, p = 2 * %d * 80, %d, 128, C.c_void_p()
+fake.cudaMalloc(C.byref(p), C.c_size_t(rows * (n + k) + n * k + 64))
+x, w = p.value, p.value + rows * k
+fake.fake_clear()
+out["rc"] = error(lambda: ctx.perturbed_projection(x, w, w + n * k + %d, rows, k, n, %d, 1, 200, 201, 7, 8, on_device=True))
+out["kernels"] = [l.split()[1] for l in log() if l.startswith("launch") and "gemm_i8" in l]
+""" % (rows_per_member, n, offset, rows_per_member))
+    if rpl is None:
+        assert out["rc"] < 0 and not out["kernels"]
+    else:
+        assert out["rc"] == 0 and len(out["kernels"]) == 1 and ("ELi0ELi%dE" % rpl) in out["kernels"][0], out
