@@ -1603,6 +1603,10 @@ extern "C" int egg_update_matrix(egg_ctx *c, int8_t *d_w_packed, void *d_opt_sta
     }
     const int amax = c->cfg.device_gaussian ? 3 * c->cfg.device_mask : c->cfg.device_mask;
     if (split && 16 * amax > 127) { set_error("noise magnitude %d does not fit the two-digit operand split", amax); return EGG_E_INVALID; }
+    if ((reinterpret_cast<uintptr_t>(d_opt_state) & 15) || (reinterpret_cast<uintptr_t>(d_fitness) & 3)) {
+        set_error("matrix update: the optimiser state needs 16-byte alignment, the fitness 4-byte (%p, %p)", d_opt_state, (const void *)d_fitness);
+        return EGG_E_INVALID;
+    }
     EGG_CUDA(cudaSetDevice(c->device));
     cudaStream_t st = c->stream;
     const int kp = (pairs + 127) / 128 * 128;
@@ -1616,12 +1620,20 @@ extern "C" int egg_update_matrix(egg_ctx *c, int8_t *d_w_packed, void *d_opt_sta
     UTRY(ctx_scratch(c, 7, (int64_t)cols_n * ktot, &u.na)); UTRY(ctx_scratch(c, 8, (int64_t)rows_k * ktot, &u.nb));
     UTRY(ctx_scratch(c, 9, (int64_t)rows_k * cols_n * splits, &u.votes));
     u.w_packed = d_w_packed; u.opt = static_cast<float *>(d_opt_state);
+    // the optimiser passes read and write words of four weights: weights anywhere else are stepped in an aligned copy
+    const bool copied = reinterpret_cast<uintptr_t>(d_w_packed) & 3;
+    const size_t wbytes = (size_t)rows_k * cols_n;
+    if (copied) {
+        UTRY(ctx_scratch(c, 10, (int64_t)wbytes, &u.w_packed));
+        EGG_CUDA(cudaMemcpyAsync(u.w_packed, d_w_packed, wbytes, cudaMemcpyDeviceToDevice, st));
+    }
     u.rows_k = rows_k; u.cols_n = cols_n; u.off_a = off_a; u.off_b = off_b; u.seed_base = seed_base;
     u.fit = d_fitness; u.pairs = pairs; u.kp = kp; u.operand_split = split ? 1 : 0;
     u.lr = lr; u.muon = optimizer;
     cudaError_t e = cudaMemsetAsync(c->d_updates, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) { set_error("cudaMemsetAsync: %s", cudaGetErrorString(e)); cleanup(); return EGG_E_CUDA; }
     UTRY(run_matrix_update(c, u, step_seed));
+    if (copied) EGG_CUDA(cudaMemcpyAsync(d_w_packed, u.w_packed, wbytes, cudaMemcpyDeviceToDevice, st));
 #undef UTRY
     return finish(c, nullptr, 0, 0, total_updates);
 }

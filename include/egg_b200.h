@@ -276,7 +276,8 @@ int egg_update_reconstruct(egg_ctx *ctx, const int32_t *fitness, int pairs,
  * d_opt_state its AdamParam{m,v,acc} (optimizer 0, 12 bytes per weight) or MuonParam{m,acc}
  * (optimizer 1, 8 bytes per weight) array in the same index order; both are updated in place.
  * d_fitness holds `pairs` int32 values; split = 1 takes the two-digit operand form for fitness
- * beyond ternary (|f| <= 127; needs 16 * noise magnitude <= 127).  All pointers are DEVICE pointers.
+ * beyond ternary (|f| <= 127; needs 16 * noise magnitude <= 127).  All pointers are DEVICE pointers;
+ * d_opt_state is 16-byte aligned, d_w_packed may lie anywhere.
  * Hyper-parameters (betas, eps, weight decay, Muon momentum and lr scale, noise mask) come from the
  * context's configuration.  *total_updates = number of weights that changed.  Its scratch (operands,
  * partial votes, Newton-Schulz workspace) is allocated on first use, kept in the context for later calls

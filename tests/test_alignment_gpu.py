@@ -27,3 +27,31 @@ def test_projection_into_words(n, rows_per_member, pairs, offset):
     assert (z[offset:offset + rows * n] == y.cpu().numpy()).all()
     assert (z[:offset] == 99).all() and (z[offset + rows * n:] == 99).all()
     ctx.close()
+
+
+@pytest.mark.parametrize("offset", [1, 2, 3, 4])
+@pytest.mark.parametrize("optimizer", [0, 1])
+def test_matrix_update_of_weights_anywhere(optimizer, offset):
+    import torch
+    pkg = load_pkg()
+    ctx = pkg.Context(pkg.default_config(device_mask=3, population_size=64), 0, 2)
+    rows, cols, pairs = 128, 384, 100
+    g = torch.Generator(device="cuda")
+    g.manual_seed(offset)
+    w = torch.randint(-127, 128, (rows * cols,), generator=g, device="cuda", dtype=torch.int8)
+    v = torch.full((rows * cols + 8,), 99, dtype=torch.int8, device="cuda")
+    v[offset:offset + rows * cols] = w
+    opt = torch.randn(rows * cols, 3 - optimizer, generator=g, device="cuda")
+    if not optimizer:
+        opt[:, 1].square_()
+    opt2 = opt.clone()
+    fit = torch.randint(-1, 2, (pairs,), generator=g, device="cuda", dtype=torch.int32)
+    torch.cuda.synchronize()
+    n = [ctx.update_matrix(p, o.data_ptr(), rows, cols, 402, 403, 0, fit.data_ptr(), pairs, 7, 0.4, optimizer, False)
+         for p, o in ((w.data_ptr(), opt), (v.data_ptr() + offset, opt2))]
+    v = v.cpu().numpy()
+    # the norm's terms are added in any order: a weight on a rounding boundary may differ under Muon
+    assert (v[offset:offset + rows * cols] != w.cpu().numpy()).sum() <= (2 if optimizer else 0)
+    assert abs(n[0] - n[1]) <= (2 if optimizer else 0) and n[0] > 0
+    assert (v[:offset] == 99).all() and (v[offset + rows * cols:] == 99).all()
+    ctx.close()

@@ -137,3 +137,25 @@ out["kernels"] = [l.split()[1] for l in log() if l.startswith("launch") and "gem
         assert out["rc"] < 0 and not out["kernels"]
     else:
         assert out["rc"] == 0 and len(out["kernels"]) == 1 and ("ELi0ELi%dE" % rpl) in out["kernels"][0], out
+
+
+@pytest.mark.parametrize("optimizer", [0, 1])
+@pytest.mark.parametrize("w_off,opt_off,copies", [(0, 0, 0), (4, 16, 0), (1, 0, 2), (2, 0, 2), (0, 4, None), (0, 8, None)])
+def test_matrix_update_of_unaligned_weights(fake_cuda, optimizer, w_off, opt_off, copies):
+    """Weights that are not word-aligned are stepped in an aligned copy; a state that is not 16-byte aligned is refused."""
+    out = fake_cuda("""
+ctx = context(hidden_dim=128, n_layers=1, seq_len=32, population_size=8)
+p = C.c_void_p()
+fake.cudaMalloc(C.byref(p), C.c_size_t(1 << 20))
+w, opt, fit = p.value + %d, p.value + (1 << 16) + %d, p.value + (1 << 19)
+update = lambda off: ctx.update_matrix(w + off, opt, 128, 128, 402, 403, 0, fit, 100, 1, 0.1, %d, False)
+for off in (-%d, 0):                  # the first call leaves the scratch behind
+    fake.fake_clear()
+    out["rc"] = error(lambda: update(off))
+    out.setdefault("copies", []).append(sum(l.startswith("copy") for l in log()))
+out["kernels"] = launches("")
+""" % (w_off, opt_off, optimizer, w_off))
+    if copies is None:
+        assert out["rc"] < 0 and out["kernels"] == 0
+    else:
+        assert out["rc"] == 0 and out["copies"][1] - out["copies"][0] == copies
