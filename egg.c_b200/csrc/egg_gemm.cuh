@@ -88,7 +88,7 @@ struct GemmParams {
     FastDiv fd_seq, fd_tiles_n, fd_third, fd_head;
     int lut_stride;              // bytes between entries of the replicated GELU table (filled by launch_gemm)
     int one;                     // 1 (filled by launch_gemm): the multiplier of additions issued as multiply-adds
-    int pow_t;                   // EPI_GELU: 2^rank1_shift when both shifts may be merged into one (0: keep two shifts)
+    int pow_t;                   // EPI_GELU, EPI_LOGITS: merged_shift()
 };
 
 template <int BN>

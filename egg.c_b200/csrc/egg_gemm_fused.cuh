@@ -49,7 +49,7 @@ struct FusedParams {
     const int32_t *xb;           // Σ_k a_k b_k per row and part: xb[r * xb_stride + part]
     int xb_stride;
     int rank1_shift, out_shift;
-    int pow_t;                   // 2^rank1_shift when both shifts may be merged into one (0: keep two), filled by launch_gemm_fused
+    int pow_t;                   // FUSED_RES: merged_shift(), filled by launch_gemm_fused
     int one;                     // 1 (filled by launch_gemm_fused): the multiplier of additions issued as multiply-adds
     const int8_t *bias;          // FUSED_RES: [H] or null
     const int2 *rope_t;          // [head_dim/2][seq_len] (cos, sin)

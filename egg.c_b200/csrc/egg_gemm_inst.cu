@@ -227,12 +227,7 @@ int launch_gemm_fused(cudaStream_t st, int mode, const int8_t *A, const int8_t *
     p.fd_head = make_fastdiv(p.head_dim > 0 ? p.head_dim : 64);
     p.fd_h = make_fastdiv(p.H);
     p.one = 1;
-    {
-        // |acc| * 2^t + |xb * a| + |(bias + noise) << (s + t)| < 2^31 for every input: |acc| <= K * 127^2, |xb| <= K * 127 * 31,
-        // |a| <= 31 (the largest noise mask), |bias + noise| <= 254
-        const int64_t bound = (int64_t)p.K * 16129 * (1ll << p.rank1_shift) + (int64_t)p.K * 127 * 961 + (254ll << (p.out_shift + p.rank1_shift));
-        p.pow_t = mode == FUSED_RES && bound < (1ll << 31) ? 1 << p.rank1_shift : 0;
-    }
+    p.pow_t = mode == FUSED_RES ? merged_shift(p.K, p.rank1_shift, p.out_shift) : 0;
     CUtensorMap ta, tb, to, tr;
     int rc;
     if ((rc = make_tmap(&ta, A, (uint64_t)p.M, (uint64_t)p.K, GEMM_BM))) return rc;
@@ -303,13 +298,7 @@ int launch_gemm(cudaStream_t st, int epi, const int8_t *A, const int8_t *B, cons
         set_error("shifts %d + %d too large for the pre-shifted bias table", p.out_shift, p.rank1_shift);
         return EGG_E_INVALID;
     }
-    p.pow_t = 0;
-    if (epi == EPI_GELU || epi == EPI_LOGITS) {
-        // both shifts as one when |acc| * 2^t + |xb * a| + |(bias + noise) << (s + t)| < 2^31 for every input:
-        // |acc| <= K * 127^2, |xb| <= K * 127 * 31, |a| <= 31 (the largest noise mask), |bias + noise| <= 254
-        const int64_t bound = (int64_t)p.K * 16129 * (1ll << p.rank1_shift) + (int64_t)p.K * 127 * 961 + (254ll << (p.out_shift + p.rank1_shift));
-        if (bound < (1ll << 31)) p.pow_t = 1 << p.rank1_shift;
-    }
+    p.pow_t = epi == EPI_GELU || epi == EPI_LOGITS ? merged_shift(p.K, p.rank1_shift, p.out_shift) : 0;
     CUtensorMap ta, tb;
     int rc;
     if ((rc = make_tmap(&ta, A, (uint64_t)p.M, (uint64_t)p.K, GEMM_BM))) return rc;

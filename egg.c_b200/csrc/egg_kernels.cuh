@@ -156,6 +156,14 @@ inline bool fused_supported(int hidden, int seq_len) { return seq_len % 32 == 0 
 // Largest output shift + rank-1 shift of the projections that add their bias before both (the row-owning residual projections
 // and MLP-up): (bias + noise) << (both shifts) joins a product below 2^30.
 constexpr int PRESHIFT_MAX = 20;
+// 2^rank1_shift where the rank-1 shift t and the output shift s of a projection over K may be merged into one, else 0:
+// |acc| * 2^t + |xb * a| + |(bias + noise) << (s + t)| < 2^31 for every input.  |acc| <= K * 127 * 128 (activations are clipped to
+// 127, a weight may be -128), |xb| <= K * 127 * 45, |a| <= 45 (three noise values of mask 15 added), |bias + noise| <= 256.
+inline int merged_shift(int K, int rank1_shift, int out_shift) {
+    if (rank1_shift > PRESHIFT_MAX || out_shift > PRESHIFT_MAX) return 0;
+    const int64_t bound = (int64_t)K * 127 * 128 * (1ll << rank1_shift) + (int64_t)K * 127 * 45 * 45 + (256ll << (out_shift + rank1_shift));
+    return bound < (1ll << 31) ? 1 << rank1_shift : 0;
+}
 // Rows that hold one member's seq_len tokens: padded to whole 32-row groups where that opens the row-owning kernels and the
 // row-per-lane epilogues for at most a third more rows (48 -> 64 costs 1.33; 16 -> 32 would double the work).
 inline int member_rows(int hidden, int seq_len) {

@@ -159,3 +159,24 @@ out["kernels"] = launches("")
         assert out["rc"] < 0 and out["kernels"] == 0
     else:
         assert out["rc"] == 0 and out["copies"][1] - out["copies"][0] == copies
+
+
+@pytest.mark.parametrize("hidden,fixed,sigma,shift_out,merged", [
+    (128, 4, 3, 9, True), (512, 4, 3, 9, True), (896, 4, 3, 9, True), (1024, 4, 3, 9, False),      # the default shifts
+    (896, 4, 3, 12, False), (256, 5, 4, 4, False), (128, 5, 5, 4, False), (128, 5, 5, 0, False),   # 2^31 within the noise of three values of 15
+])
+def test_merged_shifts_cannot_overflow(fake_cuda, hidden, fixed, sigma, shift_out, merged):
+    """The output projection shifts once instead of twice only where its accumulator times 2^t, the largest rank-1 term (Gaussian
+    noise reaches three times the mask) and the shifted bias together fit 32 bits."""
+    largest = hidden * 127 * 128 * 2 ** (fixed + sigma) + hidden * 127 * 45 * 45 + 256 * 2 ** (fixed + sigma + shift_out)
+    assert (largest < 2 ** 31) == merged
+    out = fake_cuda("""
+ctx = context(hidden_dim=%d, n_layers=1, seq_len=128, population_size=8, fixed_point=%d, sigma_shift=%d, shift_out=%d, shift_mlp_down=0, sigma_shift_vector=8,
+              device_gaussian=1)
+ctx.eval_chunk(1, 0, 0, 8)
+out["kernels"] = [l.split()[1] for l in log() if l.startswith("launch") and "gemm_fused" in l]
+""" % (hidden, fixed, sigma, shift_out))
+    # <tile width, mode (1: output projection), tables per quarter, merged>
+    got = [k.split("gemm_fused_kernelI")[1].split("EEEv")[0] for k in out["kernels"]]
+    assert any(k.endswith("Lb%d" % merged) for k in got if "ELi1E" in k), got
+    assert merged or not any(k.endswith("Lb1") for k in got if "ELi1E" in k), got
