@@ -676,14 +676,13 @@ static int gru_window_buffers(egg_gru_ctx *c, int tokens) {
 // over [population x window] rows and its products run on the tcgen05 GEMM.  Layer l of window w needs layer l of w - 1 (the
 // state) and layer l - 1 of w (the rows): layers run as a wavefront on streams of their own, so that one layer's recurrence,
 // a chain of latencies on a few SMs, hides behind the others' products.
-static int gru_windows(egg_gru_ctx *c, int64_t start_idx, int tokens) {
-    int rc = gru_window_buffers(c, tokens);
-    if (rc) return rc;
+static int gru_wavefront(egg_gru_ctx *c, int64_t start_idx, int tokens) {
     const egg_gru_config &cf = c->cfg;
     const int H = cf.hidden_dim, POP = cf.population_size, NL = cf.n_layers;
     const GruLayout &L = c->L;
     const int64_t HH = (int64_t)H * H;
     const int windows = (tokens + c->win - 1) / c->win;
+    int rc;
     EGG_CUDA(cudaEventRecord(c->fork, c->stream));
     for (int i = 0; i < c->ns; i++) EGG_CUDA(cudaStreamWaitEvent(c->lane[i].st, c->fork, 0));
     for (int d = 0; d < windows + NL - 1; d++)
@@ -747,11 +746,22 @@ static int gru_windows(egg_gru_ctx *c, int64_t start_idx, int tokens) {
             }
             EGG_CUDA(cudaEventRecord(sl.ev, st));
         }
-    for (int i = 0; i < c->ns; i++) {
-        EGG_CUDA(cudaEventRecord(c->lane[i].join, c->lane[i].st));
-        EGG_CUDA(cudaStreamWaitEvent(c->stream, c->lane[i].join, 0));
-    }
     return EGG_OK;
+}
+
+static int gru_windows(egg_gru_ctx *c, int64_t start_idx, int tokens) {
+    int rc = gru_window_buffers(c, tokens);
+    if (rc) return rc;
+    rc = gru_wavefront(c, start_idx, tokens);
+    // a call that failed half-way leaves kernels on the lanes: what follows on the context's stream waits for them all the same
+    cudaError_t e = cudaSuccess;
+    for (int i = 0; i < c->ns; i++) {
+        cudaError_t r = cudaEventRecord(c->lane[i].join, c->lane[i].st);
+        if (r == cudaSuccess) r = cudaStreamWaitEvent(c->stream, c->lane[i].join, 0);
+        if (e == cudaSuccess) e = r;
+    }
+    if (!rc && e != cudaSuccess) { set_error("joining the window streams failed: %s", cudaGetErrorString(e)); rc = EGG_E_CUDA; }
+    return rc;
 }
 
 extern "C" int egg_gru_generation(egg_gru_ctx *c, uint32_t step_seed, int64_t start_idx, int tokens, int do_update,

@@ -23,6 +23,7 @@ uintptr_t next_handle = 0x1000;
 long mallocs = 0, fail_malloc = -1, host_allocs = 0;
 std::string fail_kernel;
 long fail_kernel_after = 0;
+int last_error = 0;
 struct Config { unsigned g[3], b[3]; size_t smem; void *st; } pushed;
 
 void note(const char *what, const std::string &rest) { log_text += std::string(what) + " " + rest + "\n"; }
@@ -31,7 +32,7 @@ void *take(size_t n) { return mmap(nullptr, n ? n : 1, PROT_READ | PROT_WRITE, M
 int launch(const void *f, void *st, unsigned gx, unsigned gy, unsigned gz) {
     std::lock_guard<std::mutex> l(m);
     const std::string &name = kernels[f];
-    if (!fail_kernel.empty() && name.find(fail_kernel) != std::string::npos && fail_kernel_after-- == 0) { note("failed", name + " " + hex(st)); return 719; }
+    if (!fail_kernel.empty() && name.find(fail_kernel) != std::string::npos && fail_kernel_after-- == 0) { note("failed", name + " " + hex(st)); return last_error = 719; }
     note("launch", name + " " + hex(st) + " " + std::to_string(gx) + "," + std::to_string(gy) + "," + std::to_string(gz));
     return 0;
 }
@@ -100,7 +101,7 @@ int cudaGetDevice(int *d) { *d = 0; return 0; }
 int cudaSetDevice(int) { return 0; }
 int cudaDeviceGetAttribute(int *v, int a, int) { *v = a == 75 ? 10 : (a == 16 ? 148 : 0); return 0; }
 int cudaGetDriverEntryPoint(const char *, void **fn, unsigned long long, int *res) { *fn = (void *)encode_tiled; if (res) *res = 0; return 0; }
-int cudaGetLastError() { return 0; }
+int cudaGetLastError() { const int e = last_error; last_error = 0; return e; }
 const char *cudaGetErrorString(int e) { return e == 2 ? "out of memory" : "a failure the test asked for"; }
 int cudaFuncSetAttribute(const void *, int, int) { return 0; }
 int cudaOccupancyMaxActiveClusters(int *n, const void *, const void *) { *n = 74; return 0; }

@@ -32,6 +32,14 @@ def error(call):
     try: call()
     except pkg.EggError as e: return e.code
     return 0
+def unjoined(main):
+    # streams on which something was launched that `main` does not wait for afterwards
+    lines, left = [l.split() for l in log()], []
+    for st in {l[2] for l in lines if l[0] == "launch"} - {main}:
+        last = max(i for i, l in enumerate(lines) if l[0] == "launch" and l[2] == st)
+        marks = [(i, l[1]) for i, l in enumerate(lines) if l[0] == "record" and l[2] == st and i > last]
+        if not any(l[0] == "wait" and l[1] == main and l[2] == ev and i > at for at, ev in marks for i, l in enumerate(lines)): left.append(st)
+    return left
 out = {}
 """ % HERE
 
@@ -180,3 +188,21 @@ out["kernels"] = [l.split()[1] for l in log() if l.startswith("launch") and "gem
     got = [k.split("gemm_fused_kernelI")[1].split("EEEv")[0] for k in out["kernels"]]
     assert any(k.endswith("Lb%d" % merged) for k in got if "ELi1E" in k), got
     assert merged or not any(k.endswith("Lb1") for k in got if "ELi1E" in k), got
+
+
+@pytest.mark.parametrize("kernel,after", [(None, 0), ("gru_scan_kernel", 0), ("gru_scan_kernel", 5), ("gru_rows_kernel", 7), ("gemm_i8_kernel", 11), ("gru_loss_rows", 1)])
+def test_recurrent_windows_are_joined_also_when_a_launch_fails(fake_cuda, kernel, after):
+    """Whatever was enqueued on the window streams is waited for by the context's stream, on which the next call works."""
+    out = fake_cuda("""
+cfg = pkg.default_gru_config(hidden_dim=128, n_layers=4, population_size=32, seq_len=4096)
+ctx = pkg.GruContext(cfg, 0)
+ctx.upload_model(np.zeros(pkg.gru_model_bytes(cfg), np.int8))
+ctx.set_dataset(np.zeros(9000, np.uint8))
+kernel, after = %r, %d
+if kernel: fake.fake_fail_kernel(kernel.encode(), after)
+fake.fake_clear()
+out["rc"] = error(lambda: ctx.generation(1, 0, 4000, True))
+main = next(l.split()[2] for l in log() if "gru_noise_kernel" in l)
+out["streams"], out["left"] = len({l.split()[2] for l in log() if l.startswith("launch")}), unjoined(main)
+""" % (kernel, after))
+    assert (out["rc"] < 0) == (kernel is not None) and out["streams"] > 1 and out["left"] == [], out
