@@ -1387,6 +1387,7 @@ static int muon_steps(egg_ctx *c, int batch, float lr) {
     for (const MuonGroup &g : pl.groups) {
         if (g.batch != batch) continue;
         cudaStream_t st = c->side[g.slot];
+        c->side_used[g.slot] = true;
         EGG_CUDA(cudaStreamWaitEvent(st, c->ev_m, 0));
         NsWs ws;
         ns_ws_carve(ws, c->upd.muon_ws[g.slot], g.rows, g.cols, g.count);
@@ -1395,20 +1396,15 @@ static int muon_steps(egg_ctx *c, int batch, float lr) {
         if ((rc = launch_newton_schulz(st, ws, g.rows, g.cols, g.count, c->d_err, c->num_sms))) return rc;
         if ((rc = launch_muon_apply(st, pl.d_mats, pl.d_list + g.first, g.count, g.rows, g.cols, ws.y, c->d_model, c->d_opt, c->d_shadow,
                                     lr * cf.muon_lr_scale, cf.adam_weight_decay, c->d_updates))) return rc;
-        EGG_CUDA(cudaEventRecord(c->ev_done[g.slot], st));
-        c->side_used[g.slot] = true;
     }
     return EGG_OK;
 }
 
-static int apply_update_async(egg_ctx *c, uint32_t step_seed, float lr) {
+static int update_steps(egg_ctx *c, uint32_t step_seed, float lr) {
     const egg_config &cf = c->cfg;
     int rc;
-    if (c->upd_share != plan_share(c) && (rc = prepare_update(c))) return rc;
     const UpdPlan &pl = c->plan;
     cudaStream_t st = c->stream;
-    ChainScope chain(c->model_bytes <= CHAIN_MAX_WEIGHTS);
-    const bool sharded = update_is_sharded(c);                 // then the plan holds this rank's own parameters only
     UpdHyper h;
     h.lr = lr; h.beta1 = cf.adam_beta1; h.beta2 = cf.adam_beta2; h.eps = cf.adam_eps; h.wd = cf.adam_weight_decay; h.mu = cf.muon_momentum;
     uint8_t *changed = c->scales_on ? c->d_changed : nullptr;
@@ -1423,8 +1419,27 @@ static int apply_update_async(egg_ctx *c, uint32_t step_seed, float lr) {
     }
     // UPDATE_OVERLAY of every parameter (worker.cu:445-455)
     if (c->scales_on && (rc = PROF(EGG_PROF_OVERLAY, launch_overlay_step_all(st, c->d_scales, c->d_changed, c->d_ov_active, (int)c->SL.total, c->ov_inc, c->ov_dec)))) return rc;
-    for (int b = 0; b < 3; b++)
-        if (c->side_used[b]) { EGG_CUDA(cudaStreamWaitEvent(st, c->ev_done[b], 0)); c->side_used[b] = false; }
+    return EGG_OK;
+}
+
+static int apply_update_async(egg_ctx *c, uint32_t step_seed, float lr) {
+    int rc;
+    if (c->upd_share != plan_share(c) && (rc = prepare_update(c))) return rc;
+    cudaStream_t st = c->stream;
+    ChainScope chain(c->model_bytes <= CHAIN_MAX_WEIGHTS);
+    const bool sharded = update_is_sharded(c);                 // then the plan holds this rank's own parameters only
+    rc = update_steps(c, step_seed, lr);
+    // an update that failed half-way leaves kernels on the side streams: what follows on the context's stream waits for them all the same
+    cudaError_t e = cudaSuccess;
+    for (int b = 0; b < 3; b++) {
+        if (!c->side_used[b]) continue;
+        c->side_used[b] = false;
+        cudaError_t r = cudaEventRecord(c->ev_done[b], c->side[b]);
+        if (r == cudaSuccess) r = cudaStreamWaitEvent(st, c->ev_done[b], 0);
+        if (e == cudaSuccess) e = r;
+    }
+    if (rc) return rc;
+    EGG_CUDA(e);
     if (sharded) {
         // the new weights travel from their owners; the owners' change counts add up to the generation's
         if ((rc = broadcast_params(c, false))) return rc;

@@ -206,3 +206,18 @@ main = next(l.split()[2] for l in log() if "gru_noise_kernel" in l)
 out["streams"], out["left"] = len({l.split()[2] for l in log() if l.startswith("launch")}), unjoined(main)
 """ % (kernel, after))
     assert (out["rc"] < 0) == (kernel is not None) and out["streams"] > 1 and out["left"] == [], out
+
+
+@pytest.mark.parametrize("kernel,after", [(None, 0), ("muon_split", 0), ("muon_split", 2), ("ns_gemm", 0), ("ns_gemm", 13), ("muon_apply", 0), ("muon_apply", 1)])
+def test_muon_streams_are_joined_also_when_a_launch_fails(fake_cuda, kernel, after):
+    out = fake_cuda("""
+ctx = context(hidden_dim=128, n_layers=2, seq_len=32, population_size=64, use_muon=1)
+kernel, after = %r, %d
+if kernel: fake.fake_fail_kernel(kernel.encode(), after)
+fake.fake_clear()
+out["rc"] = error(lambda: ctx.apply_update(1, 0.1))
+main = next(l.split()[2] for l in log() if "upd_table_kernel" in l)
+out["streams"], out["left"] = len({l.split()[2] for l in log() if l.startswith("launch")}), unjoined(main)
+""" % (kernel, after))
+    assert (out["rc"] < 0) == (kernel is not None) and out["left"] == [], out
+    assert out["streams"] > 1 or (kernel, after) == ("muon_split", 0)
