@@ -39,15 +39,20 @@ struct GruStream { int rows, cols, seed_off; int64_t a_off, b_off; };   // offse
 
 __device__ __forceinline__ uint32_t xorshift32(uint32_t &x) { x ^= x << 13; x ^= x >> 17; x ^= x << 5; return x; }
 
-// gen_noise_vector_neon (full_trained_egg.c:88-104): four draws are discarded before every 16 values.
+// gen_noise_vector_neon (full_trained_egg.c:88-104): four draws are discarded before every 16 values.  Lengths are multiples of 128
+// and the vectors of neighbouring threads lie a pair's noise (tens of KB) apart, so each 16 values leave as one store: byte by
+// byte a generation took 0.39 ms longer (one token at H 512, 4 layers, 128 members: 1008 -> 622 us; 904 with vectors side by side).
 __device__ void gru_noise_vector(uint32_t &rng, int8_t *out, int count) {
     for (int i = 0; i < count; i += 16) {
         xorshift32(rng); xorshift32(rng); xorshift32(rng); xorshift32(rng);
-        for (int j = i; j < i + 16 && j < count; j++) {
+        uint32_t w[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
             const uint32_t r = xorshift32(rng);
             const int mag = (int)((r >> 1) & 31u);
-            out[j] = (int8_t)((r & 1u) ? mag : -mag);
+            w[j >> 2] |= (uint32_t)(((r & 1u) ? mag : -mag) & 0xFF) << (8 * (j & 3));
         }
+        *reinterpret_cast<uint4 *>(out + i) = make_uint4(w[0], w[1], w[2], w[3]);
     }
 }
 
