@@ -46,9 +46,9 @@ def test_update_against_oracle(kw, amp):
 ])
 def test_products_that_wrap_equal_the_isolated_update(amp, kw):
     """Fitness times noise beyond a byte wraps on the outputs' side whatever the matrix's shape: every matrix of the model
-    update equals the isolated update of that matrix, which has no other form."""
+    update equals the isolated update of that matrix, which has no other form.  Vectors do not wrap: they equal the oracle's."""
     import torch
-    pkg = load_pkg()
+    pkg, O = load_pkg(), load_oracle()
     H, V = 128, kw.get("vocab_size", 256)
     pop = 614
     cfg = pkg.default_config(hidden_dim=H, n_layers=1, seq_len=16, population_size=pop, **kw)
@@ -64,6 +64,13 @@ def test_products_that_wrap_equal_the_isolated_update(amp, kw):
     w_q = after_init + 2 * H
     w_up = w_q + 4 * H * H + 2 * H
     w_down = w_up + 4 * H * H + 4 * H
+    ocfg = O.make_config(hidden_dim=H, n_layers=1, seq_len=16, population_size=pop, **kw)
+    want, want_state = model.copy(), np.zeros(O.opt_bytes(ocfg), np.uint8)
+    O.update(ocfg, want, want_state, fit, 77, 0.4)
+    want_state = want_state.view(np.float32).reshape(-1, 3)
+    for off, length in ((V * H, 3 * H), (V * H + 3 * H + 4 * H * H, 4 * H), (after_init - H, 3 * H), (w_up - 2 * H, 2 * H), (w_down - 4 * H, 4 * H),
+                        (w_down + 4 * H * H, 3 * H)):
+        assert (state[off:off + length] == want_state[off:off + length]).all() and (got[off:off + length] == want[off:off + length]).all(), off
     d_fit = torch.from_numpy(fit).cuda()
     for off, rows, cols, a, b in ((0, H, V, 0, H), (V * H + 3 * H, H, 4 * H, 510, 511), (V * H + 3 * H + 4 * H * H + 4 * H, 4 * H, H, 512, 513),
                                   (w_q, H, H, 200, 201), (w_up, H, 4 * H, 400, 401), (w_down, 4 * H, H, 402, 403)):
