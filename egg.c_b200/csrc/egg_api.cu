@@ -82,6 +82,7 @@ struct alignas(16) Status { unsigned long long updates; int err[2]; };
 static_assert(sizeof(Status) == 16, "published as one word");
 constexpr int PIN_LOSSES = 16384;
 struct PinnedBlock { Status status; int32_t losses[PIN_LOSSES]; };
+static_assert(sizeof(PinnedBlock) <= PIN_STATUS, "a context's share of a pinned block");
 
 struct egg_ctx {
     egg_config cfg;
@@ -389,7 +390,7 @@ extern "C" void egg_ctx_destroy(egg_ctx *c) {
     if (c->comm && g_nccl.CommDestroy) g_nccl.CommDestroy(c->comm);
     void *ptrs[] = {c->arena, c->upd.base, c->pre_base, c->d_data};
     host_stage_free(c->stage);
-    pinned_give(reinterpret_cast<uint8_t *>(c->pin));
+    pinned_give_status(reinterpret_cast<uint8_t *>(c->pin));
     pinned_release();
     for (void *p : ptrs) if (p) cudaFree(p);
     for (int b = 0; b < 3; b++) {
@@ -547,7 +548,7 @@ extern "C" int egg_ctx_create(const egg_config *cfg, int device, int wave_member
     TRY(ar.commit(&c->arena));
     c->d_k = c->d_q + R * H; c->d_v = c->d_q + 2 * R * H;
     c->d_updates = &c->d_status->updates; c->d_err = c->d_status->err;
-    c->pin = reinterpret_cast<PinnedBlock *>(pinned_take());
+    c->pin = reinterpret_cast<PinnedBlock *>(pinned_take_status());
     if (!c->pin) { set_error("no pinned host memory"); egg_ctx_destroy(c); return EGG_E_NOMEM; }
     TRYC(cudaMemsetAsync(c->d_opt, 0, (size_t)c->opt_bytes, c->stream));
     TRYC(cudaMemsetAsync(c->d_loss, 0, (size_t)POP * 4, c->stream)); TRYC(cudaMemsetAsync(c->d_fit, 0, (size_t)(POP / 2) * 4, c->stream));

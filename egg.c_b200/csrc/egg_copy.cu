@@ -25,12 +25,19 @@ int DeviceArena::commit(void **base) {
 namespace {
 struct PinnedPool {
     std::mutex m;
-    int users = 0;
-    std::vector<uint8_t *> slabs, free_blocks;
+    int users = 0, copy_slabs = 0;
+    std::vector<uint8_t *> slabs, free_blocks, free_status;
+    bool grow() {
+        void *slab = nullptr;
+        if (cudaHostAlloc(&slab, PIN_SLAB, cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); return false; }
+        slabs.push_back(static_cast<uint8_t *>(slab));
+        for (int64_t o = PIN_SLAB - PIN_BLOCK; o >= 0; o -= PIN_BLOCK) free_blocks.push_back(static_cast<uint8_t *>(slab) + o);
+        return true;
+    }
+    static constexpr int64_t PIN_SLAB = 4 << 20;
 };
 PinnedPool g_pins;
-constexpr int64_t PIN_SLAB = 4 << 20;
-constexpr size_t PIN_MAX_SLABS = 64;
+constexpr int PIN_MAX_SLABS = 64;
 }  // namespace
 
 void pinned_retain() {
@@ -43,15 +50,14 @@ void pinned_release() {
     for (uint8_t *s : g_pins.slabs) cudaFreeHost(s);
     g_pins.slabs.clear();
     g_pins.free_blocks.clear();
+    g_pins.free_status.clear();
+    g_pins.copy_slabs = 0;
 }
 uint8_t *pinned_take() {
     std::lock_guard<std::mutex> l(g_pins.m);
     if (g_pins.free_blocks.empty()) {
-        if (g_pins.slabs.size() >= PIN_MAX_SLABS) return nullptr;
-        void *slab = nullptr;
-        if (cudaHostAlloc(&slab, PIN_SLAB, cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-        g_pins.slabs.push_back(static_cast<uint8_t *>(slab));
-        for (int64_t o = PIN_SLAB - PIN_BLOCK; o >= 0; o -= PIN_BLOCK) g_pins.free_blocks.push_back(static_cast<uint8_t *>(slab) + o);
+        if (g_pins.copy_slabs >= PIN_MAX_SLABS || !g_pins.grow()) return nullptr;
+        g_pins.copy_slabs++;
     }
     uint8_t *b = g_pins.free_blocks.back();
     g_pins.free_blocks.pop_back();
@@ -61,6 +67,23 @@ void pinned_give(uint8_t *block) {
     if (!block) return;
     std::lock_guard<std::mutex> l(g_pins.m);
     g_pins.free_blocks.push_back(block);
+}
+uint8_t *pinned_take_status() {
+    std::lock_guard<std::mutex> l(g_pins.m);
+    if (g_pins.free_status.empty()) {
+        if (g_pins.free_blocks.empty() && !g_pins.grow()) return nullptr;
+        uint8_t *b = g_pins.free_blocks.back();
+        g_pins.free_blocks.pop_back();
+        for (int64_t o = PIN_BLOCK / PIN_STATUS - 1; o >= 0; o--) g_pins.free_status.push_back(b + o * PIN_STATUS);
+    }
+    uint8_t *b = g_pins.free_status.back();
+    g_pins.free_status.pop_back();
+    return b;
+}
+void pinned_give_status(uint8_t *block) {
+    if (!block) return;
+    std::lock_guard<std::mutex> l(g_pins.m);
+    g_pins.free_status.push_back(block);
 }
 
 void host_stage_free(HostStage &h) {

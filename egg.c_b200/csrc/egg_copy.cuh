@@ -30,8 +30,12 @@ public:
 constexpr int64_t PIN_BLOCK = 512 << 10;
 void pinned_retain();
 void pinned_release();
-uint8_t *pinned_take();                            // null when the pool is at its bound (256 MB) or pinning fails
+uint8_t *pinned_take();                            // for copies; null when these hold 256 MB or pinning fails
 void pinned_give(uint8_t *block);
+// A context's own block, as long as it lives: seven to a block of the pool, as many as there are contexts.
+constexpr int64_t PIN_STATUS = 72 << 10;
+uint8_t *pinned_take_status();                     // null when pinning fails
+void pinned_give_status(uint8_t *block);
 
 // Copies into pageable memory: the driver moves them through one staging buffer on one CPU thread, page faults of a fresh
 // destination included: 4 to 7 GB/s, 2 to 3 ms for the 13 to 18 MB of a model.  Here a few threads each drain a pair of

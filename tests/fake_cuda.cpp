@@ -29,6 +29,14 @@ struct Config { unsigned g[3], b[3]; size_t smem; void *st; } pushed;
 void note(const char *what, const std::string &rest) { log_text += std::string(what) + " " + rest + "\n"; }
 std::string hex(const void *p) { char s[32]; snprintf(s, sizeof s, "%p", p); return s; }
 void *take(size_t n) { return mmap(nullptr, n ? n : 1, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_NORESERVE, -1, 0); }
+// zeros without holding the pages: most buffers are cleared and never touched
+void fill(void *d, int v, size_t n) {
+    const uintptr_t a = (reinterpret_cast<uintptr_t>(d) + 4095) & ~(uintptr_t)4095, e = (reinterpret_cast<uintptr_t>(d) + n) & ~(uintptr_t)4095;
+    if (v || e <= a) { memset(d, v, n); return; }
+    memset(d, 0, a - reinterpret_cast<uintptr_t>(d));
+    madvise(reinterpret_cast<void *>(a), e - a, MADV_DONTNEED);
+    memset(reinterpret_cast<void *>(e), 0, reinterpret_cast<uintptr_t>(d) + n - e);
+}
 int launch(const void *f, void *st, unsigned gx, unsigned gy, unsigned gz) {
     std::lock_guard<std::mutex> l(m);
     const std::string &name = kernels[f];
@@ -93,7 +101,7 @@ int cudaFreeHost(void *p) {
 int cudaMemcpyAsync(void *d, const void *s, size_t n, int, void *st) { memcpy(d, s, n); std::lock_guard<std::mutex> l(m); note("copy", hex(st)); return 0; }
 int cudaMemcpy(void *d, const void *s, size_t n, int) { memcpy(d, s, n); return 0; }
 int cudaMemset(void *d, int v, size_t n) { memset(d, v, n); return 0; }
-int cudaMemsetAsync(void *d, int v, size_t n, void *st) { memset(d, v, n); std::lock_guard<std::mutex> l(m); note("memset", hex(st)); return 0; }
+int cudaMemsetAsync(void *d, int v, size_t n, void *st) { fill(d, v, n); std::lock_guard<std::mutex> l(m); note("memset", hex(st)); return 0; }
 int cudaMemGetInfo(size_t *f, size_t *t) { *f = *t = (size_t)8 << 30; return 0; }
 int cudaPointerGetAttributes(void *a, const void *) { memset(a, 0, 16); return 0; }
 int cudaGetDeviceCount(int *n) { *n = 1; return 0; }

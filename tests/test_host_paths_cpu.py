@@ -221,3 +221,20 @@ out["streams"], out["left"] = len({l.split()[2] for l in log() if l.startswith("
 """ % (kernel, after))
     assert (out["rc"] < 0) == (kernel is not None) and out["left"] == [], out
     assert out["streams"] > 1 or (kernel, after) == ("muon_split", 0)
+
+
+def test_as_many_contexts_as_memory_holds(fake_cuda):
+    """The pinned pool bounds what copies hold, not how many contexts there are, and returns everything with the last of them."""
+    out = fake_cuda("""
+cfg = pkg.default_config(hidden_dim=128, n_layers=1, seq_len=16, population_size=2)
+all = [pkg.Context(cfg, 0, 2) for _ in range(600)]
+for c in all: c.upload_model(np.zeros(pkg.model_bytes(cfg), np.int8))
+out["pinned"] = fake.fake_pinned_bytes()
+for c in all[1:]: c.close()
+kept = fake.fake_pinned_bytes()
+again = [pkg.Context(cfg, 0, 2) for _ in range(599)]
+out["reused"] = fake.fake_pinned_bytes() == kept
+for c in again + all[:1]: c.close()
+out["left"] = [fake.fake_pinned_bytes(), fake.fake_device_bytes()]
+""")
+    assert out["pinned"] <= 600 * (128 << 10) and out["reused"] and out["left"] == [0, 0]
