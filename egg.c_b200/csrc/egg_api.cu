@@ -154,10 +154,11 @@ struct egg_ctx {
     int *d_err = nullptr;                          // = d_status->err
     PinnedBlock *pin = nullptr;                    // host side of the status and of short loss vectors
     HostStage stage;                    // pinned megabytes of the downloads
-    // grow-only scratch of the isolated entry points (projection, reconstruct, matrix update): allocated on first use,
-    // kept for the next call, freed with the context
-    void *scratch[18] = {};
-    size_t scratch_bytes[18] = {};
+    // scratch of one call of the isolated entry points and of sampling (they return when their work is done): the arena's share
+    // until a call needs more, then one buffer that only grows and goes with the context
+    uint8_t *scratch_start = nullptr;
+    void *scratch = nullptr, *scratch_own = nullptr;
+    int64_t scratch_bytes = 0;
     // row-owning projections with the adaptive normalisations fused (default wherever the shapes allow)
     int fused_level = 2;      // 0: two-kernel adaptive norms; 1: row-owning projections; 2: + the next mean-abs norm inside MLP-down;
                               // 3: + LN2 inside the output projection (selectable, slower: that epilogue is not hidden behind its MMAs)
@@ -185,6 +186,7 @@ struct egg_ctx {
 // 0.85 at 1024 rows, 0.93 at 16 384, 0.96 to 1.00 at 65 536, 0.99 to 1.03 at 131 072, 1.05 at 2 million; updates 0.80 at 0.4
 // million weights, 0.98 at 14.8, 1.02 at 36.
 constexpr int64_t CHAIN_MAX_ROWS = 65536, CHAIN_MAX_WEIGHTS = 16 << 20;
+constexpr int64_t SCRATCH_START = 8 << 20;
 
 // Brackets one launch (or launch group) with events when profiling is on.
 struct ProfScope {
@@ -388,7 +390,7 @@ extern "C" void egg_ctx_destroy(egg_ctx *c) {
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     if (c->comm && g_nccl.CommDestroy) g_nccl.CommDestroy(c->comm);
-    void *ptrs[] = {c->arena, c->upd.base, c->pre_base, c->d_data};
+    void *ptrs[] = {c->arena, c->upd.base, c->pre_base, c->scratch_own, c->d_data};
     host_stage_free(c->stage);
     pinned_give_status(reinterpret_cast<uint8_t *>(c->pin));
     pinned_release();
@@ -398,7 +400,6 @@ extern "C" void egg_ctx_destroy(egg_ctx *c) {
         if (c->ev_done[b]) cudaEventDestroy(c->ev_done[b]);
     }
     if (c->ev_m) cudaEventDestroy(c->ev_m);
-    for (void *p : c->scratch) if (p) cudaFree(p);
     for (cudaEvent_t e : c->prof_ev) cudaEventDestroy(e);
     if (c->t0) cudaEventDestroy(c->t0);
     if (c->t1) cudaEventDestroy(c->t1);
@@ -502,7 +503,7 @@ extern "C" int egg_ctx_create(const egg_config *cfg, int device, int wave_member
     ar.add(&c->d_exp_lut, 256); ar.add(&c->d_act_lut, 256); ar.add(&c->d_rope_lut, (int64_t)rope.size()); ar.add(&c->d_rope_t, (int64_t)rope_t.size());
     ar.add(&c->d_loss, POP); ar.add(&c->d_fit, POP / 2); ar.add(&c->d_status, 1);
     ar.add(&c->d_scales, c->SL.total); ar.add(&c->d_changed, c->SL.total); ar.add(&c->d_ov_active, c->SL.total);
-    ar.add(&c->d_segs, c->nsegs);
+    ar.add(&c->d_segs, c->nsegs); ar.add(&c->scratch_start, SCRATCH_START);
 
     // wave scratch: 23 H bytes + 40 bytes per row, noise table per pair
     // (+ a row of int32 logits per token when the head takes two passes over a vocabulary wider than one tile)
@@ -573,17 +574,23 @@ extern "C" int egg_ctx_create(const egg_config *cfg, int device, int wave_member
     return EGG_OK;
 }
 
-// Scratch slot `slot` with room for `count` elements of T: reuses the slot's buffer when it is large enough.
-template <typename T>
-static int ctx_scratch(egg_ctx *c, int slot, int64_t count, T **out) {
-    const size_t need = (size_t)(count > 0 ? count : 1) * sizeof(T);
-    if (c->scratch_bytes[slot] < need) {
-        if (c->scratch[slot]) { cudaStreamSynchronize(c->stream); cudaFree(c->scratch[slot]); c->scratch[slot] = nullptr; c->scratch_bytes[slot] = 0; }
-        cudaError_t e = cudaMalloc(&c->scratch[slot], need);
-        if (e != cudaSuccess) { set_error("cudaMalloc of %zu scratch bytes failed: %s", need, cudaGetErrorString(e)); c->scratch[slot] = nullptr; return EGG_E_NOMEM; }
-        c->scratch_bytes[slot] = need;
+// A call's scratch buffers, all of them from one piece of memory.  An allocation costs about 0.36 ms, several times a small call
+// (256 x 256 projection of 2048 rows: 60 us), so small calls find theirs in the context's arena and larger ones pay for one.
+static int ctx_scratch(egg_ctx *c, const DeviceArena &a) {
+    if (a.bytes() > c->scratch_bytes) {
+        if (c->scratch_own) { cudaStreamSynchronize(c->stream); cudaFree(c->scratch_own); c->scratch_own = nullptr; }
+        c->scratch = c->scratch_start; c->scratch_bytes = SCRATCH_START;
+        if (a.bytes() > SCRATCH_START) {
+            cudaError_t e = cudaMalloc(&c->scratch_own, (size_t)a.bytes());
+            if (e != cudaSuccess) {
+                c->scratch_own = nullptr;
+                set_error("cudaMalloc of %lld scratch bytes failed: %s", (long long)a.bytes(), cudaGetErrorString(e));
+                return EGG_E_NOMEM;
+            }
+            c->scratch = c->scratch_own; c->scratch_bytes = a.bytes();
+        }
     }
-    *out = static_cast<T *>(c->scratch[slot]);
+    a.place(c->scratch);
     return EGG_OK;
 }
 
@@ -1154,7 +1161,9 @@ extern "C" int egg_generate(egg_ctx *c, uint8_t *host_tokens, int seed_len, int 
     EGG_CUDA(cudaSetDevice(c->device));
     int8_t *kv = nullptr; uint8_t *tok = nullptr;
     int rc;
-    if ((rc = ctx_scratch(c, 16, (int64_t)cf.n_layers * 2 * 256 * cf.hidden_dim, &kv)) || (rc = ctx_scratch(c, 17, cf.seq_len + 258, &tok))) return rc;
+    DeviceArena a;
+    a.add(&kv, (int64_t)cf.n_layers * 2 * 256 * cf.hidden_dim); a.add(&tok, cf.seq_len + 258);
+    if ((rc = ctx_scratch(c, a))) return rc;
     EGG_CUDA(cudaMemsetAsync(tok, 0, (size_t)cf.seq_len + 258, c->stream));
     EGG_CUDA(cudaMemcpyAsync(tok, host_tokens, (size_t)seed_len, cudaMemcpyHostToDevice, c->stream));
     // every given token but the last only leaves its keys and values: from 12 on, one pass of the evaluation kernels over all of
@@ -1302,11 +1311,13 @@ extern "C" int egg_allgather_fitness(egg_ctx *c) {
 
 // One matrix: operands -> vote GEMM (pair index split over the GPU) -> optimiser step from the votes.
 // The isolated entry point's form; all pointers are device pointers.
+struct MuonDesc { UpdMat m; double norm2; int list; };
 struct MatrixUpdate {
     int8_t *w_packed; float *opt;
     int rows_k, cols_n, off_a, off_b, seed_base;
     const int32_t *fit; int pairs, kp, operand_split;
     int8_t *na, *nb; int32_t *votes;
+    uint8_t *desc, *ns_ws;       // Muon: descriptor and workspace
     float lr; int muon;
 };
 
@@ -1330,11 +1341,10 @@ static int run_matrix_update(egg_ctx *c, const MatrixUpdate &u, uint32_t step_se
     a.total_updates = c->d_updates;
     if (!u.muon) return PROF(EGG_PROF_UPD_APPLY, launch_adam_from_votes(c->stream, a));
     // the model update's Muon kernels on a group of one; the descriptor describes the caller's buffers from their start
-    struct { UpdMat m; double norm2; int list; } desc;
+    MuonDesc desc;
     memset(&desc, 0, sizeof(desc));
     desc.m.rows_k = u.rows_k; desc.m.cols_n = u.cols_n; desc.m.muon = 1; desc.m.lr_scale = 1.0f;
-    uint8_t *d_desc = nullptr, *wsb = nullptr;
-    if ((rc = ctx_scratch(c, 12, (int64_t)sizeof(desc), &d_desc)) || (rc = ctx_scratch(c, 13, ns_ws_bytes(u.rows_k, u.cols_n, 1), &wsb))) return rc;
+    uint8_t *d_desc = u.desc, *wsb = u.ns_ws;
     EGG_CUDA(cudaMemcpyAsync(d_desc, &desc, sizeof(desc), cudaMemcpyHostToDevice, c->stream));
     const UpdMat *dm = reinterpret_cast<const UpdMat *>(d_desc);
     double *norm2 = reinterpret_cast<double *>(d_desc + ((uint8_t *)&desc.norm2 - (uint8_t *)&desc));
@@ -1527,17 +1537,18 @@ extern "C" int egg_perturbed_projection(egg_ctx *c, const int8_t *x, const int8_
     int32_t *d_xb = nullptr;
     NoiseSeg *d_segs = nullptr;
     int rc = EGG_OK;
-    auto cleanup = [&]() { cudaStreamSynchronize(st); };      // buffers live in the context's scratch slots
+    auto cleanup = [&]() { cudaStreamSynchronize(st); };      // buffers live in the context's scratch
 #define PTRY(e) do { rc = (e); if (rc) { cleanup(); return rc; } } while (0)
 #define PTRYC(e) do { cudaError_t e_ = (e); if (e_ != cudaSuccess) { set_error("%s: %s", #e, cudaGetErrorString(e_)); cleanup(); return EGG_E_CUDA; } } while (0)
+    DeviceArena a;
+    a.add(&d_wt, (int64_t)K * N); a.add(&d_nt, pairs * stride); a.add(&d_xb, rows); a.add(&d_segs, 2);
+    if (!on_device) { a.add(&d_x, rows * K); a.add(&d_w, (int64_t)K * N); a.add(&d_y, rows * N); }
+    PTRY(ctx_scratch(c, a));
     if (on_device) { d_x = const_cast<int8_t *>(x); d_w = const_cast<int8_t *>(w_packed); d_y = y; }
     else {
-        PTRY(ctx_scratch(c, 4, rows * K, &d_x)); PTRY(ctx_scratch(c, 5, (int64_t)K * N, &d_w)); PTRY(ctx_scratch(c, 6, rows * N, &d_y));
         PTRYC(cudaMemcpyAsync(d_x, x, (size_t)(rows * K), cudaMemcpyHostToDevice, st));
         PTRYC(cudaMemcpyAsync(d_w, w_packed, (size_t)K * N, cudaMemcpyHostToDevice, st));
     }
-    PTRY(ctx_scratch(c, 0, (int64_t)K * N, &d_wt)); PTRY(ctx_scratch(c, 1, pairs * stride, &d_nt)); PTRY(ctx_scratch(c, 2, rows, &d_xb));
-    PTRY(ctx_scratch(c, 3, 2, &d_segs));
     NoiseSeg segs[2] = {{0, N, 0, off_a, 0, 0, -1, -1, 0}, {N, K, 0, off_b, 0, 0, -1, -1, 0}};
     noise_index_slices(segs, 2);
     PTRYC(cudaMemcpyAsync(d_segs, segs, sizeof(segs), cudaMemcpyHostToDevice, st));
@@ -1570,7 +1581,7 @@ extern "C" int egg_update_reconstruct(egg_ctx *c, const int32_t *fitness, int pa
     int32_t *d_fit = nullptr, *d_vote = nullptr;
     int8_t *d_na = nullptr, *d_nb = nullptr;
     int rc = EGG_OK;
-    auto cleanup = [&]() { cudaStreamSynchronize(st); };      // buffers live in the context's scratch slots
+    auto cleanup = [&]() { cudaStreamSynchronize(st); };      // buffers live in the context's scratch
 #define PTRY(e) do { rc = (e); if (rc) { cleanup(); return rc; } } while (0)
 #define PTRYC(e) do { cudaError_t e_ = (e); if (e_ != cudaSuccess) { set_error("%s: %s", #e, cudaGetErrorString(e_)); cleanup(); return EGG_E_CUDA; } } while (0)
     // fitness range decides whether f*a fits int8 directly or needs the base-16 split
@@ -1583,8 +1594,6 @@ extern "C" int egg_update_reconstruct(egg_ctx *c, const int32_t *fitness, int pa
         for (int i = 0; i < pairs; i++) { int a = hf[i] < 0 ? -hf[i] : hf[i]; if (a > fmax) fmax = a; }
     } else {
         for (int i = 0; i < pairs; i++) { int a = fitness[i] < 0 ? -fitness[i] : fitness[i]; if (a > fmax) fmax = a; }
-        PTRY(ctx_scratch(c, 10, pairs, &d_fit)); PTRY(ctx_scratch(c, 11, (int64_t)rows_k * cols_n, &d_vote));
-        PTRYC(cudaMemcpyAsync(d_fit, fitness, (size_t)pairs * 4, cudaMemcpyHostToDevice, st));
     }
     const int amax = c->cfg.device_gaussian ? 3 * c->cfg.device_mask : c->cfg.device_mask;
     if (fmax > 127) { set_error("fitness magnitude %d exceeds 127", fmax); cleanup(); return EGG_E_INVALID; }
@@ -1593,7 +1602,11 @@ extern "C" int egg_update_reconstruct(egg_ctx *c, const int32_t *fitness, int pa
         set_error("int8 fitness with noise magnitude %d does not fit the two-digit operand split", amax); cleanup(); return EGG_E_INVALID;
     }
     const int ktot = split ? 2 * kp : kp;
-    PTRY(ctx_scratch(c, 7, (int64_t)cols_n * ktot, &d_na)); PTRY(ctx_scratch(c, 8, (int64_t)rows_k * ktot, &d_nb));
+    DeviceArena a;
+    a.add(&d_na, (int64_t)cols_n * ktot); a.add(&d_nb, (int64_t)rows_k * ktot);
+    if (!on_device) { a.add(&d_fit, pairs); a.add(&d_vote, (int64_t)rows_k * cols_n); }
+    PTRY(ctx_scratch(c, a));
+    if (!on_device) PTRYC(cudaMemcpyAsync(d_fit, fitness, (size_t)pairs * 4, cudaMemcpyHostToDevice, st));
     PTRY(launch_update_operands(st, d_na, d_nb, d_fit, pairs, kp, rows_k, cols_n, off_a, off_b, seed_base, step_seed,
                                 c->cfg.device_mask, c->cfg.device_gaussian, split));
     GemmParams g;
@@ -1631,18 +1644,19 @@ extern "C" int egg_update_matrix(egg_ctx *c, int8_t *d_w_packed, void *d_opt_sta
     MatrixUpdate u;
     memset(&u, 0, sizeof(u));
     int rc = EGG_OK;
-    auto cleanup = [&]() { cudaStreamSynchronize(st); };      // buffers live in the context's scratch slots
+    auto cleanup = [&]() { cudaStreamSynchronize(st); };      // buffers live in the context's scratch
 #define UTRY(e) do { rc = (e); if (rc) { cleanup(); return rc; } } while (0)
-    UTRY(ctx_scratch(c, 7, (int64_t)cols_n * ktot, &u.na)); UTRY(ctx_scratch(c, 8, (int64_t)rows_k * ktot, &u.nb));
-    UTRY(ctx_scratch(c, 9, (int64_t)rows_k * cols_n * splits, &u.votes));
-    u.w_packed = d_w_packed; u.opt = static_cast<float *>(d_opt_state);
-    // the optimiser passes read and write words of four weights: weights anywhere else are stepped in an aligned copy
     const bool copied = reinterpret_cast<uintptr_t>(d_w_packed) & 3;
     const size_t wbytes = (size_t)rows_k * cols_n;
-    if (copied) {
-        UTRY(ctx_scratch(c, 10, (int64_t)wbytes, &u.w_packed));
-        EGG_CUDA(cudaMemcpyAsync(u.w_packed, d_w_packed, wbytes, cudaMemcpyDeviceToDevice, st));
-    }
+    DeviceArena a;
+    a.add(&u.na, (int64_t)cols_n * ktot); a.add(&u.nb, (int64_t)rows_k * ktot); a.add(&u.votes, (int64_t)rows_k * cols_n * splits);
+    if (optimizer) { a.add(&u.desc, (int64_t)sizeof(MuonDesc)); a.add(&u.ns_ws, ns_ws_bytes(rows_k, cols_n, 1)); }
+    if (copied) a.add(&u.w_packed, (int64_t)wbytes);
+    UTRY(ctx_scratch(c, a));
+    if (!copied) u.w_packed = d_w_packed;
+    u.opt = static_cast<float *>(d_opt_state);
+    // the optimiser passes read and write words of four weights: weights anywhere else are stepped in an aligned copy
+    if (copied) EGG_CUDA(cudaMemcpyAsync(u.w_packed, d_w_packed, wbytes, cudaMemcpyDeviceToDevice, st));
     u.rows_k = rows_k; u.cols_n = cols_n; u.off_a = off_a; u.off_b = off_b; u.seed_base = seed_base;
     u.fit = d_fitness; u.pairs = pairs; u.kp = kp; u.operand_split = split ? 1 : 0;
     u.lr = lr; u.muon = optimizer;

@@ -17,8 +17,7 @@ int DeviceArena::commit(void **base) {
         set_error("cudaMalloc of %lld bytes failed: %s", (long long)total, cudaGetErrorString(e));
         return EGG_E_NOMEM;
     }
-    uint8_t *at = static_cast<uint8_t *>(*base);
-    for (const Want &w : wants) { *w.p = at; at += w.bytes; }
+    place(*base);
     return EGG_OK;
 }
 

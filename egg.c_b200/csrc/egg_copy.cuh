@@ -23,6 +23,10 @@ public:
     }
     int64_t bytes() const { return total; }
     int commit(void **base);                       // EGG_OK or EGG_E_NOMEM; the caller frees *base
+    void place(void *base) const {                 // in memory that is there, bytes() long
+        uint8_t *at = static_cast<uint8_t *>(base);
+        for (const Want &w : wants) { *w.p = at; at += w.bytes; }
+    }
 };
 
 // Pinned host memory in blocks of PIN_BLOCK bytes.  Pinning costs milliseconds, so the blocks belong to the process: every context

@@ -280,8 +280,8 @@ int egg_update_reconstruct(egg_ctx *ctx, const int32_t *fitness, int pairs,
  * d_opt_state is 16-byte aligned, d_w_packed may lie anywhere.
  * Hyper-parameters (betas, eps, weight decay, Muon momentum and lr scale, noise mask) come from the
  * context's configuration.  *total_updates = number of weights that changed.  Its scratch (operands,
- * partial votes, Newton-Schulz workspace) is allocated on first use, kept in the context for later calls
- * of the same or a smaller size, and freed with the context.  Blocks until done.
+ * partial votes, Newton-Schulz workspace) is part of the context up to 8 MB; more is one allocation, kept for later
+ * calls of the same or a smaller size and freed with the context.  Blocks until done.
  */
 int egg_update_matrix(egg_ctx *ctx, int8_t *d_w_packed, void *d_opt_state, int rows_k, int cols_n,
                       int off_a, int off_b, int seed_base, const int32_t *d_fitness, int pairs,

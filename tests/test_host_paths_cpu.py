@@ -238,3 +238,30 @@ for c in again + all[:1]: c.close()
 out["left"] = [fake.fake_pinned_bytes(), fake.fake_device_bytes()]
 """)
     assert out["pinned"] <= 600 * (128 << 10) and out["reused"] and out["left"] == [0, 0]
+
+
+@pytest.mark.parametrize("call,most", [
+    ("ctx.perturbed_projection(p, p, p, 2048, 256, 256, 32, 1, 200, 201, 7, 8, on_device=True)", 0),
+    ("ctx.perturbed_projection(p, p, p, 32768, 4096, 4096, 32, 1, 200, 201, 7, 8, on_device=True)", 1),
+    ("ctx.perturbed_projection(h(65536), h(65536), h(65536), 256, 256, 256, 32, 1, 200, 201, 7, 8)", 0),
+    ("ctx.update_matrix(p, p, 256, 256, 402, 403, 0, p, 1000, 1, 0.1, 0, False)", 0),
+    ("ctx.update_matrix(p, p, 256, 256, 402, 403, 0, p, 1000, 1, 0.1, 1, True)", 0),
+    ("ctx.update_matrix(p + 1, p, 1024, 1024, 402, 403, 0, p, 1000, 1, 0.1, 1, True)", 1),
+    ("ctx.update_reconstruct(h(4000).view(np.int32), 1000, 256, 256, 402, 403, 0, 1, h(1 << 18))", 0),
+    ("ctx.generate(np.zeros(40, np.uint8), 20, 1)", 0),
+])
+def test_first_calls_allocate_once_at_most(fake_cuda, call, most):
+    """Scratch comes from the context's own memory where the work is small, in one allocation where it is not, and then stays."""
+    out = fake_cuda("""
+ctx = context(hidden_dim=512, n_layers=4, seq_len=256, population_size=8, device_mask=3)
+p = C.c_void_p()
+fake.cudaMalloc(C.byref(p), C.c_size_t(1 << 30))
+p, h = p.value, lambda n: np.zeros(n, np.int8)
+n = [fake.fake_mallocs()]
+for _ in range(3):
+    %s
+    n.append(fake.fake_mallocs())
+ctx.close()
+out["n"] = [b - a for a, b in zip(n, n[1:])]
+""" % call)
+    assert out["n"] == [most, 0, 0]
