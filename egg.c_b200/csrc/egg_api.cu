@@ -131,7 +131,7 @@ struct egg_ctx {
     int table_pairs = 0;                // pairs from which filling a wave's noise from the table is less work
     // update scratch
     void *arena = nullptr;              // the buffers of fixed size
-    void *pre_base = nullptr;           // d_pre and d_rowmax3, allocated when the two-kernel form first runs
+    void *pre_base = nullptr;           // d_pre and d_rowmax3 where the two-kernel form was chosen later (else they are in the arena, or not needed)
     UpdPlan plan;                       // of the parameters this context steps (all, or its own ones when the update is sharded)
     struct UpdBuffers {
         void *base = nullptr;           // one allocation of the plan's descriptors and all of these
@@ -448,6 +448,8 @@ static int prepare_update(egg_ctx *c) {
 
 static int noalloc_scratch_address(int device, int8_t **out);
 static bool fused_shifts(const egg_config &c);
+static bool use_fused(const egg_ctx *c);
+static void want_pre(egg_ctx *c, DeviceArena &a);
 
 extern "C" int egg_ctx_create(const egg_config *cfg, int device, int wave_members, egg_ctx **out) {
     if (!cfg || !out) { set_error("null argument"); return EGG_E_INVALID; }
@@ -532,6 +534,7 @@ extern "C" int egg_ctx_create(const egg_config *cfg, int device, int wave_member
     ar.add(&c->d_xb, R * 3); ar.add(&c->d_xb2, R); ar.add(&c->d_rowmax, R);
     ar.add(&c->d_xbo, R); ar.add(&c->d_xbn, R * 3);
     if (logit_bytes) { ar.add(&c->d_logits, R * cfg->vocab_size); ar.add(&c->d_max64, R * (cfg->vocab_size / 64)); }
+    if (!use_fused(c)) want_pre(c, ar);
     if (cfg->ntt_mode) ar.add(&c->d_coef, (int64_t)(wave_members / 2) * S);
     ar.add(&c->d_nt, (int64_t)(wave_members / 2 + 3) * c->nmap.stride);    // (a last tile's spare rows look up to 3 pairs further)
     // noise table of a wave: less work once the pairs' vectors together hold twice as many values as the table; never larger than them
@@ -823,13 +826,9 @@ extern "C" int egg_set_dataset_tokens(egg_ctx *c, const uint32_t *host_tokens, i
 
 // ---------------------------------------------------------------- evaluation
 
-// The two-kernel form's int32 rows, 12 H bytes each: only contexts that run it hold them.
-static int ensure_pre(egg_ctx *c) {
-    if (c->pre_base) return EGG_OK;
-    DeviceArena a;
-    a.add(&c->d_pre, c->R * 3 * c->cfg.hidden_dim); a.add(&c->d_rowmax3, c->R * 3);
-    return a.commit(&c->pre_base);
-}
+// The two-kernel form's int32 rows, 12 H bytes each: contexts whose shape takes that form are created with them, others get
+// them when it is chosen.
+static void want_pre(egg_ctx *c, DeviceArena &a) { a.add(&c->d_pre, c->R * 3 * c->cfg.hidden_dim); a.add(&c->d_rowmax3, c->R * 3); }
 
 // Whether the residual projections' shifts allow the row-owning form; larger ones take the two-kernel form at every shape.
 static bool fused_shifts(const egg_config &c) { return std::max(c.shift_out, c.shift_mlp_down) + c.fixed_point + c.sigma_shift <= PRESHIFT_MAX; }
@@ -946,10 +945,7 @@ static int eval_wave(egg_ctx *c, uint32_t step_seed, int64_t start_idx, int pop_
     const uint8_t *data = pf ? pf->tokens : c->d_data;
     const int64_t data_len = pf ? S + 1 : c->data_len;          // the window position is taken modulo data_len - seq_len
     int rc;
-    if (!use_fused(c)) {
-        if ((rc = ensure_pre(c))) return rc;
-        EGG_CUDA(cudaMemsetAsync(c->d_rowmax, 0, (size_t)M * 4, st));
-    }
+    if (!use_fused(c)) EGG_CUDA(cudaMemsetAsync(c->d_rowmax, 0, (size_t)M * 4, st));
     if ((rc = PROF(EGG_PROF_NOISE, launch_noise_fill(st, c->d_nt, nm.stride, c->d_segs, c->nsegs, members / 2, step_seed, pop_base / 2, mask, pf ? 0 : cf.device_gaussian, mdl, sc ? c->d_scales : nullptr, loss_dst,
                                                      members / 2 >= c->table_pairs ? c->noise_tab : NoiseTable())))) return rc;
     const int64_t data_stride = data_len / (cf.population_size / 2);
@@ -1820,6 +1816,13 @@ extern "C" int egg_measure_int8_peak(egg_ctx *c, int m, int n, int k, int iters,
 
 extern "C" int egg_set_fused_epilogues(egg_ctx *c, int enable) {
     if (!c) { set_error("null context"); return EGG_E_INVALID; }
+    if (enable <= 0 && !c->d_pre) {
+        EGG_CUDA(cudaSetDevice(c->device));
+        DeviceArena a;
+        want_pre(c, a);
+        int rc = a.commit(&c->pre_base);
+        if (rc) return rc;
+    }
     c->fused_level = enable <= 0 ? 0 : (enable >= 3 ? 3 : enable);
     return EGG_OK;
 }

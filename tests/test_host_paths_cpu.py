@@ -265,3 +265,24 @@ ctx.close()
 out["n"] = [b - a for a, b in zip(n, n[1:])]
 """ % call)
     assert out["n"] == [most, 0, 0]
+
+
+@pytest.mark.parametrize("kw,two_kernel", [(dict(seq_len=16), True), (dict(seq_len=32), False), (dict(seq_len=48, shift_out=14), True)])
+def test_memory_of_the_two_kernel_form_is_asked_for_where_it_is_chosen(fake_cuda, kw, two_kernel):
+    """At creation for shapes that take it, else by the call that switches to it; an evaluation allocates nothing and runs out of nothing."""
+    out = fake_cuda("""
+ctx = context(hidden_dim=256, n_layers=1, population_size=64, **%r)
+def evaluate():
+    fake.fake_fail_malloc(0)
+    rc = error(lambda: (ctx.eval_chunk(1, 0, 0, 64), ctx.read_losses(0, 64)))
+    fake.fake_fail_malloc(-1)
+    return rc
+out["first"] = evaluate()
+fake.fake_fail_malloc(0)
+out["refused"] = error(lambda: ctx.set_fused_epilogues(0))
+fake.fake_fail_malloc(-1)
+out["again"] = [evaluate(), ctx.fused_epilogues_active()]
+out["switched"] = [error(lambda: ctx.set_fused_epilogues(0)), evaluate(), launches("aqn_kernel")]
+""" % kw)
+    assert out["first"] == 0 and out["again"][0] == 0 and out["switched"][:2] == [0, 0] and out["switched"][2] > 0, out
+    assert (out["refused"] < 0) == (not two_kernel) and (out["again"][1] > 0) == (not two_kernel), out
