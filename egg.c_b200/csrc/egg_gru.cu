@@ -654,7 +654,12 @@ static int gru_window_buffers(egg_gru_ctx *c, int tokens) {
     c->win = 0;
     if (need > c->w_bytes) {
         if (c->w_base) { cudaFree(c->w_base); c->w_base = nullptr; c->w_bytes = 0; }
-        EGG_CUDA(cudaMalloc(&c->w_base, (size_t)need));
+        if (cudaMalloc(&c->w_base, (size_t)need) != cudaSuccess) {
+            cudaGetLastError();
+            c->w_base = nullptr;
+            set_error("cudaMalloc of %lld bytes for windows of tokens failed", (long long)need);
+            return EGG_E_NOMEM;
+        }
         c->w_bytes = need;
     }
     uint8_t *b = static_cast<uint8_t *>(c->w_base);
@@ -755,9 +760,7 @@ static int gru_wavefront(egg_gru_ctx *c, int64_t start_idx, int tokens) {
 }
 
 static int gru_windows(egg_gru_ctx *c, int64_t start_idx, int tokens) {
-    int rc = gru_window_buffers(c, tokens);
-    if (rc) return rc;
-    rc = gru_wavefront(c, start_idx, tokens);
+    int rc = gru_wavefront(c, start_idx, tokens);
     // a call that failed half-way leaves kernels on the lanes: what follows on the context's stream waits for them all the same
     cudaError_t e = cudaSuccess;
     for (int i = 0; i < c->ns; i++) {
@@ -783,10 +786,10 @@ extern "C" int egg_gru_generation(egg_gru_ctx *c, uint32_t step_seed, int64_t st
     EGG_CUDA(cudaGetLastError());
     c->launches++;
     EGG_CUDA(cudaMemsetAsync(c->d_loss, 0, (size_t)POP * 4, st));
-    int rc;
-    if (tokens >= GRU_SCAN_MIN_TOKENS) {
-        if ((rc = gru_windows(c, start_idx, tokens))) return rc;
-    } else if ((rc = gru_token_steps(c, start_idx, tokens))) return rc;
+    // token by token needs no memory beyond the context's: also where that of the windows is not to be had
+    int rc = tokens >= GRU_SCAN_MIN_TOKENS ? gru_window_buffers(c, tokens) : EGG_E_NOMEM;
+    if (rc && rc != EGG_E_NOMEM) return rc;
+    if ((rc = rc ? gru_token_steps(c, start_idx, tokens) : gru_windows(c, start_idx, tokens))) return rc;
     gru_fitness_kernel<<<(pairs + 127) / 128, 128, 0, st>>>(c->d_loss, c->d_fit, pairs);
     c->launches++;
     if (do_update) {

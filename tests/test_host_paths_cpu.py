@@ -286,3 +286,21 @@ out["switched"] = [error(lambda: ctx.set_fused_epilogues(0)), evaluate(), launch
 """ % kw)
     assert out["first"] == 0 and out["again"][0] == 0 and out["switched"][:2] == [0, 0] and out["switched"][2] > 0, out
     assert (out["refused"] < 0) == (not two_kernel) and (out["again"][1] > 0) == (not two_kernel), out
+
+
+def test_recurrent_generation_without_memory_for_windows(fake_cuda):
+    """Token by token where the windows' buffers cannot be had, in windows again when they can."""
+    out = fake_cuda("""
+cfg = pkg.default_gru_config(hidden_dim=128, n_layers=2, population_size=32, seq_len=4096)
+ctx = pkg.GruContext(cfg, 0)
+ctx.upload_model(np.zeros(pkg.gru_model_bytes(cfg), np.int8))
+ctx.set_dataset(np.zeros(9000, np.uint8))
+def generation(tokens, fails):
+    fake.fake_fail_malloc(0 if fails else -1)
+    fake.fake_clear()
+    rc = error(lambda: ctx.generation(1, 0, tokens, True))
+    fake.fake_fail_malloc(-1)
+    return [rc, launches("gru_scan_kernel") > 0, any(l.startswith("graph") for l in log())]
+out["g"] = [generation(100, True), generation(100, False), generation(4096, True), generation(100, False)]
+""")
+    assert out["g"] == [[0, False, True], [0, True, False], [0, False, True], [0, True, False]]
