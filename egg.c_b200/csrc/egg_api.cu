@@ -1224,9 +1224,11 @@ extern "C" int egg_comm_init(egg_ctx *c, const void *id128, int rank, int world)
 }
 
 // owners: parameters in order of decreasing cost, each to the rank with the least work so far; the same
-// deterministic walk on every rank.  Cost ~ weights for a matrix (tensor-core vote GEMM); a vector element costs
-// about 300 matrix elements (its votes are hashed and summed pair by pair on the ordinary cores).
-static int64_t update_cost(const ParamDesc &d) { return d.rows_k ? (int64_t)d.rows_k * d.cols_n : (int64_t)d.cols_n * 300; }
+// deterministic walk on every rank.  Cost ~ weights for a matrix (operand, vote GEMM, optimiser step).  A vector element, whose vote
+// is one row of a product that all vectors share, costs as much as about 40: measured 37 and 39 at H 256 with 163 840 and 16 384
+// pairs, 44 at H 512, 43 to 56 at H 1024.
+constexpr int VECTOR_ELEMENT_COST = 40;
+static int64_t update_cost(const ParamDesc &d) { return d.rows_k ? (int64_t)d.rows_k * d.cols_n : (int64_t)d.cols_n * VECTOR_ELEMENT_COST; }
 static void plan_owners(const std::vector<ParamDesc> &params, int world, std::vector<int> &owner) {
     std::vector<size_t> order(params.size());
     for (size_t i = 0; i < order.size(); i++) order[i] = i;

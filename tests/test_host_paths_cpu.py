@@ -304,3 +304,13 @@ def generation(tokens, fails):
 out["g"] = [generation(100, True), generation(100, False), generation(4096, True), generation(100, False)]
 """)
     assert out["g"] == [[0, False, True], [0, True, False], [0, False, True], [0, True, False]]
+
+
+def test_owner_costs_are_those_of_the_update():
+    """The sharded update deals parameters by cost: a vector element takes the time of 37 to 56 matrix weights."""
+    from common import load_pkg
+    pkg = load_pkg()
+    cfg = pkg.default_config(hidden_dim=256, n_layers=4)
+    _, costs, _, weights = pkg.update_owner_plan(cfg, 8, spans=True)
+    vector = weights <= 4 * 256
+    assert (costs[~vector] == weights[~vector]).all() and set(costs[vector] // weights[vector]) <= set(range(37, 57))
