@@ -205,18 +205,6 @@ constexpr float kMagic = 12582912.0f;          // 1.5 * 2^23
 constexpr int kMagicBits = 0x4B400000;
 // (float)v for |v| < 2^22, exact
 __device__ __forceinline__ float i2f_small(int v) { return __int_as_float(kMagicBits + v) - kMagic; }
-// the same value through the conversion unit: used for a share of the conversions so that the otherwise idle unit
-// takes load off the integer/float pipes
-__device__ __forceinline__ float i2f_cvt(int v) { return __int2float_rn(v); }
-// roundf(x) (half away from zero) as a float, for |x| < 2^22: round-to-nearest-even by the
-// magic add, then the two tie cases that differ are corrected (x - rint(x) is exact).
-__device__ __forceinline__ float roundf_small(float x) {
-    float rf = (x + kMagic) - kMagic;
-    float d = x - rf;
-    if (d == 0.5f && x > 0.0f) rf += 1.0f;
-    if (d == -0.5f && x < 0.0f) rf -= 1.0f;
-    return rf;
-}
 // integer value of a float that holds an integer, |f| < 2^22
 __device__ __forceinline__ int f2i_exact(float f) { return __float_as_int(f + kMagic) - kMagicBits; }
 

@@ -683,18 +683,11 @@ __device__ __forceinline__ void att_scores(int (&c)[4][4], const int4 (&qa)[2], 
     }
 }
 
-// exact float of an int with |v| < 2^23 (no conversion instruction)
-__device__ __forceinline__ float i2f_23(int v) {
-    float f = __int_as_float(0x4B000000 | abs(v)) - 8388608.0f;
-    return v < 0 ? -f : f;
-}
-
 // trunc(num / den) as C does, for |num/den| <= 127: the quotient is estimated in float from the three
 // limb sums and fixed up with one exact int64 remainder test.
-__device__ __forceinline__ int att_div(int p0, int p1, int p2, long long den, float rden, bool small) {
+__device__ __forceinline__ int att_div(int p0, int p1, int p2, long long den, float rden) {
     const long long num = (long long)p0 + ((long long)p1 << 7) + ((long long)p2 << 14);
-    float fn = small ? fmaf(i2f_23(p2), 16384.0f, fmaf(i2f_23(p1), 128.0f, i2f_23(p0))) : (float)num;
-    int k = f2i_exact(fn * rden);                     // nearest integer to the real quotient (|error| < 1e-3)
+    int k = f2i_exact((float)num * rden);             // nearest integer to the real quotient (|error| < 1e-3)
     long long r = num - (long long)k * den;
     if (num >= 0) { if (r < 0) k--; } else { if (r > 0) k++; }
     return k;
@@ -787,7 +780,7 @@ __device__ __forceinline__ void att_quotients(AttOut &o, int dn, const int (&acc
         }
     } else {
 #pragma unroll
-        for (int i = 0; i < 4; i++) v[i] = clip8(att_div(acc[0][i], acc[1][i], acc[2][i], i < 2 ? den0 : den1, i < 2 ? rden0 : rden1, false));
+        for (int i = 0; i < 4; i++) v[i] = clip8(att_div(acc[0][i], acc[1][i], acc[2][i], i < 2 ? den0 : den1, i < 2 ? rden0 : rden1));
     }
     if (dn & 1) {
         o.w0[dn >> 1] = __byte_perm(o.w0[dn >> 1], __byte_perm((uint32_t)v[0], (uint32_t)v[1], 0x0040), 0x5410);

@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(256) upd_vec_votes_kernel(const int8_t *tab, i
 }
 
 // The optimiser step: four consecutive elements of one vector per warp, votes as summed above.  Where they were not (Gaussian noise,
-// fitness beyond int8, more vectors than the tensor-core form takes) the warp sums them over the pairs itself; groups are
+// fitness beyond int8) the warp sums them over the pairs itself; groups are
 // ordered by index first, because all vectors share row i of the table.
 constexpr int VEC_GROUP = 4;
 
@@ -297,7 +297,7 @@ int launch_upd_vectors(cudaStream_t st, const UpdPlan &pl, const int8_t *tab, co
                        const int32_t *fit, int gaussian, int8_t *model, uint8_t *opt, const UpdHyper &h, unsigned long long *total, uint8_t *changed, int num_sms) {
     const int nvec = (int)pl.vecs.size();
     if (!nvec) return EGG_OK;
-    const bool product = pl.vec_pad > 0 && !gaussian;
+    const bool product = !gaussian;
     if (product) {
         const int rows = pl.len_long / 16, z = (pl.vec_pad / 8 + VC_TILES - 1) / VC_TILES, ncols = (int)pl.vcols.size();
         int gx = (num_sms * 6 + rows * z - 1) / (rows * z);
@@ -685,7 +685,8 @@ int upd_plan_build(UpdPlan &pl, const std::vector<ParamDesc> &params, const std:
         }
     }
     // the vectors' windows in blocks of 64 columns; tiles of eight vectors, up to 64 tiles
-    if (!pl.vecs.empty() && pl.vecs.size() <= 512) {
+    if (pl.vecs.size() > 512) { set_error("%zu vector parameters: the vote product takes 512", pl.vecs.size()); return EGG_E_INVALID; }
+    if (!pl.vecs.empty()) {
         std::stable_sort(pl.vecs.begin(), pl.vecs.end(), [](const UpdVec &a, const UpdVec &b) { return a.len != b.len ? a.len > b.len : a.x_a + a.r < b.x_a + b.r; });
         pl.vec_pad = ((int)pl.vecs.size() + 7) / 8 * 8;
         std::map<int, UpdVecCols> cover;

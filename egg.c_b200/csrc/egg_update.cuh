@@ -65,7 +65,7 @@ struct UpdPlan {
     std::vector<int2> chunks;         // table columns to fill: {first, count}, count <= UPD_CHUNK
     int W = 0, pitch = 0, kp = 0, pairs = 0;
     int vec_long = 0, len_long = 0, len_short = 0;
-    int vec_pad = 0;                  // vectors rounded up to tiles of eight (0: too many for the tensor-core form)
+    int vec_pad = 0;                  // vectors rounded up to tiles of eight
     std::vector<UpdVecCols> vcols;
     int64_t fn_bytes = 0, votes_elems = 0;
     std::vector<uint8_t> descriptors; // device image of mats | vecs | chunks | list
