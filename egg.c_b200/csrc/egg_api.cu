@@ -153,7 +153,7 @@ struct egg_ctx {
     unsigned long long *d_updates = nullptr;       // = &d_status->updates
     int *d_err = nullptr;                          // = d_status->err
     PinnedBlock *pin = nullptr;                    // host side of the status and of short loss vectors
-    HostStage stage;                    // pinned megabytes of the downloads
+    HostStage stage;                    // events of the downloads' blocks
     // scratch of one call of the isolated entry points and of sampling (they return when their work is done): the arena's share
     // until a call needs more, then one buffer that only grows and goes with the context
     uint8_t *scratch_start = nullptr;
@@ -508,7 +508,7 @@ extern "C" int egg_ctx_create(const egg_config *cfg, int device, int wave_member
     ar.add(&c->d_segs, c->nsegs); ar.add(&c->scratch_start, SCRATCH_START);
 
     // wave scratch: 23 H bytes + 40 bytes per row, noise table per pair
-    // (+ a row of int32 logits per token when the head takes two passes over a vocabulary wider than one tile)
+    // (+ a byte per logit and an int32 maximum per 64 when the head takes two passes over a vocabulary wider than one tile)
     c->tok_bytes = cfg->vocab_size == 256 ? 1 : 4;
     const int64_t logit_bytes = cfg->vocab_size == 256 ? 0 : (int64_t)cfg->vocab_size / 16 * 17;
     const int64_t per_member = SP * (23 * H + 40 + logit_bytes) + c->nmap.stride / 2 + 8;

@@ -386,12 +386,15 @@ struct egg_gru_ctx {
     cudaEvent_t fork = nullptr;
     int *d_err = nullptr;
     void *arena = nullptr;              // the buffers of fixed size
-    HostStage stage;                    // pinned megabytes of the downloads
+    HostStage stage;                    // events of the downloads' blocks
     int64_t launches = 0;
     bool have_model = false;
 };
 
-// Shorter generations replay the token-step graphs; their launch count per token is part of what callers observe.
+// Shorter generations replay the token-step graphs: their launch count per token is part of what callers observe
+// (egg_gru_launch_count), and is tested.  By time the line would lie at two tokens.  Graphs / windows in us, update included:
+//   H 512, 4 layers, 128 members: 1 token 628 / 757, 2 tokens 783 / 759, 16 tokens 2947 / 855, 63 tokens 10 239 / 1181
+//   H 128, 1 layer, 32 members: 158 / 184, 189 / 183, 604 / 200, 2043 / 258;  H 1024, 2 layers, 1024 members: 4027 / 4378, 4655 / 4441
 constexpr int GRU_SCAN_MIN_TOKENS = 64;
 // Rows of a window (population x tokens): enough for the GEMMs to fill the GPU, short enough that layers overlap.
 constexpr int GRU_WINDOW_ROWS = 32768;

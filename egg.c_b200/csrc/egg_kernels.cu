@@ -1,7 +1,6 @@
-// Non-GEMM kernels of the evaluation and update paths: per-pair noise tables,
-// row-wise embedding / adaptive-normalise / mean-abs-norm, Q/K/V requantisation,
-// causal integer-softmax attention, fitness, update operand generation, vector
-// AdamW, Muon Newton–Schulz.  "mgpu.cu" = full_cuda_train_transformer_adam_mgpu.cu.
+// Non-GEMM kernels of the evaluation: per-pair noise tables, row-wise embedding /
+// adaptive-normalise / mean-abs-norm, Q/K/V requantisation, causal integer-softmax
+// attention, cross-entropy, fitness; operands and AdamW of the isolated update.  "mgpu.cu" = full_cuda_train_transformer_adam_mgpu.cu.
 #include "egg_kernels.cuh"
 
 #include <limits.h>

@@ -184,7 +184,7 @@ struct WindowParams {
     int32_t *coef;               // [pairs][seq_len]
 };
 int launch_window_transform(cudaStream_t st, const WindowParams &p);
-// Second pass of the head over int32 logits kept in memory (vocab_size != 256): see head_loss_kernel.
+// Second pass of the head over the bytes and maxima that EPI_LOGITS leaves (vocab_size != 256): see head_loss_kernel.
 struct HeadLossParams {
     int M, V, H, seq_len, tok_len;  // rows and tokens of one member
     FastDiv fd_seq;              // filled by launch_head_loss
