@@ -208,7 +208,8 @@ int egg_allgather_fitness(egg_ctx *ctx);
  * egg_download_opt_state (and egg_save_checkpoint through it) first collects it, which makes them collective calls
  * while sharding is on.  Not combined with adaptive-noise overlays (either call refuses while the other is on).
  * Call after egg_comm_init; enable = 0 switches back and, being the moment every rank needs every state again, is
- * a collective call too.
+ * a collective call too.  A call that fails leaves this rank's setting and buffers as they were.  A communicator that
+ * replaces the one it was switched on for takes over: the next update deals the parameters over its ranks.
  */
 int egg_set_update_sharding(egg_ctx *ctx, int enable);
 /* The owner (rank), the cost weight, the byte offset inside TransformerModel and the number of int8 weights of every
@@ -518,7 +519,8 @@ int egg_wave_members(egg_ctx *ctx);
  * row-owning kernels that keep a whole output row in tensor memory and write the requantised int8 row
  * directly, for every hidden_dim (one thread block per 128-row tile up to 512; above, and for few tiles, a cluster of
  * two thread blocks that share the columns and exchange the row maxima through each other's shared memory) whenever
- * seq_len is a multiple of 32 or padding a member to one costs at most a third more rows; other lengths take the
+ * seq_len is a multiple of 32 or padding a member to one costs at most a third more rows, and the larger of shift_out
+ * and shift_mlp_down plus the rank-1 shift (fixed_point + sigma_shift) is at most 20; others take the
  * two-kernel form (int32 pre-activations + row maxima, then a requantisation kernel).  Both forms give
  * identical bytes.
  * At level 2 (the default) the MLP-down projection's epilogue also runs the mean-abs norm that follows the
@@ -527,7 +529,8 @@ int egg_wave_members(egg_ctx *ctx);
  * output projection; it is selectable and tested but not the default: that projection's epilogue is not hidden
  * behind its short contraction (K = hidden_dim), and the norm costs more there than as a kernel of its own
  * (measured on B200: +15 ms in the projections against -12 ms of row-wise kernels per 40960-member generation).
- * enable = 1 keeps the row-owning projections without either, enable = 0 forces the two-kernel form (for A/B timing and for tests that compare the forms); no
+ * enable = 1 keeps the row-owning projections without either, enable = 0 forces the two-kernel form (for A/B timing and for tests that
+ * compare the forms) and allocates its rows where the context has none (EGG_E_NOMEM leaves the level as it was); no
  * counterpart in the reference.  egg_fused_epilogues_active returns the level this context's evaluations take
  * (0 when the configuration only allows the two-kernel form).
  */
