@@ -1029,6 +1029,7 @@ static int eval_wave(egg_ctx *c, uint32_t step_seed, int64_t start_idx, int pop_
         ap.nt_stride = nm.stride; ap.nt_o_b = nb + lo.o_b; ap.xbo = c->d_xbo;
         if (c->attention_mode == 1 && attention_tc_supported(S, cf.head_dim)) rc = PROF(EGG_PROF_ATTENTION, launch_attention_tc(st, ap, c->d_err));
         else if (c->attention_mode == 2 && attention_tc_supported(S, cf.head_dim)) rc = PROF(EGG_PROF_ATTENTION, launch_attention_hy(st, ap, c->d_err));
+        else if (attention_tm_supported(S, c->SP)) rc = PROF(EGG_PROF_ATTENTION, launch_attention_tm(st, ap, c->num_sms, c->d_err));
         else rc = PROF(EGG_PROF_ATTENTION, launch_attention(st, ap));
         if (rc) return rc;
         if (sc && (rc = scaled_dot1(c, M, c->d_ao, 1, nb + lo.o_b, SL.w_o_row + lH, c->d_xbo, 1))) return rc;

@@ -146,6 +146,11 @@ static int make_tmap_box8(CUtensorMap *m, const void *ptr, uint64_t rows, uint64
     return EGG_OK;
 }
 
+int box_map(CUtensorMap *m, const void *ptr, uint64_t rows, uint64_t cols) {
+    if (!g_encode) { set_error("gemm_init() was not called"); return EGG_E_STATE; }
+    return make_tmap_box8(m, ptr, rows, cols, 64);
+}
+
 // Blocks that share a unit of the row-owning GEMM: one up to 512 columns, a cluster of two above (0: unsupported width).
 // An odd multiple of 128 is shared unevenly (640 = 384 + 256, 896 = 512 + 384).
 int fused_cluster_size(int hidden) {

@@ -114,6 +114,9 @@ struct AttnParams {
     int32_t *xbo;             // [members*seq_len] += Σ_d ao_d * noise_B_o[d]
 };
 int launch_attention(cudaStream_t st, const AttnParams &p);
+// scores, weights and sums in tensor memory (egg_attention_tm.cu)
+bool attention_tm_supported(int seq_len, int row_stride);
+int launch_attention_tm(cudaStream_t st, const AttnParams &p, int num_sms, int *err);
 // the same attention on tcgen05 (egg_attention_tc.cu): whole 128-query blocks of one member, head_dim 64, seq_len <= 512
 bool attention_tc_supported(int seq_len, int head_dim);
 int launch_attention_tc(cudaStream_t st, const AttnParams &p, int *err);
