@@ -33,7 +33,7 @@ struct GenSmem {
     alignas(16) int8_t q8[64], k8[64], v8[64];     // the new token's rows of this block's head
     alignas(16) long long part[GEN_WARPS][64];     // attention: Σ w·v of each warp's contexts
     int32_t wt[256];                               // attention weights; later the exp values of the draw
-    int32_t red[8][GEN_WARPS];
+    alignas(16) int32_t red[8][GEN_WARPS];
     int32_t exp_lut[256];
     int32_t count[256];                            // occurrences of every token so far
     int8_t act_lut[256];
@@ -67,9 +67,16 @@ __device__ __forceinline__ bool gen_wait(GenSmem &s, uint64_t *bar, uint32_t par
     if (err) atomicCAS(err, 0, (int)DEV_TIMEOUT_PEER);
     return false;
 }
+// a ring stage: filled and emptied within this block, and mostly ahead of its use
+__device__ __forceinline__ void gen_wait_ring(GenSmem &s, uint64_t *bar, uint32_t parity, int *err) {
+    if (!ptx::mbar_try_wait(bar, parity)) gen_wait(s, bar, parity, err);
+}
 __device__ __forceinline__ void gen_bar() { ptx::named_bar_sync(1, GEN_CT); }
 __device__ __forceinline__ void st_async_b32(uint32_t addr, uint32_t bar, uint32_t v) {
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %2, [%1];" ::"r"(addr), "r"(bar), "r"(v) : "memory");
+}
+__device__ __forceinline__ void st_async_v2(uint32_t addr, uint32_t bar, uint32_t a, uint32_t b) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%2, %3}, [%1];" ::"r"(addr), "r"(bar), "r"(a), "r"(b) : "memory");
 }
 __device__ __forceinline__ void st_async_v4(uint32_t addr, uint32_t bar, int a, int b, int c, int d) {
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%2, %3, %4, %5}, [%1];" ::"r"(addr), "r"(bar), "r"(a), "r"(b),
@@ -129,8 +136,30 @@ __device__ __forceinline__ int gen_dot(const int8_t *row, int lane, const int32_
     return a;
 }
 
-// out_off: byte offset of the product's exchange buffer inside GenSmem.  Every warp takes rc / 8 consecutive rows of a chunk.
-// BYTES = false: int32 results; true: GELU[clip((acc >> shift) + bias)], four consecutive rows at a time.
+// Sums of R rows over the warp, in every lane.
+template <int KW, int R>
+__device__ __forceinline__ void gen_rows(const int8_t *w, int lane, const int32_t (&x)[KW], int (&a)[R]) {
+#pragma unroll
+    for (int k = 0; k < R; k++) a[k] = gen_dot<KW>(w + k * KW * 128, lane, x);
+#pragma unroll
+    for (int k = 0; k < R; k++) a[k] = __reduce_add_sync(0xFFFFFFFFu, a[k]);
+}
+// The byte GELU[clip((sum >> shift) + bias)] of row lane & (R - 1), and four bytes to a word: one look-up a lane, not R in a row.
+template <int R>
+__device__ __forceinline__ void gen_gelu(GenSmem &s, int lane, const int (&a)[R], int bl, int i, int shift, uint32_t (&word)[R / 4]) {
+    int v = a[0];
+#pragma unroll
+    for (int k = 1; k < R; k++) v = (lane & (R - 1)) == k ? a[k] : v;
+    const int b = __shfl_sync(0xFFFFFFFFu, bl, i + (lane & (R - 1)));
+    const uint32_t byte = (uint32_t)(uint8_t)s.act_lut[(uint8_t)(int8_t)clip8((v >> shift) + b)] << (8 * (lane & 3));
+#pragma unroll
+    for (int k = 0; k < R / 4; k++) word[k] = __reduce_or_sync(0xFFFFFFFFu, (lane & (R - 1)) >> 2 == k ? byte : 0u);
+}
+
+// out_off: byte offset of the product's exchange buffer inside GenSmem.  Every warp takes rc / 8 consecutive rows of a chunk,
+// eight at a time where it has as many: their chains of loads, products and sums run side by side, and the peers get one
+// message for eight bytes or two for eight sums (up product of H 512: 3.7 -> 2.5 thousand cycles).
+// BYTES = false: int32 results; true: GELU[clip((acc >> shift) + bias)].
 template <int KW, bool BYTES>
 __device__ __forceinline__ void gen_product(GenSmem &s, GenState &g, const int8_t *vec, int rows, int group, uint32_t out_off, uint32_t bar_off, int *err,
                                             const int8_t *bias = nullptr, int shift = 0) {
@@ -144,31 +173,40 @@ __device__ __forceinline__ void gen_product(GenSmem &s, GenState &g, const int8_
         const int st = g.ring_it % GEN_STAGES;
         const int row0 = g.rank * rows + r + g.warp * per;            // row of the whole product
         const int bl = (BYTES && g.lane < per) ? (int)bias[row0 + g.lane] : 0;
-        gen_wait(s, &s.full[st], (g.ring_it / GEN_STAGES) & 1, err);
+        gen_wait_ring(s, &s.full[st], (g.ring_it / GEN_STAGES) & 1, err);
         __syncwarp();
         const int8_t *w = s.ring[st] + (int64_t)g.warp * per * K;
         for (int i = 0; i < per;) {
-            if (per - i >= 4) {
-                int a[4];
-#pragma unroll
-                for (int k = 0; k < 4; k++) a[k] = gen_dot<KW>(w + (i + k) * K, g.lane, x);
-#pragma unroll
-                for (int k = 0; k < 4; k++) a[k] = __reduce_add_sync(0xFFFFFFFFu, a[k]);
+            const uint32_t at = g.smem_base + out_off + (BYTES ? 1 : 4) * (row0 + i);
+            if (KW <= 8 && per - i >= 8 && ((row0 + i) & 7) == 0) {
+                int a[8];
+                gen_rows<KW, 8>(w + i * K, g.lane, x, a);
                 if (BYTES) {
-                    uint32_t v = 0;
-#pragma unroll
-                    for (int k = 0; k < 4; k++) v |= (uint32_t)(uint8_t)s.act_lut[(uint8_t)(int8_t)clip8((a[k] >> shift) + __shfl_sync(0xFFFFFFFFu, bl, i + k))] << (8 * k);
-                    if (half == 0) st_async_b32(ptx::mapa_u32(g.smem_base + out_off + row0 + i, dest), bar, v);
-                } else if (((row0 + i) & 3) == 0) {
-                    if (half == 0) st_async_v4(ptx::mapa_u32(g.smem_base + out_off + 4 * (row0 + i), dest), bar, a[0], a[1], a[2], a[3]);
+                    uint32_t v[2];
+                    gen_gelu<8>(s, g.lane, a, bl, i, shift, v);
+                    if (half == 0) st_async_v2(ptx::mapa_u32(at, dest), bar, v[0], v[1]);
                 } else {
-                    st_async_b32(ptx::mapa_u32(g.smem_base + out_off + 4 * (row0 + i + half), dest), bar, half ? a[1] : a[0]);
-                    st_async_b32(ptx::mapa_u32(g.smem_base + out_off + 4 * (row0 + i + 2 + half), dest), bar, half ? a[3] : a[2]);
+                    st_async_v4(ptx::mapa_u32(at + 16 * half, dest), bar, half ? a[4] : a[0], half ? a[5] : a[1], half ? a[6] : a[2], half ? a[7] : a[3]);
+                }
+                i += 8;
+            } else if (per - i >= 4) {
+                int a[4];
+                gen_rows<KW, 4>(w + i * K, g.lane, x, a);
+                if (BYTES) {
+                    uint32_t v[1];
+                    gen_gelu<4>(s, g.lane, a, bl, i, shift, v);
+                    if (half == 0) st_async_b32(ptx::mapa_u32(at, dest), bar, v[0]);
+                } else if (((row0 + i) & 3) == 0) {
+                    if (half == 0) st_async_v4(ptx::mapa_u32(at, dest), bar, a[0], a[1], a[2], a[3]);
+                } else {
+                    st_async_b32(ptx::mapa_u32(at + 4 * half, dest), bar, half ? a[1] : a[0]);
+                    st_async_b32(ptx::mapa_u32(at + 4 * (2 + half), dest), bar, half ? a[3] : a[2]);
                 }
                 i += 4;
             } else {
-                const int a = __reduce_add_sync(0xFFFFFFFFu, gen_dot<KW>(w + i * K, g.lane, x));
-                if (half == 0) st_async_b32(ptx::mapa_u32(g.smem_base + out_off + 4 * (row0 + i), dest), bar, a);
+                int a[1];
+                gen_rows<KW, 1>(w + i * K, g.lane, x, a);
+                if (half == 0) st_async_b32(ptx::mapa_u32(at, dest), bar, a[0]);
                 i++;
             }
         }
@@ -177,6 +215,38 @@ __device__ __forceinline__ void gen_product(GenSmem &s, GenState &g, const int8_
         g.ring_it++;
         r += rc;
     }
+}
+
+// q, k and v of H = 512, where a warp has four rows of each: all twelve at a time.
+template <int KW>
+__device__ __forceinline__ void gen_qkv_512(GenSmem &s, GenState &g, const int8_t *vec, uint32_t out_off, uint32_t bar_off, int *err) {
+    constexpr int K = KW * 128, H = 512, RH = H / GEN_BLOCKS;
+    int32_t x[KW];
+    gen_load_vec<KW>(vec, g.lane, x);
+    int a[3][4];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const uint32_t it = g.ring_it + (uint32_t)k;
+        gen_wait_ring(s, &s.full[it % GEN_STAGES], (it / GEN_STAGES) & 1, err);
+        __syncwarp();
+        const int8_t *w = s.ring[it % GEN_STAGES] + (int64_t)g.warp * 4 * K;
+#pragma unroll
+        for (int i = 0; i < 4; i++) a[k][i] = gen_dot<KW>(w + i * K, g.lane, x);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) a[k][i] = __reduce_add_sync(0xFFFFFFFFu, a[k][i]);
+    const int dest = g.lane & 15, half = g.lane >> 4;
+    const uint32_t bar = ptx::mapa_u32(g.smem_base + bar_off, dest), at = ptx::mapa_u32(g.smem_base + out_off + 4 * (g.rank * RH + 4 * g.warp), dest);
+    // lanes 0-15 send q and v, 16-31 k
+    st_async_v4(at + 4 * H * half, bar, half ? a[1][0] : a[0][0], half ? a[1][1] : a[0][1], half ? a[1][2] : a[0][2], half ? a[1][3] : a[0][3]);
+    if (half == 0) st_async_v4(at + 8 * H, bar, a[2][0], a[2][1], a[2][2], a[2][3]);
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+        if (g.lane == 0) ptx::mbar_arrive(&s.empty[(g.ring_it + (uint32_t)k) % GEN_STAGES]);
+    g.ring_it += 3;
 }
 
 // Waits for the exchange in flight; its barrier is armed at once for the exchange after the next one (`bytes_after`).
@@ -188,14 +258,27 @@ __device__ __forceinline__ void gen_receive(GenSmem &s, GenState &g, uint32_t by
     g.ex_it++;
 }
 
+// the eight warps' values of a slot
+__device__ __forceinline__ void gen_red(const int32_t *r, int (&v)[GEN_WARPS]) {
+    static_assert(GEN_WARPS == 8, "two 16-byte reads");
+    const int4 a = *reinterpret_cast<const int4 *>(r), b = *reinterpret_cast<const int4 *>(r + 4);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ int gen_red_max(const int32_t *r) {
+    int v[GEN_WARPS];
+    gen_red(r, v);
+    return max(max(max(v[0], v[1]), max(v[2], v[3])), max(max(v[4], v[5]), max(v[6], v[7])));
+}
+__device__ __forceinline__ int gen_red_sum(const int32_t *r) {
+    int v[GEN_WARPS];
+    gen_red(r, v);
+    return v[0] + v[1] + v[2] + v[3] + v[4] + v[5] + v[6] + v[7];
+}
 __device__ __forceinline__ int gen_block_max(GenSmem &s, const GenState &g, int slot, int v) {
     v = __reduce_max_sync(0xFFFFFFFFu, v);
     if (g.lane == 0) s.red[slot][g.warp] = v;
     gen_bar();
-    int m = s.red[slot][0];
-#pragma unroll
-    for (int i = 1; i < GEN_WARPS; i++) m = max(m, s.red[slot][i]);
-    return m;
+    return gen_red_max(s.red[slot]);
 }
 
 // Four consecutive elements of the row per thread (threads beyond H / 4 carry zeros).
@@ -205,9 +288,7 @@ __device__ __forceinline__ void gen_norm(GenSmem &s, const GenState &g, int x4, 
     const bool in = g.tid < H / 4;
     if (g.lane == 0) s.red[0][g.warp] = sum;
     gen_bar();
-    sum = 0;
-#pragma unroll
-    for (int i = 0; i < GEN_WARPS; i++) sum += s.red[0][i];
+    sum = gen_red_sum(s.red[0]);
     int mn = sum / H;
     if (!mn) mn = 1;
     const float rinv = c_rinv_up.v[mn];
@@ -232,6 +313,16 @@ __device__ __forceinline__ int gen_finish(GenSmem &s, const GenState &g, int x4,
     }
     const float scale = aln_scale(gen_block_max(s, g, 1, max(max(abs(v[0]), abs(v[1])), max(abs(v[2]), abs(v[3])))));
     return (int)pack_clip8(aln_quant_f(v[0], scale), aln_quant_f(v[1], scale), aln_quant_f(v[2], scale), aln_quant_f(v[3], scale));
+}
+
+// trunc(num / den) as C does for a weighted mean num / den of int8 values: the nearest integer to a float estimate (off by less than
+// 1e-4) and one exact remainder, where a 64-bit division takes some 500 cycles of every layer.
+__device__ __forceinline__ int gen_quotient(long long num, int den) {
+    int k = __float2int_rn((float)num / (float)den);
+    const long long r = num - (long long)k * den;
+    if (k > 0 && r < 0) k--;
+    else if (k < 0 && r > 0) k++;
+    return k;
 }
 
 template <int NJ>
@@ -335,7 +426,9 @@ __global__ void __launch_bounds__(GEN_THREADS, 1) generate_kernel(const GenParam
                 gen_norm(s, g, x4, nw, nb, H);
                 nw = row_word(M + L.ln_2 + lH); nb = row_word(M + L.ln_2_bias + lH);
                 const int4 cs = g.tid < H / 4 ? *reinterpret_cast<const int4 *>(p.rope_lut + t * 64 + (4 * g.tid) % 64) : make_int4(0, 0, 0, 0);
-                for (int k = 0; k < 3; k++) gen_product<NJ, false>(s, g, s.h, RH, 8, off_qkv + 4 * k * H, bar_off(), p.err);
+                if constexpr (H == 512) gen_qkv_512<NJ>(s, g, s.h, off_qkv, bar_off(), p.err);
+                else
+                    for (int k = 0; k < 3; k++) gen_product<NJ, false>(s, g, s.h, RH, 8, off_qkv + 4 * k * H, bar_off(), p.err);
                 gen_receive(s, g, 4 * H, p.err);               // after the attention exchange: the output product
                 // integer RoPE on q and k (apply_rope_integer, mgpu.cu:624-644), maxima of q, k, v
                 int qv[3][4];
@@ -361,10 +454,7 @@ __global__ void __launch_bounds__(GEN_THREADS, 1) generate_kernel(const GenParam
                     if (g.tid / 16 == g.rank && g.tid < H / 4) {
 #pragma unroll
                         for (int k = 0; k < 3; k++) {
-                            int m = s.red[2 + k][0];
-#pragma unroll
-                            for (int i = 1; i < GEN_WARPS; i++) m = max(m, s.red[2 + k][i]);
-                            const float sc = aln_scale(m);
+                            const float sc = aln_scale(gen_red_max(s.red[2 + k]));
                             const uint32_t w = pack_clip8(aln_quant_f(qv[k][0], sc), aln_quant_f(qv[k][1], sc), aln_quant_f(qv[k][2], sc), aln_quant_f(qv[k][3], sc));
                             const int o = 4 * (g.tid & 15);
                             *reinterpret_cast<uint32_t *>((k == 0 ? s.q8 : (k == 1 ? s.k8 : s.v8)) + o) = w;
@@ -418,10 +508,10 @@ __global__ void __launch_bounds__(GEN_THREADS, 1) generate_kernel(const GenParam
                     if (g.warp < 2) {
                         const int d = 32 * g.warp + g.lane;
                         long long wv = 0;
-                        int tot = 0;
 #pragma unroll
-                        for (int i = 0; i < GEN_WARPS; i++) { wv += s.part[i][d]; tot += s.red[6][i]; }
-                        const uint32_t o = (uint32_t)clip8((int)(wv / (tot ? (long long)tot : 1))) & 0xFF;
+                        for (int i = 0; i < GEN_WARPS; i++) wv += s.part[i][d];
+                        const int tot = gen_red_sum(s.red[6]);
+                        const uint32_t o = (uint32_t)gen_quotient(wv, tot ? tot : 1) & 0xFF;
                         // lane 4i + j -> byte j of word i; eight words go to sixteen blocks
                         uint32_t word = o << (8 * (g.lane & 3));
                         word |= __shfl_xor_sync(0xFFFFFFFFu, word, 1);
