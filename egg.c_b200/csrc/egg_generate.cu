@@ -411,7 +411,14 @@ __global__ void __launch_bounds__(GEN_THREADS, 1) generate_kernel(const GenParam
                 const bool last = l + 1 == p.n_layers;
                 int8_t *kc = p.kv + ((int64_t)(l * NH + (g.rank < NH ? g.rank : 0)) * 2) * 256 * 64, *vc = kc + 256 * 64;
                 const bool head = g.rank < NH;
-                // this thread's context row of K and its pieces of V: on their way during the product
+                gen_norm(s, g, x4, nw, nb, H);
+                nw = row_word(M + L.ln_2 + lH); nb = row_word(M + L.ln_2_bias + lH);
+                const int4 cs = g.tid < H / 4 ? *reinterpret_cast<const int4 *>(p.rope_lut + t * 64 + (4 * g.tid) % 64) : make_int4(0, 0, 0, 0);
+                if constexpr (H == 512) gen_qkv_512<NJ>(s, g, s.h, off_qkv, bar_off(), p.err);
+                else
+                    for (int k = 0; k < 3; k++) gen_product<NJ, false>(s, g, s.h, RH, 8, off_qkv + 4 * k * H, bar_off(), p.err);
+                // this thread's context row of K and its pieces of V: on their way during the exchange.  (Ahead of the norm
+                // its shared-memory accesses waited behind them, 900 cycles a layer)
                 const int d4 = g.lane & 15, c0 = 2 * g.warp + (g.lane >> 4);
                 int4 kr[4];
                 int32_t vr[16];
@@ -423,12 +430,6 @@ __global__ void __launch_bounds__(GEN_THREADS, 1) generate_kernel(const GenParam
 #pragma unroll
                     for (int i = 0; i < 16; i++) vr[i] = c0 + 16 * i < t ? *reinterpret_cast<const int32_t *>(vc + (c0 + 16 * i) * 64 + 4 * d4) : 0;
                 }
-                gen_norm(s, g, x4, nw, nb, H);
-                nw = row_word(M + L.ln_2 + lH); nb = row_word(M + L.ln_2_bias + lH);
-                const int4 cs = g.tid < H / 4 ? *reinterpret_cast<const int4 *>(p.rope_lut + t * 64 + (4 * g.tid) % 64) : make_int4(0, 0, 0, 0);
-                if constexpr (H == 512) gen_qkv_512<NJ>(s, g, s.h, off_qkv, bar_off(), p.err);
-                else
-                    for (int k = 0; k < 3; k++) gen_product<NJ, false>(s, g, s.h, RH, 8, off_qkv + 4 * k * H, bar_off(), p.err);
                 gen_receive(s, g, 4 * H, p.err);               // after the attention exchange: the output product
                 // integer RoPE on q and k (apply_rope_integer, mgpu.cu:624-644), maxima of q, k, v
                 int qv[3][4];
@@ -438,11 +439,12 @@ __global__ void __launch_bounds__(GEN_THREADS, 1) generate_kernel(const GenParam
                     if (g.tid < H / 4) {
                         a = *reinterpret_cast<const int4 *>(s.qkv + k * H + 4 * g.tid);
                         if (k < 2) {
-                            const long long half_ulp = 1ll << (p.rope_bit - 1), e0 = a.x, o0 = a.y, e1 = a.z, o1 = a.w;
-                            a.x = (int)((e0 * cs.x - o0 * cs.y + half_ulp) >> p.rope_bit);
-                            a.y = (int)((e0 * cs.y + o0 * cs.x + half_ulp) >> p.rope_bit);
-                            a.z = (int)((e1 * cs.z - o1 * cs.w + half_ulp) >> p.rope_bit);
-                            a.w = (int)((e1 * cs.w + o1 * cs.z + half_ulp) >> p.rope_bit);
+                            const long long half_ulp = 1ll << (p.rope_bit - 1);
+                            const int e0 = a.x, o0 = a.y, e1 = a.z, o1 = a.w;
+                            a.x = ptx::shr64_lo(ptx::mad_wide(-o0, cs.y, ptx::mad_wide(e0, cs.x, half_ulp)), p.rope_bit);
+                            a.y = ptx::shr64_lo(ptx::mad_wide(o0, cs.x, ptx::mad_wide(e0, cs.y, half_ulp)), p.rope_bit);
+                            a.z = ptx::shr64_lo(ptx::mad_wide(-o1, cs.w, ptx::mad_wide(e1, cs.z, half_ulp)), p.rope_bit);
+                            a.w = ptx::shr64_lo(ptx::mad_wide(o1, cs.z, ptx::mad_wide(e1, cs.w, half_ulp)), p.rope_bit);
                         }
                     }
                     qv[k][0] = a.x; qv[k][1] = a.y; qv[k][2] = a.z; qv[k][3] = a.w;
