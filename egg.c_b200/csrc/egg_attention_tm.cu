@@ -14,9 +14,10 @@
 // between maximum and weights; longer ones (seq_len > 256) form them twice.
 // Bound: the chain maximum -> weights -> sums of a tile and the instructions beside it (issue slots half busy); tensor memory has
 // room for one tile's sums only (2 x 128 + 3 x 80 of 512 columns), so that tiles overlap by one stage.  Measured against a block
-// per head with mma.sync and 96 accumulators a thread (attention_kernel), 262 144 rows, H 512: 256 tokens 525 -> 309 us; whole
-// passes: 80 tokens (H 384) 2.45 -> 1.39 ms, 512 tokens (H 1024) 18.5 -> 12.7 ms.  Sixteen weight warps that also divide: 375 us;
-// with a register split for 16-column double buffering: 338 us (a tensor-memory load is back after 45 cycles).
+// per head with mma.sync and 96 accumulators a thread (attention_kernel), 262 144 rows, H 512: 256 tokens 525 -> 298 us; whole
+// passes: 80 tokens (H 384) 2.45 -> 1.35 ms, 512 tokens (H 1024) 18.5 -> 12.5 ms.  Sixteen weight warps that also divide: 375 us;
+// with a register split for 16-column double buffering: 338 us (a tensor-memory load is back after 45 cycles); with the products of a
+// chunk in one piece instead of two: 309 us.
 // Every wait is bounded; a timeout makes all later waits fall through.  No multicast.
 #include "egg_kernels.cuh"
 #include "egg_gemm_fused.cuh"
@@ -43,7 +44,7 @@ struct AtmParams {
 struct AtmSmem {                   // behind the 1024-byte aligned stages and the table
     alignas(16) int32_t rowmax[2][2][128];
     alignas(8) uint64_t full[4], empty[4];           // Q, K, V of an item
-    uint64_t s_full[2], s_free[2], p_ready[2], pv_done, o_full, o_free;
+    uint64_t s_full[2], s_free[2], p_ready[2][2], pv_done, o_full, o_free;      // p_ready: key blocks 0 and 1, 2 and 3
     uint32_t tmem_base;
     volatile int abort_flag;
 };
@@ -128,7 +129,7 @@ __global__ void __launch_bounds__(ATM_THREADS, 1) attention_tm_kernel(const __gr
     chain_next();
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; s++) { ptx::mbar_init(&sm.full[s], 1); ptx::mbar_init(&sm.empty[s], 1); }
-        for (int b = 0; b < 2; b++) { ptx::mbar_init(&sm.s_full[b], 1); ptx::mbar_init(&sm.s_free[b], ATM_WARPS); ptx::mbar_init(&sm.p_ready[b], ATM_WARPS); }
+        for (int b = 0; b < 2; b++) { ptx::mbar_init(&sm.s_full[b], 1); ptx::mbar_init(&sm.s_free[b], ATM_WARPS); ptx::mbar_init(&sm.p_ready[b][0], ATM_WARPS); ptx::mbar_init(&sm.p_ready[b][1], ATM_WARPS); }
         ptx::mbar_init(&sm.pv_done, 1); ptx::mbar_init(&sm.o_full, 1); ptx::mbar_init(&sm.o_free, ATM_WARPS);
         sm.abort_flag = 0;
         ptx::fence_barrier_init();
@@ -194,18 +195,22 @@ __global__ void __launch_bounds__(ATM_THREADS, 1) attention_tm_kernel(const __gr
                     ptx::tc_fence_after();
                     return;
                 }
-                atm_wait(&sm.p_ready[b], phase >> b & 1, &sm.abort_flag, p.err, DEV_TIMEOUT_TMEM_EMPTY);
+                const uint32_t ready = phase >> b & 1;
                 phase ^= 1u << b;
                 if (L >> 18 & 1) {           // the last tile's sums have been read
                     atm_wait(&sm.o_free, (phase >> 5 & 1) ^ 1, &sm.abort_flag, p.err, DEV_TIMEOUT_TMEM_EMPTY);
                     phase ^= 32u;
                 }
-                if (sm.abort_flag) return;
-                ptx::tc_fence_after();
                 constexpr uint32_t i_pv = ptx::make_idesc_i8(128, 80) | ATM_B_MN;
                 const int blocks = L >> 14 & 7;
                 uint32_t v = (L & 0x3FFF) << 4, at = tmem + 128 * b, acc = (L >> 18 & 1) ^ 1;
-                for (int j = 0; j < blocks; j++, v += 2048, at += 32, acc = 1) {
+                for (int j = 0; j < 4; j++, v += 2048, at += 32, acc = 1) {
+                    if (!(j & 1)) {          // every worker has written its block of this pair: half of the products run beside the other half's weights
+                        atm_wait(&sm.p_ready[b][j >> 1], ready, &sm.abort_flag, p.err, DEV_TIMEOUT_TMEM_EMPTY);
+                        if (sm.abort_flag) return;
+                        ptx::tc_fence_after();
+                    }
+                    if (j >= blocks) continue;
                     const uint64_t dv = atm_desc_sw64(v, ones_s - v);      // dims 64..79 are the block of ones
 #pragma unroll
                     for (uint32_t l = 0; l < 3; l++) atm_mma_ts(tmem + ATM_O_COL + 80 * l, at + 8 * l, dv, i_pv, acc);
@@ -309,52 +314,53 @@ __global__ void __launch_bounds__(ATM_THREADS, 1) attention_tm_kernel(const __gr
                     ptx::tc_fence_after();
 #pragma unroll 1
                     for (int u = 0; u < 2; u++) {
-                        if (!mine) break;
-                        const int k = c < t ? 1 : (u ? kind1 : kind0);
-                        const uint32_t at = t_lane + 128 * b + 32 * half + 64 * u;
-                        uint32_t l[3][8];
-                        if (k) {
-                            uint32_t v[32];
-                            ptx::tmem_ld32(at, v);
-                            tmem_ld_wait32(v);
+                        if (mine) {
+                            const int k = c < t ? 1 : (u ? kind1 : kind0);
+                            const uint32_t at = t_lane + 128 * b + 32 * half + 64 * u;
+                            uint32_t l[3][8];
+                            if (k) {
+                                uint32_t v[32];
+                                ptx::tmem_ld32(at, v);
+                                tmem_ld_wait32(v);
 #pragma unroll
-                            for (int h = 0; h < 4; h++) {
-                                uint2 w[8];                      // the look-ups of 8 keys before the first word is put together
+                                for (int h = 0; h < 4; h++) {
+                                    uint2 w[8];                      // the look-ups of 8 keys before the first word is put together
 #pragma unroll
-                                for (int i = 0; i < 8; i++) {
-                                    // score + (255 - maximum) << sh, negative where the difference exceeds 255: entry 0
-                                    const uint32_t x = (uint32_t)__viaddmax_s32((int)v[8 * h + i], i0, 0);
-                                    w[i] = atm_entry(__dp4a(S8 ? x : x >> sh, t_mul, t_base));           // one byte of the index: a masked key's entry exists, too
+                                    for (int i = 0; i < 8; i++) {
+                                        // score + (255 - maximum) << sh, negative where the difference exceeds 255: entry 0
+                                        const uint32_t x = (uint32_t)__viaddmax_s32((int)v[8 * h + i], i0, 0);
+                                        w[i] = atm_entry(__dp4a(S8 ? x : x >> sh, t_mul, t_base));           // one byte of the index: a masked key's entry exists, too
+                                    }
+#pragma unroll
+                                    for (int g = 0; g < 2; g++) {
+                                        const uint2 *e = w + 4 * g;
+                                        const uint32_t ab = e[1].x * p.k256 + e[0].x, cd = e[3].x * p.k256 + e[2].x;       // [a0 b0 a1 b1], [c0 d0 c1 d1]
+                                        l[0][2 * h + g] = __byte_perm(ab, cd, 0x5410);
+                                        l[1][2 * h + g] = __byte_perm(ab, cd, 0x7632);
+                                        l[2][2 * h + g] = __byte_perm(e[1].y * p.k256 + e[0].y, e[3].y * p.k256 + e[2].y, 0x5410);
+                                    }
                                 }
+                                if (k == 2) {                         // keys up to the row's own stay
+                                    int lost = 24 - 8 * lane;                // bits that the first four keys' word loses
+                                    asm volatile("" : "+r"(lost));       // (masks held over the tiles cost registers that spill)
 #pragma unroll
-                                for (int g = 0; g < 2; g++) {
-                                    const uint2 *e = w + 4 * g;
-                                    const uint32_t ab = e[1].x * p.k256 + e[0].x, cd = e[3].x * p.k256 + e[2].x;       // [a0 b0 a1 b1], [c0 d0 c1 d1]
-                                    l[0][2 * h + g] = __byte_perm(ab, cd, 0x5410);
-                                    l[1][2 * h + g] = __byte_perm(ab, cd, 0x7632);
-                                    l[2][2 * h + g] = __byte_perm(e[1].y * p.k256 + e[0].y, e[3].y * p.k256 + e[2].y, 0x5410);
+                                    for (int g = 0; g < 8; g++) {
+                                        const uint32_t m = __funnelshift_rc(0xFFFFFFFFu, 0u, max(lost + 32 * g, 0));
+#pragma unroll
+                                        for (int q = 0; q < 3; q++) l[q][g] &= m;
+                                    }
                                 }
+                            } else {
+#pragma unroll
+                                for (int g = 0; g < 8; g++) l[0][g] = l[1][g] = l[2][g] = 0;
                             }
-                            if (k == 2) {                         // keys up to the row's own stay
-                                int lost = 24 - 8 * lane;                // bits that the first four keys' word loses
-                                asm volatile("" : "+r"(lost));       // (masks held over the tiles cost registers that spill)
-#pragma unroll
-                                for (int g = 0; g < 8; g++) {
-                                    const uint32_t m = __funnelshift_rc(0xFFFFFFFFu, 0u, max(lost + 32 * g, 0));
-#pragma unroll
-                                    for (int q = 0; q < 3; q++) l[q][g] &= m;
-                                }
-                            }
-                        } else {
-#pragma unroll
-                            for (int g = 0; g < 8; g++) l[0][g] = l[1][g] = l[2][g] = 0;
+                            tmem_st8(at, l[0]); tmem_st8(at + 8, l[1]); tmem_st8(at + 16, l[2]);
+                            ptx::tmem_st_wait();
                         }
-                        tmem_st8(at, l[0]); tmem_st8(at + 8, l[1]); tmem_st8(at + 16, l[2]);
+                        ptx::tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) ptx::mbar_arrive(&sm.p_ready[b][u]);
                     }
-                    ptx::tmem_st_wait();
-                    ptx::tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) ptx::mbar_arrive(&sm.p_ready[b]);
                 }
                 n += (uint32_t)nc;
             }
