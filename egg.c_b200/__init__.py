@@ -458,7 +458,7 @@ class Context:
         _check(lib().egg_set_fused_epilogues(self._h, int(level)))
 
     def set_attention_tensor_core(self, mode):
-        """0 / False: the mma.sync kernel; 1 / True: scores and weighted sums on tcgen05; 2: scores on mma.sync, weighted
+        """0 / False: the default kernel of the length; 1 / True: scores and weighted sums on tcgen05; 2: scores on mma.sync, weighted
         sums on tcgen05 with the accumulators in tensor memory."""
         _check(lib().egg_set_attention_tensor_core(self._h, int(mode)))
 

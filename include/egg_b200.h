@@ -538,13 +538,13 @@ int egg_set_fused_epilogues(egg_ctx *ctx, int enable);
 int egg_fused_epilogues_active(egg_ctx *ctx);
 /*
  * Selects the attention kernel (compute_attention's context loop, mgpu.cu:787-825); all forms give identical
- * bytes.  mode 0 (default): warp-level mma.sync kernel, accumulators in registers.  mode 1: scores and the three
- * weight-limb products as tensor-memory MMAs (tcgen05), one thread block per member and head.  mode 2: scores,
- * maxima and weights per warp on mma.sync, the weight-limb products on tcgen05 with the accumulators in tensor
- * memory (two blocks per SM, the tensor core works on one 32-key block while the warps prepare the next).
- * Modes 1 and 2 need seq_len % 128 == 0, seq_len <= 512, head_dim 64.  Off by default: as measured on B200 the
- * per-pair weight arithmetic on the CUDA cores bounds all three, and the default kernel is the fastest
- * (per 262 144 rows at seq_len 256: 0.57 ms, 1.02 ms, about 0.64 ms); kept selectable for comparison.
+ * bytes.  mode 0 (default): for windows of 33 to 512 tokens scores, weight limbs and sums in tensor memory, a
+ * persistent block per SM; for others the warp-level mma.sync kernels, accumulators in registers.  mode 1: scores and
+ * the three weight-limb products as tensor-memory MMAs (tcgen05), weights through shared memory, one thread block per
+ * member and head.  mode 2: scores, maxima and weights per warp on mma.sync, the weight-limb products on tcgen05 with
+ * the accumulators in tensor memory (two blocks per SM).  Modes 1 and 2 need seq_len % 128 == 0, seq_len <= 512,
+ * head_dim 64.  Off by default: per 262 144 rows at seq_len 256 the modes take 0.30, 1.02 and about 0.64 ms (mma.sync
+ * 0.52); kept selectable for comparison.
  */
 int egg_set_attention_tensor_core(egg_ctx *ctx, int mode);
 /*
