@@ -230,7 +230,7 @@ __device__ __forceinline__ void tab_store(const GemmParams &p, GemmSmem<BN> &sm,
 // pair slot and sign are then per-lane scalars and the per-column tables are read at warp-uniform addresses, so the
 // accumulators are consumed straight from the TMEM layout (lane = row, registers = columns) with no transpose, no
 // shuffles and about half the instructions of the transposed form.  TMEM loads are double-buffered.
-// FORM: q and k columns (EPI_QKV), both shifts as one (EPI_GELU)
+// FORM: q and k columns (EPI_QKV), both shifts as one (EPI_GELU with BN = 256)
 template <int BN, int EPI, bool FORM, bool RES_TMA>
 __device__ __forceinline__ void epilogue_rpl(const GemmParams &p, GemmSmem<BN> &sm, uint32_t taddr, int r, bool row_ok, int n0,
                                              int cbase, int slot, int sgn, int32_t (*st)[20], int lane, int m0q, int xbs,
@@ -283,7 +283,7 @@ __device__ __forceinline__ void epilogue_rpl(const GemmParams &p, GemmSmem<BN> &
                 // of 1): the integer pipe runs at half the rate of the multiply-add pipe and is the busy one here.
                 const int4 b4 = ptx::lds_v4(bcs + 4 * col);
                 uint32_t z;
-                if (FORM) {
+                if (BN == 256 ? FORM : p.pow_t != 0) {
                     // floor((acc + floor(y / 2^t)) / 2^s) == floor((acc * 2^t + y) / 2^(s+t)): one multiply-add and one shift per
                     // element; the launcher allows it only while acc * 2^t + y provably stays inside int32 (K <= 512 at t = 7)
                     const int sh2 = p.rank1_shift + p.out_shift;
@@ -788,7 +788,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     if (lane == 0 && !ptx::mbar_wait(&sm.rbar[ew], tcount & 1)) gemm_fail(p, &sm.abort_flag, DEV_TIMEOUT_FULL);
                     __syncwarp();
                 }
-                if ((EPI == EPI_QKV && n0 < 2 * p.third) || (EPI == EPI_GELU && p.pow_t))        // asked once a tile, not per four columns: 67.2 -> 66.2 ms of a generation
+                if ((EPI == EPI_QKV && n0 < 2 * p.third) || (EPI == EPI_GELU && BN == 256 && p.pow_t))        // asked once a tile, not per four columns: 68.6 -> 68.0 ms
+                    // of a generation; not for the narrow tiles of small models, where two copies of the code take longer to fetch than they save
                     epilogue_rpl<BN, EPI, true, false>(p, sm, taddr, r, row_ok, n0, cbase, slot, sgn, sm.stage[ew], lane, m0 + quarter * 32, xbs_l, rs_l,
                                                        &tmap_o, sm.ostage0[ew], sm.ostage1[ew]);
                 else

@@ -515,7 +515,7 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 const uint32_t lwb_s = ptx::smem_u32(&sm.ln_wb[qt][0]), ld4_s = ptx::smem_u32(&sm.ln_d4[qt][0]);
                 int8_t *hrow = p.h_out + (int64_t)r * p.H + cofs;
                 int dot0 = 0, dot1 = 0, dot2 = 0;
-                auto norm = [&](auto three) {           // three dots or one: asked once a unit, not per four columns (84.0 -> 82.4 ms of a generation)
+                auto norm = [&](auto dots) {           // three dots or one: asked once a unit, not per four columns (85.0 -> 83.3 ms of a generation)
                 for (int j = 0; j < NT; j++) {
                     const uint32_t box_s = ptx::smem_u32(sm.box[ew][j]) + row_ofs;
 #pragma unroll
@@ -541,14 +541,15 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                             const int y3 = __dp2a_lo(wb.w, 0x00000100, __float2int_rz(f3 * rinv));
                             yw[q4] = pack_clip8(y0, y1, y2, y3);
                             dot0 = __dp4a((int)yw[q4], d4.x, dot0);
-                            if (decltype(three)::value) { dot1 = __dp4a((int)yw[q4], d4.y, dot1); dot2 = __dp4a((int)yw[q4], d4.z, dot2); }
+                            if (decltype(dots)::value ? decltype(dots)::value == 3 : p.ndots > 1) { dot1 = __dp4a((int)yw[q4], d4.y, dot1); dot2 = __dp4a((int)yw[q4], d4.z, dot2); }
                         }
                         *reinterpret_cast<int4 *>(hrow + col) = make_int4((int)yw[0], (int)yw[1], (int)yw[2], (int)yw[3]);
                     }
                 }
                 };
-                if (p.ndots > 1) norm(std::true_type());
-                else norm(std::false_type());
+                if constexpr (MM) norm(std::integral_constant<int, 0>());          // (tiles that span members gain nothing, and small models pay for a second copy)
+                else if (p.ndots > 1) norm(std::integral_constant<int, 3>());
+                else norm(std::integral_constant<int, 1>());
                 // every warp (and both blocks of a pair) adds its columns' share: integer sums, any order
                 int32_t *xo = p.xb_out + (int64_t)r * p.xb_out_stride;
                 atomicAdd(xo, dot0);
