@@ -735,12 +735,8 @@ __global__ void __launch_bounds__(AHY_THREADS, 2) attention_hy_kernel(const Attn
 int launch_attention_hy(cudaStream_t st, const AttnParams &p, int *err) {
     if (!attention_tc_supported(p.seq_len, p.head_dim)) { set_error("tensor-core attention needs seq_len %% 128 == 0, seq_len <= 512, head_dim 64"); return EGG_E_INVALID; }
     const AhyLayout L = ahy_layout(p.seq_len);
-    static int configured[EGG_MAX_DEVICES] = {};
-    const int dev = current_device_slot();
-    if (L.total > configured[dev]) {
-        EGG_CUDA(cudaFuncSetAttribute(attention_hy_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L.total));
-        configured[dev] = L.total;
-    }
+    static std::atomic<bool> configured[EGG_MAX_DEVICES] = {};
+    EGG_CUDA(allow_all_smem(attention_hy_kernel, configured));
     const int blocks = p.members * (p.H / 64);
     attention_hy_kernel<<<blocks, AHY_THREADS, L.total, st>>>(p, L, err);
     EGG_CUDA(cudaGetLastError());
@@ -750,12 +746,8 @@ int launch_attention_hy(cudaStream_t st, const AttnParams &p, int *err) {
 int launch_attention_tc(cudaStream_t st, const AttnParams &p, int *err) {
     if (!attention_tc_supported(p.seq_len, p.head_dim)) { set_error("tensor-core attention needs seq_len %% 128 == 0, seq_len <= 512, head_dim 64"); return EGG_E_INVALID; }
     const AtcLayout L = atc_layout(p.seq_len);
-    static int configured[EGG_MAX_DEVICES] = {};
-    const int dev = current_device_slot();
-    if (L.total > configured[dev]) {
-        EGG_CUDA(cudaFuncSetAttribute(attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L.total));
-        configured[dev] = L.total;
-    }
+    static std::atomic<bool> configured[EGG_MAX_DEVICES] = {};
+    EGG_CUDA(allow_all_smem(attention_tc_kernel, configured));
     const int blocks = p.members * (p.H / 64);
     attention_tc_kernel<<<blocks, ATC_THREADS, L.total, st>>>(p, L, err);
     EGG_CUDA(cudaGetLastError());

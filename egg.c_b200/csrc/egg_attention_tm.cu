@@ -455,7 +455,7 @@ int launch_attention_tm(cudaStream_t st, const AttnParams &a, int num_sms, int *
     p.items = (a.members + p.pack - 1) / p.pack * p.heads;
     p.stage_bytes = (3 * p.rows * 64 + 1023) / 1024 * 1024;
     const int fixed = 1024 + 2048 + (int)sizeof(AtmSmem) + 16;
-    const int limit = 227 * 1024;
+    const int limit = EGG_MAX_SMEM;
     p.copies = 2 * p.stage_bytes + 32 * 1024 + fixed <= limit ? 16 : 8;      // a copy per two banks where two stages fit beside them
     p.k256 = 256;
     p.stages = (limit - fixed - 2048 * p.copies) / p.stage_bytes;
@@ -470,12 +470,8 @@ int launch_attention_tm(cudaStream_t st, const AttnParams &a, int num_sms, int *
     }
     const bool s8 = p.a.shift_attn == 8, brief = p.pack > 1;
     auto kern = s8 ? (brief ? attention_tm_kernel<true, true> : attention_tm_kernel<true, false>) : (brief ? attention_tm_kernel<false, true> : attention_tm_kernel<false, false>);
-    static size_t configured[4][EGG_MAX_DEVICES] = {};
-    size_t &have = configured[2 * s8 + brief][current_device_slot()];
-    if (smem > have) {
-        EGG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        have = smem;
-    }
+    static std::atomic<bool> configured[4][EGG_MAX_DEVICES] = {};
+    EGG_CUDA(allow_all_smem(kern, configured[2 * s8 + brief]));
     EGG_CUDA(launch_chained(kern, (unsigned)(p.items < num_sms ? p.items : num_sms), ATM_THREADS, smem, st, m[0], m[1], m[2], p));
     return EGG_OK;
 }

@@ -5,6 +5,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <atomic>
+
 #include "../../include/egg_b200.h"
 
 namespace egg {
@@ -243,6 +245,17 @@ inline int current_device_slot() {
     int d = 0;
     if (cudaGetDevice(&d) != cudaSuccess || d < 0) d = 0;
     return d % EGG_MAX_DEVICES;
+}
+// Lets a kernel use all of a block's shared memory, once per device.  For kernels whose need depends on the call: a limit that
+// followed the calls could be lowered by one thread's first launch between another thread's check and its launch.
+constexpr int EGG_MAX_SMEM = 227 * 1024;
+template <typename... P>
+inline cudaError_t allow_all_smem(void (*kern)(P...), std::atomic<bool> (&done)[EGG_MAX_DEVICES]) {
+    std::atomic<bool> &d = done[current_device_slot()];
+    if (d) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, EGG_MAX_SMEM);
+    if (e == cudaSuccess) d = true;
+    return e;
 }
 
 // ---------------------------------------------------------------- chained launches

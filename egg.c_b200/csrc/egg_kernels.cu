@@ -1013,12 +1013,8 @@ static size_t attention_smem_bytes(int SP, int heads) { return (size_t)heads * (
 
 template <typename F>
 static int launch_attention_form(cudaStream_t st, F kern, int form, unsigned blocks, size_t smem, const AttnParams &p) {
-    static size_t configured[4][EGG_MAX_DEVICES] = {};
-    size_t &have = configured[form][current_device_slot()];
-    if (smem > have) {
-        EGG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        have = smem;
-    }
+    static std::atomic<bool> configured[4][EGG_MAX_DEVICES] = {};
+    EGG_CUDA(allow_all_smem(kern, configured[form]));
     EGG_CUDA(launch_chained(kern, blocks, 128, smem, st, p));
     return EGG_OK;
 }

@@ -8,6 +8,8 @@
 #include <string.h>
 #include <sys/mman.h>
 
+#include <chrono>
+#include <condition_variable>
 #include <map>
 #include <mutex>
 #include <string>
@@ -37,9 +39,14 @@ void fill(void *d, int v, size_t n) {
     madvise(reinterpret_cast<void *>(a), e - a, MADV_DONTNEED);
     memset(reinterpret_cast<void *>(e), 0, reinterpret_cast<uintptr_t>(d) + n - e);
 }
-int launch(const void *f, void *st, unsigned gx, unsigned gy, unsigned gz) {
+std::map<const void *, int> smem_limit;
+std::string meet_kernel;
+int meeting = 0;
+std::condition_variable met;
+int launch(const void *f, void *st, unsigned gx, unsigned gy, unsigned gz, size_t smem) {
     std::lock_guard<std::mutex> l(m);
     const std::string &name = kernels[f];
+    if (smem > (smem_limit.count(f) ? (size_t)smem_limit[f] : (size_t)48 << 10)) { note("refused", name + " " + hex(st)); return last_error = 1; }
     if (!fail_kernel.empty() && name.find(fail_kernel) != std::string::npos && fail_kernel_after-- == 0) { note("failed", name + " " + hex(st)); return last_error = 719; }
     note("launch", name + " " + hex(st) + " " + std::to_string(gx) + "," + std::to_string(gy) + "," + std::to_string(gz));
     return 0;
@@ -61,6 +68,8 @@ const char *fake_log() { return log_text.c_str(); }
 void fake_clear() { log_text.clear(); }
 void fake_fail_malloc(long nth) { fail_malloc = nth < 0 ? -1 : mallocs + nth; }       // 0: the next one
 void fake_fail_kernel(const char *part, long after) { fail_kernel = part; fail_kernel_after = after; }
+// the next two settings of this kernel's shared-memory limit meet, and the smaller one takes effect last
+void fake_meet(const char *part) { meet_kernel = part; meeting = 0; }
 long fake_mallocs() { return mallocs; }
 long fake_host_allocs() { return host_allocs; }
 long long fake_device_bytes() { long long n = 0; for (auto &d : device) n += (long long)d.second; return n; }
@@ -111,7 +120,18 @@ int cudaDeviceGetAttribute(int *v, int a, int) { *v = a == 75 ? 10 : (a == 16 ? 
 int cudaGetDriverEntryPoint(const char *, void **fn, unsigned long long, int *res) { *fn = (void *)encode_tiled; if (res) *res = 0; return 0; }
 int cudaGetLastError() { const int e = last_error; last_error = 0; return e; }
 const char *cudaGetErrorString(int e) { return e == 2 ? "out of memory" : "a failure the test asked for"; }
-int cudaFuncSetAttribute(const void *, int, int) { return 0; }
+int cudaFuncSetAttribute(const void *f, int a, int v) {
+    if (a != 8) return 0;
+    std::unique_lock<std::mutex> l(m);
+    const bool meet = !meet_kernel.empty() && kernels[f].find(meet_kernel) != std::string::npos;
+    smem_limit[f] = meet && meeting ? (v < smem_limit[f] ? v : smem_limit[f]) : v;
+    if (meet) {
+        meeting++;
+        met.notify_all();
+        met.wait_for(l, std::chrono::seconds(2), [] { return meeting > 1; });
+    }
+    return 0;
+}
 int cudaOccupancyMaxActiveClusters(int *n, const void *, const void *) { *n = 74; return 0; }
 int cudaGetSymbolAddress(void **p, const void *s) {
     std::lock_guard<std::mutex> l(m);
@@ -135,10 +155,10 @@ int cudaGraphInstantiate(void **e, void *, unsigned long long) { *e = (void *)1;
 int cudaGraphDestroy(void *) { return 0; }
 int cudaGraphExecDestroy(void *) { return 0; }
 int cudaGraphLaunch(void *, void *st) { std::lock_guard<std::mutex> l(m); note("graph", hex(st)); return 0; }
-int cudaLaunchKernel(const void *f, uint64_t gxy, uint32_t gz, uint64_t, uint32_t, void **, size_t, void *st) { return launch(f, st, (unsigned)gxy, (unsigned)(gxy >> 32), gz); }
+int cudaLaunchKernel(const void *f, uint64_t gxy, uint32_t gz, uint64_t, uint32_t, void **, size_t smem, void *st) { return launch(f, st, (unsigned)gxy, (unsigned)(gxy >> 32), gz, smem); }
 int cudaLaunchKernelExC(const void *cfg, const void *f, void **) {
     const unsigned *g = static_cast<const unsigned *>(cfg);
-    return launch(f, *reinterpret_cast<void *const *>(static_cast<const char *>(cfg) + 32), g[0], g[1], g[2]);
+    return launch(f, *reinterpret_cast<void *const *>(static_cast<const char *>(cfg) + 32), g[0], g[1], g[2], *reinterpret_cast<const size_t *>(static_cast<const char *>(cfg) + 24));
 }
 
 // ---- what the compiler's start-up code calls ----

@@ -314,3 +314,24 @@ def test_owner_costs_are_those_of_the_update():
     _, costs, _, weights = pkg.update_owner_plan(cfg, 8, spans=True)
     vector = weights <= 4 * 256
     assert (costs[~vector] == weights[~vector]).all() and set(costs[vector] // weights[vector]) <= set(range(37, 57))
+
+
+@pytest.mark.parametrize("seqs,mode,kernel", [
+    ((128, 512), 0, "attention_tm_kernel"), ((528, 1024), 0, "attention_kernel"),
+    ((128, 512), 1, "attention_tc_kernel"), ((128, 512), 2, "attention_hy_kernel"),
+])
+def test_first_launches_of_two_threads(fake_cuda, seqs, mode, kernel):
+    """Two threads whose first evaluations need different amounts of shared memory for one kernel: neither lowers the other's limit."""
+    out = fake_cuda("""
+import threading
+fake.fake_meet(%r)
+ctxs = [context(hidden_dim=128, n_layers=1, seq_len=s, population_size=2) for s in %r]
+if %d:
+    for c in ctxs: c.set_attention_tensor_core(%d)
+rcs = [None, None]
+def go(i): rcs[i] = error(lambda: ctxs[i].eval_chunk(1, 0, 0, 2))
+ts = [threading.Thread(target=go, args=(i,)) for i in (0, 1)]
+[t.start() for t in ts]; [t.join() for t in ts]
+out["rcs"], out["launched"] = rcs, launches(%r)
+""" % (kernel.encode(), seqs, mode, mode, kernel))
+    assert out == {"rcs": [0, 0], "launched": 2}
