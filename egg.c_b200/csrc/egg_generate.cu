@@ -217,31 +217,45 @@ __device__ __forceinline__ void gen_product(GenSmem &s, GenState &g, const int8_
     }
 }
 
-// q, k and v of H = 512, where a warp has four rows of each: all twelve at a time.
-template <int KW>
-__device__ __forceinline__ void gen_qkv_512(GenSmem &s, GenState &g, const int8_t *vec, uint32_t out_off, uint32_t bar_off, int *err) {
-    constexpr int K = KW * 128, H = 512, RH = H / GEN_BLOCKS;
-    int32_t x[KW];
-    gen_load_vec<KW>(vec, g.lane, x);
-    int a[3][4];
+// q, k and v of a layer side by side: three ring stages are held at once, a warp forms NJ sums of each product, and the three waits,
+// products and sums overlap.  Up to twelve sums: H 256 5.54 -> 4.97 ms, 384 5.58 -> 5.23 (2 layers, 250 sampled bytes; 128 alike).
+// Fifteen (H 640, the widest whose rows fit one chunk) take longer than three products, 7.30 against 7.14 ms: a row of an odd width is
+// read by words, and a register spills.
+template <int NJ>
+constexpr bool GEN_QKV_TOGETHER = NJ <= 4;
+template <int NJ>
+__device__ __forceinline__ void gen_qkv(GenSmem &s, GenState &g, const int8_t *vec, uint32_t out_off, uint32_t bar_off, int *err) {
+    static_assert(8 * NJ * (128 * NJ) <= GEN_CHUNK && GEN_STAGES >= 3, "a block's rows are one chunk each, all held before one is released");
+    constexpr int H = NJ * 128, WORDS = NJ % 4 == 0 ? 4 : (NJ % 2 == 0 ? 2 : 1), MSGS = 3 * NJ / WORDS;       // words a message, by its alignment
+    int32_t x[NJ];
+    gen_load_vec<NJ>(vec, g.lane, x);
+    int a[3 * NJ];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         const uint32_t it = g.ring_it + (uint32_t)k;
         gen_wait_ring(s, &s.full[it % GEN_STAGES], (it / GEN_STAGES) & 1, err);
         __syncwarp();
-        const int8_t *w = s.ring[it % GEN_STAGES] + (int64_t)g.warp * 4 * K;
+        const int8_t *w = s.ring[it % GEN_STAGES] + g.warp * NJ * H;
 #pragma unroll
-        for (int i = 0; i < 4; i++) a[k][i] = gen_dot<KW>(w + i * K, g.lane, x);
+        for (int i = 0; i < NJ; i++) a[k * NJ + i] = gen_dot<NJ>(w + i * H, g.lane, x);
     }
 #pragma unroll
-    for (int k = 0; k < 3; k++)
-#pragma unroll
-        for (int i = 0; i < 4; i++) a[k][i] = __reduce_add_sync(0xFFFFFFFFu, a[k][i]);
+    for (int i = 0; i < 3 * NJ; i++) a[i] = __reduce_add_sync(0xFFFFFFFFu, a[i]);
     const int dest = g.lane & 15, half = g.lane >> 4;
-    const uint32_t bar = ptx::mapa_u32(g.smem_base + bar_off, dest), at = ptx::mapa_u32(g.smem_base + out_off + 4 * (g.rank * RH + 4 * g.warp), dest);
-    // lanes 0-15 send q and v, 16-31 k
-    st_async_v4(at + 4 * H * half, bar, half ? a[1][0] : a[0][0], half ? a[1][1] : a[0][1], half ? a[1][2] : a[0][2], half ? a[1][3] : a[0][3]);
-    if (half == 0) st_async_v4(at + 8 * H, bar, a[2][0], a[2][1], a[2][2], a[2][3]);
+    const uint32_t bar = ptx::mapa_u32(g.smem_base + bar_off, dest), at = ptx::mapa_u32(g.smem_base + out_off + 4 * NJ * (8 * g.rank + g.warp), dest);
+    // lanes 0-15 send the even messages, 16-31 the odd ones
+#pragma unroll
+    for (int m = 0; m < MSGS; m += 2) {
+        const int e = m * WORDS, o = (m + 1 < MSGS ? m + 1 : m) * WORDS;
+        const uint32_t to = at + 4 * (half ? o / NJ * H + o % NJ : e / NJ * H + e % NJ);
+        int v[4];
+#pragma unroll
+        for (int j = 0; j < WORDS; j++) v[j] = half ? a[o + j] : a[e + j];
+        if (o == e && half) continue;
+        if (WORDS == 4) st_async_v4(to, bar, v[0], v[1], v[2], v[3]);
+        else if (WORDS == 2) st_async_v2(to, bar, v[0], v[1]);
+        else st_async_b32(to, bar, v[0]);
+    }
     __syncwarp();
 #pragma unroll
     for (int k = 0; k < 3; k++)
@@ -414,7 +428,7 @@ __global__ void __launch_bounds__(GEN_THREADS, 1) generate_kernel(const GenParam
                 gen_norm(s, g, x4, nw, nb, H);
                 nw = row_word(M + L.ln_2 + lH); nb = row_word(M + L.ln_2_bias + lH);
                 const int4 cs = g.tid < H / 4 ? *reinterpret_cast<const int4 *>(p.rope_lut + t * 64 + (4 * g.tid) % 64) : make_int4(0, 0, 0, 0);
-                if constexpr (H == 512) gen_qkv_512<NJ>(s, g, s.h, off_qkv, bar_off(), p.err);
+                if constexpr (GEN_QKV_TOGETHER<NJ>) gen_qkv<NJ>(s, g, s.h, off_qkv, bar_off(), p.err);
                 else
                     for (int k = 0; k < 3; k++) gen_product<NJ, false>(s, g, s.h, RH, 8, off_qkv + 4 * k * H, bar_off(), p.err);
                 // this thread's context row of K and its pieces of V: on their way during the exchange.  (Ahead of the norm
