@@ -156,9 +156,10 @@ __device__ __forceinline__ void gen_gelu(GenSmem &s, int lane, const int (&a)[R]
     for (int k = 0; k < R / 4; k++) word[k] = __reduce_or_sync(0xFFFFFFFFu, (lane & (R - 1)) >> 2 == k ? byte : 0u);
 }
 
-// out_off: byte offset of the product's exchange buffer inside GenSmem.  Every warp takes rc / 8 consecutive rows of a chunk,
-// eight at a time where it has as many: their chains of loads, products and sums run side by side, and the peers get one
-// message for eight bytes or two for eight sums (up product of H 512: 3.7 -> 2.5 thousand cycles).
+// out_off: byte offset of the product's exchange buffer inside GenSmem.  Every warp takes rc / 8 consecutive rows of a chunk, four
+// at a time where it has as many, and eight of the up product at H 256, 384 and 512 (its share of a chunk is 4 or 8 rows, that of
+// other products at most 5): their chains of loads, products and sums run side by side, and the peers get one message for eight
+// bytes (up product of H 512: 3.7 -> 2.5 thousand cycles).
 // BYTES = false: int32 results; true: GELU[clip((acc >> shift) + bias)].
 template <int KW, bool BYTES>
 __device__ __forceinline__ void gen_product(GenSmem &s, GenState &g, const int8_t *vec, int rows, int group, uint32_t out_off, uint32_t bar_off, int *err,
@@ -178,16 +179,12 @@ __device__ __forceinline__ void gen_product(GenSmem &s, GenState &g, const int8_
         const int8_t *w = s.ring[st] + (int64_t)g.warp * per * K;
         for (int i = 0; i < per;) {
             const uint32_t at = g.smem_base + out_off + (BYTES ? 1 : 4) * (row0 + i);
-            if (KW <= 8 && per - i >= 8 && ((row0 + i) & 7) == 0) {
+            if (BYTES && per - i >= 8) {
                 int a[8];
+                uint32_t v[2];
                 gen_rows<KW, 8>(w + i * K, g.lane, x, a);
-                if (BYTES) {
-                    uint32_t v[2];
-                    gen_gelu<8>(s, g.lane, a, bl, i, shift, v);
-                    if (half == 0) st_async_v2(ptx::mapa_u32(at, dest), bar, v[0], v[1]);
-                } else {
-                    st_async_v4(ptx::mapa_u32(at + 16 * half, dest), bar, half ? a[4] : a[0], half ? a[5] : a[1], half ? a[6] : a[2], half ? a[7] : a[3]);
-                }
+                gen_gelu<8>(s, g.lane, a, bl, i, shift, v);
+                if (half == 0) st_async_v2(ptx::mapa_u32(at, dest), bar, v[0], v[1]);
                 i += 8;
             } else if (per - i >= 4) {
                 int a[4];
