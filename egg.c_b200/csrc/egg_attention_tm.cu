@@ -26,8 +26,6 @@
 
 namespace egg {
 
-int box_map(CUtensorMap *m, const void *ptr, uint64_t rows, uint64_t cols);      // egg_gemm_inst.cu: 64 columns x 32 rows, 64-byte swizzle
-
 constexpr int ATM_WARPS = 8;                           // of either kind of worker: 4 tensor-memory lane quarters x 2
 constexpr int ATM_THREADS = 32 * (2 + 2 * ATM_WARPS);      // warp 0 copies, warp 1 MMAs, 2-9 weights, 10-17 quotients
 constexpr int ATM_O_COL = 256;                         // tensor memory: two score buffers | O_l (80 each: 64 dims and the sum)
@@ -68,42 +66,16 @@ __device__ __forceinline__ void atm_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uin
         ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t *r) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),
-                 "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-                 : "memory");
-}
-__device__ __forceinline__ uint32_t tmem_ld1(uint32_t taddr) {
-    uint32_t r;
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(taddr) : "memory");
-    return r;
-}
-__device__ __forceinline__ void tmem_ld_wait32(uint32_t *r) {
-    ptx::tmem_ld_wait16(r);
-    asm volatile("" : "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]),
-                 "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31]));
-}
 __device__ __forceinline__ uint2 atm_entry(uint32_t addr) {
     uint2 v;
     asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
     return v;
 }
 
-// trunc(num / den) by an exact remainder: num = p0 + 2^7 p1 + 2^14 p2, |num / den| <= 127, limb sums below 2^23.  The nearest
-// integer to the estimate overshoots the truncated quotient exactly when the remainder, below 2^27 and so exact in wrapping
-// 32-bit arithmetic, has the opposite sign.
-__device__ __forceinline__ int atm_div(int p0, int p1, int p2, uint32_t den, float rden) {
-    const int hi = p2 * 128 + p1;
-    const float fn = fmaf(__int2float_rn(hi), 128.0f, __int2float_rn(p0));
-    const int k = __float2int_rn(fn * rden);
-    const int r = (int)((uint32_t)hi * 128u + (uint32_t)p0 - (uint32_t)k * den);
-    const int sg = (__float_as_int(fn) >> 31) | 1;
-    return k + sg * ((r * sg) >> 31);
-}
 // Four quotients from float estimates alone.  An estimate is off by less than 2^-21 of itself (num's two conversions and their sum,
 // den's conversion, the approximate reciprocal and the product: three ulps), so with the reciprocal moved 2^-20 up and down its
 // truncations enclose the quotient: where both agree that is it.  Elsewhere, one output in some 20 000 and the rows whose weight
-// all lies on one key, `differ` is set and the outputs are divided again with atm_div.
+// all lies on one key, `differ` is set and the outputs are divided again with att_div_small.
 __device__ __forceinline__ uint32_t atm_quotients(const uint32_t *p0, const uint32_t *p1, const uint32_t *p2, float up, float down, uint32_t &differ) {
     float n[4];
 #pragma unroll
@@ -279,7 +251,7 @@ __global__ void __launch_bounds__(ATM_THREADS, 1) attention_tm_kernel(const __gr
                         if (k == 0) continue;
                         uint32_t v[32];
                         ptx::tmem_ld32(t_lane + 128 * b + 32 * half + 64 * u, v);
-                        tmem_ld_wait32(v);
+                        ptx::tmem_ld_wait32(v);
                         int m[4] = {mx, INT_MIN, INT_MIN, INT_MIN};          // four chains
                         if (k == 1) {
 #pragma unroll
@@ -321,7 +293,7 @@ __global__ void __launch_bounds__(ATM_THREADS, 1) attention_tm_kernel(const __gr
                             if (k) {
                                 uint32_t v[32];
                                 ptx::tmem_ld32(at, v);
-                                tmem_ld_wait32(v);
+                                ptx::tmem_ld_wait32(v);
 #pragma unroll
                                 for (int h = 0; h < 4; h++) {
                                     uint2 w[8];                      // the look-ups of 8 keys before the first word is put together
@@ -354,7 +326,7 @@ __global__ void __launch_bounds__(ATM_THREADS, 1) attention_tm_kernel(const __gr
 #pragma unroll
                                 for (int g = 0; g < 8; g++) l[0][g] = l[1][g] = l[2][g] = 0;
                             }
-                            tmem_st8(at, l[0]); tmem_st8(at + 8, l[1]); tmem_st8(at + 16, l[2]);
+                            ptx::tmem_st8(at, l[0]); ptx::tmem_st8(at + 8, l[1]); ptx::tmem_st8(at + 16, l[2]);
                             ptx::tmem_st_wait();
                         }
                         ptx::tc_fence_before();
@@ -386,7 +358,7 @@ __global__ void __launch_bounds__(ATM_THREADS, 1) attention_tm_kernel(const __gr
                 __syncwarp();
                 ptx::tc_fence_after();
                 if (__any_sync(0xFFFFFFFFu, own)) {
-                    uint32_t s0 = tmem_ld1(t_lane + ATM_O_COL + 64), s1 = tmem_ld1(t_lane + ATM_O_COL + 144), s2 = tmem_ld1(t_lane + ATM_O_COL + 224);
+                    uint32_t s0 = ptx::tmem_ld1(t_lane + ATM_O_COL + 64), s1 = ptx::tmem_ld1(t_lane + ATM_O_COL + 144), s2 = ptx::tmem_ld1(t_lane + ATM_O_COL + 224);
                     const uint32_t at = t_lane + ATM_O_COL + (uint32_t)(half * 32);
                     float up = 0.0f, down = 0.0f;
                     uint32_t den = 1;
@@ -414,7 +386,7 @@ __global__ void __launch_bounds__(ATM_THREADS, 1) attention_tm_kernel(const __gr
                             for (int g = 0; g < 4; g++) {
                                 int k[4];
 #pragma unroll
-                                for (int i = 0; i < 4; i++) k[i] = atm_div((int)x[0][4 * g + i], (int)x[1][4 * g + i], (int)x[2][4 * g + i], den, up);
+                                for (int i = 0; i < 4; i++) k[i] = att_div_small((int)x[0][4 * g + i], (int)x[1][4 * g + i], (int)x[2][4 * g + i], den, up);
                                 o[g] = ptx::pack_sat_s8(k[0], k[1], k[2], k[3]);
                             }
                         }

@@ -219,6 +219,20 @@ __device__ __forceinline__ int div_small(int a, float rinv_up) {
     return __float2int_rz(i2f_small(a) * rinv_up);
 }
 
+// trunc(num / den) for num = p0 + 2^7 p1 + 2^14 p2, |num / den| <= 127, limb sums below 2^23 (attention over up to 512 keys, den
+// their weights' sum, rden its reciprocal to within 2^-19).  The estimate needs two conversions; the remainder num - k*den is at
+// most 2^28 in magnitude (half of 512 weights of 2^20) and rounding, so wrapping 32-bit arithmetic on the low words of num and den
+// gives its exact value.  The nearest integer k overshoots the truncated quotient exactly when the remainder's sign is
+// opposite to the numerator's (fn has the numerator's sign: below 2^31 it is exact, above its error is far smaller).
+__device__ __forceinline__ int att_div_small(int p0, int p1, int p2, uint32_t den, float rden) {
+    const int hi = p2 * 128 + p1;
+    const float fn = fmaf(__int2float_rn(hi), 128.0f, __int2float_rn(p0));
+    const int k = __float2int_rn(fn * rden);
+    const int r = (int)((uint32_t)hi * 128u + (uint32_t)p0 - (uint32_t)k * den);
+    const int sg = (__float_as_int(fn) >> 31) | 1;
+    return k + sg * ((r * sg) >> 31);
+}
+
 // [sat8(a), sat8(b), sat8(c), sat8(d)] as bytes 0..3 with the reference's clip to [-127, 127]
 __device__ __forceinline__ uint32_t pack_clip8(int a, int b, int c, int d) {
     uint32_t hi, r;

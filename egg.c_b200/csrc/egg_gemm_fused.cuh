@@ -102,17 +102,8 @@ struct FusedSmem {
     volatile int abort_flag;
 };
 
-namespace ptx {
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t *r) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-          "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-        : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-}  // namespace ptx
+// tensor map of an int8 matrix in boxes of 64 columns x 32 rows, 64-byte swizzle (egg_gemm_inst.cu)
+int box_map(CUtensorMap *m, const void *ptr, uint64_t rows, uint64_t cols);
 
 // Waits for an mbarrier phase unless the block is already draining after a timeout; a timeout here starts the drain.
 __device__ __forceinline__ void fused_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *err, int code) {

@@ -683,26 +683,13 @@ __device__ __forceinline__ void att_scores(int (&c)[4][4], const int4 (&qa)[2], 
 }
 
 // trunc(num / den) as C does, for |num/den| <= 127: the quotient is estimated in float from the three
-// limb sums and fixed up with one exact int64 remainder test.
+// limb sums and fixed up with one exact int64 remainder test.  (Limb sums below 2^23: att_div_small.)
 __device__ __forceinline__ int att_div(int p0, int p1, int p2, long long den, float rden) {
     const long long num = (long long)p0 + ((long long)p1 << 7) + ((long long)p2 << 14);
     int k = f2i_exact((float)num * rden);             // nearest integer to the real quotient (|error| < 1e-3)
     long long r = num - (long long)k * den;
     if (num >= 0) { if (r < 0) k--; } else { if (r > 0) k++; }
     return k;
-}
-
-// The same quotient when every limb sum is below 2^23 (seq_len <= 512).  The estimate needs two conversions; the remainder
-// num - k*den is below 2^27 in magnitude (den/2 and rounding), so wrapping 32-bit arithmetic on the low words of num and den
-// gives its exact value.  The nearest integer k overshoots the truncated quotient exactly when the remainder's sign is
-// opposite to the numerator's (fn has the numerator's sign: below 2^31 it is exact, above its error is far smaller).
-__device__ __forceinline__ int att_div_small(int p0, int p1, int p2, uint32_t den, float rden) {
-    const int hi = p2 * 128 + p1;
-    const float fn = fmaf(__int2float_rn(hi), 128.0f, __int2float_rn(p0));
-    const int k = __float2int_rn(fn * rden);
-    const int r = (int)((uint32_t)hi * 128u + (uint32_t)p0 - (uint32_t)k * den);
-    const int sg = (__float_as_int(fn) >> 31) | 1;
-    return k + sg * ((r * sg) >> 31);
 }
 
 // limb-packed weights of a block's 16 scores per lane; keys beyond the query's own position weigh nothing
