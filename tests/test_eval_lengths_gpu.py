@@ -1,6 +1,7 @@
-"""Evaluation at every form of the attention kernels (a warp per head up to 64 tokens, kept scores up to 128, any length
-above), at ragged ends of their key blocks, and at row tiles that span members (lengths that are multiples of 32 or padded to
-one), with and without overlays, against the CPU oracle: losses are equal."""
+"""Evaluation at every form of the attention kernels (a warp per head at 16 and 32 tokens; tensor memory where a member has 64 to 512
+rows in whole blocks of 32: two members or one in a tile, one to four tiles; for other lengths a warp per head up to 64 tokens, kept
+scores up to 128, any length above), at ragged ends of their key blocks, and at row tiles that span members (lengths that are multiples
+of 32 or padded to one), with and without overlays, against the CPU oracle: losses are equal."""
 import numpy as np
 import pytest
 
@@ -29,6 +30,9 @@ def test_losses_match_oracle(seq, hidden):
 @pytest.mark.parametrize("kw", [
     dict(hidden_dim=128, seq_len=48, shift_out=14), dict(hidden_dim=256, seq_len=128, shift_mlp_down=15, fixed_point=5),
     dict(hidden_dim=640, seq_len=32, fixed_point=6, sigma_shift=6),
+    # rows that are not padded: the attention kernels that tensor memory takes no part in
+    dict(hidden_dim=128, seq_len=80, shift_out=14), dict(hidden_dim=256, seq_len=112, shift_out=14),
+    dict(hidden_dim=256, seq_len=144, shift_out=14), dict(hidden_dim=128, seq_len=400, shift_out=14),
 ])
 def test_shifts_beyond_the_row_owning_form(kw):
     """Output shift plus rank-1 shift above 20: the two-kernel form at lengths and widths that otherwise never take it."""
