@@ -520,7 +520,7 @@ def main():
     ap.add_argument("--fused-level", type=int, default=2, choices=[0, 1, 2, 3],
                     help="A/B: 0 two-kernel adaptive norms, 1 row-owning projections, 2 (default) also the next mean-abs norm inside the MLP-down epilogue")
     ap.add_argument("--attention-tc", type=int, nargs="?", const=1, default=None, choices=[0, 1, 2],
-                    help="A/B: attention kernel: 0 mma.sync, 1 tcgen05 scores and sums, 2 mma.sync scores + tcgen05 sums (default: the library's)")
+                    help="A/B: attention kernel: 0 the default of the length, 1 tcgen05 with weights through shared memory, 2 mma.sync scores + tcgen05 sums")
     ap.add_argument("--replicated-update", action="store_true", help="N > 1: repeat the whole update on every GPU as the reference does (default: shard it by matrix)")
     ap.add_argument("--wave", type=int, default=0, help="members per internal wave (0: the library's default)")
     ap.add_argument("--small", action="store_true", help="profiling-sized run: 1024 members, one warm-up step, no end-to-end / CPU legs")

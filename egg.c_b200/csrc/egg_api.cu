@@ -162,8 +162,8 @@ struct egg_ctx {
     // row-owning projections with the adaptive normalisations fused (default wherever the shapes allow)
     int fused_level = 2;      // 0: two-kernel adaptive norms; 1: row-owning projections; 2: + the next mean-abs norm inside MLP-down;
                               // 3: + LN2 inside the output projection (selectable, slower: that epilogue is not hidden behind its MMAs)
-    // attention on tcgen05 (egg_attention_tc.cu) instead of the mma.sync kernel: correct but slower as measured, off by default
-    int attention_mode = 0;       // 0: mma.sync kernel; 1: tcgen05 scores and sums; 2: mma.sync scores, tcgen05 sums
+    // the other attentions on tcgen05 (egg_attention_tc.cu): the same bytes, slower as measured, off by default
+    int attention_mode = 0;       // 0: by length (attention_tm_supported); 1: weights through shared memory; 2: mma.sync scores, tcgen05 sums
     // measurement
     cudaEvent_t t0 = nullptr, t1 = nullptr;
     bool prof_on = false;

@@ -410,9 +410,14 @@ __global__ void __launch_bounds__(ATM_THREADS, 1) attention_tm_kernel(const __gr
     }
 }
 
-// Windows of up to 512 tokens (limb sums below 2^23) whose rows are padded to a multiple of 32.  Not those of 32 rows: four
-// members would share a tile, most of whose blocks are off the diagonal, and every quarter has a row that sees one key only and
-// is divided twice (65 536 members, H 256: 7.1 ms against 6.95 in attention_warp_kernel).
+// Members of 64 to 512 rows (limb sums below 2^23), a multiple of 32.  By length alone, measured with 2 to 16 384 members at H 128 to
+// 1024, evaluations of two layers, against the same with the mma.sync kernels.  64 tokens (two members in a tile, half of its blocks off
+// the diagonal): the kernel 0.64 to 0.99 of attention_warp_kernel's time, the evaluation 1 to 18 % shorter.  48 tokens (a quarter of
+// the rows are padding besides): the kernel 0.72 to 1.0, but 1.01 to 1.13 between 1000 and 6200 heads (20.8 -> 22.9 us); started early
+// it hides that: the evaluation is up to 15 % shorter below 1500 heads, and from there on between 4 % shorter and 0.6 % longer, by
+// which runs of one side differ too.  From 80 tokens the kernel takes 0.50 to 1.0 of attention_kernel's time.  Not 32 rows: four
+// members would share a tile, most of whose blocks are off the diagonal, and every quarter has a row that sees one key only and is
+// divided twice (65 536 members, H 256: 7.1 ms against 6.95 in attention_warp_kernel).
 bool attention_tm_supported(int seq_len, int row_stride) { return seq_len <= row_stride && row_stride % 32 == 0 && row_stride >= 64 && row_stride <= 512; }
 
 int launch_attention_tm(cudaStream_t st, const AttnParams &a, int num_sms, int *err) {

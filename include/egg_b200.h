@@ -538,8 +538,9 @@ int egg_set_fused_epilogues(egg_ctx *ctx, int enable);
 int egg_fused_epilogues_active(egg_ctx *ctx);
 /*
  * Selects the attention kernel (compute_attention's context loop, mgpu.cu:787-825); all forms give identical
- * bytes.  mode 0 (default): for windows of 33 to 512 tokens scores, weight limbs and sums in tensor memory, a
- * persistent block per SM; for others the warp-level mma.sync kernels, accumulators in registers.  mode 1: scores and
+ * bytes.  mode 0 (default): where a member has 64 to 512 rows, a multiple of 32, scores, weight limbs and sums in tensor
+ * memory, a persistent block per SM (windows of 48 to 512 tokens; an odd multiple of 16 only where its rows are padded, not
+ * with output plus rank-1 shift above 20); for others the warp-level mma.sync kernels, accumulators in registers.  mode 1: scores and
  * the three weight-limb products as tensor-memory MMAs (tcgen05), weights through shared memory, one thread block per
  * member and head.  mode 2: scores, maxima and weights per warp on mma.sync, the weight-limb products on tcgen05 with
  * the accumulators in tensor memory (two blocks per SM).  Modes 1 and 2 need seq_len % 128 == 0, seq_len <= 512,
