@@ -163,7 +163,8 @@ __device__ __forceinline__ void gen_gelu(GenSmem &s, int lane, const int (&a)[R]
 // out_off: byte offset of the product's exchange buffer inside GenSmem.  Every warp takes rc / 8 consecutive rows of a chunk, four
 // at a time where it has as many, and eight of the up product at H 256, 384 and 512 (its share of a chunk is 4 or 8 rows, that of
 // other products at most 5): their chains of loads, products and sums run side by side, and the peers get one message for eight
-// bytes (up product of H 512: 3.7 -> 2.5 thousand cycles).
+// bytes (up product of H 512: 3.7 -> 2.5 thousand cycles).  Two at a time where two or three are left, as in the down product (250
+// bytes sampled, 2 layers: H 256 4.48 -> 3.99 ms; 4 layers, H 512 7.82 -> 7.63; H 768 and 1024 +0.5 %, their rows come singly).
 // BYTES = false: int32 results; true: GELU[clip((acc >> shift) + bias)].
 template <int KW, bool BYTES>
 __device__ __forceinline__ void gen_product(GenSmem &s, GenState &g, const int8_t *vec, int rows, int group, uint32_t out_off, uint32_t bar_off, int *err,
@@ -204,6 +205,15 @@ __device__ __forceinline__ void gen_product(GenSmem &s, GenState &g, const int8_
                     st_async_b32(ptx::mapa_u32(at + 4 * (2 + half), dest), bar, half ? a[3] : a[2]);
                 }
                 i += 4;
+            } else if (!BYTES && per - i >= 2) {
+                int a[2];
+                gen_rows<KW, 2>(w + i * K, g.lane, x, a);
+                if (((row0 + i) & 1) == 0) {
+                    if (half == 0) st_async_v2(ptx::mapa_u32(at, dest), bar, (uint32_t)a[0], (uint32_t)a[1]);
+                } else {
+                    st_async_b32(ptx::mapa_u32(at + 4 * half, dest), bar, (uint32_t)(half ? a[1] : a[0]));
+                }
+                i += 2;
             } else {
                 int a[1];
                 gen_rows<KW, 1>(w + i * K, g.lane, x, a);
