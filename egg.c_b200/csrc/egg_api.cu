@@ -104,7 +104,7 @@ struct egg_ctx {
     int ov_inc = 5, ov_dec = 1;
     // tables
     int32_t *d_exp_lut = nullptr, *d_rope_lut = nullptr;
-    int2 *d_rope_t = nullptr;           // the same (cos, sin) pairs, [head_dim/2][seq_len]: consecutive tokens are consecutive in memory
+    int4 *d_rope_t = nullptr;           // the same values in the order of rope_entry()
     int8_t *d_act_lut = nullptr;
     // dataset
     uint8_t *d_data = nullptr;          // data_len tokens of tok_bytes bytes each
@@ -489,10 +489,12 @@ extern "C" int egg_ctx_create(const egg_config *cfg, int device, int wave_member
     std::vector<int32_t> exp_lut, rope;
     std::vector<int8_t> act_lut;
     host_tables(*cfg, c->SP, exp_lut, act_lut, rope);
-    const int hp = cfg->head_dim / 2;
-    std::vector<int2> rope_t((size_t)hp * SP);
+    std::vector<int4> rope_t((size_t)(SP + 31) / 32 * 32 * (HEAD_DIM / 4));
     for (int t = 0; t < SP; t++)
-        for (int i = 0; i < hp; i++) rope_t[(size_t)i * SP + t] = make_int2(rope[(size_t)t * cfg->head_dim + 2 * i], rope[(size_t)t * cfg->head_dim + 2 * i + 1]);
+        for (int q = 0; q < HEAD_DIM / 4; q++) {
+            const int32_t *v = &rope[(size_t)t * HEAD_DIM + 4 * q];
+            const_cast<int4 &>(rope_entry(rope_t.data(), t)[32 * q]) = make_int4(v[0], v[1], v[2], v[3]);
+        }
     // Muon-optimised matrices keep their overlays
     std::vector<uint8_t> active((size_t)c->SL.total, 0);
     for (const ParamDesc &d : c->params) {
@@ -559,7 +561,7 @@ extern "C" int egg_ctx_create(const egg_config *cfg, int device, int wave_member
     TRYC(cudaMemsetAsync(c->d_status, 0, sizeof(Status), c->stream)); TRYC(cudaMemsetAsync(c->d_changed, 0, (size_t)c->SL.total, c->stream));
     auto put = [&](void *d, const void *h, size_t n) { return cudaMemcpyAsync(d, h, n, cudaMemcpyHostToDevice, c->stream); };
     TRYC(put(c->d_exp_lut, exp_lut.data(), 256 * 4)); TRYC(put(c->d_act_lut, act_lut.data(), 256));
-    TRYC(put(c->d_rope_lut, rope.data(), rope.size() * 4)); TRYC(put(c->d_rope_t, rope_t.data(), rope_t.size() * sizeof(int2)));
+    TRYC(put(c->d_rope_lut, rope.data(), rope.size() * 4)); TRYC(put(c->d_rope_t, rope_t.data(), rope_t.size() * sizeof(int4)));
     TRYC(put(c->d_ov_active, active.data(), active.size())); TRYC(put(c->d_segs, segs.data(), c->nsegs * sizeof(NoiseSeg)));
 
     TRY(prepare_update(c));
@@ -843,7 +845,7 @@ static FusedParams base_fused(egg_ctx *c, int M, int K, int parts) {
     f.M = (M + 127) / 128 * 128; f.H = c->cfg.hidden_dim; f.K = K; f.parts = parts; f.seq_len = c->SP;
     f.nt = c->d_nt; f.nt_stride = c->nmap.stride; f.nt_c_off = -1;
     f.rank1_shift = c->cfg.fixed_point + c->cfg.sigma_shift;
-    f.rope_t = c->d_rope_t; f.head_dim = c->cfg.head_dim; f.rope_bit = c->cfg.rope_scale_bit;
+    f.rope_t = c->d_rope_t; f.rope_bit = c->cfg.rope_scale_bit;
     f.part_rows = c->R;
     f.err = c->d_err;
     return f;

@@ -233,12 +233,26 @@ __device__ __forceinline__ int att_div_small(int p0, int p1, int p2, uint32_t de
     return k + sg * ((r * sg) >> 31);
 }
 
+// Every byte -128 lifted to -127, the reference's clip: four instructions, where __vmaxs4 takes seven.  low is 0x80 in the bytes that
+// are 0x80: their sign is set and adding 0x7F to their other bits carries nothing into it.
+__host__ __device__ __forceinline__ uint32_t lift_min(uint32_t r) {
+    const uint32_t low = r & ~((r & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) & 0x80808080u;
+    return r + (low >> 7);
+}
+// acc + Σ |x| over four bytes, none of them -128: every byte times its sign, 0xFF or 0x01 (three instructions; __vabsss4 takes seven
+// before the sum)
+__device__ __forceinline__ int abs_sum4(uint32_t x, int acc) {
+    uint32_t neg;
+    asm("prmt.b32 %0, %1, 0, 0xba98;" : "=r"(neg) : "r"(x));          // each byte's sign, eight times
+    return __dp4a((int)x, (int)(neg | 0x01010101u), acc);
+}
+
 // [sat8(a), sat8(b), sat8(c), sat8(d)] as bytes 0..3 with the reference's clip to [-127, 127]
 __device__ __forceinline__ uint32_t pack_clip8(int a, int b, int c, int d) {
     uint32_t hi, r;
     asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, 0;" : "=r"(hi) : "r"(d), "r"(c));
     asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(b), "r"(a), "r"(hi));
-    return __vmaxs4(r, 0x81818181u);
+    return lift_min(r);
 }
 
 // (1/mn) * (1 + 2^-17) for mn = 1..127 (div_small's factor): the mean is the same for every lane of a row, so the

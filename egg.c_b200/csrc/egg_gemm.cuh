@@ -43,6 +43,12 @@ enum GemmEpi {
     EPI_NULL = 8,    // accumulators are dropped: the loop of TMA loads and tcgen05 MMAs alone (peak measurement)
 };
 
+// The rotation table for warps whose lanes are consecutive tokens: cos, sin | cos, sin of two neighbouring pairs of columns (a quad) of a
+// head, by blocks of 32 tokens, then quads, then tokens.  The quads of a token lie at compile-time distances, 32 entries apart: with
+// [pair][token] the addresses took as many instructions as the rotation.
+constexpr int HEAD_DIM = 64;            // egg_config_validate admits no other
+__host__ __device__ __forceinline__ const int4 *rope_entry(const int4 *table, int token) { return table + (token >> 5) * (32 * HEAD_DIM / 4) + (token & 31); }
+
 struct GemmParams {
     int M, N, K;
     // ---- row -> member mapping (evaluation epilogues) ----
@@ -66,7 +72,7 @@ struct GemmParams {
     const int8_t *act_lut;       // 256
     const int32_t *exp_lut;      // 256
     const int32_t *rope_lut;     // [seq_len][head_dim]
-    const int2 *rope_t;          // [head_dim/2][seq_len] (cos, sin): the same values, token index fastest
+    const int4 *rope_t;          // the same values, see rope_entry()
     int third;                   // EPI_QKV: N/3 (= hidden)
     int head_dim;
     int rope_bit;                // ROPE_SCALE_BIT
@@ -245,7 +251,7 @@ __device__ __forceinline__ void epilogue_rpl(const GemmParams &p, GemmSmem<BN> &
     const uint32_t ost_s = ptx::smem_u32(ost) + lane * 64;
     const uint32_t ost1_s = ptx::smem_u32(ost1) + lane * 64;
     const int8_t *dt = sm.d_tab[slot] + cbase;
-    const int2 *rope = p.rope_t + (rc - mem * p.seq_len);                                // column of this token position
+    const int4 *rope = rope_entry(p.rope_t, rc - mem * p.seq_len);                       // this token position
     constexpr bool do_rope = (EPI == EPI_QKV) && FORM;      // Q and K column tiles; V passes through
     const long long half_ulp = 1ll << (p.rope_bit - 1);
     int racc = 0, rmx = 0, rmn = 0;
@@ -256,12 +262,9 @@ __device__ __forceinline__ void epilogue_rpl(const GemmParams &p, GemmSmem<BN> &
         int4 cs[4];
         if (EPI == EPI_QKV && do_rope) {
             // the lanes of a warp are consecutive tokens of one member: every load below is one contiguous run
-            const int pair0 = fast_mod(n0 + cbase + 16 * c, p.fd_head) >> 1;
+            const int quad0 = ((n0 + cbase + 16 * c) & (HEAD_DIM - 1)) >> 2;
 #pragma unroll
-            for (int q4 = 0; q4 < 4; q4++) {
-                const int2 c0 = __ldg(rope + (int64_t)(pair0 + 2 * q4) * p.seq_len), c1 = __ldg(rope + (int64_t)(pair0 + 2 * q4 + 1) * p.seq_len);
-                cs[q4] = make_int4(c0.x, c0.y, c1.x, c1.y);
-            }
+            for (int q4 = 0; q4 < 4; q4++) cs[q4] = __ldg(rope + 32 * (quad0 + q4));
         }
         uint32_t *vc = v[c & 1];
         ptx::tmem_ld_wait16(vc);
@@ -315,7 +318,7 @@ __device__ __forceinline__ void epilogue_rpl(const GemmParams &p, GemmSmem<BN> &
             x3 = (int)vc[4 * q4 + 3] + ((xbs * an.w) >> p.rank1_shift);
             if (EPI == EPI_CLIP8) {
                 uint32_t w = ptx::pack_sat_s8(x0 >> p.out_shift, x1 >> p.out_shift, x2 >> p.out_shift, x3 >> p.out_shift);
-                w = __vmaxs4(w, 0x81818181u);                  // lift -128 to the reference's -127
+                w = lift_min(w);                               // lift -128 to the reference's -127
                 if (p.nt_d_off >= 0) racc = __dp4a((int)w, *reinterpret_cast<const int32_t *>(dt + col), racc);
                 outw[q4] = w;
             } else if (EPI == EPI_GELU) {
@@ -856,7 +859,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                             if (EPI == EPI_CLIP8) {
                                 // saturate to int8 and pack (two instructions), then lift -128 to the reference's -127
                                 uint32_t w = ptx::pack_sat_s8(v0 >> p.out_shift, v1 >> p.out_shift, v2 >> p.out_shift, v3 >> p.out_shift);
-                                w = __vmaxs4(w, 0x81818181u);
+                                w = lift_min(w);
                                 if (rok[i]) *reinterpret_cast<uint32_t *>(p.out8 + gofs) = w;
                             } else if (EPI == EPI_GELU) {
                                 const int2 bcw = *reinterpret_cast<const int2 *>(&sm.bc_tab[sl][sg][col]);

@@ -53,12 +53,13 @@ struct FusedParams {
     int rank1_shift, out_shift;
     int pow_t;                   // FUSED_RES: merged_shift(), filled by launch_gemm_fused
     int one;                     // 1 (filled by launch_gemm_fused): the multiplier of additions issued as multiply-adds
+    int unit[4];                 // 1 << 8i (filled by launch_gemm_fused): a dot product takes its selector from the parameters, not from a register
     const int8_t *bias;          // FUSED_RES: [H] or null
-    const int2 *rope_t;          // [head_dim/2][seq_len] (cos, sin)
-    int head_dim, rope_bit;
+    const int4 *rope_t;          // see rope_entry()
+    int rope_bit;
     int64_t part_rows;           // row distance between the parts in the output tensor map
     int *err;
-    FastDiv fd_head, fd_h, fd_seq;   // head_dim, H and seq_len as multiply-shift divisors (filled by launch_gemm_fused)
+    FastDiv fd_h, fd_seq;            // H and seq_len as multiply-shift divisors (filled by launch_gemm_fused)
     // FUSED_RES_LN: the mean-abs norm that follows the block (apply_standard_norm, mgpu.cu:646-678) and the row dots of
     // the projections after it, computed from the requantised row while it is still in shared memory
     int nt_w_m, nt_b_m;          // perturbed gain / bias tables (int16 [2][H]) in the noise table
@@ -119,8 +120,8 @@ struct FusedTabWords { int32_t a, b, d; };
 // One thread's share (4 columns) of the norm tables of a unit's member (FUSED_RES_LN).
 struct FusedLnWords { int2 w, b; int32_t d[3]; };
 
-// MERGE: both shifts of a residual projection as one (see pass 1)
-template <int BN, int MODE, bool MM, bool MERGE>
+// FORM: FUSED_RES: both shifts as one (see pass 1); FUSED_RES_LN: three row dots follow (else one)
+template <int BN, int MODE, bool MM, bool FORM>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                   const __grid_constant__ CUtensorMap tmap_o, const __grid_constant__ CUtensorMap tmap_r, const FusedParams p) {
@@ -133,6 +134,8 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     constexpr uint32_t STAGE_BYTES = GEMM_BM * GEMM_BK + BN * GEMM_BK;
     constexpr bool RES = (MODE != FUSED_QKV);   // residual + bias projections (O, MLP down)
     constexpr bool LN = (MODE == FUSED_RES_LN); // ... followed in the same epilogue by the next mean-abs norm
+    constexpr bool MERGE = (MODE == FUSED_RES) && FORM;
+    constexpr int NDOTS = LN ? (FORM ? 3 : 1) : 0;
 
     chain_next();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -285,7 +288,7 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             w.w = *reinterpret_cast<const int2 *>(reinterpret_cast<const int16_t *>(base + p.nt_w_m) + (mem & 1) * p.H + n);
             w.b = *reinterpret_cast<const int2 *>(reinterpret_cast<const int16_t *>(base + p.nt_b_m) + (mem & 1) * p.H + n);
 #pragma unroll
-            for (int q = 0; q < 3; q++) w.d[q] = q < p.ndots ? *reinterpret_cast<const int32_t *>(base + p.nt_dot[q] + n) : 0;
+            for (int q = 0; q < 3; q++) w.d[q] = q < NDOTS ? *reinterpret_cast<const int32_t *>(base + p.nt_dot[q] + n) : 0;
         };
         auto ln_store = [&](const FusedLnWords &w) {
             sm.ln_wb[tq][tn >> 2] = make_int4(w.w.x, w.w.y, w.b.x, w.b.y);
@@ -325,12 +328,14 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             if (LN && e < tab_items) ln_load(MM ? fast_div(m0 + 32 * tq, p.fd_seq) : mem, lnw);
             const uint32_t a32_s = ptx::smem_u32(&sm.a32[tb][qt][0]);
             const uint32_t bcs_s = ptx::smem_u32(&sm.bcs32[tb][qt][0]);
-            const bool do_rope = (MODE == FUSED_QKV) && part < 2;
-            const int2 *rope = p.rope_t + (r - mem * p.seq_len);           // column of this token position
+            // this token's entries of the rotation table: a warp's columns start at the same place in a head whatever the sub-tile is
+            const int4 *rope = rope_entry(p.rope_t, r - mem * p.seq_len) + 32 * (((cq * CW) & 63) >> 2);
 
             // ---------------- pass 1: values and row abs-max, written back to tensor memory ----------------
             float rmx = 0.0f;
             int imx = 0, imn = 0;
+            auto pass1 = [&](auto rope_part) {
+            constexpr bool ROPE = decltype(rope_part)::value;
             for (int j = 0; j < NT; j++) {
                 const uint32_t st = stc + (uint32_t)j;
                 const int slot = st % NS;
@@ -346,14 +351,10 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 #pragma unroll
                 for (int c = 0; c < NCH; c++) {
                     int4 cs[4];
-                    if (MODE == FUSED_QKV && do_rope) {
+                    if (ROPE) {
                         // the lanes of a warp are consecutive tokens of one member: every load below is one contiguous run
-                        const int pair0 = fast_mod(cofs + col0 + 16 * c, p.fd_head) >> 1;
 #pragma unroll
-                        for (int q4 = 0; q4 < 4; q4++) {
-                            const int2 c0 = __ldg(rope + (int64_t)(pair0 + 2 * q4) * p.seq_len), c1 = __ldg(rope + (int64_t)(pair0 + 2 * q4 + 1) * p.seq_len);
-                            cs[q4] = make_int4(c0.x, c0.y, c1.x, c1.y);
-                        }
+                        for (int q4 = 0; q4 < 4; q4++) cs[q4] = __ldg(rope + 32 * (4 * c + q4));
                     }
                     int4 rs4 = make_int4(0, 0, 0, 0);
                     if (RES) rs4 = ptx::lds_v4(box_s + (((uint32_t)c ^ swz) << 4));
@@ -386,17 +387,17 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                                 x2 = (((xbs * an.z + b4.z) >> p.rank1_shift) * p.one + (int)vc[4 * q4 + 2]) >> p.out_shift;
                                 x3 = (((xbs * an.w + b4.w) >> p.rank1_shift) * p.one + (int)vc[4 * q4 + 3]) >> p.out_shift;
                             }
-                            x0 = __dp4a(rs, 0x00000001, x0);
-                            x1 = __dp4a(rs, 0x00000100, x1);
-                            x2 = __dp4a(rs, 0x00010000, x2);
-                            x3 = __dp4a(rs, 0x01000000, x3);
+                            x0 = __dp4a(rs, p.unit[0], x0);
+                            x1 = __dp4a(rs, p.unit[1], x1);
+                            x2 = __dp4a(rs, p.unit[2], x2);
+                            x3 = __dp4a(rs, p.unit[3], x3);
                         } else {
                             x0 = ((xbs * an.x) >> p.rank1_shift) * p.one + (int)vc[4 * q4];
                             x1 = ((xbs * an.y) >> p.rank1_shift) * p.one + (int)vc[4 * q4 + 1];
                             x2 = ((xbs * an.z) >> p.rank1_shift) * p.one + (int)vc[4 * q4 + 2];
                             x3 = ((xbs * an.w) >> p.rank1_shift) * p.one + (int)vc[4 * q4 + 3];
                         }
-                        if (do_rope) {
+                        if (ROPE) {
                             // integer RoPE on adjacent (even, odd) columns (apply_rope_integer, mgpu.cu:624-644)
                             const int e0 = x0, o0 = x1, e1 = x2, o1 = x3;
                             x0 = ptx::shr64_lo(ptx::mad_wide(-o0, cs[q4].y, ptx::mad_wide(e0, cs[q4].x, half_ulp)), p.rope_bit);
@@ -418,6 +419,9 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 }
                 ptx::tmem_st_wait();
             }
+            };
+            if (MODE == FUSED_QKV && part < 2) pass1(std::integral_constant<bool, MODE == FUSED_QKV>());
+            else pass1(std::integral_constant<bool, false>());
             sm.rowpart[cq][row_in_tile] = RES ? __float_as_int(rmx) : max(imx, -imn);         // non-negative floats order like their bit patterns
             if (LN && e < tab_items) ln_store(lnw);
             ptx::named_bar_sync(2 + quarter, 128);            // the four column quarters of this lane quarter
@@ -467,7 +471,7 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                                                  aln_quant_f(val(vc[4 * q4 + 2]), scale), aln_quant_f(val(vc[4 * q4 + 3]), scale));
                     if (LN) {
 #pragma unroll
-                        for (int q4 = 0; q4 < 4; q4++) tot = __dp4a((int)__vabsss4(w[q4]), 0x01010101, tot);
+                        for (int q4 = 0; q4 < 4; q4++) tot = abs_sum4(w[q4], tot);
                     }
                     ptx::sts_v4(box_s + (((uint32_t)c ^ swz) << 4), make_int4((int)w[0], (int)w[1], (int)w[2], (int)w[3]));
                 }
@@ -506,7 +510,6 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 const uint32_t lwb_s = ptx::smem_u32(&sm.ln_wb[qt][0]), ld4_s = ptx::smem_u32(&sm.ln_d4[qt][0]);
                 int8_t *hrow = p.h_out + (int64_t)r * p.H + cofs;
                 int dot0 = 0, dot1 = 0, dot2 = 0;
-                auto norm = [&](auto dots) {           // three dots or one: asked once a unit, not per four columns (85.0 -> 83.3 ms of a generation)
                 for (int j = 0; j < NT; j++) {
                     const uint32_t box_s = ptx::smem_u32(sm.box[ew][j]) + row_ofs;
 #pragma unroll
@@ -532,19 +535,15 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                             const int y3 = __dp2a_lo(wb.w, 0x00000100, __float2int_rz(f3 * rinv));
                             yw[q4] = pack_clip8(y0, y1, y2, y3);
                             dot0 = __dp4a((int)yw[q4], d4.x, dot0);
-                            if (decltype(dots)::value ? decltype(dots)::value == 3 : p.ndots > 1) { dot1 = __dp4a((int)yw[q4], d4.y, dot1); dot2 = __dp4a((int)yw[q4], d4.z, dot2); }
+                            if (NDOTS == 3) { dot1 = __dp4a((int)yw[q4], d4.y, dot1); dot2 = __dp4a((int)yw[q4], d4.z, dot2); }
                         }
                         *reinterpret_cast<int4 *>(hrow + col) = make_int4((int)yw[0], (int)yw[1], (int)yw[2], (int)yw[3]);
                     }
                 }
-                };
-                if constexpr (MM) norm(std::integral_constant<int, 0>());          // (tiles that span members gain nothing, and small models pay for a second copy)
-                else if (p.ndots > 1) norm(std::integral_constant<int, 3>());
-                else norm(std::integral_constant<int, 1>());
                 // every warp (and both blocks of a pair) adds its columns' share: integer sums, any order
                 int32_t *xo = p.xb_out + (int64_t)r * p.xb_out_stride;
                 atomicAdd(xo, dot0);
-                if (p.ndots > 1) { atomicAdd(xo + 1, dot1); atomicAdd(xo + 2, dot2); }
+                if (NDOTS == 3) { atomicAdd(xo + 1, dot1); atomicAdd(xo + 2, dot2); }
                 __syncwarp();          // all lanes have read their boxes before lane 0 lets the next residual bytes in
             }
             if (RES && lane == 0 && nunit < num_units) {

@@ -31,6 +31,7 @@ static int set_attr_fused() {
     EGG_CUDA(cudaFuncSetAttribute(gemm_fused_kernel<BN, FUSED_RES, MM, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem_bytes<BN, MM>()));
     EGG_CUDA(cudaFuncSetAttribute(gemm_fused_kernel<BN, FUSED_RES, MM, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem_bytes<BN, MM>()));
     EGG_CUDA(cudaFuncSetAttribute(gemm_fused_kernel<BN, FUSED_RES_LN, MM, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem_bytes<BN, MM>()));
+    EGG_CUDA(cudaFuncSetAttribute(gemm_fused_kernel<BN, FUSED_RES_LN, MM, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem_bytes<BN, MM>()));
     return EGG_OK;
 }
 
@@ -160,10 +161,10 @@ int fused_cluster_size(int hidden) {
     return 0;
 }
 
-template <int BN, int MODE, bool MM, bool MERGE = false>
+template <int BN, int MODE, bool MM, bool FORM = false>
 static int launch_fused_one(cudaStream_t st, const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &to, const CUtensorMap &tr,
                             const FusedParams &p, int units, int num_sms) {
-    auto kern = gemm_fused_kernel<BN, MODE, MM, MERGE>;
+    auto kern = gemm_fused_kernel<BN, MODE, MM, FORM>;
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(GEMM_THREADS);
     cfg.dynamicSmemBytes = fused_smem_bytes<BN, MM>();
@@ -201,6 +202,7 @@ template <int BN, bool MM>
 static int launch_fused_mode(cudaStream_t st, int mode, const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &to, const CUtensorMap &tr,
                              const FusedParams &p, int units, int num_sms) {
     if (mode == FUSED_QKV) return launch_fused_one<BN, FUSED_QKV, MM>(st, ta, tb, to, tr, p, units, num_sms);
+    if (mode == FUSED_RES_LN && p.ndots == 3) return launch_fused_one<BN, FUSED_RES_LN, MM, true>(st, ta, tb, to, tr, p, units, num_sms);
     if (mode == FUSED_RES_LN) return launch_fused_one<BN, FUSED_RES_LN, MM>(st, ta, tb, to, tr, p, units, num_sms);
     if (p.pow_t) return launch_fused_one<BN, FUSED_RES, MM, true>(st, ta, tb, to, tr, p, units, num_sms);
     return launch_fused_one<BN, FUSED_RES, MM>(st, ta, tb, to, tr, p, units, num_sms);
@@ -229,9 +231,9 @@ int launch_gemm_fused(cudaStream_t st, int mode, const int8_t *A, const int8_t *
     const bool mm = p.seq_len % GEMM_BM != 0;        // a tile spans members: four table sets, see the kernel
     const int bn = (mm ? hl == 256 : hl % 256 == 0) ? 256 : 128;      // (128-column sub-tiles at H = 512 were measured: +30 % on MLP-down)
     p.fd_seq = make_fastdiv(p.seq_len);
-    p.fd_head = make_fastdiv(p.head_dim > 0 ? p.head_dim : 64);
     p.fd_h = make_fastdiv(p.H);
     p.one = 1;
+    for (int i = 0; i < 4; i++) p.unit[i] = 1 << (8 * i);
     p.pow_t = mode == FUSED_RES ? merged_shift(p.K, p.rank1_shift, p.out_shift) : 0;
     CUtensorMap ta, tb, to, tr;
     int rc;

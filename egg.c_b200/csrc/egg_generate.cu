@@ -309,7 +309,7 @@ __device__ __forceinline__ int gen_block_max(GenSmem &s, const GenState &g, int 
 // Four consecutive elements of the row per thread (threads beyond H / 4 carry zeros).
 // apply_standard_norm without noise (mgpu.cu:646-678, ns = 0): h = clip((x * w) / mean|x| + b); ends with h in place.
 __device__ __forceinline__ void gen_norm(GenSmem &s, const GenState &g, int x4, int w4, int b4, int H) {
-    int sum = __reduce_add_sync(0xFFFFFFFFu, __dp4a((int)__vabsss4((unsigned)x4), 0x01010101, 0));
+    int sum = __reduce_add_sync(0xFFFFFFFFu, abs_sum4((uint32_t)x4, 0));
     const bool in = g.tid < H / 4;
     if (g.lane == 0) s.red[0][g.warp] = sum;
     gen_bar();

@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? ROW_EMB_BLOCKS : 1) rowwise_k
                 w = ptx::pack_sat_s8(x[j][0], x[j][1], x[j][2], x[j][3]);            // |x| <= 127: the saturating pack is exact, two instructions
                 *reinterpret_cast<uint32_t *>(p.x_out + (int64_t)r * H + d) = w;
             }
-            tot = __dp4a((int)__vabsss4(w), 0x01010101, tot);    // sum of |x|, four at a time
+            tot = abs_sum4(w, tot);
         }
         // mean-abs norm with perturbed gain / bias (mgpu.cu:646-678): y = clip((x*w')/mn + b')
         tot = warp_sum(tot);

@@ -274,12 +274,9 @@ __device__ __forceinline__ float max3_abs(float a, float b, float c) {
     return d;
 }
 
-// a * b + c with a 32 x 32 -> 64-bit product (one instruction)
-__device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
-    long long d;
-    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
-    return d;
-}
+// a * b + c with a 32 x 32 -> 64-bit product: one instruction.  Left to the compiler: mad.wide.s32 written out became a product and a
+// 64-bit addition in two instructions (a rotated element 5.6 -> 3.5 instructions).
+__device__ __forceinline__ long long mad_wide(int a, int b, long long c) { return (long long)a * b + c; }
 // low 32 bits of (v >> sh) for 0 < sh < 32: exact whenever the shifted value fits 32 bits
 __device__ __forceinline__ int shr64_lo(long long v, int sh) {
     return (int)__funnelshift_r((unsigned)v, (unsigned)(v >> 32), sh);
