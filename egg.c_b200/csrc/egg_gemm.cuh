@@ -29,7 +29,6 @@ constexpr int GEMM_THREADS = 576;       // warp0 TMA, warp1 MMA, warps 2..17 epi
 constexpr int GEMM_EPI_THREADS = 512;
 constexpr int GEMM_EPI_WARPS = 16;
 constexpr int GEMM_MAX_SLOTS = 5;       // distinct population pairs a 128-row tile can touch (seq_len >= 16)
-constexpr int GEMM_RPL_SLOTS = 3;       // the same bound for the row-per-lane epilogues (seq_len a multiple of 32)
 
 enum GemmEpi {
     EPI_CLIP8 = 0,   // y = clip((acc + r1) >> out_shift)                       -> int8 (row-per-lane form with nt_d_off >= 0: Σ y·noise -> rowstat)
@@ -97,6 +96,15 @@ struct GemmParams {
     int pow_t;                   // EPI_GELU, EPI_LOGITS: merged_shift()
 };
 
+// What a row-per-lane epilogue warp reads of a tile: its own quarter of the columns, for the one member that its rows belong to.
+// Widened to int32, read as warp-uniform LDS.128.
+template <int BN>
+struct RplTables {
+    alignas(16) int32_t a32[BN / 4];        // A-noise of this projection
+    alignas(16) int32_t bcs32[BN / 4];      // (bias + bias-noise delta of the member's sign) << shift
+    alignas(16) int8_t d[BN / 4];           // B-noise of the next projection
+};
+
 template <int BN>
 struct GemmSmem {
     alignas(1024) uint8_t a[GEMM_STAGES][GEMM_BM * GEMM_BK];
@@ -122,14 +130,11 @@ struct GemmSmem {
             alignas(16) int8_t a_tab[GEMM_MAX_SLOTS][BN];       // A-noise of this projection per pair slot
             alignas(16) int16_t bc_tab[GEMM_MAX_SLOTS][2][BN];  // bias + bias-noise delta per pair slot and sign
         };
-        struct {                                            // row-per-lane epilogues: tables widened to int32, read as uniform LDS.128
-            alignas(16) int32_t a32[GEMM_RPL_SLOTS][BN];        // A-noise of this projection per pair slot
-            alignas(16) int32_t bcs32[GEMM_RPL_SLOTS][2][BN];   // (bias + bias-noise delta) << out_shift per pair slot and sign
-        } rpl;
+        RplTables<BN> rpl[GEMM_EPI_WARPS];                      // row-per-lane epilogues: each warp its own
         alignas(16) int32_t lg_a32[GEMM_MAX_SLOTS][BN];         // EPI_LOGITS: the A-noise alone, for every member length
     };
     alignas(16) int8_t d_tab[GEMM_MAX_SLOTS][BN];       // B-noise of the next projection (EPI_GELU)
-    alignas(16) int32_t rowpart[4][GEMM_BM];            // row-per-lane epilogues: per-row partial of each column quarter
+    alignas(16) int32_t rowpart[4][GEMM_BM];            // EPI_LOGITS: the row's maxima of the four column quarters
     alignas(16) int8_t act_lut[256];
     alignas(16) int32_t exp_lut[256];
     alignas(8) uint64_t full[GEMM_STAGES];
@@ -200,25 +205,12 @@ __device__ __forceinline__ bool tab_load(const GemmParams &p, int e, int m0, int
     return true;
 }
 
-template <int BN, int EPI, int RPL>
+template <int BN, int EPI>
 __device__ __forceinline__ void tab_store(const GemmParams &p, GemmSmem<BN> &sm, int e, const TabWords &w) {
     const int sl = e / (BN / 4), j = (e % (BN / 4)) * 4;
     if (EPI == EPI_LOGITS) *reinterpret_cast<int4 *>(&sm.lg_a32[sl][j]) = make_int4((int)(int8_t)w.a, (int)(int8_t)(w.a >> 8), (int)(int8_t)(w.a >> 16), w.a >> 24);
-    else if (RPL) *reinterpret_cast<int4 *>(&sm.rpl.a32[sl][j]) = make_int4((int)(int8_t)w.a, (int)(int8_t)(w.a >> 8), (int)(int8_t)(w.a >> 16), w.a >> 24);
     else *reinterpret_cast<int32_t *>(&sm.a_tab[sl][j]) = w.a;
-    if ((EPI == EPI_GELU || EPI == EPI_PRE32) && RPL) {
-        int vp[4], vn[4];
-        // GELU: shifted once more so that the sum joins the rank-1 product before its shift (see epilogue_rpl)
-        const int tsh = p.out_shift + ((EPI == EPI_GELU && GEMM_FMA_ADDS) ? p.rank1_shift : 0);
-#pragma unroll
-        for (int b = 0; b < 4; b++) {
-            const int bb = (int)(int8_t)(w.b >> (8 * b));
-            vp[b] = (bb + (int)(int8_t)(w.cp >> (8 * b))) << tsh;
-            vn[b] = (bb + (int)(int8_t)(w.cn >> (8 * b))) << tsh;
-        }
-        *reinterpret_cast<int4 *>(&sm.rpl.bcs32[sl][0][j]) = make_int4(vp[0], vp[1], vp[2], vp[3]);
-        *reinterpret_cast<int4 *>(&sm.rpl.bcs32[sl][1][j]) = make_int4(vn[0], vn[1], vn[2], vn[3]);
-    } else if (EPI == EPI_GELU || EPI == EPI_PRE32) {
+    if (EPI == EPI_GELU || EPI == EPI_PRE32) {
 #pragma unroll
         for (int b = 0; b < 4; b++) {
             const int bb = (int)(int8_t)(w.b >> (8 * b));
@@ -231,6 +223,35 @@ __device__ __forceinline__ void tab_store(const GemmParams &p, GemmSmem<BN> &sm,
     if (EPI == EPI_GELU || EPI == EPI_CLIP8) *reinterpret_cast<int32_t *>(&sm.d_tab[sl][j]) = w.d;
 }
 
+// The same for one warp of a row-per-lane epilogue: lanes below BN / 16 carry 4 of the warp's columns each, n the first of the lane's.
+template <int BN, int EPI>
+__device__ __forceinline__ void rpl_load(const GemmParams &p, int lane, int mem, int n, TabWords &w) {
+    if (lane >= BN / 16) return;
+    const int8_t *base = p.nt + (int64_t)(mem >> 1) * p.nt_stride;
+    w.a = *reinterpret_cast<const int32_t *>(base + p.nt_a_off + n);
+    w.b = 0; w.cp = 0; w.d = 0;
+    if (EPI == EPI_GELU || EPI == EPI_PRE32) {
+        if (p.bias) w.b = *reinterpret_cast<const int32_t *>(p.bias + n);
+        if (p.nt_c_off >= 0) w.cp = *reinterpret_cast<const int32_t *>(base + p.nt_c_off + (mem & 1) * p.N + n);
+    }
+    if (EPI == EPI_GELU || (EPI == EPI_CLIP8 && p.nt_d_off >= 0)) w.d = *reinterpret_cast<const int32_t *>(base + p.nt_d_off + n);
+}
+template <int BN, int EPI>
+__device__ __forceinline__ void rpl_store(const GemmParams &p, RplTables<BN> &t, int lane, const TabWords &w) {
+    if (lane >= BN / 16) return;
+    const int j = 4 * lane;
+    *reinterpret_cast<int4 *>(&t.a32[j]) = make_int4((int)(int8_t)w.a, (int)(int8_t)(w.a >> 8), (int)(int8_t)(w.a >> 16), w.a >> 24);
+    if (EPI == EPI_GELU || EPI == EPI_PRE32) {
+        int v[4];
+        // GELU: shifted once more so that the sum joins the rank-1 product before its shift (see epilogue_rpl)
+        const int tsh = p.out_shift + ((EPI == EPI_GELU && GEMM_FMA_ADDS) ? p.rank1_shift : 0);
+#pragma unroll
+        for (int b = 0; b < 4; b++) v[b] = ((int)(int8_t)(w.b >> (8 * b)) + (int)(int8_t)(w.cp >> (8 * b))) << tsh;
+        *reinterpret_cast<int4 *>(&t.bcs32[j]) = make_int4(v[0], v[1], v[2], v[3]);
+    }
+    if (EPI == EPI_GELU || EPI == EPI_CLIP8) *reinterpret_cast<int32_t *>(&t.d[j]) = w.d;
+}
+
 // ---- row-per-lane evaluation epilogues ----
 // Used when every warp's 32 accumulator rows belong to one population member (seq_len % 32 == 0): the rank-1 factor,
 // pair slot and sign are then per-lane scalars and the per-column tables are read at warp-uniform addresses, so the
@@ -238,19 +259,18 @@ __device__ __forceinline__ void tab_store(const GemmParams &p, GemmSmem<BN> &sm,
 // shuffles and about half the instructions of the transposed form.  TMEM loads are double-buffered.
 // FORM: q and k columns (EPI_QKV), both shifts as one (EPI_GELU with BN = 256)
 template <int BN, int EPI, bool FORM, bool RES_TMA>
-__device__ __forceinline__ void epilogue_rpl(const GemmParams &p, GemmSmem<BN> &sm, uint32_t taddr, int r, bool row_ok, int n0,
-                                             int cbase, int slot, int sgn, int32_t (*st)[20], int lane, int m0q, int xbs,
-                                             const int4 (&rs_pre)[BN / 4 / 16], const CUtensorMap *tmap_o, int32_t *ost, int32_t *ost1) {
+__device__ __forceinline__ int epilogue_rpl(const GemmParams &p, GemmSmem<BN> &sm, const RplTables<BN> &tab, uint32_t taddr, int r, bool row_ok, int n0,
+                                            int cbase, int lane, int m0q, int xbs, const int4 (&rs_pre)[BN / 4 / 16], const CUtensorMap *tmap_o,
+                                            int32_t *ost, int32_t *ost1) {
     constexpr int NCH = BN / 4 / 16;                       // 16-column chunks of this warp's quarter of the tile
     const int rc = row_ok ? r : (p.M - 1);
     const int mem = fast_div(rc, p.fd_seq);
     const uint32_t lut_base = ptx::smem_u32(&sm.lut32[0][lane]);
     const uint32_t lut_stride = (uint32_t)p.lut_stride;       // 128 bytes per table entry, read from the parameters
-    const uint32_t a32 = ptx::smem_u32(sm.rpl.a32[slot] + cbase);           // 32-bit shared addresses of this lane's tables
-    const uint32_t bcs = ptx::smem_u32(sm.rpl.bcs32[slot][sgn] + cbase);
+    const uint32_t a32 = ptx::smem_u32(tab.a32), bcs = ptx::smem_u32(tab.bcs32);           // 32-bit shared addresses
     const uint32_t ost_s = ptx::smem_u32(ost) + lane * 64;
     const uint32_t ost1_s = ptx::smem_u32(ost1) + lane * 64;
-    const int8_t *dt = sm.d_tab[slot] + cbase;
+    const int8_t *dt = tab.d;
     const int4 *rope = rope_entry(p.rope_t, rc - mem * p.seq_len);                       // this token position
     constexpr bool do_rope = (EPI == EPI_QKV) && FORM;      // Q and K column tiles; V passes through
     const long long half_ulp = 1ll << (p.rope_bit - 1);
@@ -421,9 +441,7 @@ __device__ __forceinline__ void epilogue_rpl(const GemmParams &p, GemmSmem<BN> &
         }
         __syncwarp();
     }
-    if (EPI == EPI_PRE32 || EPI == EPI_QKV) racc = max(rmx, -rmn);
-    // per-row partial of this column quarter; the quarters are combined after the end-of-tile barrier
-    sm.rowpart[cbase / (BN / 4)][m0q + lane - (m0q & ~(GEMM_BM - 1))] = racc;
+    return EPI == EPI_PRE32 || EPI == EPI_QKV ? max(rmx, -rmn) : racc;       // this column quarter's share of the row
 }
 
 // Logits of a vocabulary wider than one tile (mgpu.cu:969-983), row per lane, for every member length.  The cross-entropy
@@ -487,8 +505,8 @@ __device__ __forceinline__ int epilogue_logits(const GemmParams &p, GemmSmem<BN>
 // Σ exp-LUT and the target logit, and the warp of the first column quarter adds one loss term per row, reduced over
 // the warp (all its rows belong to one member) into a single atomic.
 template <int BN>
-__device__ __forceinline__ void epilogue_head_rpl(const GemmParams &p, GemmSmem<BN> &sm, uint32_t taddr, int r, bool row_ok, int cbase,
-                                                  int slot, int lane, int quarter, int row_in_tile, int xbs) {
+__device__ __forceinline__ void epilogue_head_rpl(const GemmParams &p, GemmSmem<BN> &sm, const RplTables<BN> &tab, uint32_t taddr, int r, bool row_ok, int cbase,
+                                                  int lane, int quarter, int row_in_tile, int xbs) {
     constexpr int NCH = BN / 4 / 16;
     int32_t(*hp)[4][GEMM_BM] = reinterpret_cast<int32_t(*)[4][GEMM_BM]>(&sm.stage[0][0][0]);    // [max | sum | target][quarter][row]
     const int cq = cbase / (BN / 4);
@@ -498,7 +516,7 @@ __device__ __forceinline__ void epilogue_head_rpl(const GemmParams &p, GemmSmem<
     const int64_t pair = (p.pop_base + mem) >> 1;
     const int64_t pos = p.use_same_data ? (p.start_idx % (p.data_len - p.tok_len)) : ((p.start_idx + pair * p.data_stride) % (p.data_len - p.tok_len));
     const int tgt_col = (int)p.dataset[pos + min(t, p.tok_len - 1) + 1] - cbase;                    // target column relative to this warp's quarter
-    const uint32_t a32 = ptx::smem_u32(sm.rpl.a32[slot] + cbase);
+    const uint32_t a32 = ptx::smem_u32(tab.a32);
     uint32_t v[2][16];
     int mx = INT_MIN, sum = 0, tg = 0;
 #pragma unroll 1
@@ -652,19 +670,89 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 if (ok) ptx::mma_commit(&sm.tmem_full[as]);
             }
         }
+    } else if constexpr (RPL && EPI != EPI_LOGITS) {
+        // ===================== epilogue, row per lane: 16 warps that do not wait for one another =====================
+        // A warp's rows belong to one member and its tables are its own, so that nothing has to be published to the block: a warp
+        // waits for the tile's products alone and its row results leave as atomics of its own.  (With tables of the block and two
+        // barriers a tile the warps moved in step, all of them in their loads or all of them in their arithmetic: MLP-up 6.85 -> 5.95 ms
+        // of an evaluation of 4096 members at H 512, 1.50 -> 1.29 at H 256, the head 0.41 -> 0.37.)
+        const int ew = warp - 2, quarter = warp & 3, cq = ew >> 2, cbase = cq * (BN / 4);      // lane quarter of tensor memory, column quarter of the tile
+        RplTables<BN> &tab = sm.rpl[ew];
+        // Residual bytes: with BN = 256 the warp's 32 rows x 64 columns arrive as one box through the copy engine, requested a tile
+        // ahead -- a lane loading its own row 16 bytes at a time costs 32 half-used sectors per instruction.
+        constexpr bool RES_TMA = (EPI == EPI_PRE32) && BN == 256;
+        uint32_t tcount = 0;
+        TabWords nxt = {0, 0, 0, 0, 0};
+        int pf_xb = 0;                              // the lane's rank-1 factor (raw sum of x b of its row)
+        int4 pf_rs0 = make_int4(0, 0, 0, 0);        // first chunk of residual bytes
+        auto prefetch = [&](int tile) {
+            const int tm_ = fast_div(tile, p.fd_tiles_n), rw = tm_ * GEMM_BM + quarter * 32, n0 = (tile - tm_ * tiles_n) * BN;
+            rpl_load<BN, EPI>(p, lane, fast_div(min(rw, p.M - 1), p.fd_seq), n0 + cbase + 4 * lane, nxt);
+            const int rc = min(rw + lane, p.M - 1);
+            pf_xb = p.xb[(int64_t)rc * p.xb_stride + ((EPI == EPI_QKV) ? fast_div(n0, p.fd_third) : 0)];
+            if (EPI == EPI_PRE32 && !RES_TMA) pf_rs0 = *reinterpret_cast<const int4 *>(p.resid + (int64_t)rc * p.N + n0 + cbase);
+            if (RES_TMA && lane == 0) {
+                ptx::mbar_arrive_expect_tx(&sm.rbar[ew], 32 * 64);
+                ptx::tma_load_2d(sm.ostage1[ew], &tmap_r, &sm.rbar[ew], n0 + cbase, rw);
+            }
+        };
+        if ((int)blockIdx.x < num_tiles) prefetch(blockIdx.x);
+        for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, tcount++) {
+            const int as = tcount & 1;
+            const int tm_ = fast_div(tile, p.fd_tiles_n), m0q = tm_ * GEMM_BM + quarter * 32, n0 = (tile - tm_ * tiles_n) * BN;
+            const int r = m0q + lane;
+            const bool row_ok = r < p.M;
+            __syncwarp();                           // every lane has read the previous tile's tables
+            rpl_store<BN, EPI>(p, tab, lane, nxt);
+            __syncwarp();
+            const int xbs = (fast_div(min(m0q, p.M - 1), p.fd_seq) & 1) ? -pf_xb : pf_xb;
+            int4 rs_l[BN / 4 / 16];
+            if (EPI == EPI_PRE32 && !RES_TMA) {
+                rs_l[0] = pf_rs0;
+#pragma unroll
+                for (int cc = 1; cc < BN / 4 / 16; cc++)      // used one chunk of arithmetic later each
+                    rs_l[cc] = *reinterpret_cast<const int4 *>(p.resid + (int64_t)min(r, p.M - 1) * p.N + n0 + cbase + 16 * cc);
+            }
+            const int ntile = tile + gridDim.x;
+            if (!RES_TMA && ntile < num_tiles) prefetch(ntile);          // in flight while this tile is computed
+            bool ok = ptx::mbar_wait(&sm.tmem_full[as], (tcount >> 1) & 1);
+            if (RES_TMA) ok = ok && ptx::mbar_wait(&sm.rbar[ew], tcount & 1);
+            if (!__all_sync(0xFFFFFFFFu, ok && !sm.abort_flag)) { gemm_fail(p, &sm.abort_flag, DEV_TIMEOUT_TMEM_FULL); break; }
+            ptx::tc_fence_after();
+            const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(as * BN + cbase);
+            if constexpr (EPI == EPI_HEAD) {
+                epilogue_head_rpl<BN>(p, sm, tab, taddr, r, row_ok, cbase, lane, quarter, quarter * 32 + lane, xbs);
+            } else {
+                int part;
+                if ((EPI == EPI_QKV && n0 < 2 * p.third) || (EPI == EPI_GELU && BN == 256 && p.pow_t))        // asked once a tile, not per four columns: 68.6 -> 68.0 ms
+                    // of a generation; not for the narrow tiles of small models, where two copies of the code take longer to fetch than they save
+                    part = epilogue_rpl<BN, EPI, true, false>(p, sm, tab, taddr, r, row_ok, n0, cbase, lane, m0q, xbs, rs_l, &tmap_o, sm.ostage0[ew], sm.ostage1[ew]);
+                else
+                    part = epilogue_rpl<BN, EPI, false, RES_TMA>(p, sm, tab, taddr, r, row_ok, n0, cbase, lane, m0q, xbs, rs_l, &tmap_o, sm.ostage0[ew], sm.ostage1[ew]);
+                if (row_ok) {
+                    if (EPI == EPI_GELU || (EPI == EPI_CLIP8 && p.nt_d_off >= 0)) atomicAdd(&p.rowstat[r], part);
+                    else if (EPI == EPI_PRE32) atomicMax(&p.rowstat[r], part);
+                    else if (EPI == EPI_QKV) atomicMax(&p.rowstat[(int64_t)r * 3 + fast_div(n0, p.fd_third)], part);
+                }
+            }
+            // release the accumulator stage
+            ptx::tc_fence_before();
+            __syncwarp();                           // (and every lane has read its residual bytes: the box may be refilled)
+            if (lane == 0) ptx::mbar_arrive(&sm.tmem_empty[as]);
+            if (RES_TMA && ntile < num_tiles) prefetch(ntile);
+        }
     } else {
         // ===================== epilogue (16 warps) =====================
         const int e = threadIdx.x - 64;            // 0..511
         const int ew = warp - 2;                   // 0..15
         const int quarter = warp & 3;              // TMEM lane quarter this warp may read
-        constexpr int NHALF = (EPI == EPI_HEAD && !RPL) ? 1 : 4;   // column parts per lane quarter; the transposed head keeps whole rows in one warp
+        constexpr int NHALF = EPI == EPI_HEAD ? 1 : 4;   // column parts per lane quarter; the transposed head keeps whole rows in one warp
         constexpr int COLS_PER = BN / NHALF;
         const int half = (NHALF == 4) ? (ew >> 2) : 0;     // which part of the tile's columns
         const bool active = (NHALF == 4) || ew < 4;
         const int row_in_tile = quarter * 32 + lane;
         uint32_t tcount = 0;
-        int pf_xb = 0;                              // row-per-lane form: values of the next tile, loaded a tile ahead
-        int4 pf_rs0 = make_int4(0, 0, 0, 0);
+        int pf_xb = 0;                              // EPI_LOGITS: the lane's rank-1 factor, loaded a tile ahead
         for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, tcount++) {
             const int as = tcount & 1;
             const uint32_t aph = (tcount >> 1) & 1;
@@ -684,7 +772,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 sgn = mem & 1;
                 if (tcount == 0) {
                     TabWords w;
-                    if (tab_load<BN, EPI>(p, e, m0, n0, w)) tab_store<BN, EPI, RPL>(p, sm, e, w);
+                    if (tab_load<BN, EPI>(p, e, m0, n0, w)) tab_store<BN, EPI>(p, sm, e, w);
                 }
             }
             // ---- per-row state of the 4 rows this lane owns after the transpose, and the loads that do not
@@ -718,34 +806,13 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     if (t >= p.tok_len) rok[i] = false;
                 }
             }
-            // row-per-lane form: the lane's rank-1 factor (raw Σ x·b of its row) and the first chunk of residual bytes
-            // were loaded during the previous tile (pf_*); only a block's first tile loads them here
             int xbs_l = 0;
-            int4 rs_l[BN / 4 / 16];
-            // The residual bytes of the residual projections: with BN = 256 every warp's 32 rows x 64 columns arrive as one
-            // box through the copy engine (requested a tile ahead, at the end of the previous tile's epilogue) -- a lane
-            // loading its own row 16 bytes at a time costs 32 half-used sectors per instruction (12 ms per generation).
-            constexpr bool RES_TMA = (EPI == EPI_PRE32) && RPL && BN == 256;
-            if (RES_TMA && tcount == 0 && lane == 0) {
-                ptx::mbar_arrive_expect_tx(&sm.rbar[ew], 32 * 64);
-                ptx::tma_load_2d(sm.ostage1[ew], &tmap_r, &sm.rbar[ew], n0 + cbase, m0 + quarter * 32);
-            }
-            if (RPL && active) {
-                const int rc = row_ok ? r : (p.M - 1);
-                if (tcount == 0) {
-                    pf_xb = p.xb[(int64_t)rc * p.xb_stride + ((EPI == EPI_QKV) ? fast_div(n0, p.fd_third) : 0)];
-                    if (EPI == EPI_PRE32 && !RES_TMA) pf_rs0 = *reinterpret_cast<const int4 *>(p.resid + (int64_t)rc * p.N + n0 + cbase);
-                }
+            if (EPI == EPI_LOGITS) {
+                if (tcount == 0) pf_xb = p.xb[(int64_t)(row_ok ? r : (p.M - 1)) * p.xb_stride];
                 xbs_l = sgn ? -pf_xb : pf_xb;
-                if (EPI == EPI_PRE32 && !RES_TMA) {
-                    rs_l[0] = pf_rs0;
-#pragma unroll
-                    for (int cc = 1; cc < BN / 4 / 16; cc++)      // used one chunk of arithmetic later each
-                        rs_l[cc] = *reinterpret_cast<const int4 *>(p.resid + (int64_t)rc * p.N + n0 + cbase + 16 * cc);
-                }
             }
             int32_t rs_pre[COLS_PER / 16][4];        // residual bytes of every chunk (EPI_PRE32)
-            if (EPI == EPI_PRE32 && active && !RPL) {
+            if (EPI == EPI_PRE32 && active) {
 #pragma unroll
                 for (int cc = 0; cc < COLS_PER / 16; cc++)
 #pragma unroll
@@ -769,11 +836,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 if (ntile < num_tiles) {
                     const int ntm = fast_div(ntile, p.fd_tiles_n), nm0 = ntm * GEMM_BM, nn0 = (ntile - ntm * tiles_n) * BN;
                     have_nxt = tab_load<BN, EPI>(p, e, nm0, nn0, nxt);
-                    if (RPL && active) {
-                        const int nr = nm0 + row_in_tile, nrc = nr < p.M ? nr : (p.M - 1);
-                        pf_xb = p.xb[(int64_t)nrc * p.xb_stride + ((EPI == EPI_QKV) ? fast_div(nn0, p.fd_third) : 0)];
-                        if (EPI == EPI_PRE32 && !RES_TMA) pf_rs0 = *reinterpret_cast<const int4 *>(p.resid + (int64_t)nrc * p.N + nn0 + half * COLS_PER);
-                    }
+                    if (EPI == EPI_LOGITS) pf_xb = p.xb[(int64_t)min(nm0 + row_in_tile, p.M - 1) * p.xb_stride];
                 }
             }
 
@@ -781,33 +844,9 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 
             if (!active) {
                 // nothing to compute; still takes part in the barrier protocol below
-            } else if (RPL && EPI == EPI_HEAD) {
-                epilogue_head_rpl<BN>(p, sm, taddr, r, row_ok, cbase, slot, lane, quarter, row_in_tile, xbs_l);
             } else if constexpr (EPI == EPI_LOGITS) {
                 sm.rowpart[half][row_in_tile] =
                     epilogue_logits<BN>(p, sm, taddr, n0, cbase, slot, lane, m0 + quarter * 32, xbs_l, &tmap_o, sm.ostage0[ew]);
-            } else if (RPL) {
-                if (RES_TMA) {
-                    if (lane == 0 && !ptx::mbar_wait(&sm.rbar[ew], tcount & 1)) gemm_fail(p, &sm.abort_flag, DEV_TIMEOUT_FULL);
-                    __syncwarp();
-                }
-                if ((EPI == EPI_QKV && n0 < 2 * p.third) || (EPI == EPI_GELU && BN == 256 && p.pow_t))        // asked once a tile, not per four columns: 68.6 -> 68.0 ms
-                    // of a generation; not for the narrow tiles of small models, where two copies of the code take longer to fetch than they save
-                    epilogue_rpl<BN, EPI, true, false>(p, sm, taddr, r, row_ok, n0, cbase, slot, sgn, sm.stage[ew], lane, m0 + quarter * 32, xbs_l, rs_l,
-                                                       &tmap_o, sm.ostage0[ew], sm.ostage1[ew]);
-                else
-                    epilogue_rpl<BN, EPI, false, RES_TMA>(p, sm, taddr, r, row_ok, n0, cbase, slot, sgn, sm.stage[ew], lane, m0 + quarter * 32, xbs_l,
-                                                          rs_l, &tmap_o, sm.ostage0[ew], sm.ostage1[ew]);
-                if (RES_TMA) {
-                    // every lane has read its residual bytes: the box may be refilled for the block's next tile
-                    __syncwarp();
-                    const int ntile = tile + gridDim.x;
-                    if (lane == 0 && ntile < num_tiles) {
-                        const int ntm = fast_div(ntile, p.fd_tiles_n);
-                        ptx::mbar_arrive_expect_tx(&sm.rbar[ew], 32 * 64);
-                        ptx::tma_load_2d(sm.ostage1[ew], &tmap_r, &sm.rbar[ew], (ntile - ntm * tiles_n) * BN + cbase, ntm * GEMM_BM + quarter * 32);
-                    }
-                }
             } else if (EPI <= EPI_LOGITS) {
                 // ---------------- evaluation epilogues ----------------
                 // Accumulators leave TMEM one row per lane; they are transposed through shared memory so
@@ -963,16 +1002,10 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             if (lane == 0) ptx::mbar_arrive(&sm.tmem_empty[as]);
             // tables are rewritten at the top of the next tile: everybody must be done reading them
             ptx::named_bar_sync(1, GEMM_EPI_THREADS);
-            if (RPL && EPI != EPI_HEAD && half == 0 && row_ok) {
-                // one atomic per row and tile instead of one per column quarter
-                const int a0 = sm.rowpart[0][row_in_tile], a1 = sm.rowpart[1][row_in_tile], a2 = sm.rowpart[2][row_in_tile],
-                          a3 = sm.rowpart[3][row_in_tile];
-                if (EPI == EPI_GELU || (EPI == EPI_CLIP8 && p.nt_d_off >= 0)) atomicAdd(&p.rowstat[r], a0 + a1 + a2 + a3);
-                else if (EPI == EPI_LOGITS) *reinterpret_cast<int4 *>(p.rowstat + (int64_t)r * (p.N >> 6) + (n0 >> 6)) = make_int4(a0, a1, a2, a3);
-                else if (EPI == EPI_PRE32) atomicMax(&p.rowstat[r], max(max(a0, a1), max(a2, a3)));
-                else if (EPI == EPI_QKV) atomicMax(&p.rowstat[(int64_t)r * 3 + fast_div(n0, p.fd_third)], max(max(a0, a1), max(a2, a3)));
-            }
-            if (EPI <= EPI_LOGITS && have_nxt) tab_store<BN, EPI, RPL>(p, sm, e, nxt);   // published by the next tile's barrier
+            if (EPI == EPI_LOGITS && half == 0 && row_ok)
+                *reinterpret_cast<int4 *>(p.rowstat + (int64_t)r * (p.N >> 6) + (n0 >> 6)) =
+                    make_int4(sm.rowpart[0][row_in_tile], sm.rowpart[1][row_in_tile], sm.rowpart[2][row_in_tile], sm.rowpart[3][row_in_tile]);
+            if (EPI <= EPI_LOGITS && have_nxt) tab_store<BN, EPI>(p, sm, e, nxt);   // published by the next tile's barrier
         }
     }
 

@@ -287,7 +287,7 @@ int launch_gemm(cudaStream_t st, int epi, const int8_t *A, const int8_t *B, cons
     if (epi <= EPI_LOGITS) {
         int max_slots = ((GEMM_BM - 1) / p.seq_len) / 2 + 2;
         const bool rpl = p.seq_len % 32 == 0 && p.rpl >= 0 && epi != EPI_LOGITS;
-        if (max_slots > (rpl ? GEMM_RPL_SLOTS : GEMM_MAX_SLOTS)) { set_error("seq_len %d too small for the epilogue tables", p.seq_len); return EGG_E_INVALID; }
+        if (!rpl && max_slots > GEMM_MAX_SLOTS) { set_error("seq_len %d too small for the epilogue tables", p.seq_len); return EGG_E_INVALID; }
     }
     if (epi == EPI_VOTE && p.k_splits > 1) {
         // every split must own at least one k-block: the kernel cuts ceil(num_kb / k_splits) blocks per split
