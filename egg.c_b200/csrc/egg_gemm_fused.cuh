@@ -74,7 +74,6 @@ constexpr int FUSED_MAX_H = 512;
 template <int BN, bool MM>
 struct FusedSmem {
     static constexpr int NS = 512 / BN;                 // TMEM slots = most sub-tiles a unit can have
-    static constexpr int Q = MM ? 4 : 1;                // table sets: one per lane quarter, or one
     static constexpr int WIDE = (MM && BN == 256) ? 256 : FUSED_MAX_H;      // most columns of a block
     static constexpr int NB = WIDE / BN;                // boxes per warp
     static constexpr int BOX = 32 * (BN / 4);           // bytes of one warp's int8 box: 32 rows x BN/4 columns
@@ -82,16 +81,15 @@ struct FusedSmem {
     alignas(1024) uint8_t b[GEMM_STAGES][BN * GEMM_BK];
     // per epilogue warp and sub-tile: residual bytes in (FUSED_RES), requantised bytes out
     alignas(1024) uint8_t box[GEMM_EPI_WARPS][NB][BOX];
-    alignas(16) int32_t a32[2][Q][WIDE];            // A-noise of the unit (double-buffered across units)
-    alignas(16) int32_t bcs32[2][Q][WIDE];          // (bias + bias-noise delta of the member's sign) << out_shift
-    alignas(16) int32_t rowpart[4][GEMM_BM];            // per-row abs-max of each column quarter
+    // Tables of a unit, widened to int32: the A-noise of a column quarter's columns and, for the residual projections, (bias +
+    // bias-noise delta of the member's sign) << shift behind it.  One per warp; where those do not fit (residual projections whose tiles
+    // belong to one member) one per column quarter, double-buffered across units.
+    static constexpr int TC = WIDE / 4;                 // columns of a quarter
+    alignas(16) int32_t tab[GEMM_EPI_WARPS * TC * (MM ? 2 : 1)];
+    alignas(16) int32_t rowpart[2][4][GEMM_BM];         // per-row abs-max of each column quarter (double-buffered across units)
     alignas(16) int32_t peer_max[2][GEMM_BM];           // per-row abs-max of the peer block's columns (written by the peer)
     alignas(16) uint16_t rowsum[4][GEMM_BM];            // FUSED_RES_LN: per-row Σ|x| of each column quarter (<= 127 * 128 columns)
     alignas(16) int32_t peer_sum[2][GEMM_BM];           // ... and of the peer block's columns
-    // FUSED_RES_LN, per group of 4 columns: the member's perturbed gains and biases {w0 w1 | w2 w3 | b0 b1 | b2 b3} (int16
-    // pairs), and the B-noise of the following projections {dot 0 | dot 1 | dot 2 | -} (four int8 each): one 16-byte read each
-    alignas(16) int4 ln_wb[Q][WIDE / 4];
-    alignas(16) int4 ln_d4[Q][WIDE / 4];
     alignas(8) uint64_t xbar[2];                        // arrival of the peer's maxima, one barrier per unit parity
     uint64_t xbar2[2];                                  // arrival of the peer's sums
     alignas(8) uint64_t full[GEMM_STAGES];
@@ -117,8 +115,6 @@ __device__ __forceinline__ void fused_wait(uint64_t *bar, uint32_t parity, volat
 
 // Words of the next unit's tables, loaded a unit ahead.
 struct FusedTabWords { int32_t a, b, d; };
-// One thread's share (4 columns) of the norm tables of a unit's member (FUSED_RES_LN).
-struct FusedLnWords { int2 w, b; int32_t d[3]; };
 
 // FORM: FUSED_RES: both shifts as one (see pass 1); FUSED_RES_LN: three row dots follow (else one)
 template <int BN, int MODE, bool MM, bool FORM>
@@ -231,14 +227,16 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         }
     } else {
         // ===================== epilogue (16 warps) =====================
-        const int e = threadIdx.x - 64;            // 0..511
         const int ew = warp - 2;                   // 0..15
         const int quarter = warp & 3;              // TMEM lane quarter this warp may read
         const int cq = ew >> 2;                    // column quarter of every sub-tile
         const int row_in_tile = quarter * 32 + lane;
-        const int tab_items = (HL >> 2) * Smem::Q;  // one item = 4 consecutive columns of this block's share (of one lane quarter's tables)
-        const int tq = MM ? e / (HL >> 2) : 0, tn = (MM ? e - tq * (HL >> 2) : e) << 2;        // this thread's item: table set, first column
-        const int qt = MM ? quarter : 0;           // table set of this warp's rows
+        // A warp meets the four warps of its rows (maxima, sums) and, where the tables are not its own, the four of its columns.
+        // Table items are 4 consecutive columns, one a lane.
+        constexpr bool OWN = MM || (MODE == FUSED_QKV && BN == 128);      // tables of the warp's own
+        const bool tab_mine = lane < NT * (CW / 4) && (OWN || quarter == 0);
+        const int tn = lane / (CW / 4) * BN + cq * CW + lane % (CW / 4) * 4;       // first column of this lane's item in the block's share
+        auto table = [&](int buf) { return sm.tab + (OWN ? ew * (RES ? 2 : 1) : 2 * (4 * buf + cq)) * Smem::TC; };
         const long long half_ulp = 1ll << (p.rope_bit - 1);
         // shared address of this lane's row inside a box, and the XOR that swizzles its 16-byte pieces (64-byte swizzle
         // for 64-byte rows; 32-byte rows are stored densely)
@@ -248,12 +246,11 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         int ucount = 0;
         int pf_xb = 0;
         FusedTabWords nxt = {0, 0, 0};
-        bool have_nxt = false;
 
-        auto tab_load = [&](int unit, FusedTabWords &w) -> bool {
-            if (e >= tab_items) return false;
+        auto tab_load = [&](int unit, FusedTabWords &w) {
+            if (!tab_mine) return;
             const int mt = unit / p.parts, part = unit - mt * p.parts;
-            const int mem = fast_div(mt * GEMM_BM + 32 * tq, p.fd_seq);
+            const int mem = fast_div(mt * GEMM_BM + (MM ? 32 * quarter : 0), p.fd_seq);
             const int8_t *base = p.nt + (int64_t)(mem >> 1) * p.nt_stride;
             const int n = cofs + tn;
             w.a = *reinterpret_cast<const int32_t *>(base + p.nt_a_off + part * p.H + n);
@@ -262,16 +259,17 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 if (p.bias) w.b = *reinterpret_cast<const int32_t *>(p.bias + n);
                 if (p.nt_c_off >= 0) w.d = *reinterpret_cast<const int32_t *>(base + p.nt_c_off + (mem & 1) * p.H + n);
             }
-            return true;
         };
         auto tab_store = [&](int buf, const FusedTabWords &w) {
-            *reinterpret_cast<int4 *>(&sm.a32[buf][tq][tn]) = make_int4((int)(int8_t)w.a, (int)(int8_t)(w.a >> 8), (int)(int8_t)(w.a >> 16), w.a >> 24);
+            if (!tab_mine) return;
+            int32_t *t = table(buf) + 4 * lane;
+            *reinterpret_cast<int4 *>(t) = make_int4((int)(int8_t)w.a, (int)(int8_t)(w.a >> 8), (int)(int8_t)(w.a >> 16), w.a >> 24);
             if (RES) {
                 int v[4];
 #pragma unroll
                 for (int b = 0; b < 4; b++)      // pre-shifted so that the sum joins the rank-1 product before its shift
                     v[b] = ((int)(int8_t)(w.b >> (8 * b)) + (int)(int8_t)(w.d >> (8 * b))) << (p.out_shift + p.rank1_shift);
-                *reinterpret_cast<int4 *>(&sm.bcs32[buf][tq][tn]) = make_int4(v[0], v[1], v[2], v[3]);
+                *reinterpret_cast<int4 *>(t + Smem::TC) = make_int4(v[0], v[1], v[2], v[3]);
             }
         };
         auto resid_request = [&](int unit) {      // lane 0: residual boxes of a unit, one per sub-tile
@@ -280,19 +278,6 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 ptx::mbar_arrive_expect_tx(&sm.rbar[ew][j], 32 * CW);
                 ptx::tma_load_2d(sm.box[ew][j], &tmap_r, &sm.rbar[ew][j], cofs + j * BN + cq * CW, m0 + quarter * 32);
             }
-        };
-
-        auto ln_load = [&](int mem, FusedLnWords &w) {      // threads e < tab_items: gains, biases and dot vectors of 4 columns
-            const int8_t *base = p.nt + (int64_t)(mem >> 1) * p.nt_stride;
-            const int n = cofs + tn;
-            w.w = *reinterpret_cast<const int2 *>(reinterpret_cast<const int16_t *>(base + p.nt_w_m) + (mem & 1) * p.H + n);
-            w.b = *reinterpret_cast<const int2 *>(reinterpret_cast<const int16_t *>(base + p.nt_b_m) + (mem & 1) * p.H + n);
-#pragma unroll
-            for (int q = 0; q < 3; q++) w.d[q] = q < NDOTS ? *reinterpret_cast<const int32_t *>(base + p.nt_dot[q] + n) : 0;
-        };
-        auto ln_store = [&](const FusedLnWords &w) {
-            sm.ln_wb[tq][tn >> 2] = make_int4(w.w.x, w.w.y, w.b.x, w.b.y);
-            sm.ln_d4[tq][tn >> 2] = make_int4(w.d[0], w.d[1], w.d[2], 0);
         };
 
         const uint32_t peer_max_s = p.cl > 1 ? ptx::mapa_u32(ptx::smem_u32(&sm.peer_max[0][0]), (uint32_t)(crank ^ 1)) : 0u;
@@ -307,27 +292,26 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             const int sgn = mem & 1;
             const int tb = ucount & 1;
             if (ucount == 0) {
-                FusedTabWords w;
-                if (tab_load(unit, w)) tab_store(0, w);
+                tab_load(unit, nxt);
+                if (!OWN) tab_store(0, nxt);
                 pf_xb = p.xb[(int64_t)r * p.xb_stride + part];
                 if (RES && lane == 0) resid_request(unit);
             }
-            // tables of this unit are published; everybody has left the previous unit
-            ptx::named_bar_sync(1, GEMM_EPI_THREADS);
+            if (OWN) {
+                __syncwarp();              // every lane has left the previous unit
+                tab_store(0, nxt);
+                __syncwarp();
+            } else {
+                ptx::named_bar_sync(6 + cq, 128);          // tables of this unit are published; the group has left the previous unit
+            }
             const int xbs = sgn ? -pf_xb : pf_xb;
             const int nunit = unit + unit_step;
-            have_nxt = false;
             if (nunit < num_units) {
-                have_nxt = tab_load(nunit, nxt);
+                tab_load(nunit, nxt);
                 const int nmt = nunit / p.parts;
                 pf_xb = p.xb[(int64_t)(nmt * GEMM_BM + row_in_tile) * p.xb_stride + (nunit - nmt * p.parts)];
             }
-            // the norm tables of this unit's member: requested now, stored after pass 1 (nobody reads the previous unit's
-            // any more, and this unit's readers come after a 512-thread barrier)
-            FusedLnWords lnw;
-            if (LN && e < tab_items) ln_load(MM ? fast_div(m0 + 32 * tq, p.fd_seq) : mem, lnw);
-            const uint32_t a32_s = ptx::smem_u32(&sm.a32[tb][qt][0]);
-            const uint32_t bcs_s = ptx::smem_u32(&sm.bcs32[tb][qt][0]);
+            const uint32_t tab_s = ptx::smem_u32(table(tb));
             // this token's entries of the rotation table: a warp's columns start at the same place in a head whatever the sub-tile is
             const int4 *rope = rope_entry(p.rope_t, r - mem * p.seq_len) + 32 * (((cq * CW) & 63) >> 2);
 
@@ -345,7 +329,7 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 __syncwarp();                           // lanes leave the waits at different times; the TMEM accesses are warp-wide
                 ptx::tc_fence_after();
                 const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(slot * BN + cq * CW);
-                const int col0 = j * BN + cq * CW;                     // column inside this block's share of this warp's first element
+                const uint32_t a32_s = tab_s + (uint32_t)(4 * j * CW), bcs_s = a32_s + 4 * Smem::TC;
                 uint32_t v[2][16];
                 ptx::tmem_ld16(taddr, v[0]);
 #pragma unroll
@@ -366,7 +350,7 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                     }
 #pragma unroll
                     for (int q4 = 0; q4 < 4; q4++) {
-                        const int col = col0 + 16 * c + 4 * q4;
+                        const int col = 16 * c + 4 * q4;
                         const int4 an = ptx::lds_v4(a32_s + 4 * col);
                         int x0, x1, x2, x3;
                         if (RES) {
@@ -422,11 +406,10 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             };
             if (MODE == FUSED_QKV && part < 2) pass1(std::integral_constant<bool, MODE == FUSED_QKV>());
             else pass1(std::integral_constant<bool, false>());
-            sm.rowpart[cq][row_in_tile] = RES ? __float_as_int(rmx) : max(imx, -imn);         // non-negative floats order like their bit patterns
-            if (LN && e < tab_items) ln_store(lnw);
+            sm.rowpart[tb][cq][row_in_tile] = RES ? __float_as_int(rmx) : max(imx, -imn);         // non-negative floats order like their bit patterns
             ptx::named_bar_sync(2 + quarter, 128);            // the four column quarters of this lane quarter
-            int row_max = max(max(sm.rowpart[0][row_in_tile], sm.rowpart[1][row_in_tile]),
-                              max(sm.rowpart[2][row_in_tile], sm.rowpart[3][row_in_tile]));
+            int row_max = max(max(sm.rowpart[tb][0][row_in_tile], sm.rowpart[tb][1][row_in_tile]),
+                              max(sm.rowpart[tb][2][row_in_tile], sm.rowpart[tb][3][row_in_tile]));
             if (p.cl > 1) {
                 // the other half of the row lives in the peer block: its first column quarter writes the maximum of its
                 // columns into this block's peer_max and arrives (release, cluster scope) on this block's barrier, and
@@ -491,7 +474,7 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 // y = clip((x * w') / mean|x| + b'), and the dots of y with the B-noise of the projections that read it.  The
                 // row's bytes are still in this lane's boxes; TMEM has been handed back, so the next unit's MMAs run meanwhile.
                 sm.rowsum[cq][row_in_tile] = (uint16_t)tot;
-                ptx::named_bar_sync(1, GEMM_EPI_THREADS);        // sums and norm tables of this unit are published
+                ptx::named_bar_sync(2 + quarter, 128);           // the sums of the four column quarters
                 int total = (int)sm.rowsum[0][row_in_tile] + (int)sm.rowsum[1][row_in_tile] + (int)sm.rowsum[2][row_in_tile] + (int)sm.rowsum[3][row_in_tile];
                 if (p.cl > 1) {      // the peer block's half of the row: same exchange as for the maxima
                     if (cq == 0) {
@@ -507,43 +490,76 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 int mn = fast_div(total, p.fd_h);
                 if (!mn) mn = 1;
                 const float rinv = c_rinv_up.v[mn & 127];        // mn <= 127: a mean of absolute values of int8
-                const uint32_t lwb_s = ptx::smem_u32(&sm.ln_wb[qt][0]), ld4_s = ptx::smem_u32(&sm.ln_d4[qt][0]);
-                int8_t *hrow = p.h_out + (int64_t)r * p.H + cofs;
-                int dot0 = 0, dot1 = 0, dot2 = 0;
-                for (int j = 0; j < NT; j++) {
-                    const uint32_t box_s = ptx::smem_u32(sm.box[ew][j]) + row_ofs;
+                // From here a lane has 16 columns of several rows instead of a row: their gains, biases and noise are loaded once a
+                // sub-tile, and a store covers whole rows of the box.  (A row a lane: four uniform 16-byte table reads per 16
+                // columns, and stores of 16 bytes to 32 rows each; together they took the shared-memory port a seventh of the time.)
+                constexpr int CPR = CW / 16, RPI = 32 / CPR;           // 16-byte pieces of a box row; rows of one step
+                const int pc = lane % CPR, rr = lane / CPR;
+                const int8_t *base = p.nt + (int64_t)(mem >> 1) * p.nt_stride;
+                const int16_t *gain = reinterpret_cast<const int16_t *>(base + p.nt_w_m) + sgn * p.H + cofs, *shift = reinterpret_cast<const int16_t *>(base + p.nt_b_m) + sgn * p.H + cofs;
+                int8_t *hrow = p.h_out + (int64_t)(m0 + quarter * 32 + rr) * p.H + cofs;
+                int dot[CPR][NDOTS > 0 ? NDOTS : 1];
 #pragma unroll
-                    for (int c = 0; c < NCH; c++) {
-                        const int4 xw = ptx::lds_v4(box_s + (((uint32_t)c ^ swz) << 4));
-                        const int col = j * BN + cq * CW + 16 * c;
+                for (int it = 0; it < CPR; it++)
+#pragma unroll
+                    for (int q = 0; q < NDOTS; q++) dot[it][q] = 0;
+                for (int j = 0; j < NT; j++) {
+                    const uint32_t box_s = ptx::smem_u32(sm.box[ew][j]);
+                    const int col = j * BN + cq * CW + 16 * pc;
+                    int w[8], b[8], d[NDOTS > 0 ? NDOTS : 1][4];
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const int4 wv = *reinterpret_cast<const int4 *>(gain + col + 8 * h), bv = *reinterpret_cast<const int4 *>(shift + col + 8 * h);
+                        w[4 * h] = wv.x; w[4 * h + 1] = wv.y; w[4 * h + 2] = wv.z; w[4 * h + 3] = wv.w;
+                        b[4 * h] = bv.x; b[4 * h + 1] = bv.y; b[4 * h + 2] = bv.z; b[4 * h + 3] = bv.w;
+                    }
+#pragma unroll
+                    for (int q = 0; q < NDOTS; q++) {
+                        const int4 dv = *reinterpret_cast<const int4 *>(base + p.nt_dot[q] + cofs + col);
+                        d[q][0] = dv.x; d[q][1] = dv.y; d[q][2] = dv.z; d[q][3] = dv.w;
+                    }
+#pragma unroll
+                    for (int it = 0; it < CPR; it++) {
+                        const int row = it * RPI + rr;
+                        const float ri = __shfl_sync(0xFFFFFFFFu, rinv, row);
+                        const int4 xw = ptx::lds_v4(box_s + (uint32_t)row * CW + (((uint32_t)pc ^ (BN == 256 ? (uint32_t)((row >> 1) & 3) : 0u)) << 4));
                         uint32_t yw[4];
 #pragma unroll
                         for (int q4 = 0; q4 < 4; q4++) {
                             const int xv = q4 == 0 ? xw.x : (q4 == 1 ? xw.y : (q4 == 2 ? xw.z : xw.w));
-                            const uint32_t grp = (uint32_t)(col >> 2) + (uint32_t)q4;          // group of 4 columns
-                            const int4 wb = ptx::lds_v4(lwb_s + 16u * grp), d4 = ptx::lds_v4(ld4_s + 16u * grp);
                             // x_i * w_i without widening either: a two-term dot product of the int16 pair with the word whose
                             // other byte is masked to zero, started from the bit pattern of 1.5 * 2^23 (i2f_small's addend);
                             // "+ b_i" the same way against a constant 1
-                            const float f0 = __int_as_float(__dp2a_lo(wb.x, xv & 0x000000FF, kMagicBits)) - kMagic;
-                            const float f1 = __int_as_float(__dp2a_lo(wb.x, xv & 0x0000FF00, kMagicBits)) - kMagic;
-                            const float f2 = __int_as_float(__dp2a_hi(wb.y, xv & 0x00FF0000, kMagicBits)) - kMagic;
-                            const float f3 = __int_as_float(__dp2a_hi(wb.y, xv & (int)0xFF000000, kMagicBits)) - kMagic;
-                            const int y0 = __dp2a_lo(wb.z, 0x00000001, __float2int_rz(f0 * rinv));
-                            const int y1 = __dp2a_lo(wb.z, 0x00000100, __float2int_rz(f1 * rinv));
-                            const int y2 = __dp2a_lo(wb.w, 0x00000001, __float2int_rz(f2 * rinv));
-                            const int y3 = __dp2a_lo(wb.w, 0x00000100, __float2int_rz(f3 * rinv));
+                            const float f0 = __int_as_float(__dp2a_lo(w[2 * q4], xv & 0x000000FF, kMagicBits)) - kMagic;
+                            const float f1 = __int_as_float(__dp2a_lo(w[2 * q4], xv & 0x0000FF00, kMagicBits)) - kMagic;
+                            const float f2 = __int_as_float(__dp2a_hi(w[2 * q4 + 1], xv & 0x00FF0000, kMagicBits)) - kMagic;
+                            const float f3 = __int_as_float(__dp2a_hi(w[2 * q4 + 1], xv & (int)0xFF000000, kMagicBits)) - kMagic;
+                            const int y0 = __dp2a_lo(b[2 * q4], p.unit[0], __float2int_rz(f0 * ri));
+                            const int y1 = __dp2a_lo(b[2 * q4], p.unit[1], __float2int_rz(f1 * ri));
+                            const int y2 = __dp2a_lo(b[2 * q4 + 1], p.unit[0], __float2int_rz(f2 * ri));
+                            const int y3 = __dp2a_lo(b[2 * q4 + 1], p.unit[1], __float2int_rz(f3 * ri));
                             yw[q4] = pack_clip8(y0, y1, y2, y3);
-                            dot0 = __dp4a((int)yw[q4], d4.x, dot0);
-                            if (NDOTS == 3) { dot1 = __dp4a((int)yw[q4], d4.y, dot1); dot2 = __dp4a((int)yw[q4], d4.z, dot2); }
+#pragma unroll
+                            for (int q = 0; q < NDOTS; q++) dot[it][q] = __dp4a((int)yw[q4], d[q][q4], dot[it][q]);
                         }
-                        *reinterpret_cast<int4 *>(hrow + col) = make_int4((int)yw[0], (int)yw[1], (int)yw[2], (int)yw[3]);
+                        *reinterpret_cast<int4 *>(hrow + (int64_t)(it * RPI) * p.H + col) = make_int4((int)yw[0], (int)yw[1], (int)yw[2], (int)yw[3]);
                     }
                 }
-                // every warp (and both blocks of a pair) adds its columns' share: integer sums, any order
-                int32_t *xo = p.xb_out + (int64_t)r * p.xb_out_stride;
-                atomicAdd(xo, dot0);
-                if (NDOTS == 3) { atomicAdd(xo + 1, dot1); atomicAdd(xo + 2, dot2); }
+                // the pieces of a row are neighbouring lanes: each keeps half of its rows and hands the others on, until lane pc of a
+                // row group holds the whole sum of row pc * RPI + rr
+#pragma unroll
+                for (int q = 0; q < NDOTS; q++) {
+                    if (CPR == 4) {
+                        const bool up = pc & 2;
+                        const int o0 = __shfl_xor_sync(0xFFFFFFFFu, up ? dot[0][q] : dot[2 % CPR][q], 2), o1 = __shfl_xor_sync(0xFFFFFFFFu, up ? dot[1][q] : dot[3 % CPR][q], 2);
+                        dot[0][q] = (up ? dot[2 % CPR][q] : dot[0][q]) + o0;
+                        dot[1][q] = (up ? dot[3 % CPR][q] : dot[1][q]) + o1;
+                    }
+                    const bool odd = pc & 1;
+                    const int o = __shfl_xor_sync(0xFFFFFFFFu, odd ? dot[0][q] : dot[1][q], 1);
+                    // every warp (and both blocks of a pair) adds its columns' share: integer sums, any order
+                    atomicAdd(p.xb_out + (int64_t)(m0 + quarter * 32 + pc * RPI + rr) * p.xb_out_stride + q, (odd ? dot[1][q] : dot[0][q]) + o);
+                }
                 __syncwarp();          // all lanes have read their boxes before lane 0 lets the next residual bytes in
             }
             if (RES && lane == 0 && nunit < num_units) {
@@ -551,7 +567,7 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 ptx::tma_store_wait_read<0>();
                 resid_request(nunit);
             }
-            if (have_nxt) tab_store(tb ^ 1, nxt);      // published by the next unit's barrier
+            if (!OWN && nunit < num_units) tab_store(tb ^ 1, nxt);      // published by the next unit's barrier
         }
         if (lane == 0) ptx::tma_store_wait_all<0>();     // boxes still being copied out must land before the block retires
         if (sm.abort_flag) {   // draining after a timeout: residual boxes may still be in flight towards this block
