@@ -39,9 +39,10 @@ enum FusedMode { FUSED_QKV = 0, FUSED_RES = 1, FUSED_RES_LN = 2 };
 
 struct FusedParams {
     int M, H, K;                 // rows (multiple of 128), width of one part, contraction
-    int cl;                      // thread blocks that share a unit (1 or 2, = the cluster size of the launch): each owns
+    int cl;                      // thread blocks that share a unit's columns (1 or 2): each owns
                                  // H/cl <= 512 columns of the unit's rows and the row maxima are exchanged through the
                                  // peer's shared memory
+    int pair;                    // pairs of blocks form 256 rows together (chosen by launch_gemm_fused)
     int parts;                   // 3 (q, k, v: B is [3H][K]) or 1
     int seq_len;                 // rows of one member: multiple of 32
     const int8_t *nt;            // per-pair noise table of this wave
@@ -71,14 +72,15 @@ struct FusedParams {
 
 constexpr int FUSED_MAX_H = 512;
 
-template <int BN, bool MM>
+template <int BN, bool MM, int CG>
 struct FusedSmem {
+    static constexpr int ST = CG == 2 ? 4 : GEMM_STAGES;        // ring stages: half of B in each block of a pair leaves room for a fourth
     static constexpr int NS = 512 / BN;                 // TMEM slots = most sub-tiles a unit can have
     static constexpr int WIDE = (MM && BN == 256) ? 256 : FUSED_MAX_H;      // most columns of a block
     static constexpr int NB = WIDE / BN;                // boxes per warp
     static constexpr int BOX = 32 * (BN / 4);           // bytes of one warp's int8 box: 32 rows x BN/4 columns
-    alignas(1024) uint8_t a[GEMM_STAGES][GEMM_BM * GEMM_BK];
-    alignas(1024) uint8_t b[GEMM_STAGES][BN * GEMM_BK];
+    alignas(1024) uint8_t a[ST][GEMM_BM * GEMM_BK];
+    alignas(1024) uint8_t b[ST][BN / CG * GEMM_BK];
     // per epilogue warp and sub-tile: residual bytes in (FUSED_RES), requantised bytes out
     alignas(1024) uint8_t box[GEMM_EPI_WARPS][NB][BOX];
     // Tables of a unit, widened to int32: the A-noise of a column quarter's columns and, for the residual projections, (bias +
@@ -92,8 +94,8 @@ struct FusedSmem {
     alignas(16) int32_t peer_sum[2][GEMM_BM];           // ... and of the peer block's columns
     alignas(8) uint64_t xbar[2];                        // arrival of the peer's maxima, one barrier per unit parity
     uint64_t xbar2[2];                                  // arrival of the peer's sums
-    alignas(8) uint64_t full[GEMM_STAGES];
-    uint64_t empty[GEMM_STAGES];
+    alignas(8) uint64_t full[ST];
+    uint64_t empty[ST];
     uint64_t tmem_full[NS];
     uint64_t tmem_empty[NS];
     uint64_t rbar[GEMM_EPI_WARPS][NB];                  // arrival of a residual box
@@ -117,17 +119,18 @@ __device__ __forceinline__ void fused_wait(uint64_t *bar, uint32_t parity, volat
 struct FusedTabWords { int32_t a, b, d; };
 
 // FORM: FUSED_RES: both shifts as one (see pass 1); FUSED_RES_LN: three row dots follow (else one)
-template <int BN, int MODE, bool MM, bool FORM>
+template <int BN, int MODE, bool MM, bool FORM, int CG>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                   const __grid_constant__ CUtensorMap tmap_o, const __grid_constant__ CUtensorMap tmap_r, const FusedParams p) {
     extern __shared__ uint8_t smem_raw[];
-    using Smem = FusedSmem<BN, MM>;
+    using Smem = FusedSmem<BN, MM, CG>;
     Smem &sm = *reinterpret_cast<Smem *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     constexpr int NS = Smem::NS;
     constexpr int CW = BN / 4;                  // columns of a sub-tile that one epilogue warp owns
     constexpr int NCH = CW / 16;                // 16-column chunks per warp and sub-tile
-    constexpr uint32_t STAGE_BYTES = GEMM_BM * GEMM_BK + BN * GEMM_BK;
+    constexpr int ST = Smem::ST;
+    constexpr uint32_t STAGE_BYTES = GEMM_BM * GEMM_BK + BN / CG * GEMM_BK;      // of one block
     constexpr bool RES = (MODE != FUSED_QKV);   // residual + bias projections (O, MLP down)
     constexpr bool LN = (MODE == FUSED_RES_LN); // ... followed in the same epilogue by the next mean-abs norm
     constexpr bool MERGE = (MODE == FUSED_RES) && FORM;
@@ -135,18 +138,23 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 
     chain_next();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int crank = (int)blockIdx.x % p.cl;                       // rank in the cluster (clusters are consecutive blocks)
+    // Clusters are consecutive blocks.  CG == 2: ranks that differ in the last bit are a pair, two row tiles of the same columns.
+    const int rank = (int)blockIdx.x % (p.cl * CG), crank = rank / CG, prow = rank % CG;       // share of the columns, row tile of the pair
+    const int peer = rank ^ CG;                                     // the block with the other share of this block's rows
     const int H0 = p.cl > 1 ? (p.H / 128 + 1) / 2 * 128 : p.H;      // columns of a part that the first block owns: half, rounded up to 128
     const int HL = crank ? p.H - H0 : H0;                           // ... that this block owns
     const int cofs = crank ? H0 : 0;                                // first of them
-    const int first_unit = (int)blockIdx.x / p.cl, unit_step = (int)gridDim.x / p.cl;      // both blocks of a pair walk the same units
+    const int first_unit = (int)blockIdx.x / (p.cl * CG), unit_step = (int)gridDim.x / (p.cl * CG);      // the blocks of a cluster walk the same units
     const int NT = HL / BN;                                         // sub-tiles per unit, 1..NS
-    const int num_units = (p.M / GEMM_BM) * p.parts;
+    const int tiles_m = p.M / GEMM_BM;
+    const int num_units = (tiles_m + CG - 1) / CG * p.parts;
+    // row tile of a unit: an odd last one is formed by both blocks of its pair, and the second keeps it to itself
+    auto row_tile = [&](int u) { return CG == 2 ? min(u * 2 + prow, tiles_m - 1) : u; };
     const int num_kb = (p.K + GEMM_BK - 1) / GEMM_BK;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < GEMM_STAGES; s++) { ptx::mbar_init(&sm.full[s], 1); ptx::mbar_init(&sm.empty[s], 1); }
-        for (int a = 0; a < NS; a++) { ptx::mbar_init(&sm.tmem_full[a], 1); ptx::mbar_init(&sm.tmem_empty[a], GEMM_EPI_WARPS); }
+        for (int s = 0; s < ST; s++) { ptx::mbar_init(&sm.full[s], 1); ptx::mbar_init(&sm.empty[s], 1); }
+        for (int a = 0; a < NS; a++) { ptx::mbar_init(&sm.tmem_full[a], 1); ptx::mbar_init(&sm.tmem_empty[a], CG * GEMM_EPI_WARPS); }
         for (int w = 0; w < GEMM_EPI_WARPS; w++)
             for (int a = 0; a < Smem::NB; a++) ptx::mbar_init(&sm.rbar[w][a], 1);
         ptx::mbar_init(&sm.xbar[0], GEMM_EPI_THREADS / 4);       // the peer's first column quarter: one arrival per row
@@ -157,13 +165,16 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         ptx::fence_barrier_init();
     }
     if (warp == 1) {
-        ptx::tmem_alloc(&sm.tmem_base, 512);
-        ptx::tmem_relinquish();
+        if (CG == 2) ptx::tmem_alloc_pair(&sm.tmem_base, 512);
+        else {
+            ptx::tmem_alloc(&sm.tmem_base, 512);
+            ptx::tmem_relinquish();
+        }
     }
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
-    if (p.cl > 1) ptx::cluster_sync_all();          // the peer's barriers exist before anything arrives on them
+    if (p.cl * CG > 1) ptx::cluster_sync_all();     // the peers' barriers exist before anything arrives on them
     chain_wait();
     const uint32_t tmem_base = sm.tmem_base;
 
@@ -173,19 +184,26 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             ptx::prefetch_tmap(&tmap_a);
             ptx::prefetch_tmap(&tmap_b);
             uint32_t it = 0;
+            const uint32_t full_s = CG == 2 ? ptx::mapa_u32(ptx::smem_u32(sm.full), (uint32_t)rank & ~1u) : 0u;      // of the even block
             for (int unit = first_unit; unit < num_units && !sm.abort_flag; unit += unit_step) {
                 const int mt = unit / p.parts, part = unit - mt * p.parts;
-                const int m0 = mt * GEMM_BM;
+                const int m0 = row_tile(mt) * GEMM_BM;
                 for (int j = 0; j < NT; j++) {
-                    const int n0 = part * p.H + cofs + j * BN;
+                    const int n0 = part * p.H + cofs + j * BN + prow * (BN / CG);
                     for (int kb = 0; kb < num_kb; kb++, it++) {
-                        const int s = it % GEMM_STAGES;
-                        const uint32_t ph = (it / GEMM_STAGES) & 1;
+                        const int s = it % ST;
+                        const uint32_t ph = (it / ST) & 1;
                         fused_wait(&sm.empty[s], ph ^ 1, &sm.abort_flag, p.err, DEV_TIMEOUT_EMPTY);
                         if (sm.abort_flag) break;
-                        ptx::mbar_arrive_expect_tx(&sm.full[s], STAGE_BYTES);
-                        ptx::tma_load_2d(sm.a[s], &tmap_a, &sm.full[s], kb * GEMM_BK, m0);
-                        ptx::tma_load_2d(sm.b[s], &tmap_b, &sm.full[s], kb * GEMM_BK, n0);
+                        if (CG == 2) {
+                            if (prow == 0) ptx::mbar_arrive_expect_tx(&sm.full[s], 2 * STAGE_BYTES);       // both blocks' bytes
+                            ptx::tma_load_2d_pair(sm.a[s], &tmap_a, full_s + 8 * s, kb * GEMM_BK, m0);
+                            ptx::tma_load_2d_pair(sm.b[s], &tmap_b, full_s + 8 * s, kb * GEMM_BK, n0);
+                        } else {
+                            ptx::mbar_arrive_expect_tx(&sm.full[s], STAGE_BYTES);
+                            ptx::tma_load_2d(sm.a[s], &tmap_a, &sm.full[s], kb * GEMM_BK, m0);
+                            ptx::tma_load_2d(sm.b[s], &tmap_b, &sm.full[s], kb * GEMM_BK, n0);
+                        }
                     }
                     if (sm.abort_flag) break;
                 }
@@ -197,31 +215,42 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         }
     } else if (warp == 1) {
         // ===================== MMA issuer =====================
-        if (ptx::elect_one()) {
-            constexpr uint32_t idesc = ptx::make_idesc_i8(GEMM_BM, BN);
+        if (prow == 0 && ptx::elect_one()) {
+            constexpr uint32_t idesc = ptx::make_idesc_i8(CG * GEMM_BM, BN);
             uint32_t it = 0, stc = 0;
             for (int unit = first_unit; unit < num_units && !sm.abort_flag; unit += unit_step) {
                 for (int j = 0; j < NT && !sm.abort_flag; j++, stc++) {
                     const int slot = stc % NS;
                     const uint32_t sph = (stc / NS) & 1;
-                    fused_wait(&sm.tmem_empty[slot], sph ^ 1, &sm.abort_flag, p.err, DEV_TIMEOUT_TMEM_EMPTY);
+                    if (CG == 2) {       // both blocks' epilogues arrive
+                        if (!sm.abort_flag && !ptx::mbar_wait_cluster(&sm.tmem_empty[slot], sph ^ 1, 1000000000ull)) {
+                            sm.abort_flag = 1;
+                            if (p.err) atomicCAS(p.err, 0, DEV_TIMEOUT_TMEM_EMPTY);
+                        }
+                    } else {
+                        fused_wait(&sm.tmem_empty[slot], sph ^ 1, &sm.abort_flag, p.err, DEV_TIMEOUT_TMEM_EMPTY);
+                    }
                     if (sm.abort_flag) break;
                     ptx::tc_fence_after();
                     const uint32_t d_tmem = tmem_base + (uint32_t)(slot * BN);
                     for (int kb = 0; kb < num_kb; kb++, it++) {
-                        const int s = it % GEMM_STAGES;
-                        const uint32_t ph = (it / GEMM_STAGES) & 1;
+                        const int s = it % ST;
+                        const uint32_t ph = (it / ST) & 1;
                         fused_wait(&sm.full[s], ph, &sm.abort_flag, p.err, DEV_TIMEOUT_FULL);
                         if (sm.abort_flag) break;
                         ptx::tc_fence_after();
                         const uint64_t da = ptx::make_smem_desc_sw128(ptx::smem_u32(sm.a[s]));
                         const uint64_t db = ptx::make_smem_desc_sw128(ptx::smem_u32(sm.b[s]));
 #pragma unroll
-                        for (int k = 0; k < GEMM_BK / 32; k++)
-                            ptx::mma_i8(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
-                        ptx::mma_commit(&sm.empty[s]);
+                        for (int k = 0; k < GEMM_BK / 32; k++) {
+                            if (CG == 2) ptx::mma_i8_pair(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                            else ptx::mma_i8(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                        }
+                        if (CG == 2) ptx::mma_commit_pair(&sm.empty[s], (uint32_t)rank); else ptx::mma_commit(&sm.empty[s]);
                     }
-                    if (!sm.abort_flag) ptx::mma_commit(&sm.tmem_full[slot]);
+                    if (!sm.abort_flag) {
+                        if (CG == 2) ptx::mma_commit_pair(&sm.tmem_full[slot], (uint32_t)rank); else ptx::mma_commit(&sm.tmem_full[slot]);
+                    }
                 }
             }
         }
@@ -250,7 +279,7 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         auto tab_load = [&](int unit, FusedTabWords &w) {
             if (!tab_mine) return;
             const int mt = unit / p.parts, part = unit - mt * p.parts;
-            const int mem = fast_div(mt * GEMM_BM + (MM ? 32 * quarter : 0), p.fd_seq);
+            const int mem = fast_div(row_tile(mt) * GEMM_BM + (MM ? 32 * quarter : 0), p.fd_seq);
             const int8_t *base = p.nt + (int64_t)(mem >> 1) * p.nt_stride;
             const int n = cofs + tn;
             w.a = *reinterpret_cast<const int32_t *>(base + p.nt_a_off + part * p.H + n);
@@ -273,20 +302,22 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             }
         };
         auto resid_request = [&](int unit) {      // lane 0: residual boxes of a unit, one per sub-tile
-            const int m0 = (unit / p.parts) * GEMM_BM;
+            const int m0 = row_tile(unit / p.parts) * GEMM_BM;
             for (int j = 0; j < NT; j++) {
                 ptx::mbar_arrive_expect_tx(&sm.rbar[ew][j], 32 * CW);
                 ptx::tma_load_2d(sm.box[ew][j], &tmap_r, &sm.rbar[ew][j], cofs + j * BN + cq * CW, m0 + quarter * 32);
             }
         };
 
-        const uint32_t peer_max_s = p.cl > 1 ? ptx::mapa_u32(ptx::smem_u32(&sm.peer_max[0][0]), (uint32_t)(crank ^ 1)) : 0u;
-        const uint32_t peer_bar_s = p.cl > 1 ? ptx::mapa_u32(ptx::smem_u32(&sm.xbar[0]), (uint32_t)(crank ^ 1)) : 0u;
-        const uint32_t peer_sum_s = (LN && p.cl > 1) ? ptx::mapa_u32(ptx::smem_u32(&sm.peer_sum[0][0]), (uint32_t)(crank ^ 1)) : 0u;
-        const uint32_t peer_bar2_s = (LN && p.cl > 1) ? ptx::mapa_u32(ptx::smem_u32(&sm.xbar2[0]), (uint32_t)(crank ^ 1)) : 0u;
+        const uint32_t tmem_empty_s = CG == 2 ? ptx::mapa_u32(ptx::smem_u32(sm.tmem_empty), (uint32_t)rank & ~1u) : 0u;      // of the even block
+        const uint32_t peer_max_s = p.cl > 1 ? ptx::mapa_u32(ptx::smem_u32(&sm.peer_max[0][0]), (uint32_t)peer) : 0u;
+        const uint32_t peer_bar_s = p.cl > 1 ? ptx::mapa_u32(ptx::smem_u32(&sm.xbar[0]), (uint32_t)peer) : 0u;
+        const uint32_t peer_sum_s = (LN && p.cl > 1) ? ptx::mapa_u32(ptx::smem_u32(&sm.peer_sum[0][0]), (uint32_t)peer) : 0u;
+        const uint32_t peer_bar2_s = (LN && p.cl > 1) ? ptx::mapa_u32(ptx::smem_u32(&sm.xbar2[0]), (uint32_t)peer) : 0u;
         for (int unit = first_unit; unit < num_units; unit += unit_step, ucount++) {
             const int mt = unit / p.parts, part = unit - mt * p.parts;
-            const int m0 = mt * GEMM_BM;
+            const int m0 = row_tile(mt) * GEMM_BM;
+            const bool live = CG == 1 || 2 * mt + prow < tiles_m;
             const int r = m0 + row_in_tile;
             const int mem = fast_div(m0 + (MM ? quarter * 32 : 0), p.fd_seq);       // member of this warp's rows
             const int sgn = mem & 1;
@@ -309,7 +340,7 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             if (nunit < num_units) {
                 tab_load(nunit, nxt);
                 const int nmt = nunit / p.parts;
-                pf_xb = p.xb[(int64_t)(nmt * GEMM_BM + row_in_tile) * p.xb_stride + (nunit - nmt * p.parts)];
+                pf_xb = p.xb[(int64_t)(row_tile(nmt) * GEMM_BM + row_in_tile) * p.xb_stride + (nunit - nmt * p.parts)];
             }
             const uint32_t tab_s = ptx::smem_u32(table(tb));
             // this token's entries of the rotation table: a warp's columns start at the same place in a head whatever the sub-tile is
@@ -463,8 +494,8 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 ptx::fence_proxy_async();
                 __syncwarp();
                 if (lane == 0) {
-                    ptx::mbar_arrive(&sm.tmem_empty[slot]);
-                    ptx::tma_store_2d(&tmap_o, sm.box[ew][j], cofs + j * BN + cq * CW, (int)(part * p.part_rows) + m0 + quarter * 32);
+                    if (CG == 2) ptx::mbar_arrive_cluster(tmem_empty_s + 8 * slot); else ptx::mbar_arrive(&sm.tmem_empty[slot]);
+                    if (live) ptx::tma_store_2d(&tmap_o, sm.box[ew][j], cofs + j * BN + cq * CW, (int)(part * p.part_rows) + m0 + quarter * 32);
                     ptx::tma_store_commit();
                 }
             }
@@ -542,7 +573,7 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 #pragma unroll
                             for (int q = 0; q < NDOTS; q++) dot[it][q] = __dp4a((int)yw[q4], d[q][q4], dot[it][q]);
                         }
-                        *reinterpret_cast<int4 *>(hrow + (int64_t)(it * RPI) * p.H + col) = make_int4((int)yw[0], (int)yw[1], (int)yw[2], (int)yw[3]);
+                        if (live) *reinterpret_cast<int4 *>(hrow + (int64_t)(it * RPI) * p.H + col) = make_int4((int)yw[0], (int)yw[1], (int)yw[2], (int)yw[3]);
                     }
                 }
                 // the pieces of a row are neighbouring lanes: each keeps half of its rows and hands the others on, until lane pc of a
@@ -558,7 +589,7 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                     const bool odd = pc & 1;
                     const int o = __shfl_xor_sync(0xFFFFFFFFu, odd ? dot[0][q] : dot[1][q], 1);
                     // every warp (and both blocks of a pair) adds its columns' share: integer sums, any order
-                    atomicAdd(p.xb_out + (int64_t)(m0 + quarter * 32 + pc * RPI + rr) * p.xb_out_stride + q, (odd ? dot[1][q] : dot[0][q]) + o);
+                    if (live) atomicAdd(p.xb_out + (int64_t)(m0 + quarter * 32 + pc * RPI + rr) * p.xb_out_stride + q, (odd ? dot[1][q] : dot[0][q]) + o);
                 }
                 __syncwarp();          // all lanes have read their boxes before lane 0 lets the next residual bytes in
             }
@@ -579,17 +610,20 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 
     ptx::tc_fence_before();
     __syncthreads();
+    // a pair gives its tensor memory back together, after both blocks' reads
+    if (CG == 2) ptx::cluster_sync_all();
     if (warp == 1) {
         ptx::tc_fence_after();
-        ptx::tmem_dealloc(tmem_base, 512);
+        if (CG == 2) ptx::tmem_dealloc_pair(tmem_base, 512); else ptx::tmem_dealloc(tmem_base, 512);
     }
-    // neither block of a pair retires while the other may still write its maxima into it
-    if (p.cl > 1) ptx::cluster_sync_all();
+    // no block of a cluster retires while another may still write its maxima into it
+    if (p.cl * CG > 1) { __syncwarp(); ptx::cluster_sync_all(); }
 }
 
-template <int BN, bool MM>
-constexpr size_t fused_smem_bytes() { return sizeof(FusedSmem<BN, MM>) + 1024; }
-static_assert(fused_smem_bytes<256, false>() <= 227 * 1024 && fused_smem_bytes<128, false>() <= 227 * 1024 && fused_smem_bytes<256, true>() <= 227 * 1024 &&
-                  fused_smem_bytes<128, true>() <= 227 * 1024, "fused GEMM shared memory exceeds the 227 KB a block may use");
+template <int BN, bool MM, int CG>
+constexpr size_t fused_smem_bytes() { return sizeof(FusedSmem<BN, MM, CG>) + 1024; }
+static_assert(fused_smem_bytes<256, false, 1>() <= EGG_MAX_SMEM && fused_smem_bytes<128, false, 1>() <= EGG_MAX_SMEM && fused_smem_bytes<256, true, 1>() <= EGG_MAX_SMEM &&
+                  fused_smem_bytes<128, true, 1>() <= EGG_MAX_SMEM && fused_smem_bytes<256, false, 2>() <= EGG_MAX_SMEM && fused_smem_bytes<128, false, 2>() <= EGG_MAX_SMEM &&
+                  fused_smem_bytes<256, true, 2>() <= EGG_MAX_SMEM && fused_smem_bytes<128, true, 2>() <= EGG_MAX_SMEM, "fused GEMM shared memory exceeds the 227 KB a block may use");
 
 }  // namespace egg

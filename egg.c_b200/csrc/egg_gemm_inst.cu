@@ -25,14 +25,21 @@ static int set_attr_both() {
     return set_attr<256, EPI, RPL>();
 }
 
+template <int BN, int MODE, bool MM, bool FORM, int CG = 1>
+static int set_attr_fused_one() {
+    EGG_CUDA(cudaFuncSetAttribute(gemm_fused_kernel<BN, MODE, MM, FORM, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem_bytes<BN, MM, CG>()));
+    return EGG_OK;
+}
 template <int BN, bool MM>
 static int set_attr_fused() {
-    EGG_CUDA(cudaFuncSetAttribute(gemm_fused_kernel<BN, FUSED_QKV, MM, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem_bytes<BN, MM>()));
-    EGG_CUDA(cudaFuncSetAttribute(gemm_fused_kernel<BN, FUSED_RES, MM, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem_bytes<BN, MM>()));
-    EGG_CUDA(cudaFuncSetAttribute(gemm_fused_kernel<BN, FUSED_RES, MM, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem_bytes<BN, MM>()));
-    EGG_CUDA(cudaFuncSetAttribute(gemm_fused_kernel<BN, FUSED_RES_LN, MM, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem_bytes<BN, MM>()));
-    EGG_CUDA(cudaFuncSetAttribute(gemm_fused_kernel<BN, FUSED_RES_LN, MM, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem_bytes<BN, MM>()));
-    return EGG_OK;
+    int rc;
+    if ((rc = set_attr_fused_one<BN, FUSED_QKV, MM, false>())) return rc;
+    if ((rc = set_attr_fused_one<BN, FUSED_RES, MM, false>())) return rc;
+    if ((rc = set_attr_fused_one<BN, FUSED_RES, MM, true>())) return rc;
+    if ((rc = set_attr_fused_one<BN, FUSED_RES_LN, MM, false>())) return rc;
+    if ((rc = set_attr_fused_one<BN, FUSED_RES_LN, MM, true>())) return rc;
+    if ((rc = set_attr_fused_one<BN, FUSED_RES_LN, MM, false, 2>())) return rc;
+    return set_attr_fused_one<BN, FUSED_RES_LN, MM, true, 2>();
 }
 
 int gemm_init() {
@@ -161,41 +168,51 @@ int fused_cluster_size(int hidden) {
     return 0;
 }
 
-template <int BN, int MODE, bool MM, bool FORM = false>
-static int launch_fused_one(cudaStream_t st, const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &to, const CUtensorMap &tr,
+template <int BN, int MODE, bool MM, bool FORM, int CG>
+static int launch_fused_cg(cudaStream_t st, const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &to, const CUtensorMap &tr,
                             const FusedParams &p, int units, int num_sms) {
-    auto kern = gemm_fused_kernel<BN, MODE, MM, FORM>;
+    auto kern = gemm_fused_kernel<BN, MODE, MM, FORM, CG>;
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(GEMM_THREADS);
-    cfg.dynamicSmemBytes = fused_smem_bytes<BN, MM>();
+    cfg.dynamicSmemBytes = fused_smem_bytes<BN, MM, CG>();
+    const int cluster = p.cl * CG;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
-    int groups = num_sms / p.cl;                     // resident blocks (pairs of blocks)
-    if (p.cl > 1) {
+    int groups = num_sms / cluster;                  // resident blocks (clusters of blocks)
+    if (cluster > 1) {
         attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = (unsigned)p.cl; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+        attr[0].val.clusterDim.x = (unsigned)cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr; cfg.numAttrs = 1;                  // (the occupancy question is about the cluster alone)
-        // the pairs that can be resident at once (a GPC with an odd number of free SMs leaves one out): asked once
-        static int max_pairs_dev[EGG_MAX_DEVICES] = {};
-        int &max_pairs = max_pairs_dev[current_device_slot()];
+        // the clusters that can be resident at once (a GPC whose free SMs are no multiple leaves some out): asked once a size
+        static int max_dev[2][EGG_MAX_DEVICES] = {};
+        int &max_pairs = max_dev[p.cl > 1][current_device_slot()];
         if (max_pairs == 0) {
-            cfg.gridDim = dim3((unsigned)(num_sms / p.cl * p.cl));
+            cfg.gridDim = dim3((unsigned)(num_sms / cluster * cluster));
             int n = 0;
             EGG_CUDA(cudaOccupancyMaxActiveClusters(&n, kern, &cfg));
-            if (n < 1) { set_error("no pair of blocks of the row-owning GEMM fits on the device"); return EGG_E_CUDA; }
+            if (n < 1) { set_error("no cluster of blocks of the row-owning GEMM fits on the device"); return EGG_E_CUDA; }
             max_pairs = n;
         }
         if (groups > max_pairs) groups = max_pairs;
     }
     if (groups > units) groups = units;
-    cfg.gridDim = dim3((unsigned)(groups * p.cl));
-    cfg.attrs = attr; cfg.numAttrs = p.cl > 1 ? 1 : 0;
+    cfg.gridDim = dim3((unsigned)(groups * cluster));
+    cfg.attrs = attr; cfg.numAttrs = cluster > 1 ? 1 : 0;
     if (t_chain) {
         attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
     }
     EGG_CUDA(cudaLaunchKernelEx(&cfg, kern, ta, tb, to, tr, p));
     return EGG_OK;
+}
+
+template <int BN, int MODE, bool MM, bool FORM = false>
+static int launch_fused_one(cudaStream_t st, const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &to, const CUtensorMap &tr,
+                            const FusedParams &p, int units, int num_sms) {
+    if constexpr (MODE == FUSED_RES_LN) {
+        if (p.pair) return launch_fused_cg<BN, MODE, MM, FORM, 2>(st, ta, tb, to, tr, p, units, num_sms);
+    }
+    return launch_fused_cg<BN, MODE, MM, FORM, 1>(st, ta, tb, to, tr, p, units, num_sms);
 }
 
 template <int BN, bool MM>
@@ -223,13 +240,19 @@ int launch_gemm_fused(cudaStream_t st, int mode, const int8_t *A, const int8_t *
         set_error("shifts %d + %d too large for the pre-shifted bias table", p.out_shift, p.rank1_shift);
         return EGG_E_INVALID;
     }
-    const int units = (p.M / GEMM_BM) * p.parts;
+    int units = (p.M / GEMM_BM) * p.parts;
     // few units: two blocks share each, so that a unit's products and its epilogue take half as long on SMs that would idle
     // (2048 rows, H 256: MLP-down 12.7 -> 11.3 us, Q|K|V 8.6 -> 7.2, output projection 7.4 -> 6.3)
     if (p.cl == 1 && p.H >= 256 && 2 * units <= num_sms) p.cl = 2;
     const int hl = p.H % (128 * p.cl) ? 128 : p.H / p.cl;      // columns per block (uneven shares: whole 128-column sub-tiles)
     const bool mm = p.seq_len % GEMM_BM != 0;        // a tile spans members: four table sets, see the kernel
     const int bn = (mm ? hl == 256 : hl % 256 == 0) ? 256 : 128;      // (128-column sub-tiles at H = 512 were measured: +30 % on MLP-down)
+    // Pairs of blocks where the products wait for their operands: a 128 x 256 tile takes 96 bytes a clock at the tensor cores' rate and an SM
+    // gets some 57, a pair's half needs 64.  Only below long contractions, whose epilogue is short beside them: the two blocks' epilogues
+    // wait for one another.  Residual products per evaluation of 4 or 2 layers: K 2048 8.24 -> 7.17 ms, 2560 2.43 -> 2.21, 4096 3.49 -> 3.29,
+    // 1536 1.52 -> 1.46; but K 1024 1.67 -> 1.87, and Q|K|V (K = H) 2 to 30 % longer.  Not where pairs would leave SMs without a unit.
+    p.pair = mode == FUSED_RES_LN && p.K >= 1536 && units >= 2 * num_sms;
+    if (p.pair) units = (p.M / GEMM_BM + 1) / 2 * p.parts;
     p.fd_seq = make_fastdiv(p.seq_len);
     p.fd_h = make_fastdiv(p.H);
     p.one = 1;
@@ -238,7 +261,7 @@ int launch_gemm_fused(cudaStream_t st, int mode, const int8_t *A, const int8_t *
     CUtensorMap ta, tb, to, tr;
     int rc;
     if ((rc = make_tmap(&ta, A, (uint64_t)p.M, (uint64_t)p.K, GEMM_BM))) return rc;
-    if ((rc = make_tmap(&tb, B, (uint64_t)p.parts * p.H, (uint64_t)p.K, (uint32_t)bn))) return rc;
+    if ((rc = make_tmap(&tb, B, (uint64_t)p.parts * p.H, (uint64_t)p.K, (uint32_t)(p.pair ? bn / 2 : bn)))) return rc;
     const uint64_t out_rows = p.parts > 1 ? (uint64_t)p.parts * (uint64_t)p.part_rows : (uint64_t)p.M;
     if ((rc = make_tmap_box8(&to, out, out_rows, (uint64_t)p.H, (uint32_t)bn / 4))) return rc;
     tr = to;
