@@ -105,10 +105,12 @@ struct RplTables {
     alignas(16) int8_t d[BN / 4];           // B-noise of the next projection
 };
 
-template <int BN>
+// CG: blocks that form a tile's products together (2: a pair, each with half of B's rows, which leaves room for a fourth stage)
+template <int BN, int CG = 1>
 struct GemmSmem {
-    alignas(1024) uint8_t a[GEMM_STAGES][GEMM_BM * GEMM_BK];
-    alignas(1024) uint8_t b[GEMM_STAGES][BN * GEMM_BK];
+    static constexpr int ST = CG == 2 ? 4 : GEMM_STAGES;
+    alignas(1024) uint8_t a[ST][GEMM_BM * GEMM_BK];
+    alignas(1024) uint8_t b[ST][BN / CG * GEMM_BK];
     union {
         alignas(1024) int32_t stage[GEMM_EPI_WARPS][32][20];   // transposed epilogues, per warp: 32 rows x 16 columns (+4 pad) transpose buffer
         struct {
@@ -137,8 +139,8 @@ struct GemmSmem {
     alignas(16) int32_t rowpart[4][GEMM_BM];            // EPI_LOGITS: the row's maxima of the four column quarters
     alignas(16) int8_t act_lut[256];
     alignas(16) int32_t exp_lut[256];
-    alignas(8) uint64_t full[GEMM_STAGES];
-    uint64_t empty[GEMM_STAGES];
+    alignas(8) uint64_t full[ST];
+    uint64_t empty[ST];
     uint64_t tmem_full[2];
     uint64_t tmem_empty[2];
     uint64_t rbar[GEMM_EPI_WARPS];      // per epilogue warp: arrival of its residual box (EPI_PRE32, row-per-lane, BN = 256)
@@ -258,8 +260,8 @@ __device__ __forceinline__ void rpl_store(const GemmParams &p, RplTables<BN> &t,
 // accumulators are consumed straight from the TMEM layout (lane = row, registers = columns) with no transpose, no
 // shuffles and about half the instructions of the transposed form.  TMEM loads are double-buffered.
 // FORM: q and k columns (EPI_QKV), both shifts as one (EPI_GELU with BN = 256)
-template <int BN, int EPI, bool FORM, bool RES_TMA>
-__device__ __forceinline__ int epilogue_rpl(const GemmParams &p, GemmSmem<BN> &sm, const RplTables<BN> &tab, uint32_t taddr, int r, bool row_ok, int n0,
+template <int BN, int EPI, bool FORM, bool RES_TMA, int CG>
+__device__ __forceinline__ int epilogue_rpl(const GemmParams &p, GemmSmem<BN, CG> &sm, const RplTables<BN> &tab, uint32_t taddr, int r, bool row_ok, bool live, int n0,
                                             int cbase, int lane, int m0q, int xbs, const int4 (&rs_pre)[BN / 4 / 16], const CUtensorMap *tmap_o,
                                             int32_t *ost, int32_t *ost1) {
     constexpr int NCH = BN / 4 / 16;                       // 16-column chunks of this warp's quarter of the tile
@@ -418,7 +420,7 @@ __device__ __forceinline__ int epilogue_rpl(const GemmParams &p, GemmSmem<BN> &s
     if ((EPI == EPI_GELU || EPI == EPI_CLIP8) && NCH == 4) {
         ptx::fence_proxy_async();
         __syncwarp();
-        if (lane == 0) {
+        if (lane == 0 && live) {
             ptx::tma_store_2d(tmap_o, ost, n0 + cbase, m0q);
             ptx::tma_store_commit();
         }
@@ -565,17 +567,25 @@ __device__ __forceinline__ void epilogue_head_rpl(const GemmParams &p, GemmSmem<
     }
 }
 
-template <int BN, int EPI, int RPL>
+template <int BN, int EPI, int RPL, int CG = 1>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                const __grid_constant__ CUtensorMap tmap_o, const __grid_constant__ CUtensorMap tmap_r, const GemmParams p) {
     extern __shared__ uint8_t smem_raw[];
-    GemmSmem<BN> &sm = *reinterpret_cast<GemmSmem<BN> *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    using Smem = GemmSmem<BN, CG>;
+    static_assert(CG == 1 || (BN == 256 && RPL && (EPI == EPI_GELU || EPI == EPI_CLIP8)), "pairs: outputs leave by copy engine, which a duplicate tile can skip");
+    constexpr int ST = Smem::ST;
+    Smem &sm = *reinterpret_cast<Smem *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
 
     chain_next();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tiles_n = p.N / BN;
-    const int tiles_m = (p.M + GEMM_BM - 1) / GEMM_BM;
+    const int rows_m = (p.M + GEMM_BM - 1) / GEMM_BM;              // row tiles
+    const int tiles_m = (rows_m + CG - 1) / CG;                    // row tiles of a block, or pairs of them of a pair of blocks
+    const int prow = CG == 2 ? (int)(blockIdx.x & 1) : 0;           // this block's row tile of the pair (clusters are consecutive blocks)
+    const int first_tile = (int)blockIdx.x / CG, tile_step = (int)gridDim.x / CG;
+    // an odd last row tile is formed by both blocks of its pair, and the second keeps it to itself
+    auto row_tile = [&](int t) { return CG == 2 ? min(2 * t + prow, rows_m - 1) : t; };
     const int num_kb = (p.K + GEMM_BK - 1) / GEMM_BK;
     // the vote GEMM may cut its contraction (the pair index) into k_splits parts: work item = (split, tile)
     const int k_splits = (EPI == EPI_VOTE && p.k_splits > 1) ? p.k_splits : 1;
@@ -583,19 +593,22 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     const int mn_tiles = tiles_m * tiles_n;
     const int num_tiles = mn_tiles * k_splits;
     constexpr uint32_t TMEM_COLS = (2 * BN <= 32) ? 32 : (2 * BN <= 64 ? 64 : (2 * BN <= 128 ? 128 : (2 * BN <= 256 ? 256 : 512)));
-    constexpr uint32_t STAGE_BYTES = GEMM_BM * GEMM_BK + BN * GEMM_BK;
+    constexpr uint32_t STAGE_BYTES = GEMM_BM * GEMM_BK + BN / CG * GEMM_BK;      // of one block
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < GEMM_STAGES; s++) { ptx::mbar_init(&sm.full[s], 1); ptx::mbar_init(&sm.empty[s], 1); }
-        for (int a = 0; a < 2; a++) { ptx::mbar_init(&sm.tmem_full[a], 1); ptx::mbar_init(&sm.tmem_empty[a], GEMM_EPI_WARPS); }
+        for (int s = 0; s < ST; s++) { ptx::mbar_init(&sm.full[s], 1); ptx::mbar_init(&sm.empty[s], 1); }
+        for (int a = 0; a < 2; a++) { ptx::mbar_init(&sm.tmem_full[a], 1); ptx::mbar_init(&sm.tmem_empty[a], CG * GEMM_EPI_WARPS); }
         for (int w = 0; w < GEMM_EPI_WARPS; w++) ptx::mbar_init(&sm.rbar[w], 1);
         sm.abort_flag = 0;
         sm.epi_ok = 1;
         ptx::fence_barrier_init();
     }
     if (warp == 1) {
-        ptx::tmem_alloc(&sm.tmem_base, TMEM_COLS);
-        ptx::tmem_relinquish();
+        if (CG == 2) ptx::tmem_alloc_pair(&sm.tmem_base, TMEM_COLS);
+        else {
+            ptx::tmem_alloc(&sm.tmem_base, TMEM_COLS);
+            ptx::tmem_relinquish();
+        }
     }
     if (warp >= 2) {
         int e = threadIdx.x - 64;
@@ -611,6 +624,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
+    if (CG == 2) ptx::cluster_sync_all();          // the other block's barriers exist before anything arrives on them
     chain_wait();
     const uint32_t tmem_base = sm.tmem_base;
 
@@ -621,17 +635,24 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             ptx::prefetch_tmap(&tmap_b);
             uint32_t it = 0;
             bool ok = true;
-            for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+            const uint32_t full_s = CG == 2 ? ptx::mapa_u32(ptx::smem_u32(sm.full), 0u) : 0u;          // of the even block
+            for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step) {
                 const int split = (k_splits > 1) ? tile / mn_tiles : 0, mn = tile - split * mn_tiles;
-                int tm_ = fast_div(mn, p.fd_tiles_n), m0 = tm_ * GEMM_BM, n0 = (mn - tm_ * tiles_n) * BN;
+                int tm_ = fast_div(mn, p.fd_tiles_n), m0 = row_tile(tm_) * GEMM_BM, n0 = (mn - tm_ * tiles_n) * BN + prow * (BN / CG);
                 const int kb0 = split * kb_per, kb1 = min(num_kb, kb0 + kb_per);
                 for (int kb = kb0; kb < kb1; kb++, it++) {
-                    int s = it % GEMM_STAGES;
-                    uint32_t ph = (it / GEMM_STAGES) & 1;
+                    int s = it % ST;
+                    uint32_t ph = (it / ST) & 1;
                     if (!ptx::mbar_wait(&sm.empty[s], ph ^ 1) || sm.abort_flag) { gemm_fail(p, &sm.abort_flag, DEV_TIMEOUT_EMPTY); ok = false; break; }
-                    ptx::mbar_arrive_expect_tx(&sm.full[s], STAGE_BYTES);
-                    ptx::tma_load_2d(sm.a[s], &tmap_a, &sm.full[s], kb * GEMM_BK, m0);
-                    ptx::tma_load_2d(sm.b[s], &tmap_b, &sm.full[s], kb * GEMM_BK, n0);
+                    if (CG == 2) {
+                        if (prow == 0) ptx::mbar_arrive_expect_tx(&sm.full[s], 2 * STAGE_BYTES);           // both blocks' bytes
+                        ptx::tma_load_2d_pair(sm.a[s], &tmap_a, full_s + 8 * s, kb * GEMM_BK, m0);
+                        ptx::tma_load_2d_pair(sm.b[s], &tmap_b, full_s + 8 * s, kb * GEMM_BK, n0);
+                    } else {
+                        ptx::mbar_arrive_expect_tx(&sm.full[s], STAGE_BYTES);
+                        ptx::tma_load_2d(sm.a[s], &tmap_a, &sm.full[s], kb * GEMM_BK, m0);
+                        ptx::tma_load_2d(sm.b[s], &tmap_b, &sm.full[s], kb * GEMM_BK, n0);
+                    }
                 }
             }
             if (!ok) {   // let copies already in flight land before the CTA tears down
@@ -641,21 +662,21 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         }
     } else if (warp == 1) {
         // ===================== MMA issuer =====================
-        if (ptx::elect_one()) {
-            constexpr uint32_t idesc = ptx::make_idesc_i8(GEMM_BM, BN);
+        if (prow == 0 && ptx::elect_one()) {
+            constexpr uint32_t idesc = ptx::make_idesc_i8(CG * GEMM_BM, BN);
             uint32_t it = 0, tcount = 0;
             bool ok = true;
-            for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, tcount++) {
+            for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step, tcount++) {
                 int as = tcount & 1;
                 uint32_t aph = (tcount >> 1) & 1;
-                if (!ptx::mbar_wait(&sm.tmem_empty[as], aph ^ 1) || sm.abort_flag) { gemm_fail(p, &sm.abort_flag, DEV_TIMEOUT_TMEM_EMPTY); ok = false; break; }
+                if (!(CG == 2 ? ptx::mbar_wait_cluster(&sm.tmem_empty[as], aph ^ 1, 2000000000ull) : ptx::mbar_wait(&sm.tmem_empty[as], aph ^ 1)) || sm.abort_flag) { gemm_fail(p, &sm.abort_flag, DEV_TIMEOUT_TMEM_EMPTY); ok = false; break; }
                 ptx::tc_fence_after();
                 uint32_t d_tmem = tmem_base + (uint32_t)(as * BN);
                 const int split = (k_splits > 1) ? tile / mn_tiles : 0;
                 const int kb0 = split * kb_per, kb1 = min(num_kb, kb0 + kb_per);
                 for (int kb = kb0; kb < kb1; kb++, it++) {
-                    int s = it % GEMM_STAGES;
-                    uint32_t ph = (it / GEMM_STAGES) & 1;
+                    int s = it % ST;
+                    uint32_t ph = (it / ST) & 1;
                     if (!ptx::mbar_wait(&sm.full[s], ph) || sm.abort_flag) { gemm_fail(p, &sm.abort_flag, DEV_TIMEOUT_FULL); ok = false; break; }
                     ptx::tc_fence_after();
                     uint64_t da = ptx::make_smem_desc_sw128(ptx::smem_u32(sm.a[s]));
@@ -663,11 +684,14 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 #pragma unroll
                     for (int k = 0; k < GEMM_BK / 32; k++) {
                         // +32 bytes along K inside the swizzle row = +2 in the 16-byte address field
-                        ptx::mma_i8(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+                        if (CG == 2) ptx::mma_i8_pair(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+                        else ptx::mma_i8(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
                     }
-                    ptx::mma_commit(&sm.empty[s]);
+                    if (CG == 2) ptx::mma_commit_pair(&sm.empty[s], 0); else ptx::mma_commit(&sm.empty[s]);
                 }
-                if (ok) ptx::mma_commit(&sm.tmem_full[as]);
+                if (ok) {
+                    if (CG == 2) ptx::mma_commit_pair(&sm.tmem_full[as], 0); else ptx::mma_commit(&sm.tmem_full[as]);
+                }
             }
         }
     } else if constexpr (RPL && EPI != EPI_LOGITS) {
@@ -686,7 +710,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         int pf_xb = 0;                              // the lane's rank-1 factor (raw sum of x b of its row)
         int4 pf_rs0 = make_int4(0, 0, 0, 0);        // first chunk of residual bytes
         auto prefetch = [&](int tile) {
-            const int tm_ = fast_div(tile, p.fd_tiles_n), rw = tm_ * GEMM_BM + quarter * 32, n0 = (tile - tm_ * tiles_n) * BN;
+            const int tm_ = fast_div(tile, p.fd_tiles_n), rw = row_tile(tm_) * GEMM_BM + quarter * 32, n0 = (tile - tm_ * tiles_n) * BN;
             rpl_load<BN, EPI>(p, lane, fast_div(min(rw, p.M - 1), p.fd_seq), n0 + cbase + 4 * lane, nxt);
             const int rc = min(rw + lane, p.M - 1);
             pf_xb = p.xb[(int64_t)rc * p.xb_stride + ((EPI == EPI_QKV) ? fast_div(n0, p.fd_third) : 0)];
@@ -696,12 +720,14 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 ptx::tma_load_2d(sm.ostage1[ew], &tmap_r, &sm.rbar[ew], n0 + cbase, rw);
             }
         };
-        if ((int)blockIdx.x < num_tiles) prefetch(blockIdx.x);
-        for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, tcount++) {
+        const uint32_t tmem_empty_s = CG == 2 ? ptx::mapa_u32(ptx::smem_u32(sm.tmem_empty), 0u) : 0u;        // of the even block
+        if (first_tile < num_tiles) prefetch(first_tile);
+        for (int tile = first_tile; tile < num_tiles; tile += tile_step, tcount++) {
             const int as = tcount & 1;
-            const int tm_ = fast_div(tile, p.fd_tiles_n), m0q = tm_ * GEMM_BM + quarter * 32, n0 = (tile - tm_ * tiles_n) * BN;
+            const int tm_ = fast_div(tile, p.fd_tiles_n), m0q = row_tile(tm_) * GEMM_BM + quarter * 32, n0 = (tile - tm_ * tiles_n) * BN;
+            const bool live = CG == 1 || 2 * tm_ + prow < rows_m;
             const int r = m0q + lane;
-            const bool row_ok = r < p.M;
+            const bool row_ok = r < p.M && live;
             __syncwarp();                           // every lane has read the previous tile's tables
             rpl_store<BN, EPI>(p, tab, lane, nxt);
             __syncwarp();
@@ -713,7 +739,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 for (int cc = 1; cc < BN / 4 / 16; cc++)      // used one chunk of arithmetic later each
                     rs_l[cc] = *reinterpret_cast<const int4 *>(p.resid + (int64_t)min(r, p.M - 1) * p.N + n0 + cbase + 16 * cc);
             }
-            const int ntile = tile + gridDim.x;
+            const int ntile = tile + tile_step;
             if (!RES_TMA && ntile < num_tiles) prefetch(ntile);          // in flight while this tile is computed
             bool ok = ptx::mbar_wait(&sm.tmem_full[as], (tcount >> 1) & 1);
             if (RES_TMA) ok = ok && ptx::mbar_wait(&sm.rbar[ew], tcount & 1);
@@ -726,9 +752,9 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 int part;
                 if ((EPI == EPI_QKV && n0 < 2 * p.third) || (EPI == EPI_GELU && BN == 256 && p.pow_t))        // asked once a tile, not per four columns: 68.6 -> 68.0 ms
                     // of a generation; not for the narrow tiles of small models, where two copies of the code take longer to fetch than they save
-                    part = epilogue_rpl<BN, EPI, true, false>(p, sm, tab, taddr, r, row_ok, n0, cbase, lane, m0q, xbs, rs_l, &tmap_o, sm.ostage0[ew], sm.ostage1[ew]);
+                    part = epilogue_rpl<BN, EPI, true, false, CG>(p, sm, tab, taddr, r, row_ok, live, n0, cbase, lane, m0q, xbs, rs_l, &tmap_o, sm.ostage0[ew], sm.ostage1[ew]);
                 else
-                    part = epilogue_rpl<BN, EPI, false, RES_TMA>(p, sm, tab, taddr, r, row_ok, n0, cbase, lane, m0q, xbs, rs_l, &tmap_o, sm.ostage0[ew], sm.ostage1[ew]);
+                    part = epilogue_rpl<BN, EPI, false, RES_TMA, CG>(p, sm, tab, taddr, r, row_ok, live, n0, cbase, lane, m0q, xbs, rs_l, &tmap_o, sm.ostage0[ew], sm.ostage1[ew]);
                 if (row_ok) {
                     if (EPI == EPI_GELU || (EPI == EPI_CLIP8 && p.nt_d_off >= 0)) atomicAdd(&p.rowstat[r], part);
                     else if (EPI == EPI_PRE32) atomicMax(&p.rowstat[r], part);
@@ -738,7 +764,9 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             // release the accumulator stage
             ptx::tc_fence_before();
             __syncwarp();                           // (and every lane has read its residual bytes: the box may be refilled)
-            if (lane == 0) ptx::mbar_arrive(&sm.tmem_empty[as]);
+            if (lane == 0) {
+                if (CG == 2) ptx::mbar_arrive_cluster(tmem_empty_s + 8 * as); else ptx::mbar_arrive(&sm.tmem_empty[as]);
+            }
             if (RES_TMA && ntile < num_tiles) prefetch(ntile);
         }
     } else {
@@ -1014,14 +1042,16 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     __syncwarp();
     ptx::tc_fence_before();
     __syncthreads();
+    if (CG == 2) ptx::cluster_sync_all();          // a pair gives its tensor memory back together, after both blocks' reads
     if (warp == 1) {
         ptx::tc_fence_after();
-        ptx::tmem_dealloc(tmem_base, TMEM_COLS);
+        if (CG == 2) ptx::tmem_dealloc_pair(tmem_base, TMEM_COLS); else ptx::tmem_dealloc(tmem_base, TMEM_COLS);
     }
+    if (CG == 2) { __syncwarp(); ptx::cluster_sync_all(); }          // neither block retires before the other is done with its memory
 }
 
-template <int BN>
-constexpr size_t gemm_smem_bytes() { return sizeof(GemmSmem<BN>) + 1024; }
-static_assert(gemm_smem_bytes<256>() <= 227 * 1024, "GEMM shared memory exceeds the 227 KB a block may use");
+template <int BN, int CG = 1>
+constexpr size_t gemm_smem_bytes() { return sizeof(GemmSmem<BN, CG>) + 1024; }
+static_assert(gemm_smem_bytes<256>() <= EGG_MAX_SMEM && gemm_smem_bytes<256, 2>() <= EGG_MAX_SMEM, "GEMM shared memory exceeds the 227 KB a block may use");
 
 }  // namespace egg

@@ -12,9 +12,9 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 static EncodeTiledFn g_encode = nullptr;
 
-template <int BN, int EPI, int RPL = 0>
+template <int BN, int EPI, int RPL = 0, int CG = 1>
 static int set_attr() {
-    EGG_CUDA(cudaFuncSetAttribute(gemm_i8_kernel<BN, EPI, RPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem_bytes<BN>()));
+    EGG_CUDA(cudaFuncSetAttribute(gemm_i8_kernel<BN, EPI, RPL, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem_bytes<BN, CG>()));
     return EGG_OK;
 }
 
@@ -60,6 +60,8 @@ int gemm_init() {
     if ((rc = set_attr_both<EPI_PRE32>())) return rc;
     if ((rc = set_attr_both<EPI_QKV>())) return rc;
     if ((rc = set_attr_both<EPI_GELU, 1>())) return rc;
+    if ((rc = set_attr<256, EPI_GELU, 1, 2>())) return rc;
+    if ((rc = set_attr<256, EPI_CLIP8, 1, 2>())) return rc;
     if ((rc = set_attr_both<EPI_PRE32, 1>())) return rc;
     if ((rc = set_attr_both<EPI_QKV, 1>())) return rc;
     if ((rc = set_attr<256, EPI_HEAD>())) return rc;
@@ -283,6 +285,38 @@ static int launch_one(cudaStream_t st, const CUtensorMap &ta, const CUtensorMap 
     return EGG_OK;
 }
 
+// Pairs of blocks with the tiles of 256 columns of two row tiles.
+template <int EPI>
+static int launch_pair(cudaStream_t st, const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &to, const GemmParams &p, int num_sms) {
+    auto kern = gemm_i8_kernel<256, EPI, 1, 2>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(GEMM_THREADS);
+    cfg.dynamicSmemBytes = gemm_smem_bytes<256, 2>();
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    static int max_dev[EGG_MAX_DEVICES] = {};          // pairs that can be resident at once
+    int &most = max_dev[current_device_slot()];
+    if (most == 0) {
+        cfg.gridDim = dim3((unsigned)(num_sms / 2 * 2));
+        int n = 0;
+        EGG_CUDA(cudaOccupancyMaxActiveClusters(&n, kern, &cfg));
+        if (n < 1) { set_error("no pair of blocks of the GEMM fits on the device"); return EGG_E_CUDA; }
+        most = n < num_sms / 2 ? n : num_sms / 2;
+    }
+    const int tiles = ((p.M + 2 * GEMM_BM - 1) / (2 * GEMM_BM)) * (p.N / 256);
+    cfg.gridDim = dim3((unsigned)(2 * (tiles < most ? tiles : most)));
+    if (t_chain) {
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.numAttrs = 2;
+    }
+    EGG_CUDA(cudaLaunchKernelEx(&cfg, kern, ta, tb, to, ta, p));
+    return EGG_OK;
+}
+
 template <int EPI, int RPL = 0>
 static int launch_bn(cudaStream_t st, int bn, const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &to, const GemmParams &p, int num_sms) {
     if (bn == 256) return launch_one<256, EPI, RPL>(st, ta, tb, to, p, num_sms);
@@ -295,6 +329,11 @@ static int launch_eval(cudaStream_t st, int bn, const CUtensorMap &ta, const CUt
     if (p.seq_len % 32 == 0 && p.rpl >= 0) return launch_bn<EPI, 1>(st, bn, ta, tb, to, p, num_sms);
     return launch_bn<EPI, 0>(st, bn, ta, tb, to, p, num_sms);
 }
+
+// Contractions from which pairs of blocks form the tiles (see launch_gemm_fused for what bounds them): K 1024 0.347 -> 0.330 ms and, in
+// MLP-up, 2.45 -> 2.35; 2048 0.52 -> 0.46; 4096 3.40 -> 2.97 (2.6 -> 3.0 int8 POP/s); but K 640 1.26 -> 1.45 and 512 6.2 -> 7.3: there the
+// epilogues are as long as the products, and those of a pair wait for one another.
+constexpr int PAIR_MIN_K = 1024;
 
 int launch_gemm(cudaStream_t st, int epi, const int8_t *A, const int8_t *B, const GemmParams &p_in, int num_sms) {
     GemmParams p = p_in;
@@ -331,8 +370,10 @@ int launch_gemm(cudaStream_t st, int epi, const int8_t *A, const int8_t *B, cons
     p.pow_t = epi == EPI_GELU || epi == EPI_LOGITS ? merged_shift(p.K, p.rank1_shift, p.out_shift) : 0;
     CUtensorMap ta, tb;
     int rc;
+    const bool pair = (epi == EPI_GELU || epi == EPI_CLIP8) && bn == 256 && p.seq_len % 32 == 0 && p.rpl >= 0 && p.K >= PAIR_MIN_K &&
+                      (int64_t)((p.M + GEMM_BM - 1) / GEMM_BM) * (p.N / 256) >= 4 * num_sms;
     if ((rc = make_tmap(&ta, A, (uint64_t)p.M, (uint64_t)p.K, GEMM_BM))) return rc;
-    if ((rc = make_tmap(&tb, B, (uint64_t)p.N, (uint64_t)p.K, (uint32_t)bn))) return rc;
+    if ((rc = make_tmap(&tb, B, (uint64_t)p.N, (uint64_t)p.K, (uint32_t)(pair ? bn / 2 : bn)))) return rc;
     CUtensorMap to = ta;       // only the row-per-lane int32 epilogues store through a tensor map
     if ((epi == EPI_PRE32 || epi == EPI_QKV) && p.seq_len % 32 == 0 && p.rpl >= 0) {
         if ((rc = make_tmap_out(&to, p.out32, (uint64_t)p.M, (uint64_t)p.N))) return rc;
@@ -340,6 +381,7 @@ int launch_gemm(cudaStream_t st, int epi, const int8_t *A, const int8_t *B, cons
     if (epi == EPI_LOGITS || ((epi == EPI_GELU || epi == EPI_CLIP8) && bn == 256 && p.seq_len % 32 == 0 && p.rpl >= 0)) {
         if ((rc = make_tmap_out8(&to, p.out8, (uint64_t)p.M, (uint64_t)p.N))) return rc;
     }
+    if (pair) return epi == EPI_GELU ? launch_pair<EPI_GELU>(st, ta, tb, to, p, num_sms) : launch_pair<EPI_CLIP8>(st, ta, tb, to, p, num_sms);
     switch (epi) {
         case EPI_CLIP8: return launch_eval<EPI_CLIP8>(st, bn, ta, tb, to, p, num_sms);
         case EPI_GELU: return launch_eval<EPI_GELU>(st, bn, ta, tb, to, p, num_sms);

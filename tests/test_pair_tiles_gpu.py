@@ -17,7 +17,7 @@ SEED = 0x00C0FFEE
     (512, 1, 128, 298),        # K 2048, tiles of one member, two sub-tiles of 256
     (512, 1, 96, 396),         # 297 tiles across members of 96 rows
     (640, 1, 64, 594),         # clusters of four, 384 + 256 columns
-    (1024, 1, 128, 298),       # clusters of four, 512 + 512 columns
+    (1024, 1, 128, 298),       # clusters of four, 512 + 512 columns; K 1024 in the up projection, too
 ])
 def test_pairs_equal_single_blocks_and_oracle(hidden, layers, seq, pop):
     pkg, O = load_pkg(), load_oracle()
