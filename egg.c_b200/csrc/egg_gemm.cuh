@@ -669,7 +669,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step, tcount++) {
                 int as = tcount & 1;
                 uint32_t aph = (tcount >> 1) & 1;
-                if (!(CG == 2 ? ptx::mbar_wait_cluster(&sm.tmem_empty[as], aph ^ 1, 2000000000ull) : ptx::mbar_wait(&sm.tmem_empty[as], aph ^ 1)) || sm.abort_flag) { gemm_fail(p, &sm.abort_flag, DEV_TIMEOUT_TMEM_EMPTY); ok = false; break; }
+                if (!ptx::mbar_wait(&sm.tmem_empty[as], aph ^ 1) || sm.abort_flag) { gemm_fail(p, &sm.abort_flag, DEV_TIMEOUT_TMEM_EMPTY); ok = false; break; }
                 ptx::tc_fence_after();
                 uint32_t d_tmem = tmem_base + (uint32_t)(as * BN);
                 const int split = (k_splits > 1) ? tile / mn_tiles : 0;
@@ -765,7 +765,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             ptx::tc_fence_before();
             __syncwarp();                           // (and every lane has read its residual bytes: the box may be refilled)
             if (lane == 0) {
-                if (CG == 2) ptx::mbar_arrive_cluster(tmem_empty_s + 8 * as); else ptx::mbar_arrive(&sm.tmem_empty[as]);
+                if (CG == 2) ptx::mbar_arrive_peer(tmem_empty_s + 8 * as); else ptx::mbar_arrive(&sm.tmem_empty[as]);
             }
             if (RES_TMA && ntile < num_tiles) prefetch(ntile);
         }

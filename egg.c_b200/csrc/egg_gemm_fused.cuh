@@ -222,14 +222,7 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 for (int j = 0; j < NT && !sm.abort_flag; j++, stc++) {
                     const int slot = stc % NS;
                     const uint32_t sph = (stc / NS) & 1;
-                    if (CG == 2) {       // both blocks' epilogues arrive
-                        if (!sm.abort_flag && !ptx::mbar_wait_cluster(&sm.tmem_empty[slot], sph ^ 1, 1000000000ull)) {
-                            sm.abort_flag = 1;
-                            if (p.err) atomicCAS(p.err, 0, DEV_TIMEOUT_TMEM_EMPTY);
-                        }
-                    } else {
-                        fused_wait(&sm.tmem_empty[slot], sph ^ 1, &sm.abort_flag, p.err, DEV_TIMEOUT_TMEM_EMPTY);
-                    }
+                    fused_wait(&sm.tmem_empty[slot], sph ^ 1, &sm.abort_flag, p.err, DEV_TIMEOUT_TMEM_EMPTY);          // (a pair: both blocks' epilogues arrive)
                     if (sm.abort_flag) break;
                     ptx::tc_fence_after();
                     const uint32_t d_tmem = tmem_base + (uint32_t)(slot * BN);
@@ -494,7 +487,7 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 ptx::fence_proxy_async();
                 __syncwarp();
                 if (lane == 0) {
-                    if (CG == 2) ptx::mbar_arrive_cluster(tmem_empty_s + 8 * slot); else ptx::mbar_arrive(&sm.tmem_empty[slot]);
+                    if (CG == 2) ptx::mbar_arrive_peer(tmem_empty_s + 8 * slot); else ptx::mbar_arrive(&sm.tmem_empty[slot]);
                     if (live) ptx::tma_store_2d(&tmap_o, sm.box[ew][j], cofs + j * BN + cq * CW, (int)(part * p.part_rows) + m0 + quarter * 32);
                     ptx::tma_store_commit();
                 }

@@ -86,6 +86,11 @@ __device__ __forceinline__ void st_cluster_u32(uint32_t cluster_addr, uint32_t v
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
+// the same where no memory is handed over: a reader of tensor memory that is done (its reads ordered by tc_fence_before).  A release at
+// cluster scope waits for the warp's stores and atomics: MLP-up in pairs at H 1024 2.31 ms with it, 1.99 without.
+__device__ __forceinline__ void mbar_arrive_peer(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
 // bounded wait on an own mbarrier that peer blocks arrive on (acquire at cluster scope)
 __device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity, uint64_t limit_ns) {
     const uint64_t t0 = globaltimer();
