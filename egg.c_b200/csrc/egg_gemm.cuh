@@ -207,8 +207,8 @@ __device__ __forceinline__ bool tab_load(const GemmParams &p, int e, int m0, int
     return true;
 }
 
-template <int BN, int EPI>
-__device__ __forceinline__ void tab_store(const GemmParams &p, GemmSmem<BN> &sm, int e, const TabWords &w) {
+template <int BN, int EPI, int CG>
+__device__ __forceinline__ void tab_store(const GemmParams &p, GemmSmem<BN, CG> &sm, int e, const TabWords &w) {
     const int sl = e / (BN / 4), j = (e % (BN / 4)) * 4;
     if (EPI == EPI_LOGITS) *reinterpret_cast<int4 *>(&sm.lg_a32[sl][j]) = make_int4((int)(int8_t)w.a, (int)(int8_t)(w.a >> 8), (int)(int8_t)(w.a >> 16), w.a >> 24);
     else *reinterpret_cast<int32_t *>(&sm.a_tab[sl][j]) = w.a;
@@ -573,7 +573,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                const __grid_constant__ CUtensorMap tmap_o, const __grid_constant__ CUtensorMap tmap_r, const GemmParams p) {
     extern __shared__ uint8_t smem_raw[];
     using Smem = GemmSmem<BN, CG>;
-    static_assert(CG == 1 || (BN == 256 && RPL && (EPI == EPI_GELU || EPI == EPI_CLIP8)), "pairs: outputs leave by copy engine, which a duplicate tile can skip");
+    static_assert(CG == 1 || (BN == 256 && (EPI == EPI_VOTE || (RPL && (EPI == EPI_GELU || EPI == EPI_CLIP8)))), "pairs: outputs that a duplicate tile can skip");
     constexpr int ST = Smem::ST;
     Smem &sm = *reinterpret_cast<Smem *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
 
@@ -781,13 +781,14 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         const int row_in_tile = quarter * 32 + lane;
         uint32_t tcount = 0;
         int pf_xb = 0;                              // EPI_LOGITS: the lane's rank-1 factor, loaded a tile ahead
-        for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, tcount++) {
+        const uint32_t tmem_empty_s = CG == 2 ? ptx::mapa_u32(ptx::smem_u32(sm.tmem_empty), 0u) : 0u;        // of the even block
+        for (int tile = first_tile; tile < num_tiles; tile += tile_step, tcount++) {
             const int as = tcount & 1;
             const uint32_t aph = (tcount >> 1) & 1;
             const int split = (k_splits > 1) ? tile / mn_tiles : 0, mn = tile - split * mn_tiles;
-            const int tm_ = fast_div(mn, p.fd_tiles_n), m0 = tm_ * GEMM_BM, n0 = (mn - tm_ * tiles_n) * BN;
+            const int tm_ = fast_div(mn, p.fd_tiles_n), m0 = row_tile(tm_) * GEMM_BM, n0 = (mn - tm_ * tiles_n) * BN;
             const int r = m0 + row_in_tile;
-            const bool row_ok = r < p.M;
+            const bool row_ok = r < p.M && (CG == 1 || 2 * tm_ + prow < rows_m);
 
             // ---- per-tile tables (evaluation epilogues): built here for a block's first tile, otherwise already
             // written at the end of the previous tile from words prefetched during its epilogue ----
@@ -800,7 +801,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 sgn = mem & 1;
                 if (tcount == 0) {
                     TabWords w;
-                    if (tab_load<BN, EPI>(p, e, m0, n0, w)) tab_store<BN, EPI>(p, sm, e, w);
+                    if (tab_load<BN, EPI>(p, e, m0, n0, w)) tab_store<BN, EPI, CG>(p, sm, e, w);
                 }
             }
             // ---- per-row state of the 4 rows this lane owns after the transpose, and the loads that do not
@@ -860,7 +861,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             TabWords nxt;
             bool have_nxt = false;
             if (EPI <= EPI_LOGITS) {
-                const int ntile = tile + gridDim.x;
+                const int ntile = tile + tile_step;
                 if (ntile < num_tiles) {
                     const int ntm = fast_div(ntile, p.fd_tiles_n), nm0 = ntm * GEMM_BM, nn0 = (ntile - ntm * tiles_n) * BN;
                     have_nxt = tab_load<BN, EPI>(p, e, nm0, nn0, nxt);
@@ -1027,13 +1028,15 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             // release the accumulator stage
             ptx::tc_fence_before();
             __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&sm.tmem_empty[as]);
+            if (lane == 0) {
+                if (CG == 2) ptx::mbar_arrive_peer(tmem_empty_s + 8 * as); else ptx::mbar_arrive(&sm.tmem_empty[as]);
+            }
             // tables are rewritten at the top of the next tile: everybody must be done reading them
             ptx::named_bar_sync(1, GEMM_EPI_THREADS);
             if (EPI == EPI_LOGITS && half == 0 && row_ok)
                 *reinterpret_cast<int4 *>(p.rowstat + (int64_t)r * (p.N >> 6) + (n0 >> 6)) =
                     make_int4(sm.rowpart[0][row_in_tile], sm.rowpart[1][row_in_tile], sm.rowpart[2][row_in_tile], sm.rowpart[3][row_in_tile]);
-            if (EPI <= EPI_LOGITS && have_nxt) tab_store<BN, EPI>(p, sm, e, nxt);   // published by the next tile's barrier
+            if (EPI <= EPI_LOGITS && have_nxt) tab_store<BN, EPI, CG>(p, sm, e, nxt);   // published by the next tile's barrier
         }
     }
 

@@ -62,6 +62,7 @@ int gemm_init() {
     if ((rc = set_attr_both<EPI_GELU, 1>())) return rc;
     if ((rc = set_attr<256, EPI_GELU, 1, 2>())) return rc;
     if ((rc = set_attr<256, EPI_CLIP8, 1, 2>())) return rc;
+    if ((rc = set_attr<256, EPI_VOTE, 0, 2>())) return rc;
     if ((rc = set_attr_both<EPI_PRE32, 1>())) return rc;
     if ((rc = set_attr_both<EPI_QKV, 1>())) return rc;
     if ((rc = set_attr<256, EPI_HEAD>())) return rc;
@@ -286,9 +287,9 @@ static int launch_one(cudaStream_t st, const CUtensorMap &ta, const CUtensorMap 
 }
 
 // Pairs of blocks with the tiles of 256 columns of two row tiles.
-template <int EPI>
+template <int EPI, int RPL>
 static int launch_pair(cudaStream_t st, const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &to, const GemmParams &p, int num_sms) {
-    auto kern = gemm_i8_kernel<256, EPI, 1, 2>;
+    auto kern = gemm_i8_kernel<256, EPI, RPL, 2>;
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(GEMM_THREADS);
     cfg.dynamicSmemBytes = gemm_smem_bytes<256, 2>();
@@ -306,7 +307,7 @@ static int launch_pair(cudaStream_t st, const CUtensorMap &ta, const CUtensorMap
         if (n < 1) { set_error("no pair of blocks of the GEMM fits on the device"); return EGG_E_CUDA; }
         most = n < num_sms / 2 ? n : num_sms / 2;
     }
-    const int tiles = ((p.M + 2 * GEMM_BM - 1) / (2 * GEMM_BM)) * (p.N / 256);
+    const int tiles = ((p.M + 2 * GEMM_BM - 1) / (2 * GEMM_BM)) * (p.N / 256) * ((EPI == EPI_VOTE && p.k_splits > 1) ? p.k_splits : 1);
     cfg.gridDim = dim3((unsigned)(2 * (tiles < most ? tiles : most)));
     if (t_chain) {
         attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -370,8 +371,9 @@ int launch_gemm(cudaStream_t st, int epi, const int8_t *A, const int8_t *B, cons
     p.pow_t = epi == EPI_GELU || epi == EPI_LOGITS ? merged_shift(p.K, p.rank1_shift, p.out_shift) : 0;
     CUtensorMap ta, tb;
     int rc;
-    const bool pair = (epi == EPI_GELU || epi == EPI_CLIP8) && bn == 256 && p.seq_len % 32 == 0 && p.rpl >= 0 && p.K >= PAIR_MIN_K &&
-                      (int64_t)((p.M + GEMM_BM - 1) / GEMM_BM) * (p.N / 256) >= 4 * num_sms;
+    const int rows_m = (p.M + GEMM_BM - 1) / GEMM_BM;
+    const bool pair = bn == 256 && ((epi == EPI_VOTE && p.K >= PAIR_MIN_K && rows_m % 2 == 0 && (int64_t)rows_m * (p.N / 256) * (p.k_splits > 1 ? p.k_splits : 1) >= num_sms) ||
+                                    ((epi == EPI_GELU || epi == EPI_CLIP8) && p.seq_len % 32 == 0 && p.rpl >= 0 && p.K >= PAIR_MIN_K && (int64_t)rows_m * (p.N / 256) >= 4 * num_sms));
     if ((rc = make_tmap(&ta, A, (uint64_t)p.M, (uint64_t)p.K, GEMM_BM))) return rc;
     if ((rc = make_tmap(&tb, B, (uint64_t)p.N, (uint64_t)p.K, (uint32_t)(pair ? bn / 2 : bn)))) return rc;
     CUtensorMap to = ta;       // only the row-per-lane int32 epilogues store through a tensor map
@@ -381,7 +383,10 @@ int launch_gemm(cudaStream_t st, int epi, const int8_t *A, const int8_t *B, cons
     if (epi == EPI_LOGITS || ((epi == EPI_GELU || epi == EPI_CLIP8) && bn == 256 && p.seq_len % 32 == 0 && p.rpl >= 0)) {
         if ((rc = make_tmap_out8(&to, p.out8, (uint64_t)p.M, (uint64_t)p.N))) return rc;
     }
-    if (pair) return epi == EPI_GELU ? launch_pair<EPI_GELU>(st, ta, tb, to, p, num_sms) : launch_pair<EPI_CLIP8>(st, ta, tb, to, p, num_sms);
+    if (pair) {
+        if (epi == EPI_VOTE) return launch_pair<EPI_VOTE, 0>(st, ta, tb, to, p, num_sms);
+        return epi == EPI_GELU ? launch_pair<EPI_GELU, 1>(st, ta, tb, to, p, num_sms) : launch_pair<EPI_CLIP8, 1>(st, ta, tb, to, p, num_sms);
+    }
     switch (epi) {
         case EPI_CLIP8: return launch_eval<EPI_CLIP8>(st, bn, ta, tb, to, p, num_sms);
         case EPI_GELU: return launch_eval<EPI_GELU>(st, bn, ta, tb, to, p, num_sms);

@@ -378,14 +378,18 @@ int launch_upd_operands(cudaStream_t st, const UpdPlan &pl, const UpdBatch &b, c
 // matrices is 114 to 456 tiles, where each matrix alone left the GPU mostly idle or cut its contraction into 8 to 64 pieces.
 // A tile's last 128 columns may lie beyond its matrix (rows_k an odd multiple of 128): they multiply whatever rows follow and
 // are not stored.
-constexpr int UV_BM = 128, UV_BN = 256, UV_BK = 128, UV_STAGES = 4, UV_EPI_WARPS = 8;
+// CG == 2: pairs of blocks form 256 x 256 tiles together (cta_group::2), each block with 128 rows of both operands; the second half of a
+// matrix's last tile may lie beyond it in the same way.
+constexpr int UV_BM = 128, UV_BN = 256, UV_BK = 128, UV_EPI_WARPS = 8;
 constexpr int UV_THREADS = 64 + UV_EPI_WARPS * 32;
 constexpr int UV_MAX_MATS = 512;
 
+template <int CG>
 struct UpdVoteSmem {
-    alignas(1024) uint8_t a[UV_STAGES][UV_BM * UV_BK];
-    alignas(1024) uint8_t b[UV_STAGES][UV_BN * UV_BK];
-    alignas(8) uint64_t full[UV_STAGES], empty[UV_STAGES], tmem_full[2], tmem_empty[2];
+    static constexpr int ST = CG == 2 ? 6 : 4;          // ring stages
+    alignas(1024) uint8_t a[ST][UV_BM * UV_BK];
+    alignas(1024) uint8_t b[ST][UV_BN / CG * UV_BK];
+    alignas(8) uint64_t full[ST], empty[ST], tmem_full[2], tmem_empty[2];
     int tile0[UV_MAX_MATS];
     uint32_t tmem_base;
     volatile int abort_flag;
@@ -398,28 +402,37 @@ struct UpdVoteParams {
     int *err;
 };
 
+template <int CG>
 __global__ void __launch_bounds__(UV_THREADS, 1)
 upd_votes_kernel(const __grid_constant__ CUtensorMap tab_a, const __grid_constant__ CUtensorMap tab_b, const __grid_constant__ CUtensorMap fn_a,
                  const __grid_constant__ CUtensorMap fn_b, const UpdVoteParams p) {
     extern __shared__ uint8_t uv_raw[];
-    UpdVoteSmem &sm = *reinterpret_cast<UpdVoteSmem *>((reinterpret_cast<uintptr_t>(uv_raw) + 1023) & ~uintptr_t(1023));
+    using Smem = UpdVoteSmem<CG>;
+    constexpr int ST = Smem::ST;
+    Smem &sm = *reinterpret_cast<Smem *>((reinterpret_cast<uintptr_t>(uv_raw) + 1023) & ~uintptr_t(1023));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     chain_next();
     const int items = p.tiles * p.splits, kb_per = (p.num_kb + p.splits - 1) / p.splits;
+    const int prow = CG == 2 ? (int)(blockIdx.x & 1) : 0;           // this block of the pair (clusters are consecutive blocks)
+    const int first_item = (int)blockIdx.x / CG, item_step = (int)gridDim.x / CG;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < UV_STAGES; s++) { ptx::mbar_init(&sm.full[s], 1); ptx::mbar_init(&sm.empty[s], 1); }
-        for (int a = 0; a < 2; a++) { ptx::mbar_init(&sm.tmem_full[a], 1); ptx::mbar_init(&sm.tmem_empty[a], UV_EPI_WARPS); }
+        for (int s = 0; s < ST; s++) { ptx::mbar_init(&sm.full[s], 1); ptx::mbar_init(&sm.empty[s], 1); }
+        for (int a = 0; a < 2; a++) { ptx::mbar_init(&sm.tmem_full[a], 1); ptx::mbar_init(&sm.tmem_empty[a], CG * UV_EPI_WARPS); }
         sm.abort_flag = 0;
         ptx::fence_barrier_init();
     }
     for (int i = threadIdx.x; i < p.nmats; i += UV_THREADS) sm.tile0[i] = p.mats[i].tile0;
     if (warp == 1) {
-        ptx::tmem_alloc(&sm.tmem_base, 512);
-        ptx::tmem_relinquish();
+        if (CG == 2) ptx::tmem_alloc_pair(&sm.tmem_base, 512);
+        else {
+            ptx::tmem_alloc(&sm.tmem_base, 512);
+            ptx::tmem_relinquish();
+        }
     }
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
+    if (CG == 2) ptx::cluster_sync_all();          // the other block's barriers exist before anything arrives on them
     chain_wait();
     const uint32_t tmem_base = sm.tmem_base;
     auto find = [&](int tile) {                   // matrix that owns the tile
@@ -439,21 +452,28 @@ upd_votes_kernel(const __grid_constant__ CUtensorMap tab_a, const __grid_constan
             uint32_t it = 0;
             bool ok = true;
             const int form = *p.range >> 2 & 1;
-            for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+            const uint32_t full_s = CG == 2 ? ptx::mapa_u32(ptx::smem_u32(sm.full), 0u) : 0u;          // of the even block
+            for (int item = first_item; item < items && ok; item += item_step) {
                 const int split = item / p.tiles, tile = item - split * p.tiles;
                 const UpdMat &m = p.mats[find(tile)];
                 const UpdForm f = m.form[form];
                 const int local = tile - m.tile0, tm = local / m.tiles_n, tn = local - tm * m.tiles_n;
-                const int ya = tm * UV_BM + (f.fn_is_n ? f.fn_row0 : 0), yb = tn * UV_BN + (f.fn_is_n ? 0 : f.fn_row0);
+                const int ya = (tm * CG + prow) * UV_BM + (f.fn_is_n ? f.fn_row0 : 0), yb = tn * UV_BN + prow * (UV_BN / CG) + (f.fn_is_n ? 0 : f.fn_row0);
                 const int xa = f.fn_is_n ? 0 : f.x_tab, xb = f.fn_is_n ? f.x_tab : 0;
                 const CUtensorMap *ta = f.fn_is_n ? &fn_a : &tab_a, *tb = f.fn_is_n ? &tab_b : &fn_b;
                 const int kb1 = min(p.num_kb, (split + 1) * kb_per);
                 for (int kb = split * kb_per; kb < kb1; kb++, it++) {
-                    const int s = it % UV_STAGES;
-                    if (!ptx::mbar_wait(&sm.empty[s], ((it / UV_STAGES) & 1) ^ 1) || sm.abort_flag) { fail(DEV_TIMEOUT_EMPTY); ok = false; break; }
-                    ptx::mbar_arrive_expect_tx(&sm.full[s], (UV_BM + UV_BN) * UV_BK);
-                    ptx::tma_load_2d(sm.a[s], ta, &sm.full[s], xa + kb * UV_BK, ya);
-                    ptx::tma_load_2d(sm.b[s], tb, &sm.full[s], xb + kb * UV_BK, yb);
+                    const int s = it % ST;
+                    if (!ptx::mbar_wait(&sm.empty[s], ((it / ST) & 1) ^ 1) || sm.abort_flag) { fail(DEV_TIMEOUT_EMPTY); ok = false; break; }
+                    if (CG == 2) {
+                        if (prow == 0) ptx::mbar_arrive_expect_tx(&sm.full[s], 2 * (UV_BM + UV_BN / CG) * UV_BK);          // both blocks' bytes
+                        ptx::tma_load_2d_pair(sm.a[s], ta, full_s + 8 * s, xa + kb * UV_BK, ya);
+                        ptx::tma_load_2d_pair(sm.b[s], tb, full_s + 8 * s, xb + kb * UV_BK, yb);
+                    } else {
+                        ptx::mbar_arrive_expect_tx(&sm.full[s], (UV_BM + UV_BN) * UV_BK);
+                        ptx::tma_load_2d(sm.a[s], ta, &sm.full[s], xa + kb * UV_BK, ya);
+                        ptx::tma_load_2d(sm.b[s], tb, &sm.full[s], xb + kb * UV_BK, yb);
+                    }
                 }
             }
             if (!ok) {   // let copies already in flight land before the block tears down
@@ -462,36 +482,42 @@ upd_votes_kernel(const __grid_constant__ CUtensorMap tab_a, const __grid_constan
             }
         }
     } else if (warp == 1) {
-        if (ptx::elect_one()) {
-            constexpr uint32_t idesc = ptx::make_idesc_i8(UV_BM, UV_BN);
+        if (prow == 0 && ptx::elect_one()) {
+            constexpr uint32_t idesc = ptx::make_idesc_i8(CG * UV_BM, UV_BN);
             uint32_t it = 0, tc = 0;
             bool ok = true;
-            for (int item = blockIdx.x; item < items && ok; item += gridDim.x, tc++) {
+            for (int item = first_item; item < items && ok; item += item_step, tc++) {
                 const int split = item / p.tiles, as = tc & 1;
                 if (!ptx::mbar_wait(&sm.tmem_empty[as], ((tc >> 1) & 1) ^ 1) || sm.abort_flag) { fail(DEV_TIMEOUT_TMEM_EMPTY); break; }
                 ptx::tc_fence_after();
                 const uint32_t d = tmem_base + (uint32_t)(as * UV_BN);
                 const int kb0 = split * kb_per, kb1 = min(p.num_kb, kb0 + kb_per);
                 for (int kb = kb0; kb < kb1; kb++, it++) {
-                    const int s = it % UV_STAGES;
-                    if (!ptx::mbar_wait(&sm.full[s], (it / UV_STAGES) & 1) || sm.abort_flag) { fail(DEV_TIMEOUT_FULL); ok = false; break; }
+                    const int s = it % ST;
+                    if (!ptx::mbar_wait(&sm.full[s], (it / ST) & 1) || sm.abort_flag) { fail(DEV_TIMEOUT_FULL); ok = false; break; }
                     ptx::tc_fence_after();
                     const uint64_t da = ptx::make_smem_desc_sw128(ptx::smem_u32(sm.a[s])), db = ptx::make_smem_desc_sw128(ptx::smem_u32(sm.b[s]));
 #pragma unroll
-                    for (int k = 0; k < UV_BK / 32; k++) ptx::mma_i8(d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
-                    ptx::mma_commit(&sm.empty[s]);
+                    for (int k = 0; k < UV_BK / 32; k++) {
+                        if (CG == 2) ptx::mma_i8_pair(d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+                        else ptx::mma_i8(d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+                    }
+                    if (CG == 2) ptx::mma_commit_pair(&sm.empty[s], 0); else ptx::mma_commit(&sm.empty[s]);
                 }
-                if (ok) ptx::mma_commit(&sm.tmem_full[as]);
+                if (ok) {
+                    if (CG == 2) ptx::mma_commit_pair(&sm.tmem_full[as], 0); else ptx::mma_commit(&sm.tmem_full[as]);
+                }
             }
         }
     } else {
         const int quarter = warp & 3, half = (warp - 2) >> 2;         // TMEM lane quarter, half of the tile's columns
+        const uint32_t tmem_empty_s = CG == 2 ? ptx::mapa_u32(ptx::smem_u32(sm.tmem_empty), 0u) : 0u;          // of the even block
         uint32_t tc = 0;
-        for (int item = blockIdx.x; item < items; item += gridDim.x, tc++) {
+        for (int item = first_item; item < items; item += item_step, tc++) {
             const int split = item / p.tiles, tile = item - split * p.tiles, as = tc & 1;
             const UpdMat &m = p.mats[find(tile)];
             const int local = tile - m.tile0, tm = local / m.tiles_n, tn = local - tm * m.tiles_n;
-            const int n = tm * UV_BM + quarter * 32 + lane, kbase = tn * UV_BN + half * 128;
+            const int n = (tm * CG + prow) * UV_BM + quarter * 32 + lane, kbase = tn * UV_BN + half * 128;
             const int cols_n = m.cols_n, rows_k = m.rows_k;
             int32_t *vout = p.votes + (int64_t)split * p.split_stride + m.votes_off;
             const bool ok = ptx::mbar_wait(&sm.tmem_full[as], (tc >> 1) & 1) && !sm.abort_flag;
@@ -499,7 +525,7 @@ upd_votes_kernel(const __grid_constant__ CUtensorMap tab_a, const __grid_constan
             ptx::tc_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(as * UV_BN + half * 128);
 #pragma unroll 1
-            for (int c = 0; c < 128 && kbase + c < rows_k; c += 32) {
+            for (int c = 0; c < 128 && kbase + c < rows_k && (CG == 1 || n < cols_n); c += 32) {
                 uint32_t v[32];
                 ptx::tmem_ld32(taddr + c, v);
                 ptx::tmem_ld_wait();
@@ -511,23 +537,28 @@ upd_votes_kernel(const __grid_constant__ CUtensorMap tab_a, const __grid_constan
             }
             ptx::tc_fence_before();
             __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&sm.tmem_empty[as]);
+            if (lane == 0) {
+                if (CG == 2) ptx::mbar_arrive_peer(tmem_empty_s + 8 * as); else ptx::mbar_arrive(&sm.tmem_empty[as]);
+            }
         }
     }
     __syncwarp();
     ptx::tc_fence_before();
     __syncthreads();
+    if (CG == 2) ptx::cluster_sync_all();          // a pair gives its tensor memory back together, after both blocks' reads
     if (warp == 1) {
         ptx::tc_fence_after();
-        ptx::tmem_dealloc(tmem_base, 512);
+        if (CG == 2) ptx::tmem_dealloc_pair(tmem_base, 512); else ptx::tmem_dealloc(tmem_base, 512);
     }
+    if (CG == 2) { __syncwarp(); ptx::cluster_sync_all(); }          // neither block retires before the other is done with its memory
 }
 
 int upd_init() {
     static bool done[EGG_MAX_DEVICES] = {};
     bool &d = done[current_device_slot()];
     if (d) return EGG_OK;
-    EGG_CUDA(cudaFuncSetAttribute(upd_votes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(UpdVoteSmem) + 1024));
+    EGG_CUDA(cudaFuncSetAttribute(upd_votes_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(UpdVoteSmem<1>) + 1024));
+    EGG_CUDA(cudaFuncSetAttribute(upd_votes_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(UpdVoteSmem<2>) + 1024));
     d = true;
     return EGG_OK;
 }
@@ -536,14 +567,29 @@ int launch_upd_votes(cudaStream_t st, const UpdPlan &pl, const UpdBatch &b, cons
     CUtensorMap ta, tb, fa, fb;
     int rc;
     const uint64_t fn_rows = (uint64_t)std::max(b.fn_rows[0], b.fn_rows[1]);
-    if ((rc = upd_tensor_map(&ta, tab, (uint64_t)pl.W, (uint64_t)pl.pitch, UV_BM)) || (rc = upd_tensor_map(&tb, tab, (uint64_t)pl.W, (uint64_t)pl.pitch, UV_BN)) ||
-        (rc = upd_tensor_map(&fa, fn, fn_rows, (uint64_t)pl.kp, UV_BM)) || (rc = upd_tensor_map(&fb, fn, fn_rows, (uint64_t)pl.kp, UV_BN)))
+    const uint32_t b_rows = UV_BN / pl.cg;
+    if ((rc = upd_tensor_map(&ta, tab, (uint64_t)pl.W, (uint64_t)pl.pitch, UV_BM)) || (rc = upd_tensor_map(&tb, tab, (uint64_t)pl.W, (uint64_t)pl.pitch, b_rows)) ||
+        (rc = upd_tensor_map(&fa, fn, fn_rows, (uint64_t)pl.kp, UV_BM)) || (rc = upd_tensor_map(&fb, fn, fn_rows, (uint64_t)pl.kp, b_rows)))
         return rc;
     UpdVoteParams p;
     p.mats = pl.d_mats + b.first; p.nmats = b.count; p.tiles = b.tiles; p.splits = b.splits; p.num_kb = pl.kp / UV_BK;
     p.range = range; p.votes = votes; p.split_stride = b.votes; p.err = err;
     const int items = b.tiles * b.splits;
-    EGG_CUDA(launch_chained(upd_votes_kernel, items < num_sms ? items : num_sms, UV_THREADS, sizeof(UpdVoteSmem) + 1024, st, ta, tb, fa, fb, p));
+    if (pl.cg == 1) {
+        EGG_CUDA(launch_chained(upd_votes_kernel<1>, items < num_sms ? items : num_sms, UV_THREADS, sizeof(UpdVoteSmem<1>) + 1024, st, ta, tb, fa, fb, p));
+    } else {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[2];
+        cfg.blockDim = dim3(UV_THREADS); cfg.dynamicSmemBytes = sizeof(UpdVoteSmem<2>) + 1024; cfg.stream = st;
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr; cfg.numAttrs = t_chain ? 2 : 1;
+        const int most = num_sms / 2;             // where fewer pairs are resident, the others follow
+        cfg.gridDim = dim3((unsigned)(2 * (items < most ? items : most)));
+        EGG_CUDA(cudaLaunchKernelEx(&cfg, upd_votes_kernel<2>, ta, tb, fa, fb, p));
+    }
     EGG_CUDA(cudaGetLastError());
     return EGG_OK;
 }
@@ -661,6 +707,16 @@ int upd_plan_build(UpdPlan &pl, const std::vector<ParamDesc> &params, const std:
     pl.pairs = pairs;
     pl.kp = (pairs + 15 + 127) / 128 * 128;
     pl.W = std::max(4 * hidden, vocab);
+    // Vote tiles in pairs of blocks: half of one operand's traffic from L2, which bounds the product.  Per tile of 128 columns they take 0.73
+    // to 0.82 of the time (163 840 pairs, H 256: 581 -> 427 us; 131 072, H 1024: 12.2 -> 10.0 ms; 20 480, H 512: 292 -> 211 us; 4096, H 256: 23 -> 19;
+    // 256: the same), so that a model takes them unless odd multiples of 128 outputs leave more than a fifth of their halves empty.
+    int64_t single = 0, paired = 0;
+    for (const ParamDesc &d : params)
+        if (d.rows_k) {
+            const int64_t tn = (d.rows_k + UV_BN - 1) / UV_BN;
+            single += d.cols_n / UV_BM * tn; paired += (d.cols_n + 2 * UV_BM - 1) / (2 * UV_BM) * 2 * tn;
+        }
+    pl.cg = 5 * single >= 4 * paired ? 2 : 1;
     std::vector<std::pair<int, int>> need;                   // table columns [first, last)
     auto want = [&](int s) { need.push_back({s & ~127, (s + UPD_ORIGIN + pl.kp + 64 + 127) & ~127}); };
     for (size_t i = 0; i < params.size(); i++) {
@@ -711,7 +767,7 @@ int upd_plan_build(UpdPlan &pl, const std::vector<ParamDesc> &params, const std:
             const int per = (num_kb + s - 1) / s;
             if ((num_kb + per - 1) / per != s) continue;     // no empty split
             if (b.votes * s > std::max<int64_t>(UPD_VOTE_ELEMS, b.votes)) break;
-            const int64_t waves = ((int64_t)b.tiles * s + num_sms - 1) / num_sms, cost = waves * (per + 6) * 16 + s;
+            const int64_t waves = ((int64_t)b.tiles * s + num_sms / pl.cg - 1) / (num_sms / pl.cg), cost = waves * (per + 6) * 16 + s;
             if (best < 0 || cost < best) { best = cost; b.splits = s; }
         }
         pl.fn_bytes = std::max(pl.fn_bytes, (int64_t)std::max(b.fn_rows[0], b.fn_rows[1]) * pl.kp);
@@ -740,7 +796,7 @@ int upd_plan_build(UpdPlan &pl, const std::vector<ParamDesc> &params, const std:
         m.tile0 = b.tiles; m.tiles_n = (d.rows_k + UV_BN - 1) / UV_BN; m.blk0 = b.blocks; m.muon = d.muon;
         m.lr_scale = d.lr_scale; m.model_off = d.model_off; m.opt_off = d.opt_off; m.shadow_off = d.shadow_off; m.votes_off = b.votes;
         m.ov_in = d.ov_in; m.ov_out = d.ov_out;
-        b.tiles += d.cols_n / UV_BM * m.tiles_n; b.blocks += d.cols_n / 32 * (d.rows_k / 128); b.votes += wts; b.count++;
+        b.tiles += (d.cols_n + pl.cg * UV_BM - 1) / (pl.cg * UV_BM) * m.tiles_n; b.blocks += d.cols_n / 32 * (d.rows_k / 128); b.votes += wts; b.count++;
         b.any_adam |= !d.muon;
         pl.mats.push_back(m);
         pl.mat_param.push_back((int)i);

@@ -56,6 +56,7 @@ struct MuonGroup { int batch, rows, cols, first, count, slot; };      // first: 
 
 // Host plan of an update over a set of parameters: batches of matrices that fit the workspace, device descriptors.
 struct UpdPlan {
+    int cg;                           // blocks that form a vote tile together
     std::vector<UpdMat> mats;
     std::vector<int> mat_param;       // index into the parameter list
     std::vector<UpdVec> vecs;         // the 4H-long ones first

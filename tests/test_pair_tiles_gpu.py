@@ -5,7 +5,7 @@ pair forms one twice and stores it once), tiles of one member and of several, su
 import numpy as np
 import pytest
 
-from common import load_oracle, load_pkg, make_case
+from common import cfg_pair, load_oracle, load_pkg, make_case
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +38,42 @@ def test_pairs_equal_single_blocks_and_oracle(hidden, layers, seq, pop):
     assert (got == losses(0)).all()
     for first in (0, pop - 4):
         assert (got[first:first + 4] == O.eval_losses(ocfg, model, data, seq, SEED + 5, first, 4)).all(), first
+
+
+@pytest.mark.parametrize("hidden,layers,pairs", [
+    (256, 2, 1300),            # 11 blocks of the contraction in several splits
+    (384, 1, 1501),            # three tiles of 128 outputs: the second half of the last pair's tile is not stored
+    (640, 1, 300),             # five; contraction of three blocks
+])
+def test_vote_tiles_of_pairs(hidden, layers, pairs):
+    pkg, O = load_pkg(), load_oracle()
+    kw = dict(hidden_dim=hidden, n_layers=layers, seq_len=16, population_size=2 * pairs, device_mask=15)
+    cfg, ocfg, model, data = make_case(kw, data_len=4000, model_kind="random_all", model_seed=3)
+    opt = np.zeros(O.opt_bytes(ocfg), np.uint8)
+    ctx = pkg.Context(cfg, 0, 2)
+    ctx.upload_model(model)
+    fit = np.random.RandomState(hidden).randint(-1, 2, pairs).astype(np.int32)
+    ctx.write_fitness(fit)
+    assert ctx.apply_update(SEED, 0.4) == O.update(ocfg, model, opt, fit, SEED, 0.4)
+    assert (ctx.download_model() == model).all()
+    assert (ctx.download_opt_state() == opt).all()
+    ctx.close()
+
+
+@pytest.mark.parametrize("rows,cols,pairs", [
+    (512, 1024, 2000),         # tiles and splits of the contraction enough for pairs
+    (512, 1152, 2000),         # nine row tiles of outputs: single blocks
+])
+def test_isolated_votes_of_pairs(rows, cols, pairs):
+    import torch
+    pkg, O = load_pkg(), load_oracle()
+    cfg, ocfg = cfg_pair(device_mask=3, population_size=2 * pairs)
+    fit = np.random.RandomState(rows + cols).randint(-1, 2, pairs).astype(np.int32)
+    ctx = pkg.Context(cfg, 0, 2)
+    d_fit, votes = torch.from_numpy(fit).cuda(), torch.zeros(rows * cols, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    ctx.update_reconstruct(d_fit.data_ptr(), pairs, rows, cols, 402, 403, 1000, 2, votes.data_ptr(), on_device=True)
+    ctx.close()
+    n_list = np.arange(0, cols, 37).astype(np.int32)
+    got = votes.cpu().numpy().reshape(rows // 4, cols, 4)[:, n_list, :].transpose(1, 0, 2).reshape(len(n_list), rows)      # packed order [k/4][n][4]
+    assert (got == O.vote_columns(ocfg, fit, rows, 402, 403, 1000, 2, n_list)).all()
