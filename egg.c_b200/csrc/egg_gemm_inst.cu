@@ -33,6 +33,10 @@ static int set_attr_fused_one() {
 template <int BN, bool MM>
 static int set_attr_fused() {
     int rc;
+    if constexpr (BN == 256 && !MM) {
+        if ((rc = set_attr_fused_one<BN, FUSED_QKV, MM, false, 2>()) || (rc = set_attr_fused_one<BN, FUSED_RES, MM, false, 2>()) ||
+            (rc = set_attr_fused_one<BN, FUSED_RES, MM, true, 2>())) return rc;
+    }
     if ((rc = set_attr_fused_one<BN, FUSED_QKV, MM, false>())) return rc;
     if ((rc = set_attr_fused_one<BN, FUSED_RES, MM, false>())) return rc;
     if ((rc = set_attr_fused_one<BN, FUSED_RES, MM, true>())) return rc;
@@ -212,7 +216,7 @@ static int launch_fused_cg(cudaStream_t st, const CUtensorMap &ta, const CUtenso
 template <int BN, int MODE, bool MM, bool FORM = false>
 static int launch_fused_one(cudaStream_t st, const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &to, const CUtensorMap &tr,
                             const FusedParams &p, int units, int num_sms) {
-    if constexpr (MODE == FUSED_RES_LN) {
+    if constexpr (MODE == FUSED_RES_LN || (BN == 256 && !MM)) {
         if (p.pair) return launch_fused_cg<BN, MODE, MM, FORM, 2>(st, ta, tb, to, tr, p, units, num_sms);
     }
     return launch_fused_cg<BN, MODE, MM, FORM, 1>(st, ta, tb, to, tr, p, units, num_sms);
@@ -251,10 +255,13 @@ int launch_gemm_fused(cudaStream_t st, int mode, const int8_t *A, const int8_t *
     const bool mm = p.seq_len % GEMM_BM != 0;        // a tile spans members: four table sets, see the kernel
     const int bn = (mm ? hl == 256 : hl % 256 == 0) ? 256 : 128;      // (128-column sub-tiles at H = 512 were measured: +30 % on MLP-down)
     // Pairs of blocks where the products wait for their operands: a 128 x 256 tile takes 96 bytes a clock at the tensor cores' rate and an SM
-    // gets some 57, a pair's half needs 64.  Only below long contractions, whose epilogue is short beside them: the two blocks' epilogues
-    // wait for one another.  Residual products per evaluation of 4 or 2 layers: K 2048 8.24 -> 7.17 ms, 2560 2.43 -> 2.21, 4096 3.49 -> 3.29,
-    // 1536 1.52 -> 1.46; but K 1024 1.67 -> 1.87, and Q|K|V (K = H) 2 to 30 % longer.  Not where pairs would leave SMs without a unit.
-    p.pair = mode == FUSED_RES_LN && p.K >= 1536 && units >= 2 * num_sms;
+    // gets some 57, a pair's half needs 64.  The two blocks' epilogues wait for one another, so not where those are the longer part.
+    // Down projection with the norm, per evaluation of 4 or 2 layers: K 2048 8.24 -> 7.01 ms, 2560 2.43 -> 2.17, 4096 3.49 -> 3.31, 1536 1.52 ->
+    // 1.41, but 1024 2 to 4 % longer.  Q|K|V in tiles of one member and 256 columns, one block to a row: H 512 5.94 -> 5.48, H 256 2.84 -> 2.74;
+    // output projection at H 512 5 % shorter, at H 256 as much longer.  Tiles of several members, narrower ones and rows of two
+    // blocks: Q|K|V 2 to 12 % longer.  Not where pairs would leave SMs without a unit.
+    const bool wide = p.cl == 1 && bn == 256 && !mm;
+    p.pair = units >= 2 * num_sms && (mode == FUSED_RES_LN ? p.K >= 1536 : wide && (mode == FUSED_QKV || p.K >= 512));
     if (p.pair) units = (p.M / GEMM_BM + 1) / 2 * p.parts;
     p.fd_seq = make_fastdiv(p.seq_len);
     p.fd_h = make_fastdiv(p.H);
@@ -331,10 +338,10 @@ static int launch_eval(cudaStream_t st, int bn, const CUtensorMap &ta, const CUt
     return launch_bn<EPI, 0>(st, bn, ta, tb, to, p, num_sms);
 }
 
-// Contractions from which pairs of blocks form the tiles (see launch_gemm_fused for what bounds them): K 1024 0.347 -> 0.330 ms and, in
-// MLP-up, 2.45 -> 2.35; 2048 0.52 -> 0.46; 4096 3.40 -> 2.97 (2.6 -> 3.0 int8 POP/s); but K 640 1.26 -> 1.45 and 512 6.2 -> 7.3: there the
-// epilogues are as long as the products, and those of a pair wait for one another.
-constexpr int PAIR_MIN_K = 1024;
+// Contractions from which pairs of blocks form the tiles (see launch_gemm_fused for what bounds them).  MLP-up: K 384 0.89 -> 0.87 ms,
+// 512 5.75 -> 5.45, 640 1.23 -> 1.09, 768 1.70 -> 1.45, 896 2.22 -> 1.85, 1024 2.45 -> 1.99; projections of as many columns: 512 0.155 ->
+// 0.146, 2048 0.52 -> 0.46, 4096 3.40 -> 2.92 (2.6 -> 3.0 int8 POP/s).  At K 256 between 2 % shorter and 1 % longer.
+constexpr int PAIR_MIN_K = 384;
 
 int launch_gemm(cudaStream_t st, int epi, const int8_t *A, const int8_t *B, const GemmParams &p_in, int num_sms) {
     GemmParams p = p_in;
