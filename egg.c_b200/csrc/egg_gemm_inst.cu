@@ -102,12 +102,12 @@ int upd_tensor_map(void *map, const void *ptr, uint64_t rows, uint64_t pitch, ui
 }
 
 // [rows][cols] bf16 row-major; box = 64 columns x 128 rows, 128-byte swizzle
-int bf16_tensor_map(void *map, const void *ptr, uint64_t rows, uint64_t cols) {
+int bf16_tensor_map(void *map, const void *ptr, uint64_t rows, uint64_t cols, uint32_t box_rows) {
     if (!g_encode) { set_error("gemm_init() was not called"); return EGG_E_STATE; }
     if ((reinterpret_cast<uintptr_t>(ptr) & 15) || (cols & 7)) { set_error("bf16 operand is not 16-byte aligned (ptr %p, cols %llu)", ptr, (unsigned long long)cols); return EGG_E_INVALID; }
     cuuint64_t gdim[2] = {cols, rows};
     cuuint64_t gstride[1] = {cols * 2};
-    cuuint32_t box[2] = {64, 128};
+    cuuint32_t box[2] = {64, box_rows};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = g_encode(static_cast<CUtensorMap *>(map), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(ptr), gdim, gstride, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);

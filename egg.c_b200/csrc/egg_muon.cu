@@ -8,25 +8,30 @@
 // hi*hi accumulates apart from the rest, and both leave tensor memory after every 64 contraction steps to be added to fp32
 // registers with round-to-nearest: the tensor core's own additions truncate, and a chain of 4 is short enough not to show.
 // Against fp64 the result is closer than the ordered chain of fused multiply-adds it replaces (tests/test_muon_gpu.py).
-// Bound: tensor cores, six bf16 products per fp32 product; the Gram matrix is symmetric and computed once.
+// Bound: tensor cores, six bf16 products per fp32 product; the Gram matrix is symmetric and computed once (by pairs of blocks: its diagonal
+// tile pairs with one below the diagonal, which is formed and dropped).
 #include "egg_muon.cuh"
 #include "egg_ptx.cuh"
 
 #include <cuda.h>
 
+#include <algorithm>
+
 namespace egg {
 
 constexpr int NS_T = 128;                          // tile edge
 constexpr int NS_K = 64;                           // contraction per stage: one 128-byte swizzled row of bf16
-constexpr int NS_STAGES = 2;
 constexpr int NS_EPI_WARPS = 8;
 constexpr int NS_THREADS = 64 + NS_EPI_WARPS * 32;
 constexpr int NS_BOX = NS_T * NS_K * 2;
 
+// CG == 2: pairs of blocks (cta_group::2) form two row tiles of the same columns, each with its own 128 rows of A and half of B's.
+template <int CG>
 struct NsSmem {
-    alignas(1024) uint8_t a[NS_STAGES][3][NS_BOX];
-    alignas(1024) uint8_t b[NS_STAGES][3][NS_BOX];
-    alignas(8) uint64_t full[NS_STAGES], empty[NS_STAGES], tmem_full[2], tmem_empty[2];
+    static constexpr int ST = CG == 2 ? 3 : 2;         // stages
+    alignas(1024) uint8_t a[ST][3][NS_BOX];
+    alignas(1024) uint8_t b[ST][3][NS_BOX / CG];
+    alignas(8) uint64_t full[ST], empty[ST], tmem_full[2], tmem_empty[2];
     uint32_t tmem_base;
     volatile int abort_flag;
 };
@@ -50,6 +55,15 @@ __device__ __forceinline__ void mma_bf16(uint32_t d, uint64_t a, uint64_t b, uin
         : "memory");
 }
 
+__device__ __forceinline__ void mma_bf16_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
 // v = t[0] + t[1] + t[2] exactly (while the last term is above the smallest bf16)
 __device__ __forceinline__ void split3(float v, __nv_bfloat16 (&t)[3]) {
     t[0] = __float2bfloat16_rn(v);
@@ -58,38 +72,48 @@ __device__ __forceinline__ void split3(float v, __nv_bfloat16 (&t)[3]) {
     t[2] = __float2bfloat16_rn(r1 - __bfloat162float(t[1]));
 }
 
-template <int MODE>
+template <int MODE, int CG>
 __global__ void __launch_bounds__(NS_THREADS, 1)
 ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const NsParams p) {
     extern __shared__ uint8_t ns_raw[];
-    NsSmem &sm = *reinterpret_cast<NsSmem *>((reinterpret_cast<uintptr_t>(ns_raw) + 1023) & ~uintptr_t(1023));
+    using Smem = NsSmem<CG>;
+    constexpr int ST = Smem::ST;
+    Smem &sm = *reinterpret_cast<Smem *>((reinterpret_cast<uintptr_t>(ns_raw) + 1023) & ~uintptr_t(1023));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int items = p.tiles * p.nb, chunks = p.kdim / NS_K;
+    const int prow = CG == 2 ? (int)(blockIdx.x & 1) : 0;           // this block's row tile of the pair (clusters are consecutive blocks)
+    const int first_item = (int)blockIdx.x / CG, item_step = (int)gridDim.x / CG;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < NS_STAGES; s++) { ptx::mbar_init(&sm.full[s], 1); ptx::mbar_init(&sm.empty[s], 1); }
-        for (int a = 0; a < 2; a++) { ptx::mbar_init(&sm.tmem_full[a], 1); ptx::mbar_init(&sm.tmem_empty[a], NS_EPI_WARPS); }
+        for (int s = 0; s < ST; s++) { ptx::mbar_init(&sm.full[s], 1); ptx::mbar_init(&sm.empty[s], 1); }
+        for (int a = 0; a < 2; a++) { ptx::mbar_init(&sm.tmem_full[a], 1); ptx::mbar_init(&sm.tmem_empty[a], CG * NS_EPI_WARPS); }
         sm.abort_flag = 0;
         ptx::fence_barrier_init();
     }
     if (warp == 1) {
-        ptx::tmem_alloc(&sm.tmem_base, 512);
-        ptx::tmem_relinquish();
+        if (CG == 2) ptx::tmem_alloc_pair(&sm.tmem_base, 512);
+        else {
+            ptx::tmem_alloc(&sm.tmem_base, 512);
+            ptx::tmem_relinquish();
+        }
     }
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
+    if (CG == 2) ptx::cluster_sync_all();          // the other block's barriers exist before anything arrives on them
     const uint32_t tmem_base = sm.tmem_base;
     auto decode = [&](int item, int &mat, int &ti, int &tj) {
         mat = item / p.tiles;
         int t = item - mat * p.tiles;
-        if (MODE == NS_GRAM) {                     // row ti of the upper triangle holds tiles_j - ti tiles
+        if (MODE == NS_GRAM) {                     // row ti of the upper triangle holds tiles_j - ti tiles, and so do the CG rows from it on
             ti = 0;
-            while (t >= p.tiles_j - ti) { t -= p.tiles_j - ti; ti++; }
+            while (t >= p.tiles_j - ti) { t -= p.tiles_j - ti; ti += CG; }
             tj = ti + t;
         } else {
             ti = t / p.tiles_j;
             tj = t - ti * p.tiles_j;
+            ti *= CG;
         }
+        ti += prow;
     };
     auto fail = [&](int code) {
         sm.abort_flag = 1;
@@ -99,17 +123,24 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (ptx::elect_one()) {
             uint32_t it = 0;
             bool ok = true;
-            for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+            const uint32_t full_s = CG == 2 ? ptx::mapa_u32(ptx::smem_u32(sm.full), 0u) : 0u;          // of the even block
+            for (int item = first_item; item < items && ok; item += item_step) {
                 int mat, ti, tj;
                 decode(item, mat, ti, tj);
                 for (int c = 0; c < chunks; c++, it++) {
-                    const int s = it % NS_STAGES;
-                    if (!ptx::mbar_wait(&sm.empty[s], ((it / NS_STAGES) & 1) ^ 1) || sm.abort_flag) { fail(DEV_TIMEOUT_EMPTY); ok = false; break; }
-                    ptx::mbar_arrive_expect_tx(&sm.full[s], 6 * NS_BOX);
+                    const int s = it % ST;
+                    if (!ptx::mbar_wait(&sm.empty[s], ((it / ST) & 1) ^ 1) || sm.abort_flag) { fail(DEV_TIMEOUT_EMPTY); ok = false; break; }
+                    if (prow == 0) ptx::mbar_arrive_expect_tx(&sm.full[s], 3 * CG * (NS_BOX + NS_BOX / CG));          // of both blocks
 #pragma unroll
                     for (int q = 0; q < 3; q++) {
-                        ptx::tma_load_2d(sm.a[s][q], &map_a, &sm.full[s], c * NS_K, (q * p.nb + mat) * p.rows_a + ti * NS_T);
-                        ptx::tma_load_2d(sm.b[s][q], &map_b, &sm.full[s], c * NS_K, (q * p.nb + mat) * p.rows_b + tj * NS_T);
+                        const int ya = (q * p.nb + mat) * p.rows_a + ti * NS_T, yb = (q * p.nb + mat) * p.rows_b + tj * NS_T + prow * (NS_T / CG);
+                        if (CG == 2) {
+                            ptx::tma_load_2d_pair(sm.a[s][q], &map_a, full_s + 8 * s, c * NS_K, ya);
+                            ptx::tma_load_2d_pair(sm.b[s][q], &map_b, full_s + 8 * s, c * NS_K, yb);
+                        } else {
+                            ptx::tma_load_2d(sm.a[s][q], &map_a, &sm.full[s], c * NS_K, ya);
+                            ptx::tma_load_2d(sm.b[s][q], &map_b, &sm.full[s], c * NS_K, yb);
+                        }
                     }
                 }
             }
@@ -119,16 +150,16 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
         }
     } else if (warp == 1) {
-        if (ptx::elect_one()) {
-            // bf16 x bf16 -> fp32, both operands K-major, 128 x 128
-            constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NS_T >> 3) << 17) | ((uint32_t)(NS_T >> 4) << 24);
+        if (prow == 0 && ptx::elect_one()) {
+            // bf16 x bf16 -> fp32, both operands K-major, 128 columns
+            constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NS_T >> 3) << 17) | ((uint32_t)(CG * NS_T >> 4) << 24);
             uint32_t it = 0;
             bool ok = true;
-            for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+            for (int item = first_item; item < items && ok; item += item_step) {
                 for (int c = 0; c < chunks; c++, it++) {
-                    const int s = it % NS_STAGES, as = it & 1;
+                    const int s = it % ST, as = it & 1;
                     if (!ptx::mbar_wait(&sm.tmem_empty[as], ((it >> 1) & 1) ^ 1) || sm.abort_flag) { fail(DEV_TIMEOUT_TMEM_EMPTY); ok = false; break; }
-                    if (!ptx::mbar_wait(&sm.full[s], (it / NS_STAGES) & 1) || sm.abort_flag) { fail(DEV_TIMEOUT_FULL); ok = false; break; }
+                    if (!ptx::mbar_wait(&sm.full[s], (it / ST) & 1) || sm.abort_flag) { fail(DEV_TIMEOUT_FULL); ok = false; break; }
                     ptx::tc_fence_after();
                     const uint32_t d0 = tmem_base + (uint32_t)(as * 2 * NS_T), d1 = d0 + NS_T;
                     uint64_t a[3], b[3];
@@ -140,23 +171,27 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
                     for (int k = 0; k < NS_K / 16; k++) {
                         const uint64_t o = (uint64_t)(2 * k);          // 16 bf16 = 32 bytes along the swizzled row
-                        mma_bf16(d1, a[0] + o, b[2] + o, idesc, k > 0);
-                        mma_bf16(d1, a[2] + o, b[0] + o, idesc, 1);
-                        mma_bf16(d1, a[1] + o, b[1] + o, idesc, 1);
-                        mma_bf16(d1, a[0] + o, b[1] + o, idesc, 1);
-                        mma_bf16(d1, a[1] + o, b[0] + o, idesc, 1);
-                        mma_bf16(d0, a[0] + o, b[0] + o, idesc, k > 0);
+                        auto mma = [&](uint32_t d, int i, int j, uint32_t more) {
+                            if (CG == 2) mma_bf16_pair(d, a[i] + o, b[j] + o, idesc, more); else mma_bf16(d, a[i] + o, b[j] + o, idesc, more);
+                        };
+                        mma(d1, 0, 2, k > 0);
+                        mma(d1, 2, 0, 1);
+                        mma(d1, 1, 1, 1);
+                        mma(d1, 0, 1, 1);
+                        mma(d1, 1, 0, 1);
+                        mma(d0, 0, 0, k > 0);
                     }
-                    ptx::mma_commit(&sm.empty[s]);
-                    ptx::mma_commit(&sm.tmem_full[as]);
+                    if (CG == 2) { ptx::mma_commit_pair(&sm.empty[s], 0); ptx::mma_commit_pair(&sm.tmem_full[as], 0); }
+                    else { ptx::mma_commit(&sm.empty[s]); ptx::mma_commit(&sm.tmem_full[as]); }
                 }
             }
         }
     } else {
         const int quarter = warp & 3, half = (warp - 2) >> 2;
+        const uint32_t tmem_empty_s = CG == 2 ? ptx::mapa_u32(ptx::smem_u32(sm.tmem_empty), 0u) : 0u;          // of the even block
         uint32_t it = 0;
         bool ok = true;
-        for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+        for (int item = first_item; item < items && ok; item += item_step) {
             int mat, ti, tj;
             decode(item, mat, ti, tj);
             float acc[64];
@@ -181,9 +216,12 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 }
                 ptx::tc_fence_before();
                 __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(&sm.tmem_empty[as]);
+                if (lane == 0) {
+                    if (CG == 2) ptx::mbar_arrive_peer(tmem_empty_s + 8 * as); else ptx::mbar_arrive(&sm.tmem_empty[as]);
+                }
             }
             if (!ok) break;
+            if (MODE == NS_GRAM && CG == 2 && ti > tj) continue;            // below the diagonal: the pair's other tile is the diagonal one
             const int i = ti * NS_T + quarter * 32 + lane, j0 = tj * NS_T + half * 64;
             if (MODE == NS_LAST) {
                 float *o = p.y + ((int64_t)mat * p.rows_a + i) * p.rows_b + j0;
@@ -220,19 +258,27 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     __syncwarp();
     ptx::tc_fence_before();
     __syncthreads();
+    if (CG == 2) ptx::cluster_sync_all();          // a pair gives its tensor memory back together, after both blocks' reads
     if (warp == 1) {
         ptx::tc_fence_after();
-        ptx::tmem_dealloc(tmem_base, 512);
+        if (CG == 2) ptx::tmem_dealloc_pair(tmem_base, 512); else ptx::tmem_dealloc(tmem_base, 512);
     }
+    if (CG == 2) { __syncwarp(); ptx::cluster_sync_all(); }          // neither block retires before the other is done with its memory
+}
+
+template <int MODE>
+static int ns_init() {
+    EGG_CUDA(cudaFuncSetAttribute(ns_gemm_kernel<MODE, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(NsSmem<1>) + 1024));
+    EGG_CUDA(cudaFuncSetAttribute(ns_gemm_kernel<MODE, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(NsSmem<2>) + 1024));
+    return EGG_OK;
 }
 
 int muon_init() {
     static bool done[EGG_MAX_DEVICES] = {};
     bool &d = done[current_device_slot()];
     if (d) return EGG_OK;
-    EGG_CUDA(cudaFuncSetAttribute(ns_gemm_kernel<NS_GRAM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(NsSmem) + 1024));
-    EGG_CUDA(cudaFuncSetAttribute(ns_gemm_kernel<NS_STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(NsSmem) + 1024));
-    EGG_CUDA(cudaFuncSetAttribute(ns_gemm_kernel<NS_LAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(NsSmem) + 1024));
+    int rc;
+    if ((rc = ns_init<NS_GRAM>()) || (rc = ns_init<NS_STEP>()) || (rc = ns_init<NS_LAST>())) return rc;
     d = true;
     return EGG_OK;
 }
@@ -257,12 +303,28 @@ template <int MODE>
 static int launch_ns_gemm(cudaStream_t st, const __nv_bfloat16 *a, const __nv_bfloat16 *b, NsParams p, int num_sms) {
     CUtensorMap ma, mb;
     int rc;
-    if ((rc = bf16_tensor_map(&ma, a, 3ull * p.nb * p.rows_a, (uint64_t)p.kdim)) || (rc = bf16_tensor_map(&mb, b, 3ull * p.nb * p.rows_b, (uint64_t)p.kdim))) return rc;
     p.tiles_i = p.rows_a / NS_T; p.tiles_j = p.rows_b / NS_T;
-    p.tiles = MODE == NS_GRAM ? p.tiles_i * (p.tiles_i + 1) / 2 : p.tiles_i * p.tiles_j;
+    // Pairs from a smaller side of 512 on, where row tiles come in pairs.  A 128 x 128 tile in six products reads 128 bytes a clock from shared
+    // memory and 64 from L2 at the tensor cores' rate, a pair's 96 and 48.  Five steps of one 4096 x 4096 matrix 5.1 -> 4.5 ms, of the
+    // matrices of four layers at H 1024 17.9 -> 16.6, at H 768 (two layers) 4.38 -> 4.22; at H 512 a whole update 1.44 -> 1.43, at H 256 0.440 -> 0.444.
+    const int cg = std::min(p.rows_a, std::min(p.rows_b, p.kdim)) >= 512 && p.tiles_i % 2 == 0 ? 2 : 1;
+    if ((rc = bf16_tensor_map(&ma, a, 3ull * p.nb * p.rows_a, (uint64_t)p.kdim, NS_T)) || (rc = bf16_tensor_map(&mb, b, 3ull * p.nb * p.rows_b, (uint64_t)p.kdim, NS_T / cg))) return rc;
+    if (cg == 1) {
+        p.tiles = MODE == NS_GRAM ? p.tiles_i * (p.tiles_i + 1) / 2 : p.tiles_i * p.tiles_j;
+        const int items = p.tiles * p.nb;
+        ns_gemm_kernel<MODE, 1><<<items < num_sms ? items : num_sms, NS_THREADS, sizeof(NsSmem<1>) + 1024, st>>>(ma, mb, p);
+        EGG_CUDA(cudaGetLastError());
+        return EGG_OK;
+    }
+    p.tiles = MODE == NS_GRAM ? p.tiles_i / 2 * (p.tiles_i / 2 + 1) : p.tiles_i / 2 * p.tiles_j;          // pairs of tiles
     const int items = p.tiles * p.nb;
-    ns_gemm_kernel<MODE><<<items < num_sms ? items : num_sms, NS_THREADS, sizeof(NsSmem) + 1024, st>>>(ma, mb, p);
-    EGG_CUDA(cudaGetLastError());
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.blockDim = dim3(NS_THREADS); cfg.dynamicSmemBytes = sizeof(NsSmem<2>) + 1024; cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = 1;
+    cfg.gridDim = dim3((unsigned)(2 * (items < num_sms / 2 ? items : num_sms / 2)));
+    EGG_CUDA(cudaLaunchKernelEx(&cfg, ns_gemm_kernel<MODE, 2>, ma, mb, p));
     return EGG_OK;
 }
 

@@ -33,6 +33,6 @@ int launch_newton_schulz(cudaStream_t st, const NsWs &ws, int rows, int cols, in
 int launch_muon_apply(cudaStream_t st, const UpdMat *mats, const int *list, int nb, int rows, int cols, const float *y, int8_t *model, uint8_t *opt,
                       int8_t *shadow, float lr, float wd, unsigned long long *total);
 
-int bf16_tensor_map(void *map, const void *ptr, uint64_t rows, uint64_t cols);     // egg_gemm_inst.cu: boxes of 64 columns x 128 rows
+int bf16_tensor_map(void *map, const void *ptr, uint64_t rows, uint64_t cols, uint32_t box_rows);     // egg_gemm_inst.cu: boxes of 64 columns x box_rows
 
 }  // namespace egg
