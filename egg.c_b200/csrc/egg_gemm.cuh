@@ -446,16 +446,16 @@ __device__ __forceinline__ int epilogue_rpl(const GemmParams &p, GemmSmem<BN, CG
     return EPI == EPI_PRE32 || EPI == EPI_QKV ? max(rmx, -rmn) : racc;       // this column quarter's share of the row
 }
 
-// Logits of a vocabulary wider than one tile (mgpu.cu:969-983), row per lane, for every member length.  The cross-entropy
+// Logits of a vocabulary wider than one tile (mgpu.cu:969-983), row per lane, for every member length (a32: the A-noise of the lane's
+// columns).  The cross-entropy
 // needs a logit only as min(255, row maximum - logit), so the 64 logits of a lane stay in registers and leave as one byte
 // each, min(255, their maximum - logit), with that maximum: whatever the row's maximum turns out to be, the difference
 // grows by a number that is known per 64 and the byte is exact below 255.  (Stored as int32 the logits of 2048 members of
 // 256 tokens and 8192 words were 17 GB written and read back, 3.2 + 2.4 ms, both at the memory's rate.)
 template <int BN>
-__device__ __forceinline__ int epilogue_logits(const GemmParams &p, GemmSmem<BN> &sm, uint32_t taddr, int n0, int cbase, int slot, int lane,
+__device__ __forceinline__ int epilogue_logits(const GemmParams &p, uint32_t a32, uint32_t taddr, int n0, int cbase, int lane,
                                                int m0q, int xbs, const CUtensorMap *tmap_o, int32_t *ost) {
     static_assert(BN == 256, "64 columns per lane");
-    const uint32_t a32 = ptx::smem_u32(sm.lg_a32[slot] + cbase);
     uint32_t v[4][16];
     int mx = INT_MIN;
     const int sh2 = p.rank1_shift + p.out_shift;
@@ -694,7 +694,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 }
             }
         }
-    } else if constexpr (RPL && EPI != EPI_LOGITS) {
+    } else if constexpr (RPL) {
         // ===================== epilogue, row per lane: 16 warps that do not wait for one another =====================
         // A warp's rows belong to one member and its tables are its own, so that nothing has to be published to the block: a warp
         // waits for the tile's products alone and its row results leave as atomics of its own.  (With tables of the block and two
@@ -746,7 +746,10 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             if (!__all_sync(0xFFFFFFFFu, ok && !sm.abort_flag)) { gemm_fail(p, &sm.abort_flag, DEV_TIMEOUT_TMEM_FULL); break; }
             ptx::tc_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(as * BN + cbase);
-            if constexpr (EPI == EPI_HEAD) {
+            if constexpr (EPI == EPI_LOGITS) {
+                const int mx = epilogue_logits<BN>(p, ptx::smem_u32(tab.a32), taddr, n0, cbase, lane, m0q, xbs, &tmap_o, sm.ostage0[ew]);
+                if (row_ok) p.rowstat[(int64_t)r * (p.N >> 6) + (n0 >> 6) + cq] = mx;
+            } else if constexpr (EPI == EPI_HEAD) {
                 epilogue_head_rpl<BN>(p, sm, tab, taddr, r, row_ok, cbase, lane, quarter, quarter * 32 + lane, xbs);
             } else {
                 int part;
@@ -813,7 +816,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             bool rok[4];
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                if (EPI > EPI_LOGITS || RPL) { rrow[i] = 0; xbs[i] = 0; slot_sgn[i] = 0; aux[i] = 0; rok[i] = false; continue; }
+                if (EPI >= EPI_LOGITS) { rrow[i] = 0; xbs[i] = 0; slot_sgn[i] = 0; aux[i] = 0; rok[i] = false; continue; }
                 const int rr = m0 + quarter * 32 + i * 8 + lrow;
                 rok[i] = rr < p.M;
                 const int rc = rok[i] ? rr : (p.M - 1);
@@ -875,7 +878,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 // nothing to compute; still takes part in the barrier protocol below
             } else if constexpr (EPI == EPI_LOGITS) {
                 sm.rowpart[half][row_in_tile] =
-                    epilogue_logits<BN>(p, sm, taddr, n0, cbase, slot, lane, m0 + quarter * 32, xbs_l, &tmap_o, sm.ostage0[ew]);
+                    epilogue_logits<BN>(p, ptx::smem_u32(sm.lg_a32[slot] + cbase), taddr, n0, cbase, lane, m0 + quarter * 32, xbs_l, &tmap_o, sm.ostage0[ew]);
             } else if (EPI <= EPI_LOGITS) {
                 // ---------------- evaluation epilogues ----------------
                 // Accumulators leave TMEM one row per lane; they are transposed through shared memory so
@@ -1041,7 +1044,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     }
 
     // output boxes still being copied out of shared memory must land before the block retires
-    if (RPL && (EPI == EPI_PRE32 || EPI == EPI_QKV || EPI == EPI_GELU || EPI == EPI_CLIP8 || EPI == EPI_LOGITS) && warp >= 2 && lane == 0) ptx::tma_store_wait_all<0>();
+    if ((EPI == EPI_LOGITS || (RPL && (EPI == EPI_PRE32 || EPI == EPI_QKV || EPI == EPI_GELU || EPI == EPI_CLIP8))) && warp >= 2 && lane == 0) ptx::tma_store_wait_all<0>();
     __syncwarp();
     ptx::tc_fence_before();
     __syncthreads();

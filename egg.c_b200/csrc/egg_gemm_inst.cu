@@ -71,6 +71,7 @@ int gemm_init() {
     if ((rc = set_attr_both<EPI_QKV, 1>())) return rc;
     if ((rc = set_attr<256, EPI_HEAD>())) return rc;
     if ((rc = set_attr<256, EPI_HEAD, 1>())) return rc;
+    if ((rc = set_attr<256, EPI_LOGITS>())) return rc;
     if ((rc = set_attr<256, EPI_LOGITS, 1>())) return rc;
     if ((rc = set_attr_both<EPI_VOTE>())) return rc;
     if ((rc = set_attr<256, EPI_NULL>())) return rc;
@@ -356,7 +357,7 @@ int launch_gemm(cudaStream_t st, int epi, const int8_t *A, const int8_t *B, cons
     if (epi == EPI_LOGITS && p.N % 256) { set_error("the logits GEMM needs a vocabulary that is a multiple of 256"); return EGG_E_INVALID; }
     if (epi <= EPI_LOGITS) {
         int max_slots = ((GEMM_BM - 1) / p.seq_len) / 2 + 2;
-        const bool rpl = p.seq_len % 32 == 0 && p.rpl >= 0 && epi != EPI_LOGITS;
+        const bool rpl = p.seq_len % 32 == 0 && p.rpl >= 0;
         if (!rpl && max_slots > GEMM_MAX_SLOTS) { set_error("seq_len %d too small for the epilogue tables", p.seq_len); return EGG_E_INVALID; }
     }
     if (epi == EPI_VOTE && p.k_splits > 1) {
@@ -403,7 +404,8 @@ int launch_gemm(cudaStream_t st, int epi, const int8_t *A, const int8_t *B, cons
             if (p.seq_len % 32 == 0 && p.rpl >= 0) return launch_one<256, EPI_HEAD, 1>(st, ta, tb, to, p, num_sms);
             return launch_one<256, EPI_HEAD>(st, ta, tb, to, p, num_sms);
         case EPI_LOGITS:
-            return launch_one<256, EPI_LOGITS, 1>(st, ta, tb, to, p, num_sms);
+            if (p.seq_len % 32 == 0 && p.rpl >= 0) return launch_one<256, EPI_LOGITS, 1>(st, ta, tb, to, p, num_sms);
+            return launch_one<256, EPI_LOGITS>(st, ta, tb, to, p, num_sms);
         case EPI_VOTE: return launch_bn<EPI_VOTE>(st, bn, ta, tb, to, p, num_sms);
         case EPI_NULL: return launch_one<256, EPI_NULL>(st, ta, tb, to, p, num_sms);
     }
