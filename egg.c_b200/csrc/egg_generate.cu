@@ -144,60 +144,137 @@ __device__ __forceinline__ void gen_rows(const int8_t *w, int lane, const int32_
 #pragma unroll
     for (int k = 0; k < R; k++) a[k] = __reduce_add_sync(0xFFFFFFFFu, a[k]);
 }
-// The byte GELU[clip((sum >> shift) + bias)] of row lane & (R - 1), and four bytes to a word: one look-up a lane, not R in a row.
-template <int R>
-__device__ __forceinline__ void gen_gelu(GenSmem &s, int lane, const int (&a)[R], int bl, int i, int shift, uint32_t (&word)[R / 4]) {
-    int v = a[0];
-    if (R == 4) v = lane & 2 ? (lane & 1 ? a[3] : a[2]) : (lane & 1 ? a[1] : a[0]);
-    else {
-        // becomes an indexed read of local memory: for four rows 2 % slower than the selects above (H 768, 1024), for eight 1 % faster (H 512)
-#pragma unroll
-        for (int k = 1; k < R; k++) v = (lane & (R - 1)) == k ? a[k] : v;
-    }
-    const int b = __shfl_sync(0xFFFFFFFFu, bl, i + (lane & (R - 1)));
+// The byte GELU[clip((sum >> shift) + bias)] of row lane & 3, and four bytes to a word: one look-up a lane, not four in a row.
+__device__ __forceinline__ uint32_t gen_gelu4(GenSmem &s, int lane, const int (&a)[4], int bl, int i, int shift) {
+    const int v = lane & 2 ? (lane & 1 ? a[3] : a[2]) : (lane & 1 ? a[1] : a[0]);
+    const int b = __shfl_sync(0xFFFFFFFFu, bl, i + (lane & 3));
     const uint32_t byte = (uint32_t)(uint8_t)s.act_lut[(uint8_t)(int8_t)clip8((v >> shift) + b)] << (8 * (lane & 3));
+    return __reduce_or_sync(0xFFFFFFFFu, lane < 4 ? byte : 0u);
+}
+// Eight rows with four lanes to a row: the sums meet in two shuffles, where a row a warp needs a warp-wide sum each (16 cycles of its
+// unit with eight warps).  The quads read 64 bytes of their rows at a time, in odd rows the other half of 128 first, so that eight
+// lanes cover all banks; x holds the vector's words in that order.
+template <int NJ>
+__device__ __forceinline__ void gen_load_quad(const int8_t *v, int lane, int4 (&x)[2 * NJ]) {
 #pragma unroll
-    for (int k = 0; k < R / 4; k++) word[k] = __reduce_or_sync(0xFFFFFFFFu, (lane & (R - 1)) >> 2 == k ? byte : 0u);
+    for (int c = 0; c < 2 * NJ; c++) x[c] = *reinterpret_cast<const int4 *>(v + 64 * (c ^ (lane >> 2 & 1)) + 16 * (lane & 3));
+}
+template <int NJ>
+__device__ __forceinline__ int gen_quad_dot(const int8_t *w, int lane, const int4 (&x)[2 * NJ]) {
+    const int8_t *p = w + (lane >> 2) * (128 * NJ) + 16 * (lane & 3);
+    int a = 0, b = 0;                         // two chains
+#pragma unroll
+    for (int c = 0; c < 2 * NJ; c++) {
+        const int4 r = *reinterpret_cast<const int4 *>(p + 64 * (c ^ (lane >> 2 & 1)));
+        int &t = c & 1 ? b : a;
+        t = __dp4a(r.x, x[c].x, t); t = __dp4a(r.y, x[c].y, t); t = __dp4a(r.z, x[c].z, t); t = __dp4a(r.w, x[c].w, t);
+    }
+    return a + b;
+}
+// Their bytes GELU[clip((sum >> shift) + bias)] as two words, bl the bias of row lane / 4 (in every lane; the words are right in lanes 0-15).
+__device__ __forceinline__ void gen_quad_gelu(GenSmem &s, int lane, int a, int bl, int shift, uint32_t (&word)[2]) {
+    a += __shfl_xor_sync(0xFFFFFFFFu, a, 1);
+    a += __shfl_xor_sync(0xFFFFFFFFu, a, 2);
+    uint32_t w = (uint32_t)(uint8_t)s.act_lut[(uint8_t)(int8_t)clip8((a >> shift) + bl)] << (8 * (lane >> 2 & 3));
+    w |= __shfl_xor_sync(0xFFFFFFFFu, w, 4);
+    w |= __shfl_xor_sync(0xFFFFFFFFu, w, 8);
+    word[0] = w;
+    word[1] = __shfl_xor_sync(0xFFFFFFFFu, w, 16);
 }
 
-// out_off: byte offset of the product's exchange buffer inside GenSmem.  Every warp takes rc / 8 consecutive rows of a chunk, four
-// at a time where it has as many, and eight of the up product at H 256, 384 and 512 (its share of a chunk is 4 or 8 rows, that of
-// other products at most 5): their chains of loads, products and sums run side by side, and the peers get one message for eight
-// bytes (up product of H 512: 3.7 -> 2.5 thousand cycles).  Two at a time where two or three are left, as in the down product (250
-// bytes sampled, 2 layers: H 256 4.48 -> 3.99 ms; 4 layers, H 512 7.82 -> 7.63; H 768 and 1024 +0.5 %, their rows come singly).
+// out_off: byte offset of the product's exchange buffer inside GenSmem.  Every warp takes rc / 8 consecutive rows of a chunk.  How many
+// run side by side is what a token's time hangs on (chains of loads, products, sums and a message): four rows where there are as many,
+// eight of the up product at H 256, 384 and 512 by quads of lanes, those of two chunks at H 512; one or two rows of each of two
+// neighbouring chunks, as in the down product, together.  What no chunk of a product can hold is not compiled: the instructions of a
+// token are fetched anew for every product.  Against one row or four after another (256 bytes sampled, 2 layers): H 256 4.48 -> 3.88 ms,
+// 384 4.86 -> 4.59, 640 6.45 -> 6.12, 768 7.50 -> 7.30, 1024 8.84 -> 8.41; 4 layers, H 512 7.82 -> 7.27.
 // BYTES = false: int32 results; true: GELU[clip((acc >> shift) + bias)].
 template <int KW, bool BYTES>
 __device__ __forceinline__ void gen_product(GenSmem &s, GenState &g, const int8_t *vec, int rows, int group, uint32_t out_off, uint32_t bar_off, int *err,
                                             const int8_t *bias = nullptr, int shift = 0) {
     constexpr int K = KW * 128;
-    int32_t x[KW];
-    gen_load_vec<KW>(vec, g.lane, x);
+    constexpr bool QUADS = BYTES && KW >= 2 && KW <= 4;      // chunks of 64 rows and more
+    constexpr int MOST = GEN_CHUNK / K / GEN_WARPS;          // most rows of a warp and chunk
+    constexpr bool CHUNK_PAIRS = KW != 24;                   // (H 768: 7.46 ms with them, 7.35 without)
     const int dest = g.lane & 15, half = g.lane >> 4;
     const uint32_t bar = ptx::mapa_u32(g.smem_base + bar_off, dest);
-    for (int r = 0; r < rows;) {
+    auto stage = [&](uint32_t k) { return (int)((g.ring_it + k) % GEN_STAGES); };
+    auto wait_full = [&](uint32_t k) {
+        const uint32_t it = g.ring_it + k;
+        gen_wait_ring(s, &s.full[it % GEN_STAGES], (it / GEN_STAGES) & 1, err);
+    };
+    int r = 0;
+    if constexpr (QUADS) {
+        int4 x[2 * KW];
+        gen_load_quad<KW>(vec, g.lane, x);
+        constexpr int RC = 32768 / K / 32 * 32 < 32 * KW ? 32768 / K / 32 * 32 : 32 * KW, N = 32 * KW / RC;        // rows of a chunk, whole chunks
+        static_assert(RC == 64 && GEN_CHUNK == 32768, "eight rows a warp and chunk");
+        const int row0 = g.rank * rows + 8 * g.warp;
+        int bl[N], a[N];
+#pragma unroll
+        for (int n = 0; n < N; n++) bl[n] = (int)bias[row0 + RC * n + (g.lane >> 2)];
+#pragma unroll
+        for (int n = 0; n < N; n++) {
+            wait_full((uint32_t)n);
+            __syncwarp();
+            a[n] = gen_quad_dot<KW>(s.ring[stage((uint32_t)n)] + g.warp * 8 * K, g.lane, x);
+        }
+#pragma unroll
+        for (int n = 0; n < N; n++) {
+            uint32_t v[2];
+            gen_quad_gelu(s, g.lane, a[n], bl[n], shift, v);
+            if (half == 0) st_async_v2(ptx::mapa_u32(g.smem_base + out_off + row0 + RC * n, dest), bar, v[0], v[1]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int n = 0; n < N; n++)
+            if (g.lane == 0) ptx::mbar_arrive(&s.empty[stage((uint32_t)n)]);
+        g.ring_it += N;
+        r = RC * N;
+        if (KW != 3) return;
+    }
+    int32_t x[KW];
+    gen_load_vec<KW>(vec, g.lane, x);
+    while (r < rows) {
         const int rc = gen_chunk_rows(K, rows - r, group), per = rc / GEN_WARPS;
-        const int st = g.ring_it % GEN_STAGES;
+        const int st = stage(0);
         const int row0 = g.rank * rows + r + g.warp * per;            // row of the whole product
         const int bl = (BYTES && g.lane < per) ? (int)bias[row0 + g.lane] : 0;
-        gen_wait_ring(s, &s.full[st], (g.ring_it / GEN_STAGES) & 1, err);
+        wait_full(0);
+        if (!BYTES && MOST <= 2 && CHUNK_PAIRS && per <= 2 && rows - r >= 2 * rc) {
+            // one or two rows of this chunk and as many of the next: lanes 0-15 send those, 16-31 these
+            wait_full(1);
+            __syncwarp();
+            const int8_t *w0 = s.ring[st] + g.warp * per * K, *w1 = s.ring[stage(1)] + g.warp * per * K;
+            const uint32_t at = ptx::mapa_u32(g.smem_base + out_off + 4 * (row0 + half * rc), dest);
+            int a[4];
+            a[0] = gen_dot<KW>(w0, g.lane, x); a[1] = gen_dot<KW>(w1, g.lane, x);
+            if (per == 2) {
+                a[2] = gen_dot<KW>(w0 + K, g.lane, x); a[3] = gen_dot<KW>(w1 + K, g.lane, x);
+#pragma unroll
+                for (int k = 0; k < 4; k++) a[k] = __reduce_add_sync(0xFFFFFFFFu, a[k]);
+                st_async_v2(at, bar, (uint32_t)(half ? a[1] : a[0]), (uint32_t)(half ? a[3] : a[2]));
+            } else {
+#pragma unroll
+                for (int k = 0; k < 2; k++) a[k] = __reduce_add_sync(0xFFFFFFFFu, a[k]);
+                st_async_b32(at, bar, (uint32_t)(half ? a[1] : a[0]));
+            }
+            __syncwarp();
+            if (g.lane == 0) { ptx::mbar_arrive(&s.empty[st]); ptx::mbar_arrive(&s.empty[stage(1)]); }
+            g.ring_it += 2;
+            r += 2 * rc;
+            continue;
+        }
         __syncwarp();
         const int8_t *w = s.ring[st] + (int64_t)g.warp * per * K;
         for (int i = 0; i < per;) {
             const uint32_t at = g.smem_base + out_off + (BYTES ? 1 : 4) * (row0 + i);
-            if (BYTES && per - i >= 8) {
-                int a[8];
-                uint32_t v[2];
-                gen_rows<KW, 8>(w + i * K, g.lane, x, a);
-                gen_gelu<8>(s, g.lane, a, bl, i, shift, v);
-                if (half == 0) st_async_v2(ptx::mapa_u32(at, dest), bar, v[0], v[1]);
-                i += 8;
-            } else if (per - i >= 4) {
+            if (MOST >= 4 && (BYTES || per - i >= 4)) {          // (the up product's chunks are whole groups of four rows a warp)
                 int a[4];
                 gen_rows<KW, 4>(w + i * K, g.lane, x, a);
                 if (BYTES) {
-                    uint32_t v[1];
-                    gen_gelu<4>(s, g.lane, a, bl, i, shift, v);
-                    if (half == 0) st_async_b32(ptx::mapa_u32(at, dest), bar, v[0]);
+                    const uint32_t v = gen_gelu4(s, g.lane, a, bl, i, shift);
+                    if (half == 0) st_async_b32(ptx::mapa_u32(at, dest), bar, v);
                 } else if (((row0 + i) & 3) == 0) {
                     if (half == 0) st_async_v4(ptx::mapa_u32(at, dest), bar, a[0], a[1], a[2], a[3]);
                 } else {
@@ -205,7 +282,7 @@ __device__ __forceinline__ void gen_product(GenSmem &s, GenState &g, const int8_
                     st_async_b32(ptx::mapa_u32(at + 4 * (2 + half), dest), bar, half ? a[3] : a[2]);
                 }
                 i += 4;
-            } else if (!BYTES && per - i >= 2) {
+            } else if (MOST >= 2 && !BYTES && per - i >= 2) {
                 int a[2];
                 gen_rows<KW, 2>(w + i * K, g.lane, x, a);
                 if (((row0 + i) & 1) == 0) {
@@ -214,7 +291,7 @@ __device__ __forceinline__ void gen_product(GenSmem &s, GenState &g, const int8_
                     st_async_b32(ptx::mapa_u32(at + 4 * half, dest), bar, (uint32_t)(half ? a[1] : a[0]));
                 }
                 i += 2;
-            } else {
+            } else if (!BYTES) {
                 int a[1];
                 gen_rows<KW, 1>(w + i * K, g.lane, x, a);
                 if (half == 0) st_async_b32(ptx::mapa_u32(at, dest), bar, a[0]);
@@ -427,13 +504,12 @@ __global__ void __launch_bounds__(GEN_THREADS, 1) generate_kernel(const GenParam
                 gen_receive(s, g, after_d, p.err);
                 x4 = gen_finish(s, g, x4, s.pd, p.shift_mlp_down, bd, H);
             };
-            gen_norm(s, g, x4, row_word(M + L.ln_init), row_word(M + L.ln_init_bias), H);
-            int nw = row_word(M + L.ln_1), nb = row_word(M + L.ln_1_bias);       // gains and biases of the norm after next
-            mlp(M + L.mlp_emb_bias_up, M + L.mlp_emb_bias_down, 12 * H, H);
-
-            for (int l = 0; l < p.n_layers; l++) {
+            int nw = row_word(M + L.ln_init), nb = row_word(M + L.ln_init_bias);       // gains and biases of the next norm
+            // layer -1 is the embedding's MLP: one copy of the products' code, which a token walks through many times
+            for (int l = -1; l < p.n_layers; l++) {
                 const int64_t lH = (int64_t)l * H;
                 const bool last = l + 1 == p.n_layers;
+                if (l >= 0) {
                 int8_t *kc = p.kv + ((int64_t)(l * NH + (g.rank < NH ? g.rank : 0)) * 2) * 256 * 64, *vc = kc + 256 * 64;
                 const bool head = g.rank < NH;
                 gen_norm(s, g, x4, nw, nb, H);
@@ -554,12 +630,13 @@ __global__ void __launch_bounds__(GEN_THREADS, 1) generate_kernel(const GenParam
                 gen_product<NJ, false>(s, g, s.ao, RH, 8, off_po, bar_off(), p.err);
                 gen_receive(s, g, 4 * H, p.err);               // after the activations: the down product
                 x4 = gen_finish(s, g, x4, s.po, p.shift_out, 0, H);
+                }
                 gen_norm(s, g, x4, nw, nb, H);
                 nw = row_word(last ? M + L.ln_f : M + L.ln_1 + lH + H); nb = row_word(last ? M + L.ln_f_bias : M + L.ln_1_bias + lH + H);
                 // what follows this block: the next layer's q|k|v and attention; at the end the logits (when drawing) and the next
                 // token's first two exchanges
                 const uint32_t e1 = !last ? 12 * H : (draw ? 4 * V : 4 * H), e2 = !last ? H : 4 * H;
-                mlp(M + L.mlp_bias_up + 4 * lH, M + L.mlp_bias_down + lH, e1, e2);
+                mlp(M + (l < 0 ? L.mlp_emb_bias_up : L.mlp_bias_up + 4 * lH), M + (l < 0 ? L.mlp_emb_bias_down : L.mlp_bias_down + lH), e1, e2);
             }
 
             if (draw) {

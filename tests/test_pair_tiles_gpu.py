@@ -77,3 +77,23 @@ def test_isolated_votes_of_pairs(rows, cols, pairs):
     n_list = np.arange(0, cols, 37).astype(np.int32)
     got = votes.cpu().numpy().reshape(rows // 4, cols, 4)[:, n_list, :].transpose(1, 0, 2).reshape(len(n_list), rows)      # packed order [k/4][n][4]
     assert (got == O.vote_columns(ocfg, fit, rows, 402, 403, 1000, 2, n_list)).all()
+
+
+@pytest.mark.parametrize("rows,cols", [(512, 896), (640, 1024), (1024, 1024)])
+def test_newton_schulz_in_pairs(rows, cols):
+    """Pairs of tiles in both products; an odd number of row tiles (single blocks); more pairs than fit at once in the Gram matrix."""
+    from test_muon_gpu import test_newton_schulz_against_float64 as check
+    check(rows, cols)
+
+
+@pytest.mark.parametrize("seq", [32, 48, 16])          # a warp's own tables, padded to 64 rows, tables of the tile
+def test_logits_of_short_windows(seq):
+    pkg, O = load_pkg(), load_oracle()
+    kw = dict(hidden_dim=128, n_layers=1, seq_len=seq, vocab_size=512, population_size=22, device_mask=15)
+    cfg, ocfg, model, data = make_case(kw, data_len=60000, model_kind="random_all")
+    ctx = pkg.Context(cfg, 0, 0)
+    ctx.upload_model(model)
+    ctx.set_dataset(data)
+    ctx.eval_chunk(SEED + 2, 5, 0, 22)
+    assert (ctx.read_losses(0, 22) == O.eval_losses(ocfg, model, data, 5, SEED + 2, 0, 22)).all()
+    ctx.close()
