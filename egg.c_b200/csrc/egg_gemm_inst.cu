@@ -192,8 +192,8 @@ static int launch_fused_cg(cudaStream_t st, const CUtensorMap &ta, const CUtenso
         attr[0].val.clusterDim.x = (unsigned)cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr; cfg.numAttrs = 1;                  // (the occupancy question is about the cluster alone)
         // the clusters that can be resident at once (a GPC whose free SMs are no multiple leaves some out): asked once a size
-        static int max_dev[2][EGG_MAX_DEVICES] = {};
-        int &max_pairs = max_dev[p.cl > 1][current_device_slot()];
+        static std::atomic<int> max_dev[2][EGG_MAX_DEVICES] = {};
+        std::atomic<int> &max_pairs = max_dev[p.cl > 1][current_device_slot()];
         if (max_pairs == 0) {
             cfg.gridDim = dim3((unsigned)(num_sms / cluster * cluster));
             int n = 0;
@@ -306,8 +306,8 @@ static int launch_pair(cudaStream_t st, const CUtensorMap &ta, const CUtensorMap
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
-    static int max_dev[EGG_MAX_DEVICES] = {};          // pairs that can be resident at once
-    int &most = max_dev[current_device_slot()];
+    static std::atomic<int> max_dev[EGG_MAX_DEVICES] = {};          // pairs that can be resident at once
+    std::atomic<int> &most = max_dev[current_device_slot()];
     if (most == 0) {
         cfg.gridDim = dim3((unsigned)(num_sms / 2 * 2));
         int n = 0;
@@ -316,7 +316,8 @@ static int launch_pair(cudaStream_t st, const CUtensorMap &ta, const CUtensorMap
         most = n < num_sms / 2 ? n : num_sms / 2;
     }
     const int tiles = ((p.M + 2 * GEMM_BM - 1) / (2 * GEMM_BM)) * (p.N / 256) * ((EPI == EPI_VOTE && p.k_splits > 1) ? p.k_splits : 1);
-    cfg.gridDim = dim3((unsigned)(2 * (tiles < most ? tiles : most)));
+    const int pairs = most;
+    cfg.gridDim = dim3((unsigned)(2 * (tiles < pairs ? tiles : pairs)));
     if (t_chain) {
         attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[1].val.programmaticStreamSerializationAllowed = 1;
