@@ -505,11 +505,19 @@ __global__ void __launch_bounds__(GEN_THREADS, 1) generate_kernel(const GenParam
                 x4 = gen_finish(s, g, x4, s.pd, p.shift_mlp_down, bd, H);
             };
             int nw = row_word(M + L.ln_init), nb = row_word(M + L.ln_init_bias);       // gains and biases of the next norm
-            // layer -1 is the embedding's MLP: one copy of the products' code, which a token walks through many times
-            for (int l = -1; l < p.n_layers; l++) {
+            // layer -1 is the embedding's MLP: one copy of the products' code, which a token walks through many times.  At H 128, where the
+            // code is short, two copies without the branch in the loop are the faster (224 sampled bytes, 7 layers: 9.92 against 10.03 ms)
+            int l = -1;
+            if constexpr (NJ == 1) {
+                gen_norm(s, g, x4, nw, nb, H);
+                nw = row_word(M + L.ln_1); nb = row_word(M + L.ln_1_bias);
+                mlp(M + L.mlp_emb_bias_up, M + L.mlp_emb_bias_down, 12 * H, H);
+                l = 0;
+            }
+            for (; l < p.n_layers; l++) {
                 const int64_t lH = (int64_t)l * H;
                 const bool last = l + 1 == p.n_layers;
-                if (l >= 0) {
+                if (NJ == 1 || l >= 0) {
                 int8_t *kc = p.kv + ((int64_t)(l * NH + (g.rank < NH ? g.rank : 0)) * 2) * 256 * 64, *vc = kc + 256 * 64;
                 const bool head = g.rank < NH;
                 gen_norm(s, g, x4, nw, nb, H);
