@@ -1,7 +1,8 @@
 // Persistent, warp-specialised int8 GEMM for sm_100a:
 //   D[M,N] (int32, TMEM) = A[M,K] (int8, K-major) x B[N,K]^T (int8, K-major)
-// TMA (128-byte swizzle) -> 4-stage shared-memory ring -> tcgen05.mma kind::i8 ->
-// two TMEM accumulator stages -> 8 epilogue warps.  The epilogue is where the
+// TMA (128-byte swizzle) -> shared-memory ring -> tcgen05.mma kind::i8 -> two TMEM
+// accumulator stages -> 16 epilogue warps; for long contractions two blocks of a
+// cluster form 256 rows together (cta_group::2).  The epilogue is where the
 // EGGROLL arithmetic lives: the per-member rank-1 term
 //   acc += ((x·b_p) * a_p[n] * sign) >> (FIXED_POINT + SIGMA_SHIFT)
 // (compute_linear_projection, mgpu.cu:553-572) and the call-site specific

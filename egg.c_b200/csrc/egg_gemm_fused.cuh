@@ -25,6 +25,8 @@
 // all of them; otherwise (MM, seq_len a multiple of 32) every lane quarter of 32 rows has its own member and tables, and the
 // sub-tiles are 128 wide unless the block owns exactly 256 columns, so that the tables fit beside the operands.
 // At H 256, seq_len 32 (262 144 rows) this replaces a projection with int32 output and a requantising pass: q|k|v 332 -> 200 us.
+// For long contractions and wide tiles two blocks of a cluster form 256 rows together (CG = 2, cta_group::2): an SM gets fewer bytes from
+// L2 than a 128 x 256 tile needs at the tensor cores' rate; the rule and its figures stand at launch_gemm_fused.
 // No multicast anywhere; every wait is bounded and a timeout makes all later waits fall through so that the block
 // drains, frees its tensor memory and reports.
 #pragma once
@@ -119,7 +121,7 @@ __device__ __forceinline__ void fused_wait(uint64_t *bar, uint32_t parity, volat
 struct FusedTabWords { int32_t a, b, d; };
 
 // FORM: FUSED_RES: both shifts as one (see pass 1); FUSED_RES_LN: three row dots follow (else one)
-template <int BN, int MODE, bool MM, bool FORM, int CG>
+template <int CG, int BN, int MODE, bool MM, bool FORM>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_fused_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                   const __grid_constant__ CUtensorMap tmap_o, const __grid_constant__ CUtensorMap tmap_r, const FusedParams p) {

@@ -27,7 +27,7 @@ static int set_attr_both() {
 
 template <int BN, int MODE, bool MM, bool FORM, int CG = 1>
 static int set_attr_fused_one() {
-    EGG_CUDA(cudaFuncSetAttribute(gemm_fused_kernel<BN, MODE, MM, FORM, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem_bytes<BN, MM, CG>()));
+    EGG_CUDA(cudaFuncSetAttribute(gemm_fused_kernel<CG, BN, MODE, MM, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem_bytes<BN, MM, CG>()));
     return EGG_OK;
 }
 template <int BN, bool MM>
@@ -179,7 +179,7 @@ int fused_cluster_size(int hidden) {
 template <int BN, int MODE, bool MM, bool FORM, int CG>
 static int launch_fused_cg(cudaStream_t st, const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &to, const CUtensorMap &tr,
                             const FusedParams &p, int units, int num_sms) {
-    auto kern = gemm_fused_kernel<BN, MODE, MM, FORM, CG>;
+    auto kern = gemm_fused_kernel<CG, BN, MODE, MM, FORM>;
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(GEMM_THREADS);
     cfg.dynamicSmemBytes = fused_smem_bytes<BN, MM, CG>();
