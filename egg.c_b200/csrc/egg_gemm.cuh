@@ -506,10 +506,11 @@ __device__ __forceinline__ int epilogue_logits(const GemmParams &p, uint32_t a32
 // quarter each take a quarter of the vocabulary columns of the same 32 rows: pass 0 finds the row maximum (partials
 // exchanged through shared memory under a 128-thread named barrier), pass 1 re-reads the accumulators for
 // Σ exp-LUT and the target logit, and the warp of the first column quarter adds one loss term per row, reduced over
-// the warp (all its rows belong to one member) into a single atomic.
+// the warp (all its rows belong to one member) into a single atomic.  dead: the warp gave up waiting for products; it reads no
+// accumulators, leaves its partials neutral (what the other warps look up stays inside the table) and meets both barriers.
 template <int BN>
 __device__ __forceinline__ void epilogue_head_rpl(const GemmParams &p, GemmSmem<BN> &sm, const RplTables<BN> &tab, uint32_t taddr, int r, bool row_ok, int cbase,
-                                                  int lane, int quarter, int row_in_tile, int xbs) {
+                                                  int lane, int quarter, int row_in_tile, int xbs, bool dead) {
     constexpr int NCH = BN / 4 / 16;
     int32_t(*hp)[4][GEMM_BM] = reinterpret_cast<int32_t(*)[4][GEMM_BM]>(&sm.stage[0][0][0]);    // [max | sum | target][quarter][row]
     const int cq = cbase / (BN / 4);
@@ -524,27 +525,29 @@ __device__ __forceinline__ void epilogue_head_rpl(const GemmParams &p, GemmSmem<
     int mx = INT_MIN, sum = 0, tg = 0;
 #pragma unroll 1
     for (int pass = 0; pass < 2; pass++) {
-        ptx::tmem_ld16(taddr, v[0]);
+        if (!dead) {
+            ptx::tmem_ld16(taddr, v[0]);
 #pragma unroll
-        for (int c = 0; c < NCH; c++) {
-            uint32_t *vc = v[c & 1];
-            ptx::tmem_ld_wait16(vc);
-            if (c + 1 < NCH) ptx::tmem_ld16(taddr + 16 * (c + 1), v[(c + 1) & 1]);
+            for (int c = 0; c < NCH; c++) {
+                uint32_t *vc = v[c & 1];
+                ptx::tmem_ld_wait16(vc);
+                if (c + 1 < NCH) ptx::tmem_ld16(taddr + 16 * (c + 1), v[(c + 1) & 1]);
 #pragma unroll
-            for (int q4 = 0; q4 < 4; q4++) {
-                const int col = 16 * c + 4 * q4;
-                const int4 an = ptx::lds_v4(a32 + 4 * col);
-                const int l0 = ((int)vc[4 * q4] + ((xbs * an.x) >> p.rank1_shift)) >> p.out_shift;
-                const int l1 = ((int)vc[4 * q4 + 1] + ((xbs * an.y) >> p.rank1_shift)) >> p.out_shift;
-                const int l2 = ((int)vc[4 * q4 + 2] + ((xbs * an.z) >> p.rank1_shift)) >> p.out_shift;
-                const int l3 = ((int)vc[4 * q4 + 3] + ((xbs * an.w) >> p.rank1_shift)) >> p.out_shift;
-                if (pass == 0) {
-                    mx = __vimax3_s32(__vimax3_s32(mx, l0, l1), l2, l3);
-                } else {
-                    sum += sm.exp_lut[min(255, mx - l0)] + sm.exp_lut[min(255, mx - l1)] + sm.exp_lut[min(255, mx - l2)] +
-                           sm.exp_lut[min(255, mx - l3)];
-                    const int tc = tgt_col - col;
-                    if (tc == 0) tg = l0; else if (tc == 1) tg = l1; else if (tc == 2) tg = l2; else if (tc == 3) tg = l3;
+                for (int q4 = 0; q4 < 4; q4++) {
+                    const int col = 16 * c + 4 * q4;
+                    const int4 an = ptx::lds_v4(a32 + 4 * col);
+                    const int l0 = ((int)vc[4 * q4] + ((xbs * an.x) >> p.rank1_shift)) >> p.out_shift;
+                    const int l1 = ((int)vc[4 * q4 + 1] + ((xbs * an.y) >> p.rank1_shift)) >> p.out_shift;
+                    const int l2 = ((int)vc[4 * q4 + 2] + ((xbs * an.z) >> p.rank1_shift)) >> p.out_shift;
+                    const int l3 = ((int)vc[4 * q4 + 3] + ((xbs * an.w) >> p.rank1_shift)) >> p.out_shift;
+                    if (pass == 0) {
+                        mx = __vimax3_s32(__vimax3_s32(mx, l0, l1), l2, l3);
+                    } else {
+                        sum += sm.exp_lut[min(255, mx - l0)] + sm.exp_lut[min(255, mx - l1)] + sm.exp_lut[min(255, mx - l2)] +
+                               sm.exp_lut[min(255, mx - l3)];
+                        const int tc = tgt_col - col;
+                        if (tc == 0) tg = l0; else if (tc == 1) tg = l1; else if (tc == 2) tg = l2; else if (tc == 3) tg = l3;
+                    }
                 }
             }
         }
@@ -710,6 +713,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         TabWords nxt = {0, 0, 0, 0, 0};
         int pf_xb = 0;                              // the lane's rank-1 factor (raw sum of x b of its row)
         int4 pf_rs0 = make_int4(0, 0, 0, 0);        // first chunk of residual bytes
+        bool dead = false;                          // EPI_HEAD: this warp gave up (see below)
         auto prefetch = [&](int tile) {
             const int tm_ = fast_div(tile, p.fd_tiles_n), rw = row_tile(tm_) * GEMM_BM + quarter * 32, n0 = (tile - tm_ * tiles_n) * BN;
             rpl_load<BN, EPI>(p, lane, fast_div(min(rw, p.M - 1), p.fd_seq), n0 + cbase + 4 * lane, nxt);
@@ -742,16 +746,22 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             }
             const int ntile = tile + tile_step;
             if (!RES_TMA && ntile < num_tiles) prefetch(ntile);          // in flight while this tile is computed
-            bool ok = ptx::mbar_wait(&sm.tmem_full[as], (tcount >> 1) & 1);
+            bool ok = dead || ptx::mbar_wait(&sm.tmem_full[as], (tcount >> 1) & 1);
             if (RES_TMA) ok = ok && ptx::mbar_wait(&sm.rbar[ew], tcount & 1);
-            if (!__all_sync(0xFFFFFFFFu, ok && !sm.abort_flag)) { gemm_fail(p, &sm.abort_flag, DEV_TIMEOUT_TMEM_FULL); break; }
+            if (!__all_sync(0xFFFFFFFFu, ok && !sm.abort_flag)) {
+                gemm_fail(p, &sm.abort_flag, DEV_TIMEOUT_TMEM_FULL);
+                // each warp decides by itself.  Of the head's, four meet at barriers within a tile: one that gives up walks on to the end
+                // without waiting or reading, so that nobody is left at a barrier
+                if (EPI != EPI_HEAD) break;
+                dead = true;
+            }
             ptx::tc_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(as * BN + cbase);
             if constexpr (EPI == EPI_LOGITS) {
                 const int mx = epilogue_logits<BN>(p, ptx::smem_u32(tab.a32), taddr, n0, cbase, lane, m0q, xbs, &tmap_o, sm.ostage0[ew]);
                 if (row_ok) p.rowstat[(int64_t)r * (p.N >> 6) + (n0 >> 6) + cq] = mx;
             } else if constexpr (EPI == EPI_HEAD) {
-                epilogue_head_rpl<BN>(p, sm, tab, taddr, r, row_ok, cbase, lane, quarter, quarter * 32 + lane, xbs);
+                epilogue_head_rpl<BN>(p, sm, tab, taddr, r, row_ok, cbase, lane, quarter, quarter * 32 + lane, xbs, dead);
             } else {
                 int part;
                 if ((EPI == EPI_QKV && n0 < 2 * p.third) || (EPI == EPI_GELU && BN == 256 && p.pow_t))        // asked once a tile, not per four columns: 68.6 -> 68.0 ms
