@@ -2,6 +2,7 @@
 fake_cuda.cpp, whose kernels do nothing, which logs every launch and wait and fails the call a test names."""
 import json
 import os
+import re
 import subprocess
 import sys
 
@@ -184,7 +185,7 @@ ctx = context(hidden_dim=%d, n_layers=1, seq_len=128, population_size=8, fixed_p
 ctx.eval_chunk(1, 0, 0, 8)
 out["kernels"] = [l.split()[1] for l in log() if l.startswith("launch") and "gemm_fused" in l]
 """ % (hidden, fixed, sigma, shift_out))
-    # <tile width, mode (1: output projection), tables per quarter, merged>
+    # <blocks a tile, tile width, mode (1: output projection), members across tiles, merged>
     got = [k.split("gemm_fused_kernelI")[1].split("EEEv")[0] for k in out["kernels"]]
     assert any(k.endswith("Lb%d" % merged) for k in got if "ELi1E" in k), got
     assert merged or not any(k.endswith("Lb1") for k in got if "ELi1E" in k), got
@@ -335,3 +336,77 @@ ts = [threading.Thread(target=go, args=(i,)) for i in (0, 1)]
 out["rcs"], out["launched"] = rcs, launches(%r)
 """ % (kernel.encode(), seqs, mode, mode, kernel))
     assert out == {"rcs": [0, 0], "launched": 2}
+
+
+def forms(names, kernel):
+    """Template arguments of the launches of one kernel."""
+    found = [re.search(kernel + r"I((?:L[ib]\d+E)+)E", n) for n in names]
+    return [tuple(map(int, re.findall(r"\d+", f[1]))) for f in found if f]
+
+
+def test_sizes_of_the_pair_tests_take_pairs(fake_cuda):
+    """Of every product that test_pair_tiles_gpu.py compares with single blocks, one side is formed by pairs and the other is not."""
+    from test_pair_tiles_gpu import EVALUATIONS, MATRIX_UPDATES, MODEL_UPDATES, NEWTON_SCHULZ, PROJECTIONS, RECONSTRUCTIONS, small_chunk
+    out = fake_cuda("""
+def names(): return [l.split()[1] for l in log() if l.startswith("launch")]
+for key in ("eval", "small", "projection", "aside", "votes", "update", "model", "muon"): out[key] = []
+for hidden, layers, seq, pop, other, small in %r:
+    ctx = context(wave=pop, hidden_dim=hidden, n_layers=layers, seq_len=seq, population_size=pop, **other)
+    for key, count in (("eval", pop), ("small", small)):
+        fake.fake_clear()
+        ctx.eval_chunk(1, 0, 0, count)
+        out[key].append(names())
+    ctx.close()
+p = C.c_void_p()
+fake.cudaMalloc(C.byref(p), C.c_size_t(1 << 30))
+p = p.value
+ctx = context(hidden_dim=128, n_layers=1, seq_len=32, population_size=8, device_mask=3)
+for rows, k, n in %r:
+    for key, offset in (("projection", 64), ("aside", 68)):
+        fake.fake_clear()
+        ctx.perturbed_projection(p, p, p + offset, rows, k, n, 32, 7, 200, 201, 7, 8, on_device=True)
+        out[key].append(names())
+for rows, cols, pairs, _ in %r:
+    fake.fake_clear()
+    ctx.update_reconstruct(p, pairs, rows, cols, 402, 403, 1000, 2, p, on_device=True)
+    out["votes"].append(names())
+for rows, cols, pairs, split in %r:
+    fake.fake_clear()
+    ctx.update_matrix(p, p, rows, cols, 402, 403, 1000, p, pairs, 2, 2.5, 0, split)
+    out["update"].append(names())
+for rows, cols, _ in %r:
+    fake.fake_clear()
+    ctx.update_matrix(p, p, rows, cols, 402, 403, 0, p, 32, 7, 1.0, 1, False)
+    out["muon"].append(names())
+for hidden, layers, pairs in %r:
+    ctx = context(hidden_dim=hidden, n_layers=layers, seq_len=16, population_size=2 * pairs, device_mask=15)
+    fake.fake_clear()
+    ctx.apply_update(1, 0.4)
+    out["model"].append(names())
+    ctx.close()
+""" % ([e + (small_chunk(e[0], e[2]),) for e in EVALUATIONS], PROJECTIONS, RECONSTRUCTIONS, MATRIX_UPDATES, NEWTON_SCHULZ, MODEL_UPDATES))
+
+    def fused(names, mode):                      # blocks a tile, width of the sub-tiles, last argument
+        return {(f[0], f[1], f[4]) for f in forms(names, "gemm_fused_kernel") if f[2] == mode}
+
+    def gemm(names, epi):
+        return {f[3] for f in forms(names, "gemm_i8_kernel") if f[1] == epi}
+
+    QKV, RES, RES_LN, CLIP8, GELU, VOTE = 0, 1, 2, 0, 1, 7
+    for (hidden, layers, seq, pop, other), names, small in zip(EVALUATIONS, out["eval"], out["small"]):
+        one_member = seq % 128 == 0
+        width = 256 if hidden in (256, 512, 1024) and one_member else 128
+        wide = 2 if hidden <= 512 and one_member else 1
+        assert fused(names, QKV) == {(wide, width, 0)}
+        assert fused(names, RES) == {(wide if hidden == 512 else 1, width, 0 if other or hidden == 1024 else 1)}
+        if hidden > 256:
+            assert fused(names, RES_LN) == {(2, width, 0), (2, width, 1)}
+            assert gemm(names, GELU) == {2}
+        for mode in (QKV, RES, RES_LN):
+            assert {f[0] for f in fused(small, mode)} == {1}
+        assert gemm(small, GELU) == {1}
+    assert [gemm(n, CLIP8) for n in out["projection"]] == [{2}] * 2 and [gemm(n, CLIP8) for n in out["aside"]] == [{1}] * 2
+    assert [gemm(n, VOTE) for n in out["votes"]] == [{2 if r[3] else 1} for r in RECONSTRUCTIONS]
+    assert [gemm(n, VOTE) for n in out["update"]] == [{2}] * len(MATRIX_UPDATES)
+    assert [{f[1] for f in forms(n, "ns_gemm_kernel")} for n in out["muon"]] == [{2 if r[2] else 1} for r in NEWTON_SCHULZ]
+    assert [set(forms(n, "upd_votes_kernel")) for n in out["model"]] == [{(2,)}] * len(MODEL_UPDATES)

@@ -1,7 +1,8 @@
-"""Products that pairs of thread blocks form together (cta_group::2): the same losses as the two-kernel form, whose blocks work alone, for
-every member, and as the CPU oracle for the members of the first and the last row tile.  The sizes: an odd number of row tiles (the last
-pair forms one twice and stores it once), tiles of one member and of several, sub-tiles of 256 and of 128 columns, clusters of four
-(a pair for each half of the columns), even and uneven halves."""
+"""Products that pairs of thread blocks form together (cta_group::2): the same losses as the same members in chunks too small for pairs,
+as the two-kernel form, for every member, and as the CPU oracle for the members of the first and the last row tile.  The sizes: an odd number
+of row tiles (the last pair forms one twice and stores it once) where tiles hold several members -- tiles of one member come in even
+numbers, as members do --, sub-tiles of 256 and of 128 columns, one and several of them, clusters of four (a pair for each half of the columns),
+even and uneven halves.  That these sizes do take pairs is asked in test_host_paths_cpu.py."""
 import numpy as np
 import pytest
 
@@ -12,39 +13,54 @@ pytestmark = pytest.mark.gpu
 SEED = 0x00C0FFEE
 
 
-@pytest.mark.parametrize("hidden,layers,seq,pop", [
-    (384, 2, 64, 594),         # K 1536, 297 row tiles of two members each; three sub-tiles of 128; two layers: three and one dots follow
-    (512, 1, 128, 298),        # K 2048, tiles of one member, two sub-tiles of 256
-    (512, 1, 96, 396),         # 297 tiles across members of 96 rows
-    (640, 1, 64, 594),         # clusters of four, 384 + 256 columns
-    (1024, 1, 128, 298),       # clusters of four, 512 + 512 columns; K 1024 in the up projection, too
-])
-def test_pairs_equal_single_blocks_and_oracle(hidden, layers, seq, pop):
+EVALUATIONS = [                # hidden, layers, seq, pop, other settings
+    (384, 2, 64, 594, {}),     # K 1536, 297 row tiles of two members each; three sub-tiles of 128; two layers: three and one dots follow
+    (512, 1, 128, 298, {}),    # K 2048, tiles of one member, two sub-tiles of 256
+    (512, 1, 128, 298, dict(fixed_point=5, sigma_shift=4)),          # the output projection's shifts apart
+    (512, 1, 96, 396, {}),     # 297 tiles across members of 96 rows
+    (256, 1, 128, 100, {}),    # Q|K|V alone, one sub-tile a unit
+    (640, 1, 64, 594, {}),     # clusters of four, 384 + 256 columns
+    (1024, 1, 128, 298, {}),   # clusters of four, 512 + 512 columns; K 1024 in the up projection, too
+]
+
+
+def small_chunk(hidden, seq):
+    """The most members whose products are too few tiles for pairs: MLP-up below 4 x 148, Q|K|V below 2 x 148."""
+    return min(4 * 148 * 256 // (4 * hidden) - 1, 2 * 148 // 3 - 1) * 128 // seq & ~1
+
+
+@pytest.mark.parametrize("hidden,layers,seq,pop,other", EVALUATIONS)
+def test_pairs_equal_single_blocks_and_oracle(hidden, layers, seq, pop, other):
     pkg, O = load_pkg(), load_oracle()
-    kw = dict(hidden_dim=hidden, n_layers=layers, seq_len=seq, population_size=pop, device_mask=3)
+    kw = dict(hidden_dim=hidden, n_layers=layers, seq_len=seq, population_size=pop, device_mask=3, **other)
     cfg, ocfg, model, data = make_case(kw, data_len=60000, model_kind="random_all")
 
-    def losses(level):
+    def losses(level, chunk=pop):
         ctx = pkg.Context(cfg, 0, pop)
         ctx.set_fused_epilogues(level)
         ctx.upload_model(model)
         ctx.set_dataset(data)
-        ctx.eval_chunk(SEED + 5, seq, 0, pop)
+        for first in range(0, pop, chunk):
+            ctx.eval_chunk(SEED + 5, seq, first, min(chunk, pop - first))
         out = ctx.read_losses(0, pop)
         ctx.close()
         return out
 
     got = losses(2)
+    assert (got == losses(2, small_chunk(hidden, seq))).all()
     assert (got == losses(0)).all()
     for first in (0, pop - 4):
         assert (got[first:first + 4] == O.eval_losses(ocfg, model, data, seq, SEED + 5, first, 4)).all(), first
 
 
-@pytest.mark.parametrize("hidden,layers,pairs", [
+MODEL_UPDATES = [              # hidden, layers, pairs
     (256, 2, 1300),            # 11 blocks of the contraction in several splits
     (384, 1, 1501),            # three tiles of 128 outputs: the second half of the last pair's tile is not stored
     (640, 1, 300),             # five; contraction of three blocks
-])
+]
+
+
+@pytest.mark.parametrize("hidden,layers,pairs", MODEL_UPDATES)
 def test_vote_tiles_of_pairs(hidden, layers, pairs):
     pkg, O = load_pkg(), load_oracle()
     kw = dict(hidden_dim=hidden, n_layers=layers, seq_len=16, population_size=2 * pairs, device_mask=15)
@@ -60,10 +76,15 @@ def test_vote_tiles_of_pairs(hidden, layers, pairs):
     ctx.close()
 
 
-@pytest.mark.parametrize("rows,cols,pairs", [
-    (512, 1024, 2000),         # tiles and splits of the contraction enough for pairs
-    (512, 1152, 2000),         # nine row tiles of outputs: single blocks
-])
+RECONSTRUCTIONS = [            # rows, cols, pairs, pairs of blocks
+    (2048, 2560, 500, True),   # 160 tiles
+    (2048, 2688, 500, False),  # 21 row tiles of outputs: single blocks
+    (512, 1024, 2000, False),  # 16 tiles: too few
+    (512, 1152, 2000, False),
+]
+
+
+@pytest.mark.parametrize("rows,cols,pairs", [r[:3] for r in RECONSTRUCTIONS])
 def test_isolated_votes_of_pairs(rows, cols, pairs):
     import torch
     pkg, O = load_pkg(), load_oracle()
@@ -79,9 +100,71 @@ def test_isolated_votes_of_pairs(rows, cols, pairs):
     assert (got == O.vote_columns(ocfg, fit, rows, 402, 403, 1000, 2, n_list)).all()
 
 
-@pytest.mark.parametrize("rows,cols", [(512, 896), (640, 1024), (1024, 1024)])
+MATRIX_UPDATES = [             # rows, cols, pairs, int8 fitness
+    (512, 1024, 2000, False),  # 16 tiles in 16 parts of the contraction, one block each
+    (512, 1280, 2000, True),   # 20 tiles in 11 parts of three blocks, the last of two
+]
+
+
+@pytest.mark.parametrize("rows,cols,pairs,int8fit", MATRIX_UPDATES)
+def test_matrix_update_of_pairs_with_a_split_contraction(rows, cols, pairs, int8fit):
+    import torch
+    pkg, O = load_pkg(), load_oracle()
+    cfg, ocfg = cfg_pair(device_mask=3, population_size=2 * pairs)
+    rng = np.random.default_rng(rows + int8fit)
+    w0 = rng.integers(-127, 128, rows * cols).astype(np.int8)
+    fit = (rng.integers(-127, 128, pairs) if int8fit else rng.integers(-1, 2, pairs)).astype(np.int32)
+    ctx = pkg.Context(cfg, 0, 2)
+    d_w, d_st, d_fit = torch.from_numpy(w0.copy()).cuda(), torch.zeros(rows * cols * 3, dtype=torch.float32, device="cuda"), torch.from_numpy(fit).cuda()
+    torch.cuda.synchronize()
+    n = ctx.update_matrix(d_w.data_ptr(), d_st.data_ptr(), rows, cols, 402, 403, 1000, d_fit.data_ptr(), pairs, 2, 2.5, optimizer=0, split=int8fit)
+    ctx.close()
+    w1, st1 = d_w.cpu().numpy(), d_st.cpu().numpy().reshape(-1, 3)
+    assert n == (w1 != w0).sum() > 0
+    k, n_list = np.arange(rows), np.arange(0, cols, 37).astype(np.int32)
+    for col, votes in zip(n_list, O.vote_columns(ocfg, fit, rows, 402, 403, 1000, 2, n_list)):
+        idx = ((k >> 2) * cols + col) * 4 + (k & 3)                 # packed order [k/4][n][4]
+        w, st = w0[idx].copy(), np.zeros((rows, 3), np.float32)
+        O.adam_from_votes(ocfg, w, st, votes, 2.5)
+        assert (w1[idx] == w).all() and (st1[idx].view(np.uint32) == st.view(np.uint32)).all(), col
+
+
+PROJECTIONS = [(37 * 128, 512, 4096), (37 * 128 - 64, 512, 4096)]          # rows, K, N: an odd number of row tiles, the last one whole and half
+
+
+@pytest.mark.parametrize("rows,k,n", PROJECTIONS)
+def test_projection_of_pairs_with_an_odd_row_tile(rows, k, n):
+    """Beside the transposed epilogue, which results at an odd word take and whose blocks work alone, for every row; the first and the last
+    pair of members beside the oracle; nothing is stored outside."""
+    import torch
+    pkg, O = load_pkg(), load_oracle()
+    cfg, ocfg = cfg_pair(device_mask=3, population_size=64)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(rows)
+    x = torch.clamp(torch.round(torch.randn((rows, k), generator=g, device="cuda") * 32.0), -127, 127).to(torch.int8)
+    w = torch.randint(-127, 128, (k * n,), generator=g, device="cuda", dtype=torch.int8)
+    out = torch.full((2, rows * n + 128 * n), 99, dtype=torch.int8, device="cuda")
+    ctx = pkg.Context(cfg, 0, 2)
+    torch.cuda.synchronize()
+    for o, offset in zip(out, (64, 68)):
+        ctx.perturbed_projection(x.data_ptr(), w.data_ptr(), o.data_ptr() + offset, rows, k, n, 32, 7, 200, 201, 7, 8, on_device=True)
+    ctx.close()
+    y, z = (o[f:f + rows * n].view(rows, n) for o, f in zip(out, (64, 68)))
+    assert torch.equal(y, z)
+    for o, f in zip(out, (64, 68)):
+        assert (o[:f] == 99).all() and (o[f + rows * n:] == 99).all()
+    xs, ws = x.cpu().numpy(), w.cpu().numpy()
+    for j in (0, rows // 64 - 1):
+        assert (y[64 * j:64 * j + 64].cpu().numpy() == O.projection(ocfg, xs[64 * j:64 * j + 64], ws, k, n, 32, 7 + j, 200, 201, 7, 8)).all(), j
+
+
+NEWTON_SCHULZ = [(512, 896, True), (640, 1024, False), (1024, 1024, True), (2304, 2304, True)]          # rows, cols, pairs of blocks
+
+
+@pytest.mark.parametrize("rows,cols", [n[:2] for n in NEWTON_SCHULZ])
 def test_newton_schulz_in_pairs(rows, cols):
-    """Pairs of tiles in both products; an odd number of row tiles (single blocks); more pairs than fit at once in the Gram matrix."""
+    """Pairs of tiles in both products; an odd number of row tiles (single blocks); a square matrix; 90 pairs in the Gram matrix and 162 in the
+    step, more than fit at once, so that a pair goes on to another item, also after a tile below the diagonal."""
     from test_muon_gpu import test_newton_schulz_against_float64 as check
     check(rows, cols)
 
