@@ -340,10 +340,17 @@ static int launch_eval(cudaStream_t st, int bn, const CUtensorMap &ta, const CUt
     return launch_bn<EPI, 0>(st, bn, ta, tb, to, p, num_sms);
 }
 
-// Contractions from which pairs of blocks form the tiles (see launch_gemm_fused for what bounds them).  MLP-up: K 384 0.89 -> 0.87 ms,
+// Whether pairs of blocks form the tiles of 256 columns (see launch_gemm_fused for what bounds them).  MLP-up: K 384 0.89 -> 0.87 ms,
 // 512 5.75 -> 5.45, 640 1.23 -> 1.09, 768 1.70 -> 1.45, 896 2.22 -> 1.85, 1024 2.45 -> 1.99; projections of as many columns: 512 0.155 ->
 // 0.146, 2048 0.52 -> 0.46, 4096 3.40 -> 2.92 (2.6 -> 3.0 int8 POP/s).  At K 256 between 2 % shorter and 1 % longer.
-constexpr int PAIR_MIN_K = 384;
+// Votes of one matrix: by the contraction of one item, which has to make up for a launch of clusters (whole calls of 40 to 60 us): up to 384
+// 2 us longer, at 512 the same, above up to 10 % shorter (4096 x 4096 from 16 384 pairs 463 -> 415 us).
+static bool pairs_form(int epi, const GemmParams &p, int rows_m, int num_sms) {
+    const int splits = epi == EPI_VOTE && p.k_splits > 1 ? p.k_splits : 1;
+    const int64_t tiles = (int64_t)rows_m * (p.N / 256) * splits;
+    if (epi == EPI_VOTE) return p.K > 512 * splits && rows_m % 2 == 0 && tiles >= num_sms;
+    return (epi == EPI_GELU || epi == EPI_CLIP8) && p.seq_len % 32 == 0 && p.rpl >= 0 && p.K >= 384 && tiles >= 4 * num_sms;
+}
 
 int launch_gemm(cudaStream_t st, int epi, const int8_t *A, const int8_t *B, const GemmParams &p_in, int num_sms) {
     GemmParams p = p_in;
@@ -381,8 +388,7 @@ int launch_gemm(cudaStream_t st, int epi, const int8_t *A, const int8_t *B, cons
     CUtensorMap ta, tb;
     int rc;
     const int rows_m = (p.M + GEMM_BM - 1) / GEMM_BM;
-    const bool pair = bn == 256 && ((epi == EPI_VOTE && p.K >= PAIR_MIN_K && rows_m % 2 == 0 && (int64_t)rows_m * (p.N / 256) * (p.k_splits > 1 ? p.k_splits : 1) >= num_sms) ||
-                                    ((epi == EPI_GELU || epi == EPI_CLIP8) && p.seq_len % 32 == 0 && p.rpl >= 0 && p.K >= PAIR_MIN_K && (int64_t)rows_m * (p.N / 256) >= 4 * num_sms));
+    const bool pair = bn == 256 && pairs_form(epi, p, rows_m, num_sms);
     if ((rc = make_tmap(&ta, A, (uint64_t)p.M, (uint64_t)p.K, GEMM_BM))) return rc;
     if ((rc = make_tmap(&tb, B, (uint64_t)p.N, (uint64_t)p.K, (uint32_t)(pair ? bn / 2 : bn)))) return rc;
     CUtensorMap to = ta;       // only the row-per-lane int32 epilogues store through a tensor map

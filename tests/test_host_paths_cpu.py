@@ -410,3 +410,25 @@ for hidden, layers, pairs in %r:
     assert [gemm(n, VOTE) for n in out["update"]] == [{2}] * len(MATRIX_UPDATES)
     assert [{f[1] for f in forms(n, "ns_gemm_kernel")} for n in out["muon"]] == [{2 if r[2] else 1} for r in NEWTON_SCHULZ]
     assert [set(forms(n, "upd_votes_kernel")) for n in out["model"]] == [{(2,)}] * len(MODEL_UPDATES)
+
+
+@pytest.mark.parametrize("call,kernel,blocks", [
+    # votes of one matrix: the contraction of one item
+    ("ctx.update_matrix(p, p, 2048, 2048, 402, 403, 0, p, 1024, 1, 0.1, 0, False)", "gemm_i8_kernel", 1),          # 384
+    ("ctx.update_matrix(p, p, 512, 512, 402, 403, 0, p, 16384, 1, 0.1, 0, False)", "gemm_i8_kernel", 1),           # 512
+    ("ctx.update_matrix(p, p, 2048, 2048, 402, 403, 0, p, 2000, 1, 0.1, 0, False)", "gemm_i8_kernel", 2),          # 683
+    ("ctx.update_reconstruct(p, 512, 2048, 3072, 402, 403, 0, 1, p, on_device=True)", "gemm_i8_kernel", 1),
+    ("ctx.update_reconstruct(p, 513, 2048, 3072, 402, 403, 0, 1, p, on_device=True)", "gemm_i8_kernel", 2),
+])
+def test_pairs_of_blocks_where_they_gain(fake_cuda, call, kernel, blocks):
+    out = fake_cuda("""
+ctx = context(hidden_dim=128, n_layers=1, seq_len=32, population_size=8, device_mask=3)
+p = C.c_void_p()
+fake.cudaMalloc(C.byref(p), C.c_size_t(1 << 30))
+p = p.value
+fake.fake_clear()
+%s
+out["names"] = [l.split()[1] for l in log() if l.startswith("launch")]
+""" % call)
+    at = {"gemm_i8_kernel": 3, "ns_gemm_kernel": 1}[kernel]
+    assert {f[at] for f in forms(out["names"], kernel)} == {blocks}

@@ -77,8 +77,9 @@ def test_vote_tiles_of_pairs(hidden, layers, pairs):
 
 
 RECONSTRUCTIONS = [            # rows, cols, pairs, pairs of blocks
-    (2048, 2560, 500, True),   # 160 tiles
-    (2048, 2688, 500, False),  # 21 row tiles of outputs: single blocks
+    (2048, 2560, 1000, True),  # 160 tiles
+    (2048, 2688, 1000, False), # 21 row tiles of outputs: single blocks
+    (2048, 2560, 500, False),  # a short contraction
     (512, 1024, 2000, False),  # 16 tiles: too few
     (512, 1152, 2000, False),
 ]
@@ -101,8 +102,8 @@ def test_isolated_votes_of_pairs(rows, cols, pairs):
 
 
 MATRIX_UPDATES = [             # rows, cols, pairs, int8 fitness
-    (512, 1024, 2000, False),  # 16 tiles in 16 parts of the contraction, one block each
-    (512, 1280, 2000, True),   # 20 tiles in 11 parts of three blocks, the last of two
+    (1024, 1024, 16384, False),          # 32 tiles in 10 parts of the contraction, of 13 blocks, the last of 11
+    (1024, 1280, 10000, True),           # 40 tiles in 8 parts of 20 blocks, the last of 18
 ]
 
 
