@@ -345,11 +345,15 @@ static int launch_eval(cudaStream_t st, int bn, const CUtensorMap &ta, const CUt
 // 0.146, 2048 0.52 -> 0.46, 4096 3.40 -> 2.92 (2.6 -> 3.0 int8 POP/s).  At K 256 between 2 % shorter and 1 % longer.
 // Votes of one matrix: by the contraction of one item, which has to make up for a launch of clusters (whole calls of 40 to 60 us): up to 384
 // 2 us longer, at 512 the same, above up to 10 % shorter (4096 x 4096 from 16 384 pairs 463 -> 415 us).
+// Projections of their own (and the recurrent model's): the same launch against some (K - 256) / 150 ns a tile.  K 384 1.2 us longer up to 2368
+// tiles, the same at 4736; 512 0.7 longer at 1184, 1.0 shorter at 1776 (85 us), 30 at 9472 (309); 768 1.5 longer at 592, 1.0 shorter at 888;
+// 1024 0.9 shorter at 592 (58).  MLP-up stands in a chain of launches, where the clusters' cost does not show: K 384 and 512 the same from 592 tiles on.
 static bool pairs_form(int epi, const GemmParams &p, int rows_m, int num_sms) {
     const int splits = epi == EPI_VOTE && p.k_splits > 1 ? p.k_splits : 1;
     const int64_t tiles = (int64_t)rows_m * (p.N / 256) * splits;
     if (epi == EPI_VOTE) return p.K > 512 * splits && rows_m % 2 == 0 && tiles >= num_sms;
-    return (epi == EPI_GELU || epi == EPI_CLIP8) && p.seq_len % 32 == 0 && p.rpl >= 0 && p.K >= 384 && tiles >= 4 * num_sms;
+    if (p.seq_len % 32 || p.rpl < 0 || p.K < 384 || tiles < 4 * num_sms) return false;
+    return epi == EPI_GELU || (epi == EPI_CLIP8 && (p.K - 256) * tiles >= 2560 * num_sms);
 }
 
 int launch_gemm(cudaStream_t st, int epi, const int8_t *A, const int8_t *B, const GemmParams &p_in, int num_sms) {

@@ -419,6 +419,12 @@ for hidden, layers, pairs in %r:
     ("ctx.update_matrix(p, p, 2048, 2048, 402, 403, 0, p, 2000, 1, 0.1, 0, False)", "gemm_i8_kernel", 2),          # 683
     ("ctx.update_reconstruct(p, 512, 2048, 3072, 402, 403, 0, 1, p, on_device=True)", "gemm_i8_kernel", 1),
     ("ctx.update_reconstruct(p, 513, 2048, 3072, 402, 403, 0, 1, p, on_device=True)", "gemm_i8_kernel", 2),
+    # projections: rows and contraction
+    ("ctx.perturbed_projection(p, p, p, 296 * 128, 384, 2048, 64, 7, 200, 201, 7, 8, on_device=True)", "gemm_i8_kernel", 1),
+    ("ctx.perturbed_projection(p, p, p, 148 * 128, 512, 2048, 64, 7, 200, 201, 7, 8, on_device=True)", "gemm_i8_kernel", 1),
+    ("ctx.perturbed_projection(p, p, p, 222 * 128, 512, 2048, 64, 7, 200, 201, 7, 8, on_device=True)", "gemm_i8_kernel", 2),
+    ("ctx.perturbed_projection(p, p, p, 198 * 128, 768, 768, 64, 7, 200, 201, 7, 8, on_device=True)", "gemm_i8_kernel", 1),
+    ("ctx.perturbed_projection(p, p, p, 148 * 128, 1024, 1024, 64, 7, 200, 201, 7, 8, on_device=True)", "gemm_i8_kernel", 2),
 ])
 def test_pairs_of_blocks_where_they_gain(fake_cuda, call, kernel, blocks):
     out = fake_cuda("""

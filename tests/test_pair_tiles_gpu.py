@@ -130,7 +130,7 @@ def test_matrix_update_of_pairs_with_a_split_contraction(rows, cols, pairs, int8
         assert (w1[idx] == w).all() and (st1[idx].view(np.uint32) == st.view(np.uint32)).all(), col
 
 
-PROJECTIONS = [(37 * 128, 512, 4096), (37 * 128 - 64, 512, 4096)]          # rows, K, N: an odd number of row tiles, the last one whole and half
+PROJECTIONS = [(37 * 128, 1024, 4096), (37 * 128 - 64, 1024, 4096)]          # rows, K, N: an odd number of row tiles, the last one whole and half
 
 
 @pytest.mark.parametrize("rows,k,n", PROJECTIONS)
