@@ -722,15 +722,17 @@ int upd_plan_build(UpdPlan &pl, const std::vector<ParamDesc> &params, const std:
     pl.kp = (pairs + 15 + 127) / 128 * 128;
     pl.W = std::max(4 * hidden, vocab);
     // Vote tiles in pairs of blocks: half of one operand's traffic from L2, which bounds the product.  Per tile of 128 columns they take 0.73
-    // to 0.82 of the time (163 840 pairs, H 256: 581 -> 427 us; 131 072, H 1024: 12.2 -> 10.0 ms; 20 480, H 512: 292 -> 211 us; 4096, H 256: 23 -> 19;
-    // 256: the same), so that a model takes them unless odd multiples of 128 outputs leave more than a fifth of their halves empty.
+    // to 0.82 of the time (163 840 pairs, H 256: 581 -> 427 us; 131 072, H 1024: 12.2 -> 10.0 ms; 20 480, H 512: 292 -> 211 us; 4096, H 256: 23 -> 19),
+    // so that a model takes them unless odd multiples of 128 outputs leave more than a fifth of their halves empty, and not for few pairs, which a
+    // launch of clusters does not pay for: whole updates of 32 to 368 pairs 1 to 3 us longer at H 256 to 1024 (H 256, 2 layers: 46.1 -> 47.2; H 896
+    // 228.5 -> 231.5; at most 1.4 shorter at H 512, 4 layers), of 480 (four blocks of the contraction) 1.5 shorter at H 512, 2.8 at 1024, of 512 up to 20.
     int64_t single = 0, paired = 0;
     for (const ParamDesc &d : params)
         if (d.rows_k) {
             const int64_t tn = (d.rows_k + UV_BN - 1) / UV_BN;
             single += d.cols_n / UV_BM * tn; paired += (d.cols_n + 2 * UV_BM - 1) / (2 * UV_BM) * 2 * tn;
         }
-    pl.cg = 5 * single >= 4 * paired ? 2 : 1;
+    pl.cg = pl.kp >= 512 && 5 * single >= 4 * paired ? 2 : 1;
     std::vector<std::pair<int, int>> need;                   // table columns [first, last)
     auto want = [&](int s) { need.push_back({s & ~127, (s + UPD_ORIGIN + pl.kp + 64 + 127) & ~127}); };
     for (size_t i = 0; i < params.size(); i++) {

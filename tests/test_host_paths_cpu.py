@@ -378,7 +378,7 @@ for rows, cols, _ in %r:
     fake.fake_clear()
     ctx.update_matrix(p, p, rows, cols, 402, 403, 0, p, 32, 7, 1.0, 1, False)
     out["muon"].append(names())
-for hidden, layers, pairs in %r:
+for hidden, layers, pairs, _ in %r:
     ctx = context(hidden_dim=hidden, n_layers=layers, seq_len=16, population_size=2 * pairs, device_mask=15)
     fake.fake_clear()
     ctx.apply_update(1, 0.4)
@@ -409,7 +409,7 @@ for hidden, layers, pairs in %r:
     assert [gemm(n, VOTE) for n in out["votes"]] == [{2 if r[3] else 1} for r in RECONSTRUCTIONS]
     assert [gemm(n, VOTE) for n in out["update"]] == [{2}] * len(MATRIX_UPDATES)
     assert [{f[1] for f in forms(n, "ns_gemm_kernel")} for n in out["muon"]] == [{2 if r[2] else 1} for r in NEWTON_SCHULZ]
-    assert [set(forms(n, "upd_votes_kernel")) for n in out["model"]] == [{(2,)}] * len(MODEL_UPDATES)
+    assert [set(forms(n, "upd_votes_kernel")) for n in out["model"]] == [{(2 if u[3] else 1,)} for u in MODEL_UPDATES]
 
 
 @pytest.mark.parametrize("call,kernel,blocks", [
@@ -425,6 +425,10 @@ for hidden, layers, pairs in %r:
     ("ctx.perturbed_projection(p, p, p, 222 * 128, 512, 2048, 64, 7, 200, 201, 7, 8, on_device=True)", "gemm_i8_kernel", 2),
     ("ctx.perturbed_projection(p, p, p, 198 * 128, 768, 768, 64, 7, 200, 201, 7, 8, on_device=True)", "gemm_i8_kernel", 1),
     ("ctx.perturbed_projection(p, p, p, 148 * 128, 1024, 1024, 64, 7, 200, 201, 7, 8, on_device=True)", "gemm_i8_kernel", 2),
+    # votes of a model
+    ("context(hidden_dim=256, n_layers=2, seq_len=32, population_size=64).apply_update(1, 0.1)", "upd_votes_kernel", 1),
+    ("context(hidden_dim=896, n_layers=1, seq_len=32, population_size=738).apply_update(1, 0.1)", "upd_votes_kernel", 1),
+    ("context(hidden_dim=896, n_layers=1, seq_len=32, population_size=740).apply_update(1, 0.1)", "upd_votes_kernel", 2),
 ])
 def test_pairs_of_blocks_where_they_gain(fake_cuda, call, kernel, blocks):
     out = fake_cuda("""
@@ -436,5 +440,5 @@ fake.fake_clear()
 %s
 out["names"] = [l.split()[1] for l in log() if l.startswith("launch")]
 """ % call)
-    at = {"gemm_i8_kernel": 3, "ns_gemm_kernel": 1}[kernel]
+    at = {"gemm_i8_kernel": 3, "upd_votes_kernel": 0}[kernel]
     assert {f[at] for f in forms(out["names"], kernel)} == {blocks}

@@ -53,14 +53,15 @@ def test_pairs_equal_single_blocks_and_oracle(hidden, layers, seq, pop, other):
         assert (got[first:first + 4] == O.eval_losses(ocfg, model, data, seq, SEED + 5, first, 4)).all(), first
 
 
-MODEL_UPDATES = [              # hidden, layers, pairs
-    (256, 2, 1300),            # 11 blocks of the contraction in several splits
-    (384, 1, 1501),            # three tiles of 128 outputs: the second half of the last pair's tile is not stored
-    (640, 1, 300),             # five; contraction of three blocks
+MODEL_UPDATES = [              # hidden, layers, pairs, pairs of blocks
+    (256, 2, 1300, True),      # 11 blocks of the contraction in several splits
+    (384, 1, 1501, True),      # three tiles of 128 outputs: the second half of the last pair's tile is not stored
+    (640, 1, 370, True),       # five; the shortest contraction
+    (640, 1, 300, False),      # single blocks
 ]
 
 
-@pytest.mark.parametrize("hidden,layers,pairs", MODEL_UPDATES)
+@pytest.mark.parametrize("hidden,layers,pairs", [u[:3] for u in MODEL_UPDATES])
 def test_vote_tiles_of_pairs(hidden, layers, pairs):
     pkg, O = load_pkg(), load_oracle()
     kw = dict(hidden_dim=hidden, n_layers=layers, seq_len=16, population_size=2 * pairs, device_mask=15)
