@@ -21,14 +21,15 @@
 //   pass 2 (per sub-tile): requantise (aln_quant_f), pack, write the warp's 32 x BN/4 int8 box to shared memory, release
 //          the TMEM slot to the MMA warp, store the box with one TMA store.
 // So the MMAs of the next unit's first sub-tile overlap pass 2 of this unit's last, and no int32 intermediate ever
-// reaches HBM.  When seq_len is a multiple of 128 a tile's rows belong to one population member and one set of tables serves
-// all of them; otherwise (MM, seq_len a multiple of 32) every lane quarter of 32 rows has its own member and tables, and the
-// sub-tiles are 128 wide unless the block owns exactly 256 columns, so that the tables fit beside the operands.
+// reaches HBM.  When seq_len is a multiple of 128 a tile's rows belong to one population member; otherwise (MM, seq_len a
+// multiple of 32) every lane quarter of 32 rows has its own member.  Tables are the warp's own (MM, and q, k, v in 128-column
+// sub-tiles), else those of a column quarter, shared by its four warps and double-buffered across units.  With MM the sub-tiles are
+// 128 wide unless the block owns exactly 256 columns, so that the tables fit beside the operands.
 // At H 256, seq_len 32 (262 144 rows) this replaces a projection with int32 output and a requantising pass: q|k|v 332 -> 200 us.
 // For long contractions and wide tiles two blocks of a cluster form 256 rows together (CG = 2, cta_group::2): an SM gets fewer bytes from
 // L2 than a 128 x 256 tile needs at the tensor cores' rate; the rule and its figures stand at launch_gemm_fused.
-// No multicast anywhere; every wait is bounded and a timeout makes all later waits fall through so that the block
-// drains, frees its tensor memory and reports.
+// Operands come by plain loads, no multicast; only tcgen05.commit of a pair arrives on both blocks' barriers.  Every wait is bounded and
+// a timeout makes all later waits fall through so that the block drains, frees its tensor memory and reports.
 #pragma once
 
 #include "egg_gemm.cuh"

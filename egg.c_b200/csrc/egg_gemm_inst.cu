@@ -42,8 +42,10 @@ static int set_attr_fused() {
     if ((rc = set_attr_fused_one<BN, FUSED_RES, MM, true>())) return rc;
     if ((rc = set_attr_fused_one<BN, FUSED_RES_LN, MM, false>())) return rc;
     if ((rc = set_attr_fused_one<BN, FUSED_RES_LN, MM, true>())) return rc;
-    if ((rc = set_attr_fused_one<BN, FUSED_RES_LN, MM, false, 2>())) return rc;
-    return set_attr_fused_one<BN, FUSED_RES_LN, MM, true, 2>();
+    if constexpr (BN == 128 || !MM) {
+        if ((rc = set_attr_fused_one<BN, FUSED_RES_LN, MM, false, 2>()) || (rc = set_attr_fused_one<BN, FUSED_RES_LN, MM, true, 2>())) return rc;
+    }
+    return EGG_OK;
 }
 
 int gemm_init() {
@@ -217,7 +219,7 @@ static int launch_fused_cg(cudaStream_t st, const CUtensorMap &ta, const CUtenso
 template <int BN, int MODE, bool MM, bool FORM = false>
 static int launch_fused_one(cudaStream_t st, const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &to, const CUtensorMap &tr,
                             const FusedParams &p, int units, int num_sms) {
-    if constexpr (MODE == FUSED_RES_LN || (BN == 256 && !MM)) {
+    if constexpr (MODE == FUSED_RES_LN ? BN == 128 || !MM : BN == 256 && !MM) {
         if (p.pair) return launch_fused_cg<BN, MODE, MM, FORM, 2>(st, ta, tb, to, tr, p, units, num_sms);
     }
     return launch_fused_cg<BN, MODE, MM, FORM, 1>(st, ta, tb, to, tr, p, units, num_sms);
@@ -253,16 +255,18 @@ int launch_gemm_fused(cudaStream_t st, int mode, const int8_t *A, const int8_t *
     // (2048 rows, H 256: MLP-down 12.7 -> 11.3 us, Q|K|V 8.6 -> 7.2, output projection 7.4 -> 6.3)
     if (p.cl == 1 && p.H >= 256 && 2 * units <= num_sms) p.cl = 2;
     const int hl = p.H % (128 * p.cl) ? 128 : p.H / p.cl;      // columns per block (uneven shares: whole 128-column sub-tiles)
-    const bool mm = p.seq_len % GEMM_BM != 0;        // a tile spans members: four table sets, see the kernel
+    const bool mm = p.seq_len % GEMM_BM != 0;        // a tile spans members: tables of the warp's own, see the kernel
     const int bn = (mm ? hl == 256 : hl % 256 == 0) ? 256 : 128;      // (128-column sub-tiles at H = 512 were measured: +30 % on MLP-down)
     // Pairs of blocks where the products wait for their operands: a 128 x 256 tile takes 96 bytes a clock at the tensor cores' rate and an SM
     // gets some 57, a pair's half needs 64.  The two blocks' epilogues wait for one another, so not where those are the longer part.
     // Down projection with the norm, per evaluation of 4 or 2 layers: K 2048 8.24 -> 7.01 ms, 2560 2.43 -> 2.17, 4096 3.49 -> 3.31, 1536 1.52 ->
     // 1.41, but 1024 2 to 4 % longer.  Q|K|V in tiles of one member and 256 columns, one block to a row: H 512 5.94 -> 5.48, H 256 2.84 -> 2.74;
     // output projection at H 512 5 % shorter, at H 256 as much longer.  Tiles of several members, narrower ones and rows of two
-    // blocks: Q|K|V 2 to 12 % longer.  Not where pairs would leave SMs without a unit.
+    // blocks: Q|K|V 2 to 12 % longer.  From two units an SM on, for clusters of four: the down projection of 148 and 222 row tiles 9 to 11 and 2 to 6 us
+    // a launch longer (H 640 to 1024), of 296 up to 2 us shorter, of 592 17 to 32.  Clusters of two would gain from 98 row tiles on (H 384 and 512: 1 to 8 us),
+    // Q|K|V at H 256 not before 222 (148: 0.4 us a launch longer).
     const bool wide = p.cl == 1 && bn == 256 && !mm;
-    p.pair = units >= 2 * num_sms && (mode == FUSED_RES_LN ? p.K >= 1536 : wide && (mode == FUSED_QKV || p.K >= 512));
+    p.pair = units >= 2 * num_sms && (mode == FUSED_RES_LN ? p.K >= 1536 && (bn == 128 || !mm) : wide && (mode == FUSED_QKV || p.K >= 512));
     if (p.pair) units = (p.M / GEMM_BM + 1) / 2 * p.parts;
     p.fd_seq = make_fastdiv(p.seq_len);
     p.fd_h = make_fastdiv(p.H);
