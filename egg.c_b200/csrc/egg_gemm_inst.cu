@@ -263,8 +263,7 @@ int launch_gemm_fused(cudaStream_t st, int mode, const int8_t *A, const int8_t *
     // 1.41, but 1024 2 to 4 % longer.  Q|K|V in tiles of one member and 256 columns, one block to a row: H 512 5.94 -> 5.48, H 256 2.84 -> 2.74;
     // output projection at H 512 5 % shorter, at H 256 as much longer.  Tiles of several members, narrower ones and rows of two
     // blocks: Q|K|V 2 to 12 % longer.  From two units an SM on, for clusters of four: the down projection of 148 and 222 row tiles 9 to 11 and 2 to 6 us
-    // a launch longer (H 640 to 1024), of 296 up to 2 us shorter, of 592 17 to 32.  Clusters of two would gain from 98 row tiles on (H 384 and 512: 1 to 8 us),
-    // Q|K|V at H 256 not before 222 (148: 0.4 us a launch longer).
+    // a launch longer (H 640 to 1024), of 296 up to 2 us shorter, of 592 17 to 32; Q|K|V at H 256 of 100 to 592 the same within 0.4 us.
     const bool wide = p.cl == 1 && bn == 256 && !mm;
     p.pair = units >= 2 * num_sms && (mode == FUSED_RES_LN ? p.K >= 1536 && (bn == 128 || !mm) : wide && (mode == FUSED_QKV || p.K >= 512));
     if (p.pair) units = (p.M / GEMM_BM + 1) / 2 * p.parts;

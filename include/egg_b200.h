@@ -527,8 +527,10 @@ int egg_wave_members(egg_ctx *ctx);
  * block (apply_standard_norm, mgpu.cu:646-678: LN1 of the next layer or the final norm) and the row dots of the
  * projections after it, so that row-wise kernel launch disappears.  Level 3 does the same for LN2 inside the
  * output projection; it is selectable and tested but not the default: that projection's epilogue is not hidden
- * behind its short contraction (K = hidden_dim), and the norm costs more there than as a kernel of its own
- * (measured on B200: +15 ms in the projections against -12 ms of row-wise kernels per 40960-member generation).
+ * behind its short contraction (K = hidden_dim), it forms no pairs of blocks there, and the norm costs as much as a kernel
+ * of its own (evaluations at level 2 and 3 on B200: H 256, 32 tokens 3.07 and 3.11 ms; H 384, 80 tokens 4.36 and 4.43;
+ * H 512, 64 tokens 14.6 and 14.9; the same within the runs at 256 tokens, H 256 12.33 and 12.33, H 512 27.7 and 27.6, and at
+ * H 1024, 512 tokens 12.2 and 12.2).
  * enable = 1 keeps the row-owning projections without either, enable = 0 forces the two-kernel form (for A/B timing and for tests that
  * compare the forms) and allocates its rows where the context has none (EGG_E_NOMEM leaves the level as it was); no
  * counterpart in the reference.  egg_fused_epilogues_active returns the level this context's evaluations take
